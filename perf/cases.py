@@ -82,8 +82,9 @@ def draw(rng):
         batch = rng.choice([1, 2, 4, 8])
         return {"kind": "layer", "model": rng.choice(["llama", "qwen", "mixtral"]), "batch": batch,
                 "seq": _spread(rng, 16, 8192 // batch)}
-    return {"kind": "weight", "n": 8 * _spread(rng, 64, 3584), "k": 128 * _spread(rng, 4, 148),
-            "quant": rng.choice(["SHARQ", "NVFP4"])}
+    quant = rng.choice(["SHARQ", "NVFP4"])
+    n = 8 * _spread(rng, 64, 3584)
+    return {"kind": "weight", "n": n if quant == "SHARQ" else -(-n // 128) * 128, "k": 128 * _spread(rng, 4, 148), "quant": quant}
 
 
 # ------------------------------------------------------------------------------------------ inputs
@@ -178,7 +179,9 @@ def run(state):
         return state["layer"](state["x"], state["cos"], state["sin"])
     if state["quant"] == "SHARQ":
         return quantize_weight_shared_nvfp4(state["w"])
-    return quantize_weight_nvfp4(state["w"])
+    q, sf, scale = quantize_weight_nvfp4(state["w"])
+    # the spare band behind the scale factors of the N rows (a multiple of 128 here) is not part of the result
+    return q, sf[: state["w"].numel() // 16], scale
 
 
 # ------------------------------------------------------------------------------------------ work
