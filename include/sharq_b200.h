@@ -151,6 +151,17 @@ int sharq_duplicate_sfa32_to_sfa16(const void *sfa_sparse, int m, int n, int k, 
  * of the scale buffer are written, as in the reference.  bindings.cpp:74-160 */
 int sharq_quantize_nvfp4(const void *x_bf16, int rows, int k, void *q, void *sf, void *stream);
 
+/* The two with their host-side passes folded in (model/quantize.py:43-44,141-169): scale = clamp(max|x|/2688, 1e-9)
+ * and the quantisation of (x / scale).to(bf16) as torch evaluates it on a CUDA device (the 0-dim divisor is cast
+ * to bf16 first), in two launches.  x 16-byte aligned; workspace: sharq_scaled_quantize_workspace_bytes() bytes with
+ * any content; scale_out: one device float.  nvfp4: K % 64 == 0, padding bytes of sf untouched.  w32_shared:
+ * K % 128 == 0 and K/32 <= 1024, every byte of both scale buffers is written. */
+size_t sharq_scaled_quantize_workspace_bytes(void);
+int sharq_scaled_quantize_nvfp4(const void *x_bf16, int rows, int k, void *workspace, size_t workspace_bytes, void *q, void *sf,
+                                float *scale_out, void *stream);
+int sharq_scaled_quantize_w32_shared(const void *w_bf16, int n, int k, void *workspace, size_t workspace_bytes, void *qw,
+                                     void *sfw_sparse, void *sfw_dense, float *scale_out, void *stream);
+
 /* compress_sparse_a(A_q_dense, N): dense payload with at most two non-zero bytes per
  * 4-byte chunk -> A_comp, E.  bindings.cpp:164-230 */
 int sharq_compress_sparse_a(const void *a_q_dense, int m, int n, int k, void *a_comp, void *e, void *stream);

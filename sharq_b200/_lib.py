@@ -39,6 +39,9 @@ SIGNATURES = {
     "sharq_quantize_w32_shared": (c_int, [_P, c_int, c_int, _P, _P, _P, _P]),
     "sharq_duplicate_sfa32_to_sfa16": (c_int, [_P, c_int, c_int, c_int, _P, _P]),
     "sharq_quantize_nvfp4": (c_int, [_P, c_int, c_int, _P, _P, _P]),
+    "sharq_scaled_quantize_workspace_bytes": (c_size_t, []),
+    "sharq_scaled_quantize_nvfp4": (c_int, [_P, c_int, c_int, _P, c_size_t, _P, _P, _P, _P]),
+    "sharq_scaled_quantize_w32_shared": (c_int, [_P, c_int, c_int, _P, c_size_t, _P, _P, _P, _P, _P]),
     "sharq_compress_sparse_a": (c_int, [_P, c_int, c_int, c_int, _P, _P, _P]),
     "sharq_matmul": (c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, c_float, _P, _P, _P]),
     "sharq_sparse_matmul": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, c_float, _P, _P, _P]),

@@ -229,6 +229,33 @@ int sharq_quantize_nvfp4(const void *x, int rows, int k, void *q, void *sf, void
   return check_cuda(sharq::run_quantize_dense_nvfp4(x, rows, k, q, sf, as_stream(stream)), "quantize_nvfp4");
 }
 
+int sharq_scaled_quantize_nvfp4(const void *x, int rows, int k, void *workspace, size_t workspace_bytes, void *q, void *sf,
+                                float *scale_out, void *stream) {
+  SHARQ_REQUIRE(rows > 0 && k > 0, "X must be shaped [rows, K]");
+  SHARQ_REQUIRE(k % 64 == 0, "scaled_quantize_nvfp4 requires K to be a multiple of 64, got %d", k);
+  SHARQ_REQUIRE(x && workspace && q && sf && scale_out, "null buffer");
+  SHARQ_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0, "X must be 16-byte aligned");
+  SHARQ_REQUIRE(workspace_bytes >= sharq_scaled_quantize_workspace_bytes(), "workspace is too small");
+  return check_cuda(sharq::run_scaled_quantize(x, rows, k, false, static_cast<float *>(workspace), q, sf, nullptr, scale_out,
+                                               as_stream(stream)),
+                    "scaled_quantize_nvfp4");
+}
+
+int sharq_scaled_quantize_w32_shared(const void *w, int n, int k, void *workspace, size_t workspace_bytes, void *qw,
+                                     void *sfw_sparse, void *sfw_dense, float *scale_out, void *stream) {
+  SHARQ_REQUIRE(n > 0 && k > 0, "W must be shaped [N, K]");
+  SHARQ_REQUIRE(k % 128 == 0, "scaled_quantize_w32_shared requires K to be a multiple of 128, got %d", k);
+  SHARQ_REQUIRE(k / 32 <= 1024, "scaled_quantize_w32_shared requires K / 32 <= 1024");
+  SHARQ_REQUIRE(w && workspace && qw && sfw_sparse && sfw_dense && scale_out, "null buffer");
+  SHARQ_REQUIRE((reinterpret_cast<uintptr_t>(w) & 15) == 0, "W must be 16-byte aligned");
+  SHARQ_REQUIRE(workspace_bytes >= sharq_scaled_quantize_workspace_bytes(), "workspace is too small");
+  return check_cuda(sharq::run_scaled_quantize(w, n, k, true, static_cast<float *>(workspace), qw, sfw_sparse, sfw_dense,
+                                               scale_out, as_stream(stream)),
+                    "scaled_quantize_w32_shared");
+}
+
+size_t sharq_scaled_quantize_workspace_bytes(void) { return sizeof(float) * (size_t)sharq::kScaledQuantPartials; }
+
 int sharq_compress_sparse_a(const void *a_q_dense, int m, int n, int k, void *a_comp, void *e, void *stream) {
   (void)n;
   SHARQ_REQUIRE(m > 0 && k > 0, "A_q_dense must be shaped [M, K/2]");

@@ -5,8 +5,9 @@
 //   kernels/src/reorder.cu:69-203,381-555 and kernels/src/down.cu:72-233 with identity
 //   reorder and KE == 0                         (dense NVFP4 quantisation, 16-group scales)
 //   kernels/src/bindings.cpp:164-230            (structured-sparse compressor, debug path)
-// These run offline (weights) or in the dense-NVFP4 baseline mode, so they are written
-// for clarity: one thread per scale group, 16-byte loads and stores.
+//   model/quantize.py:43-44,141-169             (tensor scale and division in front of the two)
+// The kernels that take an already scaled input are written for clarity: one thread per scale
+// group, 16-byte loads and stores.
 #include "common.cuh"
 #include "quant.cuh"
 
@@ -140,6 +141,144 @@ __global__ void __launch_bounds__(256) compress_sparse_a_kernel(const uint8_t *_
       (uint16_t)meta;
 }
 
+// ---------------------------------------------------------------------------
+// Unscaled bf16 matrix -> tensor scale, division and quantisation in two launches.
+//
+// HBM-bound: x has to be read twice (the scale depends on all of it), 4 B + 0.6 B per element.
+// Launch 1 leaves one maximum per CTA in `partials`, so nothing has to be zeroed first; launch 2
+// reduces them again in every CTA and walks the matrix from its END, so that the last ~100 MB launch 1
+// read come from L2.  As ATen passes (abs, max, float, divide, clamp, divide, cast) and a
+// quantisation kernel this took 668 us at 28672 x 4096, of which 442 us were ATen's division by a
+// 0-dim tensor; now 102 us (absmax 37 us = 6.4 TB/s, quantisation 65 us), and 85 -> 16 us at 1000 x 14336
+// (dense).
+//
+// Arithmetic: dividing a bf16 CUDA tensor by a 0-dim float32 tensor casts the divisor to bf16 first, so
+// y = bf16(x / float(bf16(scale))).  Quotients of two 8-bit significands are either representable
+// or at least 2^-17 (relative) away from every bf16 rounding boundary, and x * (1 / div) is within
+// 2^-22 of them: the product rounds to the same y.  A subnormal quotient may round differently,
+// but its group's scale is clamped to >= 2^-9, under which it becomes a zero of the same sign either way.
+// A NaN in x makes the scale and with it every y NaN, as the ATen passes do.
+// ---------------------------------------------------------------------------
+constexpr int kScaledThreads = 256;
+
+__device__ __forceinline__ float block_max_nan(float mx, float *warp_max) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float other = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = (mx != mx || other != other) ? __int_as_float(0x7fffffff) : fmaxf(mx, other);
+  }
+  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  mx = warp_max[0];
+#pragma unroll
+  for (int w = 1; w < kScaledThreads / 32; ++w) {
+    const float other = warp_max[w];
+    mx = (mx != mx || other != other) ? __int_as_float(0x7fffffff) : fmaxf(mx, other);
+  }
+  return mx;
+}
+
+__global__ void __launch_bounds__(kScaledThreads) absmax_partials_kernel(const uint4 *__restrict__ x, size_t n16,
+                                                                         float *__restrict__ partials) {
+  __shared__ float warp_max[kScaledThreads / 32];
+  __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
+  const size_t stride = (size_t)gridDim.x * kScaledThreads;
+  for (size_t i = (size_t)blockIdx.x * kScaledThreads + threadIdx.x; i < n16; i += 4 * stride) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = (i + u * stride < n16) ? __ldg(x + i + u * stride) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+      for (int t = 0; t < 4; ++t) m2 = __hmax2_nan(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&w[t])));
+    }
+  }
+  const float lo = __bfloat162float(m2.x), hi = __bfloat162float(m2.y);
+  const float mx = block_max_nan((lo != lo || hi != hi) ? __int_as_float(0x7fffffff) : fmaxf(lo, hi), warp_max);
+  if (threadIdx.x == 0) partials[blockIdx.x] = mx;
+}
+
+// The bytes of both scale views of a shared weight that belong to no row: rows [n, ceil128(n)) of the
+// last band and everything behind the bands (K % 128 == 0, so whole 32-bit words).
+__device__ __forceinline__ void zero_scale_padding(int n, int k, uint8_t *sf_sparse, uint8_t *sf_dense) {
+  const size_t alloc = sf_alloc_bytes(n, k) / 4;
+  const int bands = (n + 127) / 128, t_sp = k / 128, t_d = k / 64;  // 512-byte scale tiles per band
+  const size_t worker = (size_t)blockIdx.x * blockDim.x + threadIdx.x, workers = (size_t)gridDim.x * blockDim.x;
+  uint32_t *w_sp = reinterpret_cast<uint32_t *>(sf_sparse), *w_d = reinterpret_cast<uint32_t *>(sf_dense);
+  for (size_t i = (size_t)bands * t_sp * 128 + worker; i < alloc; i += workers) w_sp[i] = 0u;
+  for (size_t i = (size_t)bands * t_d * 128 + worker; i < alloc; i += workers) w_d[i] = 0u;
+  const size_t pad = (size_t)(bands * 128 - n);
+  for (size_t i = worker; i < pad * t_sp; i += workers) w_sp[sf_offset(n + (int)(i / t_sp), 4 * (int)(i % t_sp), k / 32) / 4] = 0u;
+  for (size_t i = worker; i < pad * t_d; i += workers) w_d[sf_offset(n + (int)(i / t_d), 4 * (int)(i % t_d), k / 16) / 4] = 0u;
+}
+
+// kShared: 32 elements per thread, scale of 32, both scale views.  Else 16 elements per thread.
+// The groups of a row are a multiple of 4, so four neighbouring lanes' scale bytes form a 32-bit word of
+// the blocked layout: gathered by shuffles and stored once.
+template <bool kShared>
+__global__ void __launch_bounds__(kScaledThreads) scaled_quantize_kernel(const uint4 *__restrict__ x, int rows, int k,
+                                                                         const float *__restrict__ partials, int n_partials,
+                                                                         uint8_t *__restrict__ q,
+                                                                         uint8_t *__restrict__ sf, uint8_t *__restrict__ sf2,
+                                                                         float *__restrict__ scale_out) {
+  constexpr int kVecs = kShared ? 4 : 2;  // 16-byte vectors of a group
+  __shared__ float warp_max[kScaledThreads / 32];
+  if (kShared) zero_scale_padding(rows, k, sf, sf2);
+  float mx = 0.0f;
+  for (int i = threadIdx.x; i < n_partials; i += kScaledThreads) {
+    const float p = partials[i];
+    mx = (mx != mx || p != p) ? __int_as_float(0x7fffffff) : fmaxf(mx, p);
+  }
+  const float amax = block_max_nan(mx, warp_max);
+  // ATen divides by a host scalar by multiplying with its float reciprocal; clamp keeps a NaN
+  const float raw = __fmul_rn(amax, 1.0f / 2688.0f);
+  const float scale = raw != raw ? raw : fmaxf(raw, 1.0e-9f);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *scale_out = scale;
+  const float recip = __frcp_rn(__bfloat162float(__float2bfloat16_rn(scale)));
+
+  const int groups = k / (8 * kVecs);
+  const long long total = (long long)rows * groups;
+  const long long chunks = (total + kScaledThreads - 1) / kScaledThreads;
+  for (long long c = chunks - 1 - blockIdx.x; c >= 0; c -= gridDim.x) {
+    const long long idx = c * kScaledThreads + threadIdx.x;
+    const bool live = idx < total;
+    const int row = live ? (int)(idx / groups) : 0, g = live ? (int)(idx - (long long)row * groups) : 0;
+    uint32_t code = 0;
+    if (live) {
+      float v[8 * kVecs];
+#pragma unroll
+      for (int j = 0; j < kVecs; ++j) unpack8(__ldg(x + idx * kVecs + j), v + 8 * j);
+      float gm = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 8 * kVecs; ++i) {
+        v[i] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(v[i], recip)));
+        gm = fmaxf(gm, fabsf(v[i]));
+      }
+      code = float_to_ue4m3(clamp_val(__fdiv_rn(gm, kFp4Max), kScaleEps, kFp8Max));
+      const float inv = __frcp_rn(ue4m3_to_float(code));
+      uint32_t o[kVecs];
+#pragma unroll
+      for (int j = 0; j < kVecs; ++j)
+        o[j] = pack_e2m1x8(__fmul_rn(v[8 * j + 0], inv), __fmul_rn(v[8 * j + 1], inv), __fmul_rn(v[8 * j + 2], inv),
+                           __fmul_rn(v[8 * j + 3], inv), __fmul_rn(v[8 * j + 4], inv), __fmul_rn(v[8 * j + 5], inv),
+                           __fmul_rn(v[8 * j + 6], inv), __fmul_rn(v[8 * j + 7], inv));
+      uint8_t *dst = q + (size_t)idx * (4 * kVecs);
+      if (kShared)
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[kVecs - 1]);
+      else
+        *reinterpret_cast<uint2 *>(dst) = make_uint2(o[0], o[1]);
+    }
+    const uint32_t s1 = __shfl_down_sync(0xffffffffu, code, 1);
+    const uint32_t s2 = __shfl_down_sync(0xffffffffu, code, 2);
+    const uint32_t s3 = __shfl_down_sync(0xffffffffu, code, 3);
+    if (live && (g & 3) == 0)
+      *reinterpret_cast<uint32_t *>(sf + sf_offset(row, g, groups)) = code | (s1 << 8) | (s2 << 16) | (s3 << 24);
+    if (kShared && live && (g & 1) == 0)  // the two 16-group slots of a 32-group are neighbours
+      *reinterpret_cast<uint32_t *>(sf2 + sf_offset(row, 2 * g, k / 16)) = code * 0x101u | (s1 * 0x1010000u);
+  }
+}
+
 inline unsigned blocks_for(long long items) { return (unsigned)((items + 255) / 256); }
 
 }  // namespace
@@ -167,6 +306,32 @@ cudaError_t run_duplicate_sf32_to_sf16(const void *sf32, int rows, int k, void *
 cudaError_t run_quantize_dense_nvfp4(const void *x, int rows, int k, void *q, void *sf, cudaStream_t stream) {
   quantize_dense_nvfp4_kernel<<<blocks_for((long long)rows * (k / 16)), 256, 0, stream>>>(
       static_cast<const __nv_bfloat16 *>(x), rows, k, static_cast<uint8_t *>(q), static_cast<uint8_t *>(sf));
+  return cudaGetLastError();
+}
+
+cudaError_t run_scaled_quantize(const void *x, int rows, int k, bool shared, float *partials, void *q, void *sf, void *sf2,
+                                float *scale_out, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err != cudaSuccess) return err;
+  if ((err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return err;
+  const size_t n16 = (size_t)rows * k / 8;
+  // four 16-byte loads in flight per thread, six CTAs per SM
+  size_t parts = (n16 + 4 * kScaledThreads - 1) / (4 * kScaledThreads);
+  const size_t cap = (size_t)6 * sms < (size_t)kScaledQuantPartials ? (size_t)6 * sms : (size_t)kScaledQuantPartials;
+  if (parts > cap) parts = cap;
+  absmax_partials_kernel<<<(unsigned)parts, kScaledThreads, 0, stream>>>(static_cast<const uint4 *>(x), n16, partials);
+  const long long chunks = ((long long)rows * (k / (shared ? 32 : 16)) + kScaledThreads - 1) / kScaledThreads;
+  const long long full = 6LL * sms;
+  const unsigned grid = (unsigned)(chunks < full ? chunks : full);
+  if (shared)
+    scaled_quantize_kernel<true><<<grid, kScaledThreads, 0, stream>>>(
+        static_cast<const uint4 *>(x), rows, k, partials, (int)parts, static_cast<uint8_t *>(q), static_cast<uint8_t *>(sf),
+        static_cast<uint8_t *>(sf2), scale_out);
+  else
+    scaled_quantize_kernel<false><<<grid, kScaledThreads, 0, stream>>>(
+        static_cast<const uint4 *>(x), rows, k, partials, (int)parts, static_cast<uint8_t *>(q), static_cast<uint8_t *>(sf),
+        nullptr, scale_out);
   return cudaGetLastError();
 }
 

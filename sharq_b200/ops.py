@@ -379,6 +379,43 @@ def quantize_w_nvfp4(W: torch.Tensor):
     return _quantize_nvfp4(W, "reorder_quantize_w")
 
 
+def _scaled_quantize_input(X: torch.Tensor, name: str) -> torch.Tensor:
+    _check(X.is_cuda and X.dtype == torch.bfloat16 and X.dim() == 2 and X.numel() > 0,
+           f"{name} must be a non-empty CUDA bfloat16 matrix")
+    X = X.contiguous()
+    return X if X.data_ptr() % 16 == 0 else X.clone()
+
+
+def scaled_quantize_nvfp4(X: torch.Tensor):
+    """Unscaled bf16 X [rows, K], K % 64 == 0 -> (QX [rows, K/2], SFX, scale [0-dim float32]): tensor scale,
+    division and dense NVFP4 quantisation in two launches (extra op, not in the reference)."""
+    X = _scaled_quantize_input(X, "X")
+    rows, K = int(X.shape[0]), int(X.shape[1])
+    dev, ws_bytes = X.device, int(_lib.lib().sharq_scaled_quantize_workspace_bytes())
+    Q = torch.empty((rows, K // 2), dtype=torch.uint8, device=dev)
+    SF, ws = _u8(_sf_bytes(rows, K), dev), _u8(ws_bytes, dev)
+    scale = torch.empty((), dtype=torch.float32, device=dev)
+    with _on_device(dev):
+        _lib.check(_lib.lib().sharq_scaled_quantize_nvfp4(_ptr(X), rows, K, _ptr(ws), ws_bytes, _ptr(Q), _ptr(SF), _ptr(scale),
+                                                          _stream(dev)))
+    return Q, SF, scale
+
+
+def scaled_quantize_w32_shared(W: torch.Tensor):
+    """Unscaled bf16 W [N, K], K % 128 == 0 -> (QW [N, K/2], SFW_sparse, SFW_dense, scale [0-dim float32]):
+    tensor scale, division and shared weight quantisation in two launches (extra op, not in the reference)."""
+    W = _scaled_quantize_input(W, "W")
+    N, K = int(W.shape[0]), int(W.shape[1])
+    dev, ws_bytes = W.device, int(_lib.lib().sharq_scaled_quantize_workspace_bytes())
+    QW = torch.empty((N, K // 2), dtype=torch.uint8, device=dev)
+    SFS, SFD, ws = _u8(_sf_bytes(N, K), dev), _u8(_sf_bytes(N, K), dev), _u8(ws_bytes, dev)
+    scale = torch.empty((), dtype=torch.float32, device=dev)
+    with _on_device(dev):
+        _lib.check(_lib.lib().sharq_scaled_quantize_w32_shared(_ptr(W), N, K, _ptr(ws), ws_bytes, _ptr(QW), _ptr(SFS), _ptr(SFD),
+                                                               _ptr(scale), _stream(dev)))
+    return QW, SFS, SFD, scale
+
+
 def _check_identity(reorder_index: torch.Tensor, K: int, KE: int) -> None:
     _check(int(KE) == 0, "sharq_b200 supports the deprecated reorder ops only with KE == 0")
     _check(reorder_index.numel() == K, "reorder_index must have K entries")

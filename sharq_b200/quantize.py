@@ -1,9 +1,9 @@
 """Host-side quantisation helpers with the names and meaning of the reference's
 model/quantize.py (lines 43-44, 141-200), running on the sm_100a ops.
 
-Differences in mechanism only: the activation helpers fold the tensor-scale passes
-(amax, divide) into the kernels instead of running them as separate PyTorch ops; the
-returned tuples are the same.
+Differences in mechanism only: the helpers fold the tensor-scale passes (amax, divide) into
+the kernels instead of running them as separate PyTorch ops; the returned tuples are the same.
+Other dtypes than bf16 and widths that the folded kernels do not take keep the PyTorch passes.
 """
 from __future__ import annotations
 
@@ -17,9 +17,17 @@ def global_nvfp4_scale(x: torch.Tensor) -> torch.Tensor:
     return torch.clamp(x.abs().max().float() / (448.0 * 6.0), min=1e-9)
 
 
+def _folds(x: torch.Tensor, k_multiple: int) -> bool:
+    """Whether the scaled quantisation kernels take x as it is."""
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.numel() > 0 and x.shape[1] % k_multiple == 0
+            and x.shape[1] <= 32768)
+
+
 @torch.no_grad()
 def quantize_weight_shared_nvfp4(weight: torch.Tensor):
     """-> (q_weight, scale_weight_sparse, scale_weight_dense, scale) (model/quantize.py:149-153)."""
+    if _folds(weight, 128):
+        return ops.scaled_quantize_w32_shared(weight)
     scale = global_nvfp4_scale(weight)
     q, sfs, sfd = ops.quantize_w32_shared((weight / scale).to(torch.bfloat16).contiguous())
     return q, sfs, sfd, scale
@@ -28,6 +36,8 @@ def quantize_weight_shared_nvfp4(weight: torch.Tensor):
 @torch.no_grad()
 def quantize_weight_nvfp4(weight: torch.Tensor):
     """-> (q_weight, scale_weight, scale) (model/quantize.py:141-145)."""
+    if _folds(weight, 64):
+        return ops.scaled_quantize_nvfp4(weight)
     scale = global_nvfp4_scale(weight)
     q, sf = ops.quantize_w_nvfp4((weight / scale).to(torch.bfloat16).contiguous())
     return q, sf, scale
@@ -36,6 +46,8 @@ def quantize_weight_nvfp4(weight: torch.Tensor):
 @torch.no_grad()
 def quantize_activation_nvfp4(x: torch.Tensor):
     """-> (q_x, scale_x, scale) (model/quantize.py:165-169)."""
+    if _folds(x, 64):
+        return ops.scaled_quantize_nvfp4(x)
     scale = global_nvfp4_scale(x)
     q, sf = ops.quantize_x_nvfp4((x / scale).to(torch.bfloat16).contiguous())
     return q, sf, scale

@@ -62,3 +62,40 @@ def test_compress_sparse_a(oracle):
     want = oracle.compress_sparse_a(dense)
     assert np.array_equal(got[0], want[0])
     assert np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("rows,k", [(1, 128), (7, 384), (127, 14336), (128, 4096), (129, 256), (1000, 18944)])
+@pytest.mark.parametrize("peak", [1.0, 1.90625, 3e38, 1e-30])
+def test_scaled_quantisation_equals_the_torch_passes(rows, k, peak):
+    """Edges of the 128-row scale bands and of the 256-group chunks; absmax values whose bf16(scale) is a power of
+    two, a short significand, near overflow and clamped to 1e-9.  Bytes equal those of torch's own absmax and division
+    in front of the quantisation of the scaled tensor."""
+    from sharq_b200 import ops, quantize
+
+    x = H.config0_x(rows, k, seed=rows)
+    x = (x.float() * (peak / x.float().abs().max())).to(torch.bfloat16).cuda()
+    scale = quantize.global_nvfp4_scale(x)
+    scaled = (x / scale).to(torch.bfloat16).contiguous()
+    qw, sfs, sfd, got_scale = ops.scaled_quantize_w32_shared(x)
+    for got, want in zip((qw, sfs, sfd), ops.quantize_w32_shared(scaled)):
+        assert torch.equal(got, want)
+    assert torch.equal(got_scale, scale)
+    q, sf, got_scale = ops.scaled_quantize_nvfp4(x)
+    want_q, want_sf = ops.quantize_x_nvfp4(scaled)
+    assert torch.equal(q, want_q) and torch.equal(got_scale, scale)
+    r = torch.arange(rows, device="cuda")[:, None]
+    g = torch.arange(k // 16, device="cuda")[None]
+    at = (r // 128) * (k // 64) * 512 + (g // 4) * 512 + (r % 32) * 16 + ((r // 32) % 4) * 4 + g % 4  # padding is not written
+    assert torch.equal(sf[at], want_sf[at])
+
+
+def test_scaled_quantisation_keeps_a_nan_like_the_torch_passes():
+    from sharq_b200 import ops, quantize
+
+    x = H.config0_x(40, 256, seed=3).cuda()
+    x[7, 100] = float("nan")
+    scaled = (x / quantize.global_nvfp4_scale(x)).to(torch.bfloat16).contiguous()
+    qw, sfs, sfd, scale = ops.scaled_quantize_w32_shared(x)
+    assert bool(torch.isnan(scale))
+    for got, want in zip((qw, sfs, sfd), ops.quantize_w32_shared(scaled)):
+        assert torch.equal(got, want)
