@@ -210,6 +210,19 @@ int sharq_linear_gemm_ws(const void *a_comp, const void *e, const void *sfa_spar
                          int k, float alpha, const float *alpha_dev, const void *bias_bf16, void *d, void *workspace,
                          size_t workspace_bytes, int *error_flag, void *stream);
 
+/* Fused SharQ GEMM of a merged gate_up weight [2*ffn, K] (gate rows first, ffn % 128 == 0, no bias) whose epilogue
+ * applies SwiGLU: h[m, ffn] = bf16(bf16(silu(gate)) * up), gate and up rounded to bf16 first, and the bits of max|h| go to
+ * amax_bits (one uint32 word, 16-byte aligned rows of h).  The same bits as sharq_linear_gemm followed by sharq_swiglu, without the [m, 2*ffn]
+ * intermediate.  sharq_absmax_sparse_residual_quantize_x is sharq_scaled_sparse_residual_quantize_x for an X whose max|X|
+ * is already in amax_bits (no statistics pass).  sharq_gemm_swiglu_pays: 1 where this form is the faster one. */
+int sharq_gemm_swiglu_pays(int m, int ffn, int k);
+int sharq_linear_gemm_swiglu(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res,
+                             const void *qw, const void *sfw_sparse, const void *sfw_dense, int m, int ffn, int k, float alpha,
+                             const float *alpha_dev, void *h, void *amax_bits, int *error_flag, void *stream);
+int sharq_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, int n, int k, const void *amax_bits, void *a_comp,
+                                            void *e, void *sfa_sparse, void *q_res, void *sf_res, float *scale_out,
+                                            void *stream);
+
 /* No counterpart in the reference.  Same work and outputs as
  * sharq_fused_rmsnorm_sparse_residual_quantize_x, for callers that cannot allocate device
  * memory and have no spare buffer to pass as workspace (a server that has given all free
@@ -268,6 +281,8 @@ int sharq_allreduce_bf16_peer(void *const *rank_data_ptrs, void *const *rank_fla
  *   sharq_linear_gemm_grouped: D[r] = alpha * alpha_vec[g] * (A_sparse[r] + A_res[r]) . W_g^T for every
  *     row r of a unit of expert g (one launch; qw / sfw_sparse / sfw_dense: host arrays of `groups`
  *     device pointers; alpha_vec: device, e.g. activation scale x weight scale per expert).
+ *   sharq_linear_gemm_grouped_swiglu / sharq_grouped_absmax_sparse_residual_quantize_x: the grouped
+ *     forms of sharq_linear_gemm_swiglu and sharq_absmax_sparse_residual_quantize_x (amax_workspace: `groups` words).
  *   sharq_moe_combine: out[t] = sum over the top_k slots of token t, in ascending expert order, of
  *     y[dest[t,j]] * w[t,j] with bf16 rounding after every product and addition, which is what the
  *     reference's sequence of index_add_ calls on a zero buffer computes. */
@@ -282,6 +297,13 @@ int sharq_linear_gemm_grouped(const void *a_comp, const void *e, const void *sfa
                               int groups, const void *const *qw, const void *const *sfw_sparse, const void *const *sfw_dense,
                               const int *unit_group, const float *alpha_vec, float alpha, int m, int n, int k, void *d,
                               int *error_flag, void *stream);
+int sharq_linear_gemm_grouped_swiglu(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res,
+                                     const void *sf_res, int groups, const void *const *qw, const void *const *sfw_sparse,
+                                     const void *const *sfw_dense, const int *unit_group, const float *alpha_vec, float alpha,
+                                     int m, int ffn, int k, void *h, void *amax_workspace, int *error_flag, void *stream);
+int sharq_grouped_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, int n, int k, const int *unit_group, int groups,
+                                                    const void *amax_workspace, void *a_comp, void *e, void *sfa_sparse,
+                                                    void *q_res, void *sf_res, float *scale_vec_out, void *stream);
 int sharq_moe_combine(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
                       int tokens, int top_k, int width, void *stream);
 

@@ -53,6 +53,10 @@ SIGNATURES = {
         c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, c_float, _P, _P, c_size_t, _P, _P]),
     "sharq_linear_gemm_ws": (
         c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, _P, _P, c_size_t, _P, _P]),
+    "sharq_gemm_swiglu_pays": (c_int, [c_int, c_int, c_int]),
+    "sharq_linear_gemm_swiglu": (
+        c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, _P, _P, _P]),
+    "sharq_absmax_sparse_residual_quantize_x": (c_int, [_P, c_int, c_int, c_int, _P, _P, _P, _P, _P, _P, _P, _P]),
     "sharq_set_gemm_tile_n": (c_int, [c_int]),
     "sharq_set_wait_limit_cycles": (c_int, [c_longlong]),
     "sharq_allreduce_bf16_multimem": (c_int, [_P, POINTER(c_void_p), c_int, c_int, c_size_t, c_int, _P, _P]),
@@ -64,6 +68,11 @@ SIGNATURES = {
     "sharq_linear_gemm_grouped": (
         c_int, [_P, _P, _P, _P, _P, c_int, POINTER(c_void_p), POINTER(c_void_p), POINTER(c_void_p), _P, _P, c_float, c_int,
                 c_int, c_int, _P, _P, _P]),
+    "sharq_linear_gemm_grouped_swiglu": (
+        c_int, [_P, _P, _P, _P, _P, c_int, POINTER(c_void_p), POINTER(c_void_p), POINTER(c_void_p), _P, _P, c_float, c_int,
+                c_int, c_int, _P, _P, _P, _P]),
+    "sharq_grouped_absmax_sparse_residual_quantize_x": (
+        c_int, [_P, c_int, c_int, c_int, _P, c_int, _P, _P, _P, _P, _P, _P, _P, _P]),
     "sharq_moe_combine": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, _P]),
     "sharq_linear_gemm_scatter": (
         c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, POINTER(c_void_p), c_int, c_int, _P, _P]),

@@ -139,6 +139,17 @@ int sharq_scaled_sparse_residual_quantize_x(const void *x, int m, int n, int k, 
                     "scaled_sparse_residual_quantize_x");
 }
 
+int sharq_absmax_sparse_residual_quantize_x(const void *x, int m, int n, int k, const void *amax_bits, void *a_comp, void *e,
+                                            void *sfa_sparse, void *q_res, void *sf_res, float *scale_out, void *stream) {
+  (void)n;
+  SHARQ_REQUIRE(m > 0 && k > 0, "X must be shaped [M, K]");
+  SHARQ_REQUIRE(k % 128 == 0, "absmax_sparse_residual_quantize_x requires K to be a multiple of 128, got %d", k);
+  SHARQ_REQUIRE(x && amax_bits && a_comp && e && sfa_sparse && q_res && sf_res, "null buffer");
+  return check_cuda(sharq::run_scaled_prepare(x, nullptr, 0.0f, m, k, const_cast<void *>(amax_bits), nullptr, a_comp, e,
+                                              sfa_sparse, q_res, sf_res, scale_out, as_stream(stream), /*absmax_ready=*/true),
+                    "absmax_sparse_residual_quantize_x");
+}
+
 int sharq_rope_inplace(void *x_bf16, int rows, int row_stride, int seq_len, int heads, int head_dim, const void *cos_bf16,
                        const void *sin_bf16, void *stream) {
   SHARQ_REQUIRE(x_bf16 && cos_bf16 && sin_bf16, "null buffer");
@@ -332,10 +343,12 @@ int sharq_grouped_swiglu_sparse_residual_quantize_x(const void *gate_up_bf16, in
                     "grouped_swiglu_sparse_residual_quantize_x");
 }
 
-int sharq_linear_gemm_grouped(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res,
-                              int groups, const void *const *qw, const void *const *sfw_sparse, const void *const *sfw_dense,
-                              const int *unit_group, const float *alpha_vec, float alpha, int m, int n, int k, void *d,
-                              int *error_flag, void *stream) {
+namespace {
+
+int gemm_grouped(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res, int groups,
+                 const void *const *qw, const void *const *sfw_sparse, const void *const *sfw_dense, const int *unit_group,
+                 const float *alpha_vec, float alpha, int m, int n, int k, void *d, unsigned int *amax_bits, int *error_flag,
+                 void *stream) {
   SHARQ_REQUIRE(m > 0 && m % 256 == 0 && n > 0 && k > 0 && k % 128 == 0,
                 "M must be a positive multiple of 256, K a multiple of 128");
   SHARQ_REQUIRE(groups >= 1 && groups <= sharq::kGemmMaxGroups, "groups must be in [1, %d]", sharq::kGemmMaxGroups);
@@ -363,7 +376,41 @@ int sharq_linear_gemm_grouped(const void *a_comp, const void *e, const void *sfa
   g.n = n;
   g.k = k;
   g.error_flag = error_flag;
+  g.amax_bits = amax_bits;
   return check_cuda(sharq::run_gemm_grouped(g, as_stream(stream)), "linear_gemm_grouped");
+}
+
+}  // namespace
+
+int sharq_linear_gemm_grouped(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res,
+                              int groups, const void *const *qw, const void *const *sfw_sparse, const void *const *sfw_dense,
+                              const int *unit_group, const float *alpha_vec, float alpha, int m, int n, int k, void *d,
+                              int *error_flag, void *stream) {
+  return gemm_grouped(a_comp, e, sfa_sparse, q_res, sf_res, groups, qw, sfw_sparse, sfw_dense, unit_group, alpha_vec, alpha, m, n,
+                      k, d, nullptr, error_flag, stream);
+}
+
+int sharq_linear_gemm_grouped_swiglu(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res,
+                                     const void *sf_res, int groups, const void *const *qw, const void *const *sfw_sparse,
+                                     const void *const *sfw_dense, const int *unit_group, const float *alpha_vec, float alpha,
+                                     int m, int ffn, int k, void *h, void *amax_workspace, int *error_flag, void *stream) {
+  SHARQ_REQUIRE(ffn > 0 && ffn % 128 == 0, "ffn must be a positive multiple of 128, got %d", ffn);
+  SHARQ_REQUIRE(h && amax_workspace && (reinterpret_cast<uintptr_t>(h) & 15) == 0, "h must be 16-byte aligned, amax_workspace set");
+  return gemm_grouped(a_comp, e, sfa_sparse, q_res, sf_res, groups, qw, sfw_sparse, sfw_dense, unit_group, alpha_vec, alpha, m,
+                      2 * ffn, k, h, static_cast<unsigned int *>(amax_workspace), error_flag, stream);
+}
+
+int sharq_grouped_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, int n, int k, const int *unit_group, int groups,
+                                                    const void *amax_workspace, void *a_comp, void *e, void *sfa_sparse,
+                                                    void *q_res, void *sf_res, float *scale_vec_out, void *stream) {
+  (void)n;
+  SHARQ_REQUIRE(m > 0 && m % 256 == 0 && k > 0 && k % 128 == 0, "M must be a positive multiple of 256 and K of 128");
+  SHARQ_REQUIRE(groups >= 1 && groups <= sharq::kGemmMaxGroups, "groups must be in [1, %d]", sharq::kGemmMaxGroups);
+  SHARQ_REQUIRE(x_bf16 && unit_group && amax_workspace && a_comp && e && sfa_sparse && q_res && sf_res && scale_vec_out,
+                "null buffer");
+  return check_cuda(sharq::run_grouped_prepare(x_bf16, m, k, static_cast<const unsigned int *>(amax_workspace), unit_group, groups,
+                                               a_comp, e, sfa_sparse, q_res, sf_res, scale_vec_out, as_stream(stream)),
+                    "grouped_absmax_sparse_residual_quantize_x");
 }
 
 int sharq_moe_combine(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
@@ -589,6 +636,37 @@ int sharq_linear_gemm_ws(const void *a_comp, const void *e, const void *sfa_spar
   SHARQ_REQUIRE(workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15) == 0,
                 "workspace must be 16-byte aligned");
   return check_cuda(sharq::run_gemm(g, as_stream(stream)), "linear_gemm");
+}
+
+int sharq_gemm_swiglu_pays(int m, int ffn, int k) { return m > 0 && ffn > 0 && k > 0 && sharq::gemm_swiglu_pays(m, ffn, k); }
+
+int sharq_linear_gemm_swiglu(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res,
+                             const void *qw, const void *sfw_sparse, const void *sfw_dense, int m, int ffn, int k, float alpha,
+                             const float *alpha_dev, void *h, void *amax_bits, int *error_flag, void *stream) {
+  SHARQ_REQUIRE(m > 0 && ffn > 0 && k > 0, "M, ffn, K must be positive");
+  SHARQ_REQUIRE(k % 128 == 0, "linear_gemm_swiglu requires K to be a multiple of 128, got %d", k);
+  SHARQ_REQUIRE(ffn % 128 == 0, "linear_gemm_swiglu requires ffn to be a multiple of 128, got %d", ffn);
+  SHARQ_REQUIRE(a_comp && e && sfa_sparse && q_res && sf_res && qw && sfw_sparse && sfw_dense && h && amax_bits && error_flag,
+                "null buffer");
+  SHARQ_REQUIRE((reinterpret_cast<uintptr_t>(h) & 15) == 0, "h must be 16-byte aligned");
+  sharq::GemmArgs g;
+  g.a_comp = a_comp;
+  g.e = e;
+  g.sfa_sparse = sfa_sparse;
+  g.a_dense = q_res;
+  g.sfa_dense = sf_res;
+  g.b = qw;
+  g.sfb_sparse = sfw_sparse;
+  g.sfb_dense = sfw_dense;
+  g.d = h;
+  g.alpha = alpha;
+  g.alpha_ptr = alpha_dev;
+  g.m = m;
+  g.n = 2 * ffn;
+  g.k = k;
+  g.amax_bits = static_cast<unsigned int *>(amax_bits);
+  g.error_flag = error_flag;
+  return check_cuda(sharq::run_gemm_swiglu(g, as_stream(stream)), "linear_gemm_swiglu");
 }
 
 }  // extern "C"

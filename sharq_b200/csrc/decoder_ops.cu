@@ -19,6 +19,7 @@
 #include <cstdint>
 
 #include "decoder_ops.cuh"
+#include "silu.cuh"
 
 namespace sharq {
 
@@ -28,18 +29,6 @@ __device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 
 __device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
 __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
-__device__ __forceinline__ float exp2f_approx(float v) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
-}
-
-__device__ __forceinline__ float rcp_approx(float v) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
-}
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
@@ -90,25 +79,6 @@ __global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16 *__restrict__ x
     *reinterpret_cast<uint4 *>(p) = make_uint4(oa[0], oa[1], oa[2], oa[3]);
     *reinterpret_cast<uint4 *>(p + half) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
   }
-}
-
-// silu as ATen computes it for a bf16 tensor: x / (1 + exp(-x)) in float, rounded to bf16.
-// The kernel would be bound by the accurate expf and the IEEE division, so the value is first
-// formed with the approximate exp2 and reciprocal units: for |x| <= 16 that result is within
-// (1.5 |x| + 8) * 2^-24 <= 2^-19 relative (32 float ulps) of the true value (argument
-// rounding 1.5 |x|, ex2.approx 4, the addition 1, rcp.approx 2, the product 1), and the
-// accurate formula within 3 ulps.  When the fast value lies more than 40 ulps from every bf16
-// rounding boundary (float bits ...8000) both round to the same bf16 number; otherwise, and
-// for |x| > 16, the accurate formula is evaluated.
-__device__ __forceinline__ float silu_accurate(float x) { return x / (1.0f + expf(-x)); }
-
-__device__ __forceinline__ float silu_bf16(float x) {
-  const float e = exp2f_approx(-1.4426950408889634f * x);
-  const float fast = x * rcp_approx(1.0f + e);
-  const uint32_t t = (__float_as_uint(fast) + 0x8000u + 40u) & 0xFFFFu;
-  float v = fast;
-  if (!(fabsf(x) <= 16.0f && t >= 81u)) v = silu_accurate(x);
-  return round_bf16(v);
 }
 
 // One CTA walks rows; its 256 threads hold up to four 16-byte vectors of the row each (K <= 8192)
@@ -251,7 +221,8 @@ __global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           // the product of two bf16 values is exact in float; the packed conversion rounds it once
-          o[j] = pack2(__fmul_rn(silu_bf16(lo_f(gw[j])), lo_f(uw[j])), __fmul_rn(silu_bf16(hi_f(gw[j])), hi_f(uw[j])));
+          const uint32_t sw = pack2(silu_f32(lo_f(gw[j])), silu_f32(hi_f(gw[j])));
+          o[j] = pack2(__fmul_rn(lo_f(sw), lo_f(uw[j])), __fmul_rn(hi_f(sw), hi_f(uw[j])));
           mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<__nv_bfloat162 *>(&o[j])));
         }
         *reinterpret_cast<uint4 *>(hrow + v * 8) = make_uint4(o[0], o[1], o[2], o[3]);

@@ -33,6 +33,7 @@
 // to the common exit, where tensor memory is released.
 #include "common.cuh"
 #include "gemm.cuh"
+#include "silu.cuh"
 #include "sm100_ptx.cuh"
 
 #include <cstring>
@@ -113,6 +114,7 @@ struct GemmParams {
   // source GPU.  scatter_rows is a multiple of 128, so a tile has one owner.  scatter_rows == 0: plain output.
   __nv_bfloat16 *d_peer[kGemmMaxPeers];
   int scatter_rows, scatter_rank;
+  unsigned int *amax_bits;  // SWIGLU: bits of max|h| are raised here (one word per group when grouped)
 };
 
 // Grouped launch (mixture-of-experts layers): the rows of the activation are sorted by group
@@ -211,7 +213,46 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams &p, const uint32
   }
 }
 
-template <int BN, bool SPARSE, bool DENSE, bool PAIR, bool GROUPED, bool WIDE = false>
+// SwiGLU of 32 columns held in registers: h = bf16(bf16(silu(g)) * u), g and u rounded to bf16 as the plain epilogue
+// stores them, into the warp's staging tile (layout of epilogue_chunk); returns the packed max |h| of this row.
+__device__ __forceinline__ __nv_bfloat162 swiglu_chunk(const uint32_t *gate, const uint32_t *up, float alpha, uint8_t *stage,
+                                                       int stage_row) {
+  __nv_bfloat162 mx = __floats2bfloat162_rn(0.0f, 0.0f);
+#pragma unroll
+  for (int v = 0; v < 4; ++v) {
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int j = 8 * v + 2 * i;
+      const float2 g = __bfloat1622float2(
+          __floats2bfloat162_rn(alpha * __uint_as_float(gate[j]), alpha * __uint_as_float(gate[j + 1])));
+      const float2 w = __bfloat1622float2(__floats2bfloat162_rn(alpha * __uint_as_float(up[j]), alpha * __uint_as_float(up[j + 1])));
+      const float2 s = __bfloat1622float2(__floats2bfloat162_rn(silu_f32(g.x), silu_f32(g.y)));
+      const __nv_bfloat162 h = __floats2bfloat162_rn(__fmul_rn(s.x, w.x), __fmul_rn(s.y, w.y));
+      mx = __hmax2(mx, __habs2(h));
+      o[i] = *reinterpret_cast<const uint32_t *>(&h);
+    }
+    *reinterpret_cast<uint4 *>(stage + stage_row * 64 + ((v ^ ((stage_row >> 1) & 3)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  return mx;
+}
+
+// Warp-wide maximum raised into *amax_bits (non-negative floats order like their bit patterns); the read first keeps
+// most warps from an atomic once the maximum has settled.
+__device__ __forceinline__ void raise_absmax(unsigned int *amax_bits, __nv_bfloat162 mx2, int lane) {
+  float mx = fmaxf(__bfloat162float(mx2.x), __bfloat162float(mx2.y));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  const unsigned int bits = __float_as_uint(mx);
+  if (lane == 0 && bits > *reinterpret_cast<volatile unsigned int *>(amax_bits)) atomicMax(amax_bits, bits);
+}
+
+// SWIGLU: the weight is a merged gate_up matrix [2F, k] and the launch writes h = silu(gate) * up [m, F] and max|h|
+// instead of the product: a pair tile takes 128 gate rows (CTA 0's half of the weight tile) and the 128 up rows of the
+// same columns (CTA 1's half), so that an epilogue thread holds both factors of its elements.  The separate SwiGLU pass reads
+// and writes 6 bytes per element of h (41 us at 2048 x 14336, 300 us at 16384 x 18944, about its memory time); here the
+// arithmetic hides behind the next tile's MMAs: whole layers 518 -> 487 us (2048 tokens) and 4.26 -> 3.85 ms (16384).
+template <int BN, bool SPARSE, bool DENSE, bool PAIR, bool GROUPED, bool WIDE = false, bool SWIGLU = false>
 __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtensorMap &tm_a_dense, const CUtensorMap &tm_a_comp,
                                           const GemmParams &p, const GroupTable *gt) {
   using L = StageLayout<BN, SPARSE, DENSE, PAIR>;
@@ -242,6 +283,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   // work units: a unit is one output tile of a CTA (128 x BN) or of a pair (256 x BN)
   const int m_units = PAIR ? (p.m + 255) / 256 : (p.m + kBM - 1) / kBM;
   const int n_tiles = (p.n + BN - 1) / BN;
+  const int ffn = p.n >> 1;  // SWIGLU: columns of h (a multiple of 128)
   const int k_splits = p.k_splits;
   const int num_units = m_units * n_tiles * k_splits;
   // unit -> (K share, tile); tiles M-fastest
@@ -291,7 +333,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         const uint8_t *sfb_sparse = GROUPED ? gt->sfb_sparse[grp] : p.sfb_sparse;
         const int m_tile = PAIR ? 2 * (tile % m_units) + (int)cta_rank : (tile % m_units);
         const int n_tile = tile / m_units;
-        const int w_row = n_tile * BN + (PAIR ? (int)cta_rank * (BN / 2) : 0);
+        const int w_row = SWIGLU ? n_tile * 128 + (int)cta_rank * ffn : n_tile * BN + (PAIR ? (int)cta_rank * (BN / 2) : 0);
         // The metadata and scale-factor copies are plain bulk copies without bounds checks.  A
         // tile may hang over the last 128-row band (the second CTA of a pair when ceil(M/128) is
         // odd, the second weight band of a 256-wide tile when ceil(N/128) is odd): such a band
@@ -299,7 +341,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         const int a_band = min(m_tile, a_bands - 1);
         int b_band[L::kBands];
 #pragma unroll
-        for (int b = 0; b < L::kBands; ++b) b_band[b] = min(n_tile * L::kBands + b, b_bands - 1);
+        for (int b = 0; b < L::kBands; ++b)
+          b_band[b] = SWIGLU ? n_tile + b * (ffn / 128) : min(n_tile * L::kBands + b, b_bands - 1);
         for (int it = k_begin(u), it_end = k_end(u); it < it_end; ++it, ++g) {
           const int s = (int)(g % S);
           const uint32_t ph = (g / S) & 1u;
@@ -480,6 +523,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     // stored as 8 rows x 64 contiguous bytes per instruction.
     uint8_t *stage = p.staged_store ? smem + S * L::kStageBytes + 512 + ew * 2048 : nullptr;
     uint32_t tile_iter = 0;
+    __nv_bfloat162 h_max = __floats2bfloat162_rn(0.0f, 0.0f);  // SWIGLU: running max |h|
     for (int u = unit0; u < num_units; u += unit_stride) {
       const int tile = u / k_splits;
       const int grp = GROUPED ? gt->unit_group[tile % m_units] : 0;
@@ -497,10 +541,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
       if (!ok) break;
       ptx::tc_fence_after();
       uint32_t acc[kColsPerEpiWarp];
-      const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::kColAcc + half * kColsPerEpiWarp);
+      // SWIGLU: 64 gate columns and the 64 up columns that belong to them, else neighbouring columns
+      const uint32_t taddr =
+          tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::kColAcc + half * (SWIGLU ? 64 : kColsPerEpiWarp));
 #pragma unroll
       for (int c = 0; c < kColsPerEpiWarp / 32; ++c)
-        ptx::tmem_ld_32x32b_x32(taddr + 32 * c, *reinterpret_cast<uint32_t(*)[32]>(&acc[32 * c]));
+        ptx::tmem_ld_32x32b_x32(taddr + (SWIGLU ? 32 * (c & 1) + 128 * (c >> 1) : 32 * c),
+                                *reinterpret_cast<uint32_t(*)[32]>(&acc[32 * c]));
       ptx::tmem_ld_wait();
       // the accumulator is in registers: give tensor memory back before the slow part
       ptx::tc_fence_before();
@@ -513,6 +560,28 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
       }
       const int row = m_tile * kBM + quad * 32 + lane;
       const int col_base = n_tile * BN + half * kColsPerEpiWarp;
+      if constexpr (SWIGLU) {
+        const int row0 = m_tile * kBM + quad * 32;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const __nv_bfloat162 mx = swiglu_chunk(&acc[32 * c], &acc[64 + 32 * c], alpha, stage, lane);
+          if (row < p.m) h_max = __hmax2(h_max, mx);
+          __syncwarp();
+          const int gcol = n_tile * 128 + half * 64 + 32 * c + (lane & 3) * 8;
+#pragma unroll
+          for (int it = 0; it < 4; ++it) {
+            const int r = it * 8 + (lane >> 2);
+            const uint4 v = *reinterpret_cast<const uint4 *>(stage + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4));
+            if (row0 + r < p.m) *reinterpret_cast<uint4 *>(p.d + (size_t)(row0 + r) * ffn + gcol) = v;
+          }
+          __syncwarp();
+        }
+        if (GROUPED) {  // the unit's rows belong to one group
+          raise_absmax(p.amax_bits + grp, h_max, lane);
+          h_max = __floats2bfloat162_rn(0.0f, 0.0f);
+        }
+        continue;
+      }
       if (k_splits > 1) {
         // partial sums of this K share: fp32 vector reductions into the accumulation buffer
         if (row < p.m) {
@@ -588,6 +657,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
           epilogue_chunk(p, &acc[32 * c], row, col_base + 32 * c, alpha, beta, has_c);
       }
     }
+    if (SWIGLU && !GROUPED) raise_absmax(p.amax_bits, h_max, lane);
   }
 
   ptx::tc_fence_before();
@@ -601,18 +671,19 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
 
 // WIDE: the scatter-mode epilogue (128-byte row pieces for the peer stores), its own instantiation so
 // that the other kernels keep their register allocation.
-template <int BN, bool SPARSE, bool DENSE, bool PAIR, bool WIDE = false>
+template <int BN, bool SPARSE, bool DENSE, bool PAIR, bool WIDE = false, bool SWIGLU = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a_dense,
                 const __grid_constant__ CUtensorMap tm_a_comp, const GemmParams p) {
-  gemm_body<BN, SPARSE, DENSE, PAIR, false, WIDE>(tm_w, tm_a_dense, tm_a_comp, p, nullptr);
+  gemm_body<BN, SPARSE, DENSE, PAIR, false, WIDE, SWIGLU>(tm_w, tm_a_dense, tm_a_comp, p, nullptr);
 }
 
 // The fused SharQ GEMM of all groups (experts) of a mixture-of-experts layer in one launch, CTA pairs.
+template <bool SWIGLU>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_grouped_kernel(const __grid_constant__ GroupTable groups, const __grid_constant__ CUtensorMap tm_a_dense,
                         const __grid_constant__ CUtensorMap tm_a_comp, const GemmParams p) {
-  gemm_body<256, true, true, true, true>(groups.tm_w[0], tm_a_dense, tm_a_comp, p, &groups);
+  gemm_body<256, true, true, true, true, false, SWIGLU>(groups.tm_w[0], tm_a_dense, tm_a_comp, p, &groups);
 }
 
 // Second kernel of a split-K GEMM: the epilogue on the accumulated fp32 sums, 32 columns per thread.
@@ -700,11 +771,11 @@ cudaError_t device_info(int *dev_out, int *sms_out) {
   return cudaSuccess;
 }
 
-template <int BN, bool SPARSE, bool DENSE, bool PAIR, bool WIDE = false>
+template <int BN, bool SPARSE, bool DENSE, bool PAIR, bool WIDE = false, bool SWIGLU = false>
 cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
   using L = StageLayout<BN, SPARSE, DENSE, PAIR>;
   static bool attr_set[64] = {};
-  auto kernel = gemm_kernel<BN, SPARSE, DENSE, PAIR, WIDE>;
+  auto kernel = gemm_kernel<BN, SPARSE, DENSE, PAIR, WIDE, SWIGLU>;
   int dev = 0, sms = 0;
   cudaError_t e = device_info(&dev, &sms);
   if (e != cudaSuccess) return e;
@@ -739,6 +810,7 @@ cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
   p.n = a.n;
   p.k = a.k;
   p.error_flag = a.error_flag;
+  p.amax_bits = a.amax_bits;
   p.scatter_rows = 0;
   if (a.scatter_world > 1) {
     // dealing rows to their owners needs whole 128-row tiles per owner and the coalesced store path
@@ -802,16 +874,18 @@ cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
 
 }  // namespace
 
-cudaError_t run_gemm_grouped(const GroupedGemmArgs &a, cudaStream_t stream) {
+template <bool SWIGLU>
+static cudaError_t launch_grouped(const GroupedGemmArgs &a, cudaStream_t stream) {
   using L = StageLayout<256, true, true, true>;
   static bool attr_set[64] = {};
+  auto kernel = gemm_grouped_kernel<SWIGLU>;
   if (a.groups < 1 || a.groups > kMaxGroups || a.m <= 0 || a.m % 256 != 0 || a.n <= 0 || a.k <= 0 || a.k % 128 != 0)
     return cudaErrorInvalidValue;
   int dev = 0, sms = 0;
   cudaError_t e = device_info(&dev, &sms);
   if (e != cudaSuccess) return e;
   if (!attr_set[dev]) {
-    e = cudaFuncSetAttribute(gemm_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
@@ -841,6 +915,7 @@ cudaError_t run_gemm_grouped(const GroupedGemmArgs &a, cudaStream_t stream) {
   p.n = a.n;
   p.k = a.k;
   p.error_flag = a.error_flag;
+  p.amax_bits = a.amax_bits;
   p.k_splits = 1;
   const int units = (a.m / 256) * ((a.n + 255) / 256);
   const int clusters = units < sms / 2 ? units : sms / 2;
@@ -856,7 +931,51 @@ cudaError_t run_gemm_grouped(const GroupedGemmArgs &a, cudaStream_t stream) {
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_grouped_kernel, gt, tm_ad, tm_ac, p);
+  return cudaLaunchKernelEx(&cfg, kernel, gt, tm_ad, tm_ac, p);
+}
+
+// What the SWIGLU epilogue takes: whole 128-column bands of gate and up, 16-byte aligned rows of h.
+static bool swiglu_ok(int n, const void *d, const unsigned int *amax_bits) {
+  return n > 0 && n % 256 == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0 && amax_bits != nullptr;
+}
+
+cudaError_t run_gemm_grouped(const GroupedGemmArgs &a, cudaStream_t stream) {
+  if (a.amax_bits == nullptr) return launch_grouped<false>(a, stream);
+  if (a.groups < 1 || a.groups > kMaxGroups || !swiglu_ok(a.n, a.d, a.amax_bits)) return cudaErrorInvalidValue;
+  cudaError_t e = cudaMemsetAsync(a.amax_bits, 0, sizeof(unsigned int) * a.groups, stream);
+  return e != cudaSuccess ? e : launch_grouped<true>(a, stream);
+}
+
+// Tile width of a fused or single GEMM (128 / 256 = single CTAs, 512 = CTA pairs of 256 x 256).
+static cudaError_t choose_tile_n(int m, int n, int k, int *tile_n) {
+  int dev = 0, sms = 0;
+  cudaError_t e = device_info(&dev, &sms);
+  if (e != cudaSuccess) return e;
+  const int pair_units = ((m + 255) / 256) * ((n + 255) / 256);
+  if (m <= 128 || n <= 128) {
+    *tile_n = n > 128 ? 256 : 128;
+  } else if (pair_units * 4 <= sms || k <= 512) {
+    // 256 x 256 pair tiles would keep at most half of the SMs busy, or the K loop is too
+    // short to hide the drain of a 256-wide accumulator: 128 x 128 tiles (measured at the
+    // 8-way tensor-parallel shapes: 14.6 vs 18.8 us for N = 768, 12.7 vs 16.7 us for K = 512)
+    *tile_n = 128;
+  } else {
+    *tile_n = 512;
+  }
+  return cudaSuccess;
+}
+
+bool gemm_swiglu_pays(int m, int ffn, int k) {
+  int tile_n = 0;
+  return ffn % 128 == 0 && choose_tile_n(m, 2 * ffn, k, &tile_n) == cudaSuccess && tile_n == 512;
+}
+
+cudaError_t run_gemm_swiglu(const GemmArgs &a, cudaStream_t stream) {
+  if (a.a_comp == nullptr || a.a_dense == nullptr || a.bias != nullptr || a.c_in != nullptr || a.scatter_world > 1 ||
+      !swiglu_ok(a.n, a.d, a.amax_bits))
+    return cudaErrorInvalidValue;
+  cudaError_t e = cudaMemsetAsync(a.amax_bits, 0, sizeof(unsigned int), stream);
+  return e != cudaSuccess ? e : launch<256, true, true, true, false, true>(a, stream);
 }
 
 cudaError_t run_gemm(const GemmArgs &a, cudaStream_t stream) {
@@ -866,20 +985,8 @@ cudaError_t run_gemm(const GemmArgs &a, cudaStream_t stream) {
   // tile_n: 0 = automatic, 128 / 256 = single-CTA tiles of that width, 512 = CTA pairs (256 x 256)
   int tile_n = a.tile_n;
   if (tile_n == 0) {
-    int dev = 0, sms = 0;
-    cudaError_t e = device_info(&dev, &sms);
+    cudaError_t e = choose_tile_n(a.m, a.n, a.k, &tile_n);
     if (e != cudaSuccess) return e;
-    const int pair_units = ((a.m + 255) / 256) * ((a.n + 255) / 256);
-    if (a.m <= 128 || a.n <= 128) {
-      tile_n = a.n > 128 ? 256 : 128;
-    } else if (pair_units * 4 <= sms || a.k <= 512) {
-      // 256 x 256 pair tiles would keep at most half of the SMs busy, or the K loop is too
-      // short to hide the drain of a 256-wide accumulator: 128 x 128 tiles (measured at the
-      // 8-way tensor-parallel shapes: 14.6 vs 18.8 us for N = 768, 12.7 vs 16.7 us for K = 512)
-      tile_n = 128;
-    } else {
-      tile_n = 512;
-    }
   }
   const bool pair = tile_n == 512;
   const bool scatter = a.scatter_world > 1;  // validated by launch(): fused GEMM, staged stores, whole tiles per owner

@@ -39,9 +39,19 @@ struct GemmArgs {
   // block scatter_rank.  Needs m % (128 * scatter_world) == 0 and n % 8 == 0.
   void *d_peer[kGemmMaxPeers] = {};
   int scatter_world = 0, scatter_rank = 0;
+  unsigned int *amax_bits = nullptr;  // run_gemm_swiglu only: bits of max|h|
 };
 
 cudaError_t run_gemm(const GemmArgs &args, cudaStream_t stream);
+
+// Fused SharQ GEMM of a merged gate_up weight [2F, k] (n = 2F, F % 128 == 0, no bias) whose epilogue writes
+// h = bf16(bf16(silu(gate)) * up) [m, F] to d and the bits of max|h| to *amax_bits: the bits that the plain
+// GEMM followed by the SwiGLU kernel gives.
+cudaError_t run_gemm_swiglu(const GemmArgs &args, cudaStream_t stream);
+
+// Whether that epilogue is the better form: where the plain GEMM would run CTA pairs.  With fewer or shorter tiles the
+// GEMM runs 128-wide (or split-K) tiles that hold no gate / up pairs, and gate_up is small enough to stay in L2.
+bool gemm_swiglu_pays(int m, int ffn, int k);
 
 // Fused SharQ GEMM over the groups (experts) of a mixture-of-experts layer in one launch.  The
 // activation rows are sorted by group, every group's segment padded to a multiple of 256 rows
@@ -59,6 +69,7 @@ struct GroupedGemmArgs {
   void *d = nullptr;
   int m = 0, n = 0, k = 0;
   int *error_flag = nullptr;
+  unsigned int *amax_bits = nullptr;  // set: the SwiGLU epilogue of run_gemm_swiglu, max|h| per group
 };
 cudaError_t run_gemm_grouped(const GroupedGemmArgs &args, cudaStream_t stream);
 

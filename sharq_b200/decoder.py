@@ -231,10 +231,10 @@ class SharqDecoderLayer(torch.nn.Module):
         else:
             x2 = x2 + o
             prep = self.gate_up.prepare_input_rmsnorm(x2, self.post_norm, cfg.eps)
-        gu = self.gate_up.apply_prepared(prep)
         if self.fused_glue:
-            d = self.down.apply_prepared_reduced(self.down.local.prepare_input_swiglu(gu))
+            d = self.down.apply_prepared_reduced(self.gate_up.apply_prepared_swiglu(prep, self.down.local))
         else:
+            gu = self.gate_up.apply_prepared(prep)
             f = gu.shape[1] // 2
             d = self.down(F.silu(gu[:, :f]) * gu[:, f:])
         if return_delta:
@@ -257,8 +257,7 @@ class SharqDecoderLayer(torch.nn.Module):
         attn2 = attn.transpose(1, 2).reshape(b * s, self.local_heads * cfg.head_dim)
         self.o_proj.local.apply_prepared(self.o_proj.local.prepare_input(attn2), scatter=sp.scatter)
         prepared, x_local = sp.transition(x_local, self.post_norm, cfg.eps)
-        gu = self.gate_up.apply_prepared(prepared)
-        self.down.local.apply_prepared(self.down.local.prepare_input_swiglu(gu), scatter=sp.scatter)
+        self.down.local.apply_prepared(self.gate_up.apply_prepared_swiglu(prepared, self.down.local), scatter=sp.scatter)
         return sp.transition(x_local, next_gamma, cfg.eps)
 
     @torch.no_grad()
@@ -338,8 +337,13 @@ class SharqDecoderLayer(torch.nn.Module):
                                           torch.stack([d.weight_scale.reshape(()) for _, d in self.experts]).float().contiguous())
         ws13, ws2 = self._expert_weight_scales
         p1 = ops.grouped_sparse_residual_quantize_x(hn.contiguous(), unit_group, e, src_row=src_row)
-        gu = ops.linear_gemm_grouped(*p1[:5], w13, unit_group, (p1[5] * ws13).contiguous())
-        p2 = ops.grouped_swiglu_sparse_residual_quantize_x(gu, unit_group, e)
+        alpha13 = (p1[5] * ws13).contiguous()
+        if w13[0][0].shape[0] % 256 == 0:
+            hmid, amax = ops.linear_gemm_grouped_swiglu(*p1[:5], w13, unit_group, alpha13)
+            p2 = ops.grouped_absmax_sparse_residual_quantize_x(hmid, unit_group, e, amax)
+        else:
+            p2 = ops.grouped_swiglu_sparse_residual_quantize_x(ops.linear_gemm_grouped(*p1[:5], w13, unit_group, alpha13),
+                                                               unit_group, e)
         y = ops.linear_gemm_grouped(*p2[:5], w2, unit_group, (p2[5] * ws2).contiguous())
         return ops.moe_combine(y, dest, selected.contiguous(), routing.contiguous())
 

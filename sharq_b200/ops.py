@@ -320,6 +320,23 @@ def swiglu_sparse_residual_quantize_x(gate_up: torch.Tensor, N: int):
     return A_comp, E, SFA, Q_res, SF_res, scale
 
 
+def absmax_sparse_residual_quantize_x(X: torch.Tensor, N: int, amax_bits: torch.Tensor):
+    """scaled_sparse_residual_quantize_x of an X whose max|X| is already known (amax_bits: the float's bits, as
+    linear_gemm_swiglu leaves them): one launch, no statistics pass."""
+    M, K = _check_x(X)
+    _check(K % 128 == 0, f"absmax_sparse_residual_quantize_x requires K to be a multiple of 128, got {K}")
+    _check(amax_bits.is_cuda and amax_bits.device == X.device and amax_bits.dtype == torch.int32 and amax_bits.numel() == 1,
+           "amax_bits must be one CUDA int32 on X's device")
+    dev = X.device
+    A_comp, E, SFA, Q_res, SF_res, tail = _prepare_buffers(M, K, dev, extra=256)
+    scale = tail[:4].view(torch.float32).reshape(())
+    with _on_device(dev):
+        _lib.check(_lib.lib().sharq_absmax_sparse_residual_quantize_x(
+            _ptr(X), M, int(N), K, _ptr(amax_bits), _ptr(A_comp), _ptr(E), _ptr(SFA), _ptr(Q_res), _ptr(SF_res), _ptr(scale),
+            _stream(dev)))
+    return A_comp, E, SFA, Q_res, SF_res, scale
+
+
 def scaled_sparse_residual_quantize_x(X: torch.Tensor, N: int):
     """Unscaled bf16 X -> (A_comp, E, SFA_sparse, Q_res, SF_res, scale): tensor scale,
     division and prepare in two launches (extra op, not in the reference)."""
@@ -556,6 +573,19 @@ def sparse_matmul_tensor_scale(A_comp, B, E, SFA, SFB, M: int, N: int, K: int, a
     return _sparse_gemm("sparse_matmul_tensor_scale", A_comp, B, E, SFA, SFB, M, N, K, 1.0, alpha, beta)
 
 
+def _check_fused_operands(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense) -> None:
+    M, K = int(Q_res.shape[0]), int(Q_res.shape[1]) * 2
+    N = int(QW.shape[0])
+    dev = Q_res.device
+    ea, ee, esf, eq, _ = get_fused_sparse_residual_buffer_sizes(M, N, K)
+    for t, want, nm in ((A_comp, ea, "A_comp"), (E, ee, "E"), (SFA_sparse, esf, "SFA_sparse"), (Q_res, eq, "Q_res"),
+                        (SF_res, esf, "SF_res"), (QW, N * (K // 2), "QW"), (SFW_sparse, _sf_bytes(N, K), "SFW_sparse"),
+                        (SFW_dense, _sf_bytes(N, K), "SFW_dense")):
+        _check(t.is_cuda and t.device == dev and t.dtype == torch.uint8 and t.is_contiguous(),
+               f"{nm} must be a contiguous CUDA uint8 tensor on the device of Q_res")
+        _check(t.numel() == want, f"{nm}.numel() mismatch: expected {want}, got {t.numel()}")
+
+
 def sharq_linear_gemm(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense, alpha,
                       bias: Optional[torch.Tensor] = None, alpha_host: float = 1.0,
                       out: Optional[torch.Tensor] = None, scatter=None) -> Optional[torch.Tensor]:
@@ -568,13 +598,7 @@ def sharq_linear_gemm(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_
     M, K = int(Q_res.shape[0]), int(Q_res.shape[1]) * 2
     N = int(QW.shape[0])
     dev = Q_res.device
-    ea, ee, esf, eq, _ = get_fused_sparse_residual_buffer_sizes(M, N, K)
-    for t, want, nm in ((A_comp, ea, "A_comp"), (E, ee, "E"), (SFA_sparse, esf, "SFA_sparse"), (Q_res, eq, "Q_res"),
-                        (SF_res, esf, "SF_res"), (QW, N * (K // 2), "QW"), (SFW_sparse, _sf_bytes(N, K), "SFW_sparse"),
-                        (SFW_dense, _sf_bytes(N, K), "SFW_dense")):
-        _check(t.is_cuda and t.device == dev and t.dtype == torch.uint8 and t.is_contiguous(),
-               f"{nm} must be a contiguous CUDA uint8 tensor on the device of Q_res")
-        _check(t.numel() == want, f"{nm}.numel() mismatch: expected {want}, got {t.numel()}")
+    _check_fused_operands(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense)
     if bias is not None:
         _check(bias.is_cuda and bias.dtype == torch.bfloat16 and bias.numel() == N and bias.is_contiguous(),
                "bias must be a contiguous CUDA bfloat16 tensor with N elements")
@@ -603,6 +627,30 @@ def sharq_linear_gemm(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_
             None if alpha_t is None else _scale_ptr(alpha_t, Q_res, "alpha"), _ptr(bias), _ptr(D),
             _ptr(ws), ws_bytes, _ptr(_error_flag(dev)), _stream(dev)))
     return D
+
+
+def linear_gemm_swiglu_pays(M: int, ffn: int, K: int) -> bool:
+    """Whether linear_gemm_swiglu takes the shape and is faster than the GEMM and the SwiGLU kernel."""
+    return bool(_lib.lib().sharq_gemm_swiglu_pays(int(M), int(ffn), int(K)))
+
+
+def linear_gemm_swiglu(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense, alpha: torch.Tensor,
+                       alpha_host: float = 1.0):
+    """Fused SharQ GEMM of a merged gate_up weight [2F, K] (F % 128 == 0, no bias) with SwiGLU in its epilogue:
+    -> (H [M, F] bf16, amax_bits [1] int32 with the bits of max|H|); the bits of swiglu(sharq_linear_gemm(...))."""
+    M, K = int(Q_res.shape[0]), int(Q_res.shape[1]) * 2
+    N = int(QW.shape[0])
+    dev = Q_res.device
+    _check(N % 256 == 0, f"the merged gate_up weight must have a multiple of 256 rows, got {N}")
+    _check_fused_operands(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense)
+    H = torch.empty((M, N // 2), dtype=torch.bfloat16, device=dev)
+    amax_bits = torch.empty(1, dtype=torch.int32, device=dev)
+    with _on_device(dev):
+        _lib.check(_lib.lib().sharq_linear_gemm_swiglu(
+            _ptr(A_comp), _ptr(E), _ptr(SFA_sparse), _ptr(Q_res), _ptr(SF_res), _ptr(QW), _ptr(SFW_sparse), _ptr(SFW_dense),
+            M, N // 2, K, float(alpha_host), _scale_ptr(alpha, Q_res, "alpha"), _ptr(H), _ptr(amax_bits),
+            _ptr(_error_flag(dev)), _stream(dev)))
+    return H, amax_bits
 
 
 def sharq_linear_forward(x: torch.Tensor, qw: torch.Tensor, sfw_sparse: torch.Tensor, sfw_dense: torch.Tensor,
@@ -676,10 +724,26 @@ def grouped_swiglu_sparse_residual_quantize_x(gate_up: torch.Tensor, unit_group:
     return A_comp, E, SFA, Q_res, SF_res, scales
 
 
-def linear_gemm_grouped(A_comp, E, SFA_sparse, Q_res, SF_res, weights, unit_group: torch.Tensor, alpha_vec: torch.Tensor,
-                        alpha: float = 1.0) -> torch.Tensor:
-    """Fused SharQ GEMM of a grouped activation against one weight per group in one launch.  weights: list of
-    (QW [N, K/2], SFW_sparse, SFW_dense), all of the same shape; alpha_vec: CUDA float32 [groups]."""
+def grouped_absmax_sparse_residual_quantize_x(X: torch.Tensor, unit_group: torch.Tensor, groups: int, amax_bits: torch.Tensor,
+                                              N: int = 0):
+    """grouped_sparse_residual_quantize_x of an X whose max|X| per group is already known (amax_bits int32 [groups])."""
+    _check_grouped(X, unit_group, groups, "X")
+    M, K = int(X.shape[0]), int(X.shape[1])
+    _check(K % 128 == 0, f"K must be a multiple of 128, got {K}")
+    _check(amax_bits.is_cuda and amax_bits.device == X.device and amax_bits.dtype == torch.int32 and amax_bits.is_contiguous()
+           and amax_bits.numel() == groups, "amax_bits must be a contiguous CUDA int32 vector with one entry per group")
+    dev = X.device
+    A_comp, E, SFA, Q_res, SF_res, tail = _prepare_buffers(M, K, dev, extra=256)
+    scales = tail[:4 * groups].view(torch.float32)
+    with _on_device(dev):
+        _lib.check(_lib.lib().sharq_grouped_absmax_sparse_residual_quantize_x(
+            _ptr(X), M, int(N), K, _ptr(unit_group), int(groups), _ptr(amax_bits), _ptr(A_comp), _ptr(E), _ptr(SFA),
+            _ptr(Q_res), _ptr(SF_res), _ptr(scales), _stream(dev)))
+    return A_comp, E, SFA, Q_res, SF_res, scales
+
+
+def _grouped_operands(Q_res, weights, alpha_vec):
+    """Checks shared by the grouped GEMMs -> (M, K, groups, host pointer arrays of the weight buffers)."""
     M, K = int(Q_res.shape[0]), int(Q_res.shape[1]) * 2
     groups = len(weights)
     N = int(weights[0][0].shape[0])
@@ -690,13 +754,39 @@ def linear_gemm_grouped(A_comp, E, SFA_sparse, Q_res, SF_res, weights, unit_grou
     for qw, sfs, sfd in weights:
         _check(tuple(qw.shape) == (N, K // 2) and qw.is_contiguous() and qw.device == dev, "weights must share one shape [N, K/2]")
     arr = ctypes.c_void_p * groups
-    qws, sfss, sfds = (arr(*[w[i].data_ptr() for w in weights]) for i in range(3))
+    return M, K, groups, tuple(arr(*[w[i].data_ptr() for w in weights]) for i in range(3))
+
+
+def linear_gemm_grouped(A_comp, E, SFA_sparse, Q_res, SF_res, weights, unit_group: torch.Tensor, alpha_vec: torch.Tensor,
+                        alpha: float = 1.0) -> torch.Tensor:
+    """Fused SharQ GEMM of a grouped activation against one weight per group in one launch.  weights: list of
+    (QW [N, K/2], SFW_sparse, SFW_dense), all of the same shape; alpha_vec: CUDA float32 [groups]."""
+    N = int(weights[0][0].shape[0])
+    M, K, groups, pointers = _grouped_operands(Q_res, weights, alpha_vec)
+    dev = Q_res.device
     D = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
     with _on_device(dev):
         _lib.check(_lib.lib().sharq_linear_gemm_grouped(
-            _ptr(A_comp), _ptr(E), _ptr(SFA_sparse), _ptr(Q_res), _ptr(SF_res), groups, qws, sfss, sfds, _ptr(unit_group),
+            _ptr(A_comp), _ptr(E), _ptr(SFA_sparse), _ptr(Q_res), _ptr(SF_res), groups, *pointers, _ptr(unit_group),
             _ptr(alpha_vec), float(alpha), M, N, K, _ptr(D), _ptr(_error_flag(dev)), _stream(dev)))
     return D
+
+
+def linear_gemm_grouped_swiglu(A_comp, E, SFA_sparse, Q_res, SF_res, weights, unit_group: torch.Tensor,
+                               alpha_vec: torch.Tensor, alpha: float = 1.0):
+    """linear_gemm_grouped of merged gate_up weights [2F, K] (F % 128 == 0) with SwiGLU in its epilogue:
+    -> (H [M, F] bf16, amax_bits [groups] int32 with the bits of max|H| per group; rows of empty units are not written)."""
+    N = int(weights[0][0].shape[0])
+    _check(N % 256 == 0, f"the merged gate_up weights must have a multiple of 256 rows, got {N}")
+    M, K, groups, pointers = _grouped_operands(Q_res, weights, alpha_vec)
+    dev = Q_res.device
+    H = torch.empty((M, N // 2), dtype=torch.bfloat16, device=dev)
+    amax_bits = torch.empty(groups, dtype=torch.int32, device=dev)
+    with _on_device(dev):
+        _lib.check(_lib.lib().sharq_linear_gemm_grouped_swiglu(
+            _ptr(A_comp), _ptr(E), _ptr(SFA_sparse), _ptr(Q_res), _ptr(SF_res), groups, *pointers, _ptr(unit_group),
+            _ptr(alpha_vec), float(alpha), M, N // 2, K, _ptr(H), _ptr(amax_bits), _ptr(_error_flag(dev)), _stream(dev)))
+    return H, amax_bits
 
 
 def moe_combine(y: torch.Tensor, dest: torch.Tensor, selected: torch.Tensor, w: torch.Tensor) -> torch.Tensor:

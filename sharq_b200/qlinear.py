@@ -177,6 +177,20 @@ class QLinearLayer(nn.Module):
         return y
 
     @torch.no_grad()
+    def apply_prepared_swiglu(self, prepared, down: "QLinearLayer"):
+        """down.prepare_input_swiglu(self.apply_prepared(prepared)) for a merged gate_up layer whose output nothing
+        else reads: where the shape allows, SwiGLU and the absmax run in the GEMM epilogue and the [M, 2F] product
+        is never stored (same bits)."""
+        if (prepared[0] == "SHARQ" and down.quant_type == "SHARQ" and self.fused_gemm and self.bias is None
+                and self.out_features % 256 == 0
+                and ops.linear_gemm_swiglu_pays(prepared[4].shape[0], self.out_features // 2, self.in_features)):
+            _, a_comp, e, sfa, q_res, sf_res, scale_x = prepared
+            h, amax_bits = ops.linear_gemm_swiglu(a_comp, e, sfa, q_res, sf_res, self.weight_q, self.scale_w_sparse,
+                                                  self.scale_w_dense, scale_x.reshape(1), alpha_host=self.weight_scale_host)
+            return ("SHARQ", *ops.absmax_sparse_residual_quantize_x(h, down.out_features, amax_bits))
+        return down.prepare_input_swiglu(self.apply_prepared(prepared))
+
+    @torch.no_grad()
     def forward(self, x):
         if isinstance(x, tuple):
             x_orig, bsz, q_len = x
