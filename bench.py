@@ -147,7 +147,7 @@ def kernel_category(name: str) -> str:
         return "sharq_kernel+collective"  # reduce-scatter sum, RMSNorm prepare and all-gather in one kernel
     if "allreduce" in n or "nccl" in n:
         return "collective"
-    if "gemm" in n or "splitk_finalize" in n or "nvjet" in n or "cutlass" in n or "cublas" in n:
+    if "gemm" in n or "nvjet" in n or "cutlass" in n or "cublas" in n:
         return "gemm"
     if "prepare_" in n or "rms_stats" in n or "abs_stats" in n:
         return "sharq_kernel"

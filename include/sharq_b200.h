@@ -191,13 +191,11 @@ int sharq_linear_gemm(const void *a_comp, const void *e, const void *sfa_sparse,
                       int k, float alpha, const float *alpha_dev, const void *bias_bf16, void *d, int *error_flag,
                       void *stream);
 
-/* The three GEMMs with caller-provided scratch (no counterpart in the reference).  With
- * sharq_gemm_workspace_bytes(M, N) bytes (non-zero for M <= 128: M * N floats; contents
- * need not be initialised) a small-M GEMM, which is bound by streaming the weights, splits K
- * over the SMs: units add their fp32 partial sums into the scratch with vector reductions
- * and a second kernel applies alpha / beta / bias and writes bf16.  The order of those fp32
- * additions is not fixed, so the last bits of the sums may vary from call to call.  With
- * workspace == NULL, or M > 128, these are the plain entry points. */
+/* The three GEMMs with leave to split K (no counterpart in the reference).  With a workspace of
+ * sharq_gemm_workspace_bytes(M, N) bytes (nothing is written to it: any 16-byte aligned device pointer will do) a GEMM
+ * whose tiles alone would leave SMs idle, bound by streaming the weights, splits K over the CTAs of a cluster, which sum their fp32
+ * partial tiles on chip in a fixed order: results are the same from call to call, in another order of additions
+ * than the unsplit launch.  With workspace == NULL these are the plain entry points. */
 size_t sharq_gemm_workspace_bytes(int m, int n);
 int sharq_matmul_ws(const void *a, const void *b, const void *sfa, const void *sfb, int m, int n, int k, float alpha,
                     const float *alpha_dev, const void *c_in, float beta, void *d, void *workspace,

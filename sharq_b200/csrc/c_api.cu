@@ -528,7 +528,7 @@ int sharq_set_gemm_tile_n(int tile_n) {
 }
 
 size_t sharq_gemm_workspace_bytes(int m, int n) {
-  return (m > 0 && m <= 128 && n > 0) ? (size_t)m * (size_t)n * sizeof(float) : 0;
+  return m > 0 && n > 0 ? 16 : 0;  // a split launch keeps its partial sums on chip; the workspace only says that it may split
 }
 
 int sharq_matmul(const void *a, const void *b, const void *sfa, const void *sfb, int m, int n, int k, float alpha,
@@ -558,8 +558,7 @@ int sharq_matmul_ws(const void *a, const void *b, const void *sfa, const void *s
   g.k = k;
   g.tile_n = g_tile_n;
   g.error_flag = error_flag;
-  g.workspace = workspace;
-  g.workspace_bytes = workspace ? workspace_bytes : 0;
+  g.split_k = workspace != nullptr && workspace_bytes >= sharq_gemm_workspace_bytes(m, n);
   SHARQ_REQUIRE(workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15) == 0,
                 "workspace must be 16-byte aligned");
   return check_cuda(sharq::run_gemm(g, as_stream(stream)), "matmul");
@@ -591,8 +590,7 @@ int sharq_sparse_matmul_ws(const void *a_comp, const void *b, const void *e, con
   g.k = k;
   g.tile_n = g_tile_n;
   g.error_flag = error_flag;
-  g.workspace = workspace;
-  g.workspace_bytes = workspace ? workspace_bytes : 0;
+  g.split_k = workspace != nullptr && workspace_bytes >= sharq_gemm_workspace_bytes(m, n);
   SHARQ_REQUIRE(workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15) == 0,
                 "workspace must be 16-byte aligned");
   return check_cuda(sharq::run_gemm(g, as_stream(stream)), "sparse_matmul");
@@ -631,8 +629,7 @@ int sharq_linear_gemm_ws(const void *a_comp, const void *e, const void *sfa_spar
   g.k = k;
   g.tile_n = g_tile_n;
   g.error_flag = error_flag;
-  g.workspace = workspace;
-  g.workspace_bytes = workspace ? workspace_bytes : 0;
+  g.split_k = workspace != nullptr && workspace_bytes >= sharq_gemm_workspace_bytes(m, n);
   SHARQ_REQUIRE(workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15) == 0,
                 "workspace must be 16-byte aligned");
   return check_cuda(sharq::run_gemm(g, as_stream(stream)), "linear_gemm");

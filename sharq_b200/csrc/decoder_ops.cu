@@ -183,6 +183,7 @@ __device__ __forceinline__ void cta_absmax_to(float *warp_max, __nv_bfloat162 mx
 // group, 256-row units, unit_group[u] < 0 = no rows) a CTA takes chunks of kGroupedChunkRows
 // consecutive rows, skips chunks of empty units and raises amax_bits[group of the chunk].
 constexpr int kGroupedChunkRows = 64;
+constexpr int kSwigluPieceVecs = 512;  // two vectors for each of the 256 threads
 
 __global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 *__restrict__ gate_up, long long rows,
                                                             int ffn, long long row_stride, __nv_bfloat16 *__restrict__ h,
@@ -192,22 +193,25 @@ __global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 
   const int vecs = ffn >> 3;
   __nv_bfloat162 mx2 = __floats2bfloat162_rn(0.0f, 0.0f);  // running max of |h|, two lanes
   const bool grouped = unit_group != nullptr;
-  const long long n_chunks = grouped ? (rows + kGroupedChunkRows - 1) / kGroupedChunkRows : rows;
-  // a CTA walks rows (chunks of rows when grouped), its threads the 16-byte vectors of a row, two vectors in flight per thread
+  const int pieces = grouped ? 1 : (vecs + kSwigluPieceVecs - 1) / kSwigluPieceVecs;  // pieces of a row, so that few rows fill the SMs too
+  const long long n_chunks = grouped ? (rows + kGroupedChunkRows - 1) / kGroupedChunkRows : rows * pieces;
+  // a CTA walks pieces of rows (chunks of rows when grouped), its threads the 16-byte vectors, two vectors in flight per thread
   for (long long chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
-   const long long row_lo = grouped ? chunk * kGroupedChunkRows : chunk;
-   const long long row_hi = grouped ? min(rows, row_lo + kGroupedChunkRows) : chunk + 1;
+   const long long row_lo = grouped ? chunk * kGroupedChunkRows : chunk / pieces;
+   const long long row_hi = grouped ? min(rows, row_lo + kGroupedChunkRows) : row_lo + 1;
+   const int v_lo = grouped ? 0 : (int)(chunk % pieces) * kSwigluPieceVecs;
+   const int v_hi = grouped ? vecs : min(vecs, v_lo + kSwigluPieceVecs);
    const int grp = grouped ? unit_group[row_lo / 256] : 0;
    if (grp < 0) continue;
    for (long long row = row_lo; row < row_hi; ++row) {
     const __nv_bfloat16 *grow = gate_up + row * row_stride;
     __nv_bfloat16 *hrow = h + row * (long long)ffn;
-    for (int v0 = threadIdx.x; v0 < vecs; v0 += 2 * blockDim.x) {
+    for (int v0 = v_lo + threadIdx.x; v0 < v_hi; v0 += 2 * blockDim.x) {
       uint4 g4[2], u4[2];
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const int v = v0 + t * blockDim.x;
-        if (v < vecs) {
+        if (v < v_hi) {
           g4[t] = __ldg(reinterpret_cast<const uint4 *>(grow + v * 8));
           u4[t] = __ldg(reinterpret_cast<const uint4 *>(grow + ffn + v * 8));
         }
@@ -215,7 +219,7 @@ __global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const int v = v0 + t * blockDim.x;
-        if (v >= vecs) break;
+        if (v >= v_hi) break;
         const uint32_t gw[4] = {g4[t].x, g4[t].y, g4[t].z, g4[t].w}, uw[4] = {u4[t].x, u4[t].y, u4[t].z, u4[t].w};
         uint32_t o[4];
 #pragma unroll
@@ -397,7 +401,8 @@ cudaError_t run_swiglu_absmax(const void *gate_up, long long rows, int ffn, long
     if (err != cudaSuccess) return err;
   }
   long long ctas = (long long)sm_count() * 8;
-  const long long work = unit_group != nullptr ? (rows + kGroupedChunkRows - 1) / kGroupedChunkRows : rows;
+  const long long work = unit_group != nullptr ? (rows + kGroupedChunkRows - 1) / kGroupedChunkRows
+                                               : rows * ((ffn / 8 + kSwigluPieceVecs - 1) / kSwigluPieceVecs);
   if (ctas > work) ctas = work;
   swiglu_absmax_kernel<<<(unsigned)ctas, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(gate_up), rows, ffn,
                                                             row_stride, static_cast<__nv_bfloat16 *>(h), amax_bits, unit_group);

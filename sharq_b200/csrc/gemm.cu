@@ -21,8 +21,9 @@
 //              tensor memory back to the MMA warp at once, then alpha/beta/bias, bf16 (packed
 //              conversions), a transpose through a small shared-memory tile and coalesced
 //              global stores overlap the next tile's MMAs.
-// Small M with caller scratch: K is split over the SMs, units add fp32 partial sums into the
-// scratch and splitk_finalize_kernel applies the epilogue.
+// Few tiles (decode batches, short chunks): K is split over the CTAs of a cluster, one tile per cluster; every
+// CTA leaves its fp32 partial tile in its own shared memory and the cluster's epilogue threads sum the tiles
+// in rank order through distributed shared memory (no scratch, no second kernel, a fixed order of additions).
 // CTA-pair mode (cta_group::2, cluster of 2): the pair computes a 256 x 256 tile; CTA r owns
 // rows [128r,128r+128) (its A operands, scales, metadata, accumulator) and loads weight rows
 // [128r,128r+128) of the tile; the tensor cores of both SMs read both halves.  Every CTA
@@ -46,6 +47,8 @@ namespace {
 constexpr int kBM = 128;
 constexpr int kBK = 256;  // logical K per stage
 constexpr int kEpiWarps = 8;
+constexpr int kPrefetchStages = 8;  // K stages of weights a CTA prefetches into L2 while the activation is still being prepared
+constexpr int kMaxSplits = 8;  // CTAs of a split-K cluster (the portable cluster size)
 constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 
 // Shared-memory stage and tensor-memory column layout.  In pair mode BN is the pair's tile
@@ -84,6 +87,8 @@ struct StageLayout {
   static constexpr int kColSfbD = kColSfaD + 16;
   static constexpr int kColEnd = kColSfbD + 4 * (BN / 32);
   static constexpr int kTmemCols = kColEnd <= 256 ? 256 : 512;
+  static constexpr int kPartStride = BN + 4;  // floats per row of a split launch's partial tile (row starts on distinct banks)
+  static_assert(PAIR || kBM * kPartStride * 4 <= kStages * kStageBytes, "the partial tile takes the place of the stages");
   static constexpr int kSmemBytes =
       kStages * kStageBytes + kOutStageBytes + 1024 /*alignment slack*/ + 512 /*barriers*/;
 };
@@ -102,11 +107,8 @@ struct GemmParams {
   float beta;
   int m, n, k;
   int *error_flag;
-  // Split K (small M): every output tile is computed by k_splits units, each over its share of
-  // the K stages; their fp32 partial sums are added into splitk_acc [m, n] (zero-filled by the
-  // launcher) with vector reductions and a second kernel applies the epilogue.
+  // Split K: the k_splits CTAs of a cluster compute one output tile, each over its share of the K stages.
   int k_splits;
-  float *splitk_acc;
   int staged_store;  // output tiles are transposed through shared memory for coalesced stores (N % 8 == 0)
   // Scatter mode (row-parallel linear under tensor parallelism): the output rows are dealt to their owner GPUs.
   // Row r belongs to GPU o = r / scatter_rows and is stored, through the peer mapping, into d_peer[o] at row
@@ -129,9 +131,76 @@ struct GroupTable {
   const float *alpha;     // [groups] on the device: per-group factor (activation scale x weight scale)
 };
 
-// Epilogue of 32 accumulator columns held in registers: d = bf16(alpha * acc + beta * c_in),
-// then (+ bias) in bf16; rows >= M and columns >= N are masked.  A thread owns one row and
-// stores 64 contiguous bytes.
+// Epilogue of 8 accumulator columns: o = bf16(alpha * acc + beta * c_in), then (+ bias) in bf16, packed.  Columns >= N
+// read nothing; what they hold is masked by the caller's store.
+__device__ __forceinline__ void epilogue_8(const GemmParams &p, const float (&acc)[8], int row, int col, float alpha, float beta,
+                                           bool has_c, uint32_t (&o)[4]) {
+  const bool full = (col + 8 <= p.n) && ((p.n & 7) == 0);
+  float f[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) f[i] = alpha * acc[i];
+  if (has_c) {
+    const __nv_bfloat16 *c = p.c_in + (size_t)row * p.n + col;
+    if (full && (reinterpret_cast<uintptr_t>(p.c_in) & 15) == 0) {
+      uint4 cv = *reinterpret_cast<const uint4 *>(c);
+      uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        f[2 * i] = __fmaf_rn(beta, bf16_bits_to_float(cw[i] & 0xFFFFu), f[2 * i]);
+        f[2 * i + 1] = __fmaf_rn(beta, bf16_bits_to_float(cw[i] >> 16), f[2 * i + 1]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (col + i < p.n) f[i] = __fmaf_rn(beta, __bfloat162float(c[i]), f[i]);
+    }
+  }
+  // two values per conversion instruction (the scalar conversion unit is the slow pipe here)
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    __nv_bfloat162 pair = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+    o[i] = *reinterpret_cast<uint32_t *>(&pair);
+  }
+  if (p.bias != nullptr) {
+    // bias is added to the bf16 result, as a separate bf16 add would (a bf16 add rounds the
+    // exact sum once, which is what the fp32 add + rounding of two bf16 values gives)
+    if (full && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
+      const uint4 bv = __ldg(reinterpret_cast<const uint4 *>(p.bias + col));
+      const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        __nv_bfloat162 sum = __hadd2(*reinterpret_cast<__nv_bfloat162 *>(&o[i]),
+                                     *reinterpret_cast<const __nv_bfloat162 *>(&bw[i]));
+        o[i] = *reinterpret_cast<uint32_t *>(&sum);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int cc = col + 2 * i;
+        const float b0 = cc < p.n ? __bfloat162float(p.bias[cc]) : 0.0f;
+        const float b1 = cc + 1 < p.n ? __bfloat162float(p.bias[cc + 1]) : 0.0f;
+        const uint32_t lo = float_to_bf16_bits(bf16_bits_to_float(o[i] & 0xFFFFu) + b0);
+        const uint32_t hi = float_to_bf16_bits(bf16_bits_to_float(o[i] >> 16) + b1);
+        o[i] = lo | (hi << 16);
+      }
+    }
+  }
+}
+
+// 8 packed columns to row `row` of D; columns >= N are masked.
+__device__ __forceinline__ void store_8(const GemmParams &p, const uint32_t (&o)[4], int row, int col) {
+  __nv_bfloat16 *d = p.d + (size_t)row * p.n + col;
+  if (col + 8 <= p.n && (p.n & 7) == 0 && (reinterpret_cast<uintptr_t>(p.d) & 15) == 0) {
+    *reinterpret_cast<uint4 *>(d) = make_uint4(o[0], o[1], o[2], o[3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (col + i < p.n) d[i] = __ushort_as_bfloat16((unsigned short)((o[i >> 1] >> (16 * (i & 1))) & 0xFFFFu));
+  }
+}
+
+// Epilogue of 32 accumulator columns held in registers; rows >= M and columns >= N are masked.  A thread owns one row
+// and stores 64 contiguous bytes.
 // With `stage` non-null the 64 bytes go to row `stage_row` of a 32-row x 64-byte shared-memory
 // tile instead, 16-byte chunk v at position v ^ ((row >> 1) & 3) (no bank conflicts on the way in
 // or out); the caller stores the tile and masks rows >= M and columns >= N; requires N % 8 == 0.
@@ -142,73 +211,20 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams &p, const uint32
                                                float beta, bool has_c, uint8_t *stage = nullptr, int stage_row = 0,
                                                int chunk_base = 0) {
   if (stage == nullptr && (row >= p.m || col0 >= p.n)) return;
-  if (stage != nullptr && (row >= p.m || col0 >= p.n)) {
-    has_c = false;  // masked by the caller's store; C_in must not be read out of range
-  }
-  const size_t off = (size_t)row * p.n + col0;
-  const bool full = (col0 + 32 <= p.n) && ((p.n & 7) == 0);
+  if (row >= p.m || col0 >= p.n) has_c = false;  // masked by the caller's store; C_in must not be read out of range
 #pragma unroll
   for (int v = 0; v < 4; ++v) {  // 8 columns per 16-byte store
     float f[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = alpha * __uint_as_float(acc[8 * v + i]);
-    if (has_c) {
-      if (full) {
-        uint4 cv = *reinterpret_cast<const uint4 *>(p.c_in + off + 8 * v);
-        uint32_t cw[4] = {cv.x, cv.y, cv.z, cv.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          f[2 * i] = __fmaf_rn(beta, bf16_bits_to_float(cw[i] & 0xFFFFu), f[2 * i]);
-          f[2 * i + 1] = __fmaf_rn(beta, bf16_bits_to_float(cw[i] >> 16), f[2 * i + 1]);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (col0 + 8 * v + i < p.n) f[i] = __fmaf_rn(beta, __bfloat162float(p.c_in[off + 8 * v + i]), f[i]);
-      }
-    }
-    // two values per conversion instruction (the scalar conversion unit is the slow pipe here)
+    for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(acc[8 * v + i]);
     uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      __nv_bfloat162 pair = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-      o[i] = *reinterpret_cast<uint32_t *>(&pair);
-    }
-    if (p.bias != nullptr) {
-      // bias is added to the bf16 result, as a separate bf16 add would (a bf16 add rounds the
-      // exact sum once, which is what the fp32 add + rounding of two bf16 values gives)
-      if (full && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
-        const uint4 bv = __ldg(reinterpret_cast<const uint4 *>(p.bias + col0 + 8 * v));
-        const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          __nv_bfloat162 sum = __hadd2(*reinterpret_cast<__nv_bfloat162 *>(&o[i]),
-                                       *reinterpret_cast<const __nv_bfloat162 *>(&bw[i]));
-          o[i] = *reinterpret_cast<uint32_t *>(&sum);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int cc = col0 + 8 * v + 2 * i;
-          const float b0 = cc < p.n ? __bfloat162float(p.bias[cc]) : 0.0f;
-          const float b1 = cc + 1 < p.n ? __bfloat162float(p.bias[cc + 1]) : 0.0f;
-          const uint32_t lo = float_to_bf16_bits(bf16_bits_to_float(o[i] & 0xFFFFu) + b0);
-          const uint32_t hi = float_to_bf16_bits(bf16_bits_to_float(o[i] >> 16) + b1);
-          o[i] = lo | (hi << 16);
-        }
-      }
-    }
+    epilogue_8(p, f, row, col0 + 8 * v, alpha, beta, has_c, o);
     if (stage != nullptr) {
       uint8_t *slot = kWide ? stage + stage_row * 128 + (((chunk_base + v) ^ (stage_row & 7)) << 4)
                             : stage + stage_row * 64 + ((v ^ ((stage_row >> 1) & 3)) << 4);
       *reinterpret_cast<uint4 *>(slot) = make_uint4(o[0], o[1], o[2], o[3]);
-    } else if (full) {
-      *reinterpret_cast<uint4 *>(p.d + off + 8 * v) = make_uint4(o[0], o[1], o[2], o[3]);
     } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (col0 + 8 * v + i < p.n)
-          p.d[off + 8 * v + i] = __ushort_as_bfloat16((unsigned short)((o[i >> 1] >> (16 * (i & 1))) & 0xFFFFu));
+      store_8(p, o, row, col0 + 8 * v);
     }
   }
 }
@@ -285,12 +301,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   const int n_tiles = (p.n + BN - 1) / BN;
   const int ffn = p.n >> 1;  // SWIGLU: columns of h (a multiple of 128)
   const int k_splits = p.k_splits;
-  const int num_units = m_units * n_tiles * k_splits;
-  // unit -> (K share, tile); tiles M-fastest
-  auto k_begin = [&](int u) { return (int)((long long)k_stages * (u % k_splits) / k_splits); };
-  auto k_end = [&](int u) { return (int)((long long)k_stages * (u % k_splits + 1) / k_splits); };
-  const int unit0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-  const int unit_stride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  const int num_units = m_units * n_tiles;  // tiles M-fastest
+  const int unit0 = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x / k_splits;
+  const int unit_stride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x / k_splits;
+  // this CTA's share of the K stages
+  const int k_rank = PAIR ? 0 : (int)blockIdx.x % k_splits;  // the rank in the cluster of a split launch
+  const int it_begin = k_stages * k_rank / k_splits, it_end = k_stages * (k_rank + 1) / k_splits;
 
   if (threadIdx.x == 32) {
     // fetch the tensor maps while the barriers and tensor memory are being set up
@@ -319,13 +335,37 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  // The set-up above and the prefetch below overlap the end of the kernel that prepares the activation; from here on
+  // every role reads or writes what earlier kernels may still use.
+  if (!PAIR && warp == 0 && unit0 < num_units) {
+    // weight tiles of this CTA's first stages into L2: nothing of them depends on the activation
+    if (ptx::elect_one()) {
+      const int n_tile = unit0 / m_units;
+      const int ahead = min(it_end, it_begin + kPrefetchStages);
+      for (int it = it_begin; it < ahead; ++it) {
+        ptx::tma_prefetch_l2_2d(&tm_w, it * 128, n_tile * BN);
+#pragma unroll
+        for (int b = 0; b < L::kBands; ++b) {
+          const size_t band = (size_t)min(n_tile * L::kBands + b, b_bands - 1);
+          if (DENSE)
+            ptx::bulk_prefetch_l2(p.sfb_dense + (band * tiles_d + 4 * (size_t)it) * 512, (uint32_t)min(4, tiles_d - 4 * it) * 512);
+          if (SPARSE)
+            ptx::bulk_prefetch_l2(p.sfb_sparse + (band * tiles_sp + 2 * (size_t)it) * 512, (uint32_t)min(2, tiles_sp - 2 * it) * 512);
+        }
+      }
+    }
+    __syncwarp();
+  }
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();
+
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (ptx::elect_one()) {
       uint32_t g = 0;  // stages issued so far, across tiles
       bool ok = true;
       for (int u = unit0; u < num_units && ok; u += unit_stride) {
-        const int tile = u / k_splits;
+        const int tile = u;
         const int grp = GROUPED ? gt->unit_group[tile % m_units] : 0;
         if (GROUPED && grp < 0) continue;
         const CUtensorMap *tw = GROUPED ? &gt->tm_w[grp] : &tm_w;
@@ -343,7 +383,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
 #pragma unroll
         for (int b = 0; b < L::kBands; ++b)
           b_band[b] = SWIGLU ? n_tile + b * (ffn / 128) : min(n_tile * L::kBands + b, b_bands - 1);
-        for (int it = k_begin(u), it_end = k_end(u); it < it_end; ++it, ++g) {
+        for (int it = it_begin; it < it_end; ++it, ++g) {
           const int s = (int)(g % S);
           const uint32_t ph = (g / S) & 1u;
           if (!ptx::mbar_wait(empty_bar + s, ph ^ 1u, abort_flag)) {
@@ -391,8 +431,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         uint32_t g = 0;
         bool ok = true;
         for (int u = unit0; u < num_units && ok; u += unit_stride) {
-          if (GROUPED && gt->unit_group[(u / k_splits) % m_units] < 0) continue;
-          for (int it = k_begin(u), it_end = k_end(u); it < it_end; ++it, ++g) {
+          if (GROUPED && gt->unit_group[u % m_units] < 0) continue;
+          for (int it = it_begin; it < it_end; ++it, ++g) {
             const int s = (int)(g % S);
             if (!ptx::mbar_wait(full_bar + s, (g / S) & 1u, abort_flag)) {
               *abort_flag = 1;
@@ -411,7 +451,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         uint32_t tile_iter = 0;
         bool ok = true;
         for (int u = unit0; u < num_units && ok; u += unit_stride) {
-          if (GROUPED && gt->unit_group[(u / k_splits) % m_units] < 0) continue;
+          if (GROUPED && gt->unit_group[u % m_units] < 0) continue;
           // the epilogue warps must have pulled the previous tile out of tensor memory
           const bool drained = PAIR ? ptx::mbar_wait_cluster(acc_empty_bar, (tile_iter & 1u) ^ 1u, abort_flag)
                                     : ptx::mbar_wait(acc_empty_bar, (tile_iter & 1u) ^ 1u, abort_flag);
@@ -422,7 +462,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
           }
           ptx::tc_fence_after();
           uint32_t accumulate = 0;
-          for (int it = k_begin(u), it_end = k_end(u); it < it_end; ++it, ++g) {
+          for (int it = it_begin; it < it_end; ++it, ++g) {
             const int s = (int)(g % S);
             const uint32_t ph = (g / S) & 1u;
             bool got = ptx::mbar_wait(full_bar + s, ph, abort_flag);
@@ -525,7 +565,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     uint32_t tile_iter = 0;
     __nv_bfloat162 h_max = __floats2bfloat162_rn(0.0f, 0.0f);  // SWIGLU: running max |h|
     for (int u = unit0; u < num_units; u += unit_stride) {
-      const int tile = u / k_splits;
+      const int tile = u;
       const int grp = GROUPED ? gt->unit_group[tile % m_units] : 0;
       if (GROUPED && grp < 0) continue;
       const float alpha = GROUPED ? alpha0 * gt->alpha[grp] : alpha0;
@@ -582,22 +622,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         }
         continue;
       }
-      if (k_splits > 1) {
-        // partial sums of this K share: fp32 vector reductions into the accumulation buffer
+      if (!PAIR && k_splits > 1) {
+        // this CTA's partial tile into its own shared memory: the last stage has been consumed, nothing else is loaded
         if (row < p.m) {
-          float *dst = p.splitk_acc + (size_t)row * p.n + col_base;
-          const bool vec = (p.n & 3) == 0;
+          float *dst = reinterpret_cast<float *>(smem) + (size_t)(quad * 32 + lane) * L::kPartStride + half * kColsPerEpiWarp;
 #pragma unroll
-          for (int i = 0; i < kColsPerEpiWarp; i += 4) {
-            if (vec && col_base + i + 4 <= p.n) {
-              ptx::red_add_v4_f32(dst + i, __uint_as_float(acc[i]), __uint_as_float(acc[i + 1]),
-                                  __uint_as_float(acc[i + 2]), __uint_as_float(acc[i + 3]));
-            } else {
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                if (col_base + i + j < p.n) atomicAdd(dst + i + j, __uint_as_float(acc[i + j]));
-            }
-          }
+          for (int i = 0; i < kColsPerEpiWarp; i += 4)
+            *reinterpret_cast<uint4 *>(dst + i) = make_uint4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
         }
         continue;
       }
@@ -662,6 +693,44 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
 
   ptx::tc_fence_before();
   __syncthreads();
+  if (!PAIR && k_splits > 1) {
+    ptx::cluster_sync();  // every CTA's partial tile is written
+    if (threadIdx.x >= 64) {
+      const int m_tile = unit0 % m_units, n_tile = unit0 / m_units;
+      const int rows = min(kBM, p.m - m_tile * kBM);
+      const float alpha = p.alpha_ptr ? p.alpha * (*p.alpha_ptr) : p.alpha;
+      const bool has_c = (p.c_in != nullptr) && (p.beta != 0.0f);
+      const uint32_t part = ptx::smem_u32(smem);
+      // 8 columns per thread, dealt over the threads of all CTAs: neighbouring lanes read neighbouring 32 bytes
+      for (int i = (int)threadIdx.x - 64 + k_rank * 32 * kEpiWarps; i < rows * (BN / 8); i += k_splits * 32 * kEpiWarps) {
+        const int r = i / (BN / 8), c8 = i % (BN / 8);
+        const int row = m_tile * kBM + r, col = n_tile * BN + 8 * c8;
+        if (col >= p.n) continue;
+        const uint32_t at = part + (uint32_t)(r * L::kPartStride + 8 * c8) * 4u;
+        float4 lo[kMaxSplits], hi[kMaxSplits];
+#pragma unroll
+        for (int s = 0; s < kMaxSplits; ++s) {
+          if (s < k_splits) {
+            lo[s] = ptx::ld_cluster_f32x4(at, s);
+            hi[s] = ptx::ld_cluster_f32x4(at + 16, s);
+          }
+        }
+        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int s = 0; s < kMaxSplits; ++s) {
+          if (s < k_splits) {
+            f[0] += lo[s].x, f[1] += lo[s].y, f[2] += lo[s].z, f[3] += lo[s].w;
+            f[4] += hi[s].x, f[5] += hi[s].y, f[6] += hi[s].z, f[7] += hi[s].w;
+          }
+        }
+        uint32_t o[4];
+        epilogue_8(p, f, row, col, alpha, p.beta, has_c, o);
+        store_8(p, o, row, col);
+      }
+    }
+    __syncwarp();
+    ptx::cluster_sync();  // no CTA leaves while another may still read its partial tile
+  }
   if (PAIR) ptx::cluster_sync();  // neither CTA leaves (or frees tensor memory) while its peer may still use it
   if (warp == 1) {
     ptx::tc_fence_after();
@@ -684,34 +753,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_grouped_kernel(const __grid_constant__ GroupTable groups, const __grid_constant__ CUtensorMap tm_a_dense,
                         const __grid_constant__ CUtensorMap tm_a_comp, const GemmParams p) {
   gemm_body<256, true, true, true, true, false, SWIGLU>(groups.tm_w[0], tm_a_dense, tm_a_comp, p, &groups);
-}
-
-// Second kernel of a split-K GEMM: the epilogue on the accumulated fp32 sums, 32 columns per thread.
-__global__ void __launch_bounds__(256) splitk_finalize_kernel(const GemmParams p) {
-  const int chunks = (p.n + 31) / 32;
-  const long long total = (long long)p.m * chunks;
-  const float alpha = p.alpha_ptr ? p.alpha * (*p.alpha_ptr) : p.alpha;
-  const bool has_c = (p.c_in != nullptr) && (p.beta != 0.0f);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int row = (int)(i / chunks);
-    const int col0 = (int)(i % chunks) * 32;
-    const float *src = p.splitk_acc + (size_t)row * p.n + col0;
-    uint32_t acc[32];
-    if ((p.n & 3) == 0 && col0 + 32 <= p.n) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const float4 t = __ldcg(reinterpret_cast<const float4 *>(src) + v);
-        acc[4 * v] = __float_as_uint(t.x);
-        acc[4 * v + 1] = __float_as_uint(t.y);
-        acc[4 * v + 2] = __float_as_uint(t.z);
-        acc[4 * v + 3] = __float_as_uint(t.w);
-      }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = col0 + j < p.n ? __float_as_uint(__ldcg(src + j)) : 0u;
-    }
-    epilogue_chunk(p, acc, row, col0, alpha, p.beta, has_c);
-  }
 }
 
 // ------------------------------------------------------------------ host side
@@ -825,51 +866,59 @@ cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
   }
   const int n_tiles = (a.n + BN - 1) / BN;
   const int m_units = PAIR ? (a.m + 255) / 256 : (a.m + kBM - 1) / kBM;
-  int units = m_units * n_tiles;
-  // Split K when one row of tiles cannot fill the GPU (M <= 128 is weight-bandwidth-bound: the
-  // weights must stream through as many SMs as possible) and the caller gave scratch.
-  p.k_splits = 1;
-  p.splitk_acc = nullptr;
-  const int k_stages = (a.k + kBK - 1) / kBK;
-  if (!PAIR && m_units == 1 && a.scatter_world <= 1 && a.workspace != nullptr &&
-      a.workspace_bytes >= (size_t)a.m * a.n * sizeof(float)) {
-    int splits = sms / units;
-    if (splits > k_stages / 2) splits = k_stages / 2;  // at least two K stages per unit
-    // the fp32 reductions cost M x N x splits atomics: measured worth it for M <= 64 (qkv
-    // 16.2 -> 13.3 us, down 39.9 -> 17.3 us at M = 16) and for long K (down at M = 128:
-    // 41.0 -> 22.9 us), not for M = 128 with K = 4096 (17.8 -> 19.0 us)
-    if (splits >= 2 && (a.m <= 64 || k_stages >= 32)) {
-      p.k_splits = splits;
-      p.splitk_acc = static_cast<float *>(a.workspace);
-      units *= splits;
-      e = cudaMemsetAsync(a.workspace, 0, (size_t)a.m * a.n * sizeof(float), stream);
-      if (e != cudaSuccess) return e;
-    }
-  }
+  const int units = m_units * n_tiles;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  if (PAIR) {
-    const int clusters = units < sms / 2 ? units : sms / 2;
-    cfg.gridDim = dim3(2 * clusters);
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-  } else {
-    cfg.gridDim = dim3(units < sms ? units : sms);
-  }
+  cudaLaunchAttribute attr[2];
+  // see grid_dependency_wait in gemm_body; the linears of a 32-token decode step, with split K and the cluster prepare: 123 -> 100 us
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
   cfg.blockDim = dim3(kGemmThreads);
   cfg.dynamicSmemBytes = L::kSmemBytes;
   cfg.stream = stream;
-  e = cudaLaunchKernelEx(&cfg, kernel, tm_w, tm_ad, tm_ac, p);
-  if (e != cudaSuccess || p.k_splits == 1) return e;
-  const long long chunks = (long long)a.m * ((a.n + 31) / 32);
-  long long blocks = (chunks + 255) / 256;
-  if (blocks > 4LL * sms) blocks = 4LL * sms;
-  splitk_finalize_kernel<<<(unsigned)blocks, 256, 0, stream>>>(p);
-  return cudaGetLastError();
+  p.k_splits = 1;
+  if (PAIR) {
+    const int clusters = units < sms / 2 ? units : sms / 2;
+    cfg.gridDim = dim3(2 * clusters);
+    attr[1].val.clusterDim.x = 2;
+  } else {
+    // Split K where the tiles alone leave SMs idle (few rows: the launch is bound by streaming the weights, which
+    // takes as many SMs as possible): the most CTAs per tile for which all clusters run at the same time, each
+    // with at least two K stages.  Sums through distributed shared memory took the place of a memset, fp32 atomics and a
+    // second kernel (4.5 us of 20 per launch at M = 32), for which only M <= 64 or K >= 8192 had paid.
+    if (a.split_k && a.scatter_world <= 1) {
+      static int capacity[64][kMaxSplits + 1] = {};  // clusters of a size that the device holds at once; 0 = not asked yet
+      const int k_stages = (a.k + kBK - 1) / kBK;
+      int s = k_stages / 2 < kMaxSplits ? k_stages / 2 : kMaxSplits;
+      if (s > sms / units) s = sms / units;
+      for (; s >= 2; --s) {
+        if (capacity[dev][s] == 0) {
+          attr[1].val.clusterDim.x = (unsigned)s;
+          cudaLaunchConfig_t ask = cfg;
+          ask.gridDim = dim3((unsigned)s);
+          ask.attrs = attr + 1;
+          ask.numAttrs = 1;
+          int n = 0;
+          if (cudaOccupancyMaxActiveClusters(&n, kernel, &ask) != cudaSuccess) {
+            (void)cudaGetLastError();
+            n = 0;
+          }
+          capacity[dev][s] = n > 0 ? n : -1;
+        }
+        if (capacity[dev][s] >= units) break;
+      }
+      if (s >= 2) p.k_splits = s;
+    }
+    attr[1].val.clusterDim.x = (unsigned)p.k_splits;
+    cfg.gridDim = dim3(p.k_splits > 1 ? units * p.k_splits : (units < sms ? units : sms));
+    if (p.k_splits == 1) cfg.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, tm_w, tm_ad, tm_ac, p);
 }
 
 }  // namespace

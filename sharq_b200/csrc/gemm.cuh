@@ -30,10 +30,7 @@ struct GemmArgs {
   int m = 0, n = 0, k = 0;
   int tile_n = 0;             // 0 = choose, else 128 or 256
   int *error_flag = nullptr;  // device int, set non-zero when a bounded wait ran out
-  // Optional scratch of at least m * n * 4 bytes: lets a GEMM with M <= 128 split K over the SMs
-  // (fp32 partial sums are accumulated there, a second kernel applies the epilogue).
-  void *workspace = nullptr;
-  size_t workspace_bytes = 0;
+  bool split_k = false;  // K may be split over the CTAs of a cluster (another order of the fp32 additions)
   // Scatter mode (scatter_world > 1, `d` unused): the m / scatter_world rows owned by GPU o are stored into
   // d_peer[o] (GPU o's collection buffer as mapped on this GPU, [scatter_world][m / scatter_world][n] bf16) at
   // block scatter_rank.  Needs m % (128 * scatter_world) == 0 and n % 8 == 0.

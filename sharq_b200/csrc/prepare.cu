@@ -27,6 +27,7 @@
 #include "common.cuh"
 #include "prepare.cuh"
 #include "prepare_device.cuh"
+#include "sm100_ptx.cuh"
 
 #include <cstdlib>
 
@@ -216,7 +217,11 @@ struct PrepareParams {
 };
 
 constexpr int kPrepareCtasPerSm = 3;
-constexpr size_t kInlineAbsmaxElements = 256 * 1024;  // up to 512 KB of input is scanned by every CTA
+// Up to the first size every CTA scans the whole input for its maximum, up to the second one cluster prepares it (us per launch at
+// K = 4096, scan / cluster / cooperative grid: 16 rows 5.9 / 6.7 / 9; 32 rows 8.1 / 6.9 / 9; 64 rows 11.8 / 8.0 / 9; 128 rows - / - / 9.0;
+// RMSNorm, cluster / cooperative grid: 16 rows 8.1 / 10.8, 64 rows 9.7 / 10.8).
+constexpr size_t kInlineAbsmaxElements = 64 * 1024;
+constexpr size_t kClusterElements = 256 * 1024;
 
 // kCtas: resident CTAs per SM the register allocation aims at.  The tensor-scale mode runs
 // fastest with two (no spills) except on a gathered activation (src_row), where the third CTA
@@ -228,6 +233,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
   const int groups32 = k >> 5;
   const int aligned_m = (m + 127) / 128 * 128;
 
+  ptx::grid_launch_dependents();
   __shared__ ScaleTables tbl;
   extern __shared__ uint4 gamma_smem[];  // mode 1: the whole RMSNorm weight, k bf16
   if (threadIdx.x < 128) {
@@ -235,6 +241,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
     tbl.value[threadIdx.x] = v;
     tbl.recip[threadIdx.x] = __frcp_rn(v);  // code 0 is never looked up (scales are clamped to >= 2^-9)
   }
+  ptx::grid_dependency_wait();
   if (kMode == 1) {
     const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
     for (int i = threadIdx.x; i < k / 8; i += blockDim.x) gamma_smem[i] = __ldg(gsrc + i);
@@ -484,7 +491,11 @@ __device__ __forceinline__ void store_group(const FusedParams &p, const GroupOut
   }
 }
 
-template <int kMode, bool kAdd, int kFusedThreads>
+//
+// kCluster: the same kernel as one thread-block cluster for small inputs (decode steps).  The tensor absmax goes
+// through distributed shared memory and a cluster barrier, so nothing has to be zeroed before the launch, and the other SMs are free for
+// the CTAs of the GEMM that follows, which start early and fetch their weights meanwhile.
+template <int kMode, bool kAdd, int kFusedThreads, bool kCluster>
 __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const FusedParams p) {
   static_assert(kMode == 1 || kMode == 2, "modes with a statistics pass");
   constexpr int kFusedWarps = kFusedThreads / 32;
@@ -498,17 +509,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
 
   __shared__ ScaleTables tbl;
   __shared__ float warp_red[32];
+  __shared__ float cta_amax;  // kCluster
   extern __shared__ uint4 fused_smem[];
   uint4 *gamma_s = fused_smem;                                      // mode 1: k bf16, pieces permuted like the cache
   uint4 *cache = fused_smem + (kMode == 1 ? row_vecs : 0);          // chunk_rows x k bf16
   float *partial = reinterpret_cast<float *>(cache + (size_t)p.chunk_rows * row_vecs);  // mode 1: chunk_rows x partial_stride
   float *inv_s = partial + (kMode == 1 ? p.chunk_rows * partial_stride : 0);            // mode 1: rows_per_cta
 
+  ptx::grid_launch_dependents();
   if (threadIdx.x < 128) {
     const float v = ue4m3_to_float(threadIdx.x);
     tbl.value[threadIdx.x] = v;
     tbl.recip[threadIdx.x] = __frcp_rn(v);  // code 0 is never looked up (scales are clamped to >= 2^-9)
   }
+  ptx::grid_dependency_wait();
   if (kMode == 1) {
     const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
     for (int i = threadIdx.x; i < row_vecs; i += kFusedThreads) gamma_s[cache_slot(i >> 2, i & 3)] = __ldg(gsrc + i);
@@ -676,20 +690,35 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int w = 1; w < kFusedWarps; ++w) mx = fmaxf(mx, warp_red[w]);
-      if (mx > 0.0f) atomicMax(p.amax_bits, __float_as_uint(mx));
-      __threadfence();
-      atomicAdd(p.arrive, 1u);
-      const long long t0 = clock64();
-      while (ld_acquire_gpu(p.arrive) < gridDim.x) {
-        if (clock64() - t0 > kGridBarrierLimitCycles) {
-          atomicAdd(&g_prepare_timeouts, 1);
-          break;
+      if (kCluster) {
+        cta_amax = mx;
+      } else {
+        if (mx > 0.0f) atomicMax(p.amax_bits, __float_as_uint(mx));
+        __threadfence();
+        atomicAdd(p.arrive, 1u);
+        const long long t0 = clock64();
+        while (ld_acquire_gpu(p.arrive) < gridDim.x) {
+          if (clock64() - t0 > kGridBarrierLimitCycles) {
+            atomicAdd(&g_prepare_timeouts, 1);
+            break;
+          }
         }
       }
     }
     __syncthreads();
   }
-  const float amax = __uint_as_float(ld_acquire_gpu(p.amax_bits));
+  float amax = 0.0f;
+  if (kCluster) {
+    ptx::cluster_sync();
+    const uint32_t at = ptx::smem_u32(&cta_amax);
+    if (lane < (int)gridDim.x) amax = ptx::ld_cluster_f32(at, lane);  // at most 16 CTAs, one per lane
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    ptx::cluster_arrive();  // the wait is at the end: no CTA leaves while another may still read its maximum
+    if (blockIdx.x == 0 && threadIdx.x == 0) *p.amax_bits = __float_as_uint(amax);
+  } else {
+    amax = __uint_as_float(ld_acquire_gpu(p.amax_bits));
+  }
   // ATen divides a CUDA tensor by a host scalar by multiplying with the float
   // reciprocal; clamp(min=1e-9) follows (kernels/src/bindings.cpp:337 of the reference).
   const float scale = fmaxf(__fmul_rn(amax, 1.0f / 2688.0f), 1.0e-9f);
@@ -763,6 +792,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
       store_group(p, o, row, group, live, group < groups_padded, aligned_m, lane);
     }
   }
+  if (kCluster) {
+    __syncwarp();
+    ptx::cluster_wait();
+  }
 }
 
 }  // namespace
@@ -795,13 +828,18 @@ static int prepare_grid(const PrepareParams &p) {
 }
 
 static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, cudaStream_t stream) {
-  dim3 grid(prepare_grid(p));
-  dim3 block(kPrepareThreads);
-  if (debug) {
-    prepare_kernel<0, true><<<grid, block, 0, stream>>>(p);
-  } else if (mode == 0) {
-    prepare_kernel<0, false><<<grid, block, 0, stream>>>(p);
-  } else if (mode == 1) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the table set-up overlaps the kernel before
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(prepare_grid(p));
+  cfg.blockDim = dim3(kPrepareThreads);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (debug) return cudaLaunchKernelEx(&cfg, prepare_kernel<0, true>, p);
+  if (mode == 0) return cudaLaunchKernelEx(&cfg, prepare_kernel<0, false>, p);
+  if (mode == 1) {
     const size_t gamma_bytes = (size_t)p.k * sizeof(__nv_bfloat16);
     static bool attr_set[64] = {};
     int dev = 0;
@@ -810,13 +848,11 @@ static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, 
       if (e != cudaSuccess) return e;
       attr_set[dev] = true;
     }
-    prepare_kernel<1, false><<<grid, block, gamma_bytes, stream>>>(p);
-  } else if (p.src_row != nullptr) {
-    prepare_kernel<2, false><<<grid, block, 0, stream>>>(p);
-  } else {
-    prepare_kernel<2, false, 2><<<grid, block, 0, stream>>>(p);
+    cfg.dynamicSmemBytes = gamma_bytes;
+    return cudaLaunchKernelEx(&cfg, prepare_kernel<1, false>, p);
   }
-  return cudaGetLastError();
+  if (p.src_row != nullptr) return cudaLaunchKernelEx(&cfg, prepare_kernel<2, false>, p);
+  return cudaLaunchKernelEx(&cfg, prepare_kernel<2, false, 2>, p);
 }
 
 cudaError_t run_prepare(const void *x, int m, int k, void *a_comp, void *e, void *q_sparse_dense,
@@ -835,54 +871,77 @@ cudaError_t run_prepare(const void *x, int m, int k, void *a_comp, void *e, void
   return launch_prepare(0, q_sparse_dense != nullptr, p, stream);
 }
 
-// One cooperative launch for statistics + prepare (see prepare_fused_kernel).  Returns
-// cudaErrorNotSupported when the shape does not fit or the device cannot launch it, in which
-// case the caller falls back to the separate statistics and prepare kernels.
-template <int kMode, bool kAdd, int kThreads>
-static cudaError_t launch_fused_t(const FusedParams &p_in, cudaStream_t stream) {
+// One launch for statistics + prepare (see prepare_fused_kernel): a cooperative grid over all SMs, or one cluster.
+// Returns cudaErrorNotSupported when the shape does not fit or the device cannot launch it, in which
+// case the caller falls back to the other forms.
+// 512 threads per CTA: measured against 448, 768 and 896 (more threads spill or idle in the
+// partly filled last round of 56 warp tasks per CTA at 2048 x 4096)
+template <int kMode, bool kAdd, bool kCluster>
+static cudaError_t launch_fused(const FusedParams &p_in, cudaStream_t stream) {
+  constexpr int kThreads = 512;
   static bool attr_set[64] = {};
-  static int coop[64] = {};  // 0 unknown, 1 yes, -1 no
+  static int usable[64] = {};  // 0 unknown, else the CTAs of the launch, -1 no
   int dev = 0, sms = 0;
   cudaError_t e = current_sms(&dev, &sms);
   if (e != cudaSuccess) return e;
-  if (coop[dev] == 0) {
-    int v = 0;
-    coop[dev] = (cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && v) ? 1 : -1;
+  auto kernel = prepare_fused_kernel<kMode, kAdd, kThreads, kCluster>;
+  if (!attr_set[dev]) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedSmemBudget + 16);
+    if (e == cudaSuccess && kCluster) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    attr_set[dev] = true;
   }
-  if (coop[dev] < 0) return cudaErrorNotSupported;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  cfg.blockDim = dim3(kThreads);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (kCluster) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    for (int c = 16; usable[dev] == 0; c /= 2) {
+      attr[0].val.clusterDim.x = (unsigned)c;
+      cfg.gridDim = dim3((unsigned)c);
+      cfg.dynamicSmemBytes = kFusedSmemBudget + 16;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) (void)cudaGetLastError();
+      if (n > 0 || c == 4) usable[dev] = n > 0 ? c : -1;
+    }
+  } else {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    if (usable[dev] == 0) {
+      int v = 0;
+      usable[dev] = (cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && v) ? sms : -1;
+    }
+  }
+  if (usable[dev] < 0) return cudaErrorNotSupported;
+  const int ctas = usable[dev];
   FusedParams p = p_in;
   const int groups32 = p.k / 32;
-  p.rows_per_cta = (p.m + sms - 1) / sms;
+  p.rows_per_cta = (p.m + ctas - 1) / ctas;
   const size_t row_bytes = (size_t)p.k * 2 + (kMode == 1 ? (size_t)(groups32 + 4) * 4 : 0);
   const size_t fixed = (kMode == 1 ? (size_t)p.k * 2 + (size_t)p.rows_per_cta * 4 : 0);
   if (fixed + row_bytes > (size_t)kFusedSmemBudget) return cudaErrorNotSupported;
   const size_t capacity = ((size_t)kFusedSmemBudget - fixed) / row_bytes;
   p.chunk_rows = (int)(capacity < (size_t)p.rows_per_cta ? capacity : (size_t)p.rows_per_cta);
-  const size_t smem = fixed + (size_t)p.chunk_rows * row_bytes + 16;
-  auto kernel = prepare_fused_kernel<kMode, kAdd, kThreads>;
-  if (!attr_set[dev]) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedSmemBudget + 16);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.dynamicSmemBytes = fixed + (size_t)p.chunk_rows * row_bytes + 16;
+  if (kCluster) {
+    attr[0].val.clusterDim.x = (unsigned)ctas;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
   }
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.gridDim = dim3(sms);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
-// 512 threads per CTA: measured against 448, 768 and 896 (more threads spill or idle in the
-// partly filled last round of 56 warp tasks per CTA at 2048 x 4096)
-template <int kMode, bool kAdd>
-static cudaError_t launch_fused(const FusedParams &p, cudaStream_t stream) {
-  return launch_fused_t<kMode, kAdd, 512>(p, stream);
+template <bool kCluster>
+static cudaError_t launch_fused_mode(const FusedParams &p, bool rms, cudaStream_t stream) {
+  if (!rms) return launch_fused<2, false, kCluster>(p, stream);
+  return p.residual != nullptr ? launch_fused<1, true, kCluster>(p, stream) : launch_fused<1, false, kCluster>(p, stream);
 }
 
 static bool fused_prepare_enabled() {
@@ -912,13 +971,14 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   const bool rms = gamma != nullptr;
   // a small non-RMSNorm input (a decode step): the prepare kernel finds max|x| itself
   const bool inline_absmax = !rms && !absmax_ready && (size_t)m * k <= kInlineAbsmaxElements;
+  const size_t elements = (size_t)m * (size_t)k;
+  const bool one_cluster = !absmax_ready && elements <= kClusterElements && (rms || elements > kInlineAbsmaxElements);
   // One cooperative launch pays while the per-SM row caches hold most of the tensor; beyond that
   // the separate statistics and prepare kernels (more resident warps per SM) are faster.  Measured
   // crossovers (us, one launch / separate): RMSNorm 4096 x 4096 35.0 / 37.0, 8192 x 4096
   // 65.7 / 63.8, 16384 x 4096 136 / 118; tensor scale 2048 x 7168 24.9 / 25.0, 4096 x 4096 28.7 / 27.0.
-  const size_t elements = (size_t)m * (size_t)k;
   const bool one_launch_pays = elements < (rms ? ((size_t)1 << 25) : ((size_t)1 << 24));
-  if (!absmax_ready && !inline_absmax && one_launch_pays && fused_prepare_enabled()) {
+  if (!absmax_ready && !inline_absmax && (one_launch_pays || one_cluster) && fused_prepare_enabled()) {
     FusedParams f{};
     f.x = static_cast<const __nv_bfloat16 *>(x);
     f.residual = static_cast<const __nv_bfloat16 *>(residual);
@@ -936,10 +996,12 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
     f.sf_res = static_cast<uint8_t *>(sf_res);
     f.m = m;
     f.k = k;
+    if (one_cluster) {
+      if ((err = launch_fused_mode<true>(f, rms, stream)) == cudaSuccess) return cudaSuccess;
+      (void)cudaGetLastError();
+    }
     if ((err = cudaMemsetAsync(amax_bits, 0, 2 * sizeof(unsigned int), stream)) != cudaSuccess) return err;
-    err = !rms ? launch_fused<2, false>(f, stream)
-               : (residual != nullptr ? launch_fused<1, true>(f, stream) : launch_fused<1, false>(f, stream));
-    if (err == cudaSuccess) return cudaSuccess;
+    if ((err = launch_fused_mode<false>(f, rms, stream)) == cudaSuccess) return cudaSuccess;
     (void)cudaGetLastError();  // not launchable here: the separate kernels below do the same work
     if (err != cudaErrorNotSupported && err != cudaErrorCooperativeLaunchTooLarge) return err;
     err = cudaSuccess;

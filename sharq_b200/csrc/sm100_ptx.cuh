@@ -123,7 +123,53 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// A float / 16 bytes of another CTA's shared memory (addr: this CTA's address of the same variable).
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t cta_rank) {
+  float v;
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %1, %2;\n\t"
+      "ld.shared::cluster.f32 %0, [remote];\n\t"
+      "}"
+      : "=f"(v)
+      : "r"(addr), "r"(cta_rank)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr, uint32_t cta_rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [remote];\n\t"
+      "}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(addr), "r"(cta_rank)
+      : "memory");
+  return v;
+}
+
+// ---------------------------------------------------------------- programmatic dependent launch
+// Waits until the kernels this launch depends on have finished and their writes are visible; returns at once in a
+// kernel that was launched without the attribute.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets a dependent kernel that was launched with the attribute start its blocks (it waits itself before it reads).
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- TMA
+// L2 prefetch of a tile / of `bytes` contiguous bytes (a multiple of 16, 16-byte aligned).  L2 is where every write of
+// the GPU lands, so a prefetch ahead of a dependency wait cannot make stale data visible.
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap *m, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(m), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }

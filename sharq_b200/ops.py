@@ -478,12 +478,9 @@ def _scale_ptr(scale: torch.Tensor, reference: torch.Tensor, name: str):
     return _ptr(scale)
 
 
-def _gemm_scratch(M: int, N: int, dev):
-    """Scratch that lets a small-M GEMM split K over the SMs: (tensor or None, bytes)."""
-    if M > 128 or os.environ.get("SHARQ_GEMM_SPLIT_K", "1") == "0":
-        return None, 0
-    nbytes = int(_lib.lib().sharq_gemm_workspace_bytes(M, N))
-    return (torch.empty(nbytes, dtype=torch.uint8, device=dev), nbytes) if nbytes else (None, 0)
+def _split_k(dev):
+    """(workspace, bytes) arguments that let a GEMM of few tiles split K over the SMs: nothing is written to it."""
+    return (None, 0) if os.environ.get("SHARQ_GEMM_SPLIT_K", "1") == "0" else (_error_flag(dev), 16)
 
 
 def _dense_gemm(A, B, SFA, SFB, alpha, alpha_t, C_in, beta, out=None):
@@ -495,7 +492,7 @@ def _dense_gemm(A, B, SFA, SFB, alpha, alpha_t, C_in, beta, out=None):
         _check(out.is_cuda and out.device == dev and out.dtype == torch.bfloat16 and out.is_contiguous()
                and tuple(out.shape) == (M, N), "out must be a contiguous CUDA bfloat16 tensor shaped [M, N]")
         D = out
-    ws, ws_bytes = _gemm_scratch(M, N, dev)
+    ws, ws_bytes = _split_k(dev)
     with _on_device(dev):
         _lib.check(_lib.lib().sharq_matmul_ws(
             _ptr(A), _ptr(B), _ptr(SFA), _ptr(SFB), M, N, K, float(alpha),
@@ -554,7 +551,7 @@ def _sparse_gemm(name, A_comp, B, E, SFA, SFB, M, N, K, alpha, alpha_t, beta):
     _check(B.shape[1] == K // 2, f"B.size(1) mismatch: expected {K // 2}, got {B.shape[1]}")
     dev = A_comp.device
     D = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
-    ws, ws_bytes = _gemm_scratch(M, N, dev)
+    ws, ws_bytes = _split_k(dev)
     with _on_device(dev):
         _lib.check(_lib.lib().sharq_sparse_matmul_ws(
             _ptr(A_comp), _ptr(B), _ptr(E), _ptr(SFA), _ptr(SFB), M, N, K, float(alpha),
@@ -619,7 +616,7 @@ def sharq_linear_gemm(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_
         _check(out.is_cuda and out.device == dev and out.dtype == torch.bfloat16 and out.is_contiguous()
                and tuple(out.shape) == (M, N), "out must be a contiguous CUDA bfloat16 tensor shaped [M, N]")
         D = out
-    ws, ws_bytes = _gemm_scratch(M, N, dev)
+    ws, ws_bytes = _split_k(dev)
     with _on_device(dev):
         _lib.check(_lib.lib().sharq_linear_gemm_ws(
             _ptr(A_comp), _ptr(E), _ptr(SFA_sparse), _ptr(Q_res), _ptr(SF_res), _ptr(QW), _ptr(SFW_sparse),
