@@ -1,7 +1,8 @@
-"""In-tree build of the CUDA library (nvcc, sm_100a only).
+"""In-tree build of the CUDA library (nvcc, sm_100a only) and of its torch binding (g++).
 
 `python -m sharq_b200._build` compiles sharq_b200/csrc/*.cu into
-sharq_b200/lib/libsharq_b200.so.  nvcc cross-compiles without a GPU.
+sharq_b200/lib/libsharq_b200.so (nvcc cross-compiles without a GPU) and sharq_b200/csrc/torch_bind.cpp
+into sharq_b200/lib/sharq_native.so.
 """
 from __future__ import annotations
 
@@ -15,6 +16,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB_PATH = LIB_DIR / "libsharq_b200.so"
+BIND_PATH = LIB_DIR / "sharq_native.so"
 SOURCES = ["prepare.cu", "prepare_static.cu", "sp_transition.cu", "quant.cu", "gemm.cu", "allreduce.cu", "decoder_ops.cu",
            "c_api.cu"]
 NVCC_FLAGS = [
@@ -32,11 +34,25 @@ def find_nvcc() -> str:
 
 
 def _stale() -> bool:
-    if not LIB_PATH.exists():
+    if not LIB_PATH.exists() or not BIND_PATH.exists():
         return True
-    t = LIB_PATH.stat().st_mtime
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "sharq_b200.h"]
+    t = min(LIB_PATH.stat().st_mtime, BIND_PATH.stat().st_mtime)
+    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.cpp")) + [PKG.parent / "include" / "sharq_b200.h"]
     return any(d.stat().st_mtime > t for d in deps)
+
+
+def _bind_command(out: Path) -> list[str]:
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(find_nvcc()).resolve().parent.parent / "include"
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"], cuda]
+    return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            *[a for i in includes for a in ("-isystem", str(i))], str(CSRC / "torch_bind.cpp"), "-o", str(out),
+            f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", f"-L{LIB_DIR}", "-l:" + LIB_PATH.name,
+            "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -63,6 +79,9 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     cmd = [nvcc, "-shared", "-o", str(tmp)] + [str(obj_dir / (s + ".o")) for s in SOURCES]
     subprocess.run(cmd, check=True)
     os.replace(tmp, LIB_PATH)
+    tmp = BIND_PATH.with_suffix(".so.tmp")
+    subprocess.run(_bind_command(tmp), check=True)
+    os.replace(tmp, BIND_PATH)
     return LIB_PATH
 
 

@@ -11,7 +11,9 @@ from pathlib import Path
 
 _PKG = Path(__file__).resolve().parent
 LIB_PATH = _PKG / "lib" / "libsharq_b200.so"
+NATIVE_PATH = _PKG / "lib" / "sharq_native.so"
 _LIB = None
+_NATIVE = None
 
 # name -> (restype, argtypes); mirrors include/sharq_b200.h one to one
 _P = c_void_p
@@ -106,6 +108,24 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _LIB = L
     return _LIB
+
+
+def native():
+    """The torch binding of the hot operators (csrc/torch_bind.cpp)."""
+    global _NATIVE
+    if _NATIVE is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (the binding links against its libraries)
+
+        lib()  # the library it calls; also the check that the build is there
+        if not NATIVE_PATH.exists():
+            raise ImportError(f"{NATIVE_PATH} is missing: build it with `python -m sharq_b200._build`")
+        spec = importlib.util.spec_from_file_location("sharq_native", NATIVE_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _NATIVE = module
+    return _NATIVE
 
 
 def check(status: int) -> None:

@@ -26,6 +26,7 @@ import torch
 from . import _lib
 
 _ERROR_FLAGS: dict[int, torch.Tensor] = {}
+_NO_FLAG = torch.zeros(1, dtype=torch.int32)
 _PREPARE_TIMEOUTS_SEEN = 0
 
 
@@ -43,6 +44,8 @@ def _stream(device: torch.device):
 
 
 def _error_flag(device: torch.device) -> torch.Tensor:
+    if device.type != "cuda":
+        return _NO_FLAG  # the operator refuses the tensor
     idx = device.index if device.index is not None else torch.cuda.current_device()
     flag = _ERROR_FLAGS.get(idx)
     if flag is None:
@@ -160,53 +163,13 @@ def _on_device(dev):
     return torch.cuda.device(dev)
 
 
-def _scaled_prepare(X, gamma, eps, N, return_workspace, residual=None):
-    M, K = int(X.shape[0]), int(X.shape[1])
-    dev = X.device
-    ws_bytes = 256 + 4 * M
-    A_comp, E, SFA, Q_res, SF_res, tail = _prepare_buffers(M, K, dev, extra=_round256(ws_bytes) + 256)
-    ws = tail[:ws_bytes]
-    scale = tail[_round256(ws_bytes):_round256(ws_bytes) + 4].view(torch.float32).reshape(())
-    L = _lib.lib()
-    with _on_device(dev):
-        if residual is not None:
-            total = torch.empty_like(X)
-            _lib.check(L.sharq_fused_add_rmsnorm_sparse_residual_quantize_x(
-                X.data_ptr(), residual.data_ptr(), total.data_ptr(), gamma.data_ptr(), float(eps), M, N, K, ws.data_ptr(),
-                ws_bytes, A_comp.data_ptr(), E.data_ptr(), SFA.data_ptr(), Q_res.data_ptr(), SF_res.data_ptr(),
-                scale.data_ptr(), _stream(dev)))
-            return A_comp, E, SFA, Q_res, SF_res, scale, total
-        if gamma is not None:
-            _lib.check(L.sharq_fused_rmsnorm_sparse_residual_quantize_x(
-                X.data_ptr(), gamma.data_ptr(), float(eps), M, N, K, ws.data_ptr(), ws_bytes, A_comp.data_ptr(),
-                E.data_ptr(), SFA.data_ptr(), Q_res.data_ptr(), SF_res.data_ptr(), scale.data_ptr(), _stream(dev)))
-        else:
-            _lib.check(L.sharq_scaled_sparse_residual_quantize_x(
-                X.data_ptr(), M, N, K, ws.data_ptr(), ws_bytes, A_comp.data_ptr(), E.data_ptr(), SFA.data_ptr(),
-                Q_res.data_ptr(), SF_res.data_ptr(), scale.data_ptr(), _stream(dev)))
-    if return_workspace:
-        return A_comp, E, SFA, Q_res, SF_res, scale, ws
-    return A_comp, E, SFA, Q_res, SF_res, scale
-
-
 def fused_rmsnorm_sparse_residual_quantize_x(X: torch.Tensor, rmsnorm_weight: torch.Tensor, rmsnorm_eps: float,
                                              N: int, return_workspace: bool = False):
     """-> (A_comp, E, SFA_sparse, Q_res, SF_res, scale [0-dim float32]).
 
     With return_workspace=True the scratch buffer is appended (bytes [256, 256+4M) hold
     the per-row inv_rms as float32)."""
-    M, K = _check_x(X)
-    w = rmsnorm_weight
-    _check(w.is_cuda, "rmsnorm_weight must be a CUDA tensor")
-    _check(w.is_contiguous(), "rmsnorm_weight must be contiguous")
-    _check(w.dtype == torch.bfloat16, "rmsnorm_weight must be torch.bfloat16")
-    _check(w.dim() == 1, "rmsnorm_weight must be shaped [K]")
-    _check(w.device == X.device, "rmsnorm_weight must be on the same device as X")
-    _check(w.shape[0] == K, f"rmsnorm_weight size mismatch: expected {K}, got {w.shape[0]}")
-    _check(K % 128 == 0,
-           f"fused_rmsnorm_sparse_residual_quantize_x currently requires K to be a multiple of 128, got {K}")
-    _check(K // 32 <= 1024, f"fused_rmsnorm_sparse_residual_quantize_x requires K/32 <= 1024, got {K // 32}")
-    return _scaled_prepare(X, w, rmsnorm_eps, N, return_workspace)
+    return _lib.native().scaled_prepare(X, rmsnorm_weight, rmsnorm_eps, N, None, return_workspace)
 
 
 def fused_add_rmsnorm_sparse_residual_quantize_x(X: torch.Tensor, residual: torch.Tensor, rmsnorm_weight: torch.Tensor,
@@ -214,16 +177,7 @@ def fused_add_rmsnorm_sparse_residual_quantize_x(X: torch.Tensor, residual: torc
     """-> (A_comp, E, SFA_sparse, Q_res, SF_res, scale, S) with S = X + residual (bf16, as the ATen
     add rounds) and the first six the RMSNorm-fused prepare of S.  The add rides on the row
     statistics pass, so S costs no extra read of X."""
-    M, K = _check_x(X)
-    _check(residual.is_cuda and residual.dtype == torch.bfloat16 and residual.is_contiguous()
-           and tuple(residual.shape) == (M, K) and residual.device == X.device,
-           "residual must be a contiguous CUDA bfloat16 tensor shaped like X on the same device")
-    w = rmsnorm_weight
-    _check(w.is_cuda and w.is_contiguous() and w.dtype == torch.bfloat16 and w.dim() == 1 and w.shape[0] == K
-           and w.device == X.device, "rmsnorm_weight must be a contiguous CUDA bfloat16 tensor shaped [K] on X's device")
-    _check(K % 128 == 0, f"fused_add_rmsnorm_sparse_residual_quantize_x requires K to be a multiple of 128, got {K}")
-    _check(K // 32 <= 1024, f"fused_add_rmsnorm_sparse_residual_quantize_x requires K/32 <= 1024, got {K // 32}")
-    return _scaled_prepare(X, w, rmsnorm_eps, N, False, residual=residual)
+    return _lib.native().scaled_prepare(X, rmsnorm_weight, rmsnorm_eps, N, residual, False)
 
 
 def rope_inplace_(qkv: torch.Tensor, heads: int, head_dim: int, cos: torch.Tensor, sin: torch.Tensor,
@@ -231,16 +185,7 @@ def rope_inplace_(qkv: torch.Tensor, heads: int, head_dim: int, cos: torch.Tenso
     """Rotary embedding in place on the first `heads` heads of every row of qkv [rows, width]
     (bf16, unit column stride); cos/sin bf16 [seq_len, head_dim]; position = row % seq_len.
     Equals `x * cos + rotate_half(x) * sin` of the ATen ops, head by head."""
-    _check(qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.stride(1) == 1,
-           "qkv must be a CUDA bfloat16 matrix with unit column stride")
-    for t, name in ((cos, "cos"), (sin, "sin")):
-        _check(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and tuple(t.shape) == (seq_len, head_dim),
-               f"{name} must be a contiguous CUDA bfloat16 tensor shaped [seq_len, head_dim]")
-    _check(heads * head_dim <= qkv.shape[1], "heads * head_dim exceeds the row width")
-    dev = qkv.device
-    with _on_device(dev):
-        _lib.check(_lib.lib().sharq_rope_inplace(_ptr(qkv), int(qkv.shape[0]), int(qkv.stride(0)), int(seq_len), int(heads),
-                                                 int(head_dim), _ptr(cos), _ptr(sin), _stream(dev)))
+    _lib.native().rope_inplace(qkv, heads, head_dim, cos, sin, seq_len)
     return qkv
 
 
@@ -301,48 +246,19 @@ def swiglu_sparse_residual_quantize_x(gate_up: torch.Tensor, N: int):
     -> (A_comp, E, SFA_sparse, Q_res, SF_res, scale).  Equals
     scaled_sparse_residual_quantize_x(swiglu(gate_up), N) in two launches: the SwiGLU kernel
     also produces the tensor absmax, so the prepare needs no statistics pass."""
-    _check(gate_up.is_cuda and gate_up.dtype == torch.bfloat16 and gate_up.dim() == 2 and gate_up.is_contiguous(),
-           "gate_up must be a contiguous CUDA bfloat16 matrix")
-    M, F2 = int(gate_up.shape[0]), int(gate_up.shape[1])
-    K = F2 // 2
-    _check(F2 % 2 == 0 and K % 128 == 0, f"swiglu_sparse_residual_quantize_x requires K to be a multiple of 128, got {K}")
-    dev = gate_up.device
-    ws_bytes = 256
-    h_bytes = M * K * 2
-    A_comp, E, SFA, Q_res, SF_res, tail = _prepare_buffers(M, K, dev, extra=512 + h_bytes)
-    ws = tail[:ws_bytes]
-    scale = tail[256:260].view(torch.float32).reshape(())
-    H = tail[512:512 + h_bytes]
-    with _on_device(dev):
-        _lib.check(_lib.lib().sharq_swiglu_sparse_residual_quantize_x(
-            _ptr(gate_up), M, int(N), K, _ptr(H), _ptr(ws), ws_bytes, _ptr(A_comp), _ptr(E), _ptr(SFA), _ptr(Q_res),
-            _ptr(SF_res), _ptr(scale), _stream(dev)))
-    return A_comp, E, SFA, Q_res, SF_res, scale
+    return _lib.native().swiglu_prepare(gate_up, N)
 
 
 def absmax_sparse_residual_quantize_x(X: torch.Tensor, N: int, amax_bits: torch.Tensor):
     """scaled_sparse_residual_quantize_x of an X whose max|X| is already known (amax_bits: the float's bits, as
     linear_gemm_swiglu leaves them): one launch, no statistics pass."""
-    M, K = _check_x(X)
-    _check(K % 128 == 0, f"absmax_sparse_residual_quantize_x requires K to be a multiple of 128, got {K}")
-    _check(amax_bits.is_cuda and amax_bits.device == X.device and amax_bits.dtype == torch.int32 and amax_bits.numel() == 1,
-           "amax_bits must be one CUDA int32 on X's device")
-    dev = X.device
-    A_comp, E, SFA, Q_res, SF_res, tail = _prepare_buffers(M, K, dev, extra=256)
-    scale = tail[:4].view(torch.float32).reshape(())
-    with _on_device(dev):
-        _lib.check(_lib.lib().sharq_absmax_sparse_residual_quantize_x(
-            _ptr(X), M, int(N), K, _ptr(amax_bits), _ptr(A_comp), _ptr(E), _ptr(SFA), _ptr(Q_res), _ptr(SF_res), _ptr(scale),
-            _stream(dev)))
-    return A_comp, E, SFA, Q_res, SF_res, scale
+    return _lib.native().absmax_prepare(X, N, amax_bits)
 
 
 def scaled_sparse_residual_quantize_x(X: torch.Tensor, N: int):
     """Unscaled bf16 X -> (A_comp, E, SFA_sparse, Q_res, SF_res, scale): tensor scale,
     division and prepare in two launches (extra op, not in the reference)."""
-    M, K = _check_x(X)
-    _check(K % 128 == 0, f"scaled_sparse_residual_quantize_x requires K to be a multiple of 128, got {K}")
-    return _scaled_prepare(X, None, 0.0, N, False)
+    return _lib.native().scaled_prepare(X, None, 0.0, N, None, False)
 
 
 # --------------------------------------------------------------------------- weights / dense quant
@@ -407,30 +323,14 @@ def scaled_quantize_nvfp4(X: torch.Tensor):
     """Unscaled bf16 X [rows, K], K % 64 == 0 -> (QX [rows, K/2], SFX, scale [0-dim float32]): tensor scale,
     division and dense NVFP4 quantisation in two launches (extra op, not in the reference)."""
     X = _scaled_quantize_input(X, "X")
-    rows, K = int(X.shape[0]), int(X.shape[1])
-    dev, ws_bytes = X.device, int(_lib.lib().sharq_scaled_quantize_workspace_bytes())
-    Q = torch.empty((rows, K // 2), dtype=torch.uint8, device=dev)
-    SF, ws = _u8(_sf_bytes(rows, K), dev), _u8(ws_bytes, dev)
-    scale = torch.empty((), dtype=torch.float32, device=dev)
-    with _on_device(dev):
-        _lib.check(_lib.lib().sharq_scaled_quantize_nvfp4(_ptr(X), rows, K, _ptr(ws), ws_bytes, _ptr(Q), _ptr(SF), _ptr(scale),
-                                                          _stream(dev)))
-    return Q, SF, scale
+    return _lib.native().scaled_quantize(X, False)
 
 
 def scaled_quantize_w32_shared(W: torch.Tensor):
     """Unscaled bf16 W [N, K], K % 128 == 0 -> (QW [N, K/2], SFW_sparse, SFW_dense, scale [0-dim float32]):
     tensor scale, division and shared weight quantisation in two launches (extra op, not in the reference)."""
     W = _scaled_quantize_input(W, "W")
-    N, K = int(W.shape[0]), int(W.shape[1])
-    dev, ws_bytes = W.device, int(_lib.lib().sharq_scaled_quantize_workspace_bytes())
-    QW = torch.empty((N, K // 2), dtype=torch.uint8, device=dev)
-    SFS, SFD, ws = _u8(_sf_bytes(N, K), dev), _u8(_sf_bytes(N, K), dev), _u8(ws_bytes, dev)
-    scale = torch.empty((), dtype=torch.float32, device=dev)
-    with _on_device(dev):
-        _lib.check(_lib.lib().sharq_scaled_quantize_w32_shared(_ptr(W), N, K, _ptr(ws), ws_bytes, _ptr(QW), _ptr(SFS), _ptr(SFD),
-                                                               _ptr(scale), _stream(dev)))
-    return QW, SFS, SFD, scale
+    return _lib.native().scaled_quantize(W, True)
 
 
 def _check_identity(reorder_index: torch.Tensor, K: int, KE: int) -> None:
@@ -478,27 +378,13 @@ def _scale_ptr(scale: torch.Tensor, reference: torch.Tensor, name: str):
     return _ptr(scale)
 
 
-def _split_k(dev):
-    """(workspace, bytes) arguments that let a GEMM of few tiles split K over the SMs: nothing is written to it."""
-    return (None, 0) if os.environ.get("SHARQ_GEMM_SPLIT_K", "1") == "0" else (_error_flag(dev), 16)
+def _split_k() -> bool:
+    """Whether a GEMM of few tiles may split K over the SMs."""
+    return os.environ.get("SHARQ_GEMM_SPLIT_K", "1") != "0"
 
 
 def _dense_gemm(A, B, SFA, SFB, alpha, alpha_t, C_in, beta, out=None):
-    M, N, K = int(A.shape[0]), int(B.shape[0]), int(A.shape[1]) * 2
-    dev = A.device
-    if out is None:
-        D = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
-    else:
-        _check(out.is_cuda and out.device == dev and out.dtype == torch.bfloat16 and out.is_contiguous()
-               and tuple(out.shape) == (M, N), "out must be a contiguous CUDA bfloat16 tensor shaped [M, N]")
-        D = out
-    ws, ws_bytes = _split_k(dev)
-    with _on_device(dev):
-        _lib.check(_lib.lib().sharq_matmul_ws(
-            _ptr(A), _ptr(B), _ptr(SFA), _ptr(SFB), M, N, K, float(alpha),
-            None if alpha_t is None else _scale_ptr(alpha_t, A, "scale"), _ptr(C_in), float(beta), _ptr(D),
-            _ptr(ws), ws_bytes, _ptr(_error_flag(dev)), _stream(dev)))
-    return D
+    return _lib.native().dense_gemm(A, B, SFA, SFB, alpha, alpha_t, C_in, beta, out, _error_flag(A.device), _split_k())
 
 
 def _check_c_in(C_in, A, M, N):
@@ -533,31 +419,8 @@ def matmul_accum_tensor_scale(A, B, SFA, SFB, scale: torch.Tensor, C_in, beta: f
 
 
 def _sparse_gemm(name, A_comp, B, E, SFA, SFB, M, N, K, alpha, alpha_t, beta):
-    _check(M > 0 and N > 0 and K > 0, "M, N, K must be positive")
-    _check(beta == 0.0, f"{name} currently requires beta == 0")
-    ts = (A_comp, B, E, SFA, SFB)
-    _check(all(t.is_cuda for t in ts), f"{name} inputs must be CUDA tensors")
-    _check(all(t.is_contiguous() for t in ts), f"{name} inputs must be contiguous")
-    for t, nm in zip(ts, ("A_comp", "B", "E", "SFA", "SFB")):
-        _check(t.dtype == torch.uint8, f"{nm} must be torch.uint8")
-    _check(all(t.device == A_comp.device for t in ts), f"{name} inputs must be on the same device")
-    ea, ee, esfa, esfb = get_sparse_nvfp4_buffer_sizes(M, N, K)
-    _check(A_comp.numel() == ea, f"A_comp.numel() mismatch: expected {ea}, got {A_comp.numel()}")
-    _check(E.numel() == ee, f"E.numel() mismatch: expected {ee}, got {E.numel()}")
-    _check(SFA.numel() == esfa, f"SFA.numel() mismatch: expected {esfa}, got {SFA.numel()}")
-    _check(SFB.numel() == esfb, f"SFB.numel() mismatch: expected {esfb}, got {SFB.numel()}")
-    _check(B.dim() == 2, "B must be a 2D tensor shaped [N, K/2]")
-    _check(B.shape[0] == N, f"B.size(0) mismatch: expected {N}, got {B.shape[0]}")
-    _check(B.shape[1] == K // 2, f"B.size(1) mismatch: expected {K // 2}, got {B.shape[1]}")
-    dev = A_comp.device
-    D = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
-    ws, ws_bytes = _split_k(dev)
-    with _on_device(dev):
-        _lib.check(_lib.lib().sharq_sparse_matmul_ws(
-            _ptr(A_comp), _ptr(B), _ptr(E), _ptr(SFA), _ptr(SFB), M, N, K, float(alpha),
-            None if alpha_t is None else _scale_ptr(alpha_t, A_comp, "alpha"), float(beta), _ptr(D),
-            _ptr(ws), ws_bytes, _ptr(_error_flag(dev)), _stream(dev)))
-    return D
+    return _lib.native().sparse_gemm(name, A_comp, B, E, SFA, SFB, M, N, K, alpha, alpha_t, beta, _error_flag(A_comp.device),
+                                     _split_k())
 
 
 def sparse_matmul(A_comp, B, E, SFA, SFB, M: int, N: int, K: int, alpha: float = 1.0, beta: float = 0.0):
@@ -592,38 +455,25 @@ def sharq_linear_gemm(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_
     scatter=(rank_ptrs, rank, world): row-parallel output under tensor parallelism; the rows are dealt to the
     collection buffers of their owner GPUs (rank_ptrs: ctypes array of their mappings, see
     sharq_linear_gemm_scatter); nothing is returned."""
+    alpha_t = alpha if isinstance(alpha, torch.Tensor) else None
+    if scatter is None:
+        return _lib.native().linear_gemm(
+            A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense, alpha_t,
+            float(alpha_host) if alpha_t is not None else float(alpha) * float(alpha_host), bias, out,
+            _error_flag(Q_res.device), _split_k())
     M, K = int(Q_res.shape[0]), int(Q_res.shape[1]) * 2
     N = int(QW.shape[0])
     dev = Q_res.device
     _check_fused_operands(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense)
-    if bias is not None:
-        _check(bias.is_cuda and bias.dtype == torch.bfloat16 and bias.numel() == N and bias.is_contiguous(),
-               "bias must be a contiguous CUDA bfloat16 tensor with N elements")
-    alpha_t = alpha if isinstance(alpha, torch.Tensor) else None
-    if scatter is not None:
-        _check(bias is None and out is None, "scatter mode takes neither bias nor out")
-        rank_ptrs, rank, world = scatter
-        with _on_device(dev):
-            _lib.check(_lib.lib().sharq_linear_gemm_scatter(
-                _ptr(A_comp), _ptr(E), _ptr(SFA_sparse), _ptr(Q_res), _ptr(SF_res), _ptr(QW), _ptr(SFW_sparse),
-                _ptr(SFW_dense), M, N, K, float(alpha_host) if alpha_t is not None else float(alpha) * float(alpha_host),
-                None if alpha_t is None else _scale_ptr(alpha_t, Q_res, "alpha"), rank_ptrs, int(rank), int(world),
-                _ptr(_error_flag(dev)), _stream(dev)))
-        return None
-    if out is None:
-        D = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
-    else:
-        _check(out.is_cuda and out.device == dev and out.dtype == torch.bfloat16 and out.is_contiguous()
-               and tuple(out.shape) == (M, N), "out must be a contiguous CUDA bfloat16 tensor shaped [M, N]")
-        D = out
-    ws, ws_bytes = _split_k(dev)
+    _check(bias is None and out is None, "scatter mode takes neither bias nor out")
+    rank_ptrs, rank, world = scatter
     with _on_device(dev):
-        _lib.check(_lib.lib().sharq_linear_gemm_ws(
+        _lib.check(_lib.lib().sharq_linear_gemm_scatter(
             _ptr(A_comp), _ptr(E), _ptr(SFA_sparse), _ptr(Q_res), _ptr(SF_res), _ptr(QW), _ptr(SFW_sparse),
             _ptr(SFW_dense), M, N, K, float(alpha_host) if alpha_t is not None else float(alpha) * float(alpha_host),
-            None if alpha_t is None else _scale_ptr(alpha_t, Q_res, "alpha"), _ptr(bias), _ptr(D),
-            _ptr(ws), ws_bytes, _ptr(_error_flag(dev)), _stream(dev)))
-    return D
+            None if alpha_t is None else _scale_ptr(alpha_t, Q_res, "alpha"), rank_ptrs, int(rank), int(world),
+            _ptr(_error_flag(dev)), _stream(dev)))
+    return None
 
 
 def linear_gemm_swiglu_pays(M: int, ffn: int, K: int) -> bool:
@@ -635,32 +485,18 @@ def linear_gemm_swiglu(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW
                        alpha_host: float = 1.0):
     """Fused SharQ GEMM of a merged gate_up weight [2F, K] (F % 128 == 0, no bias) with SwiGLU in its epilogue:
     -> (H [M, F] bf16, amax_bits [1] int32 with the bits of max|H|); the bits of swiglu(sharq_linear_gemm(...))."""
-    M, K = int(Q_res.shape[0]), int(Q_res.shape[1]) * 2
-    N = int(QW.shape[0])
-    dev = Q_res.device
-    _check(N % 256 == 0, f"the merged gate_up weight must have a multiple of 256 rows, got {N}")
-    _check_fused_operands(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense)
-    H = torch.empty((M, N // 2), dtype=torch.bfloat16, device=dev)
-    amax_bits = torch.empty(1, dtype=torch.int32, device=dev)
-    with _on_device(dev):
-        _lib.check(_lib.lib().sharq_linear_gemm_swiglu(
-            _ptr(A_comp), _ptr(E), _ptr(SFA_sparse), _ptr(Q_res), _ptr(SF_res), _ptr(QW), _ptr(SFW_sparse), _ptr(SFW_dense),
-            M, N // 2, K, float(alpha_host), _scale_ptr(alpha, Q_res, "alpha"), _ptr(H), _ptr(amax_bits),
-            _ptr(_error_flag(dev)), _stream(dev)))
-    return H, amax_bits
+    return _lib.native().linear_gemm_swiglu(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense, alpha, alpha_host,
+                                            _error_flag(Q_res.device))
 
 
 def sharq_linear_forward(x: torch.Tensor, qw: torch.Tensor, sfw_sparse: torch.Tensor, sfw_dense: torch.Tensor,
-                         weight_scale: float) -> torch.Tensor:
+                         weight_scale: float, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Whole SharQ linear on an unscaled bf16 activation [M,K] -> bf16 [M,N]: the optional
     op the reference's vLLM plugin calls when present (benchmarks/vllm/sharq.py:199-213).
     Two prepare launches and one GEMM launch; the activation scale stays on the device."""
     _check(x.dim() == 2, "x must be shaped [M, K]")
     x = x.contiguous().to(torch.bfloat16)
-    N = int(qw.shape[0])
-    a_comp, e, sfa, q_res, sf_res, scale = scaled_sparse_residual_quantize_x(x, N)
-    return sharq_linear_gemm(a_comp, e, sfa, q_res, sf_res, qw, sfw_sparse, sfw_dense, scale.reshape(1),
-                             alpha_host=float(weight_scale))
+    return _lib.native().linear_forward(x, qw, sfw_sparse, sfw_dense, weight_scale, bias, _error_flag(x.device), _split_k())
 
 
 # --------------------------------------------------------------------------- grouped (mixture-of-experts) launches

@@ -197,7 +197,11 @@ class QLinearLayer(nn.Module):
         else:
             x_orig, bsz, q_len = x, None, x.shape[0]
         x2 = x_orig.reshape(-1, x_orig.shape[-1]).to(torch.bfloat16)
-        y = self.apply_prepared(self.prepare_input(x2))
+        if self.quant_type == "SHARQ" and self.fused_gemm:
+            y = ops.sharq_linear_forward(x2, self.weight_q, self.scale_w_sparse, self.scale_w_dense, self.weight_scale_host,
+                                         bias=self.bias)
+        else:
+            y = self.apply_prepared(self.prepare_input(x2))
         if bsz is not None:
             return y.reshape(bsz, q_len, -1)
         return y.reshape(q_len, -1)
