@@ -281,6 +281,9 @@ int sharq_allreduce_bf16_peer(void *const *rank_data_ptrs, void *const *rank_fla
  *     device pointers; alpha_vec: device, e.g. activation scale x weight scale per expert).
  *   sharq_linear_gemm_grouped_swiglu / sharq_grouped_absmax_sparse_residual_quantize_x: the grouped
  *     forms of sharq_linear_gemm_swiglu and sharq_absmax_sparse_residual_quantize_x (amax_workspace: `groups` words).
+ *   sharq_moe_plan: the grouping itself from selected [tokens * top_k] (expert of every token slot, experts <= 16, unit 256
+ *     for the entry points below): dest[slot] = its grouped row (ascending slots inside an expert), src_row[row] = its
+ *     token or -1, unit_group as above; rows >= (ceil(slots / unit) + experts) * unit, a multiple of unit.
  *   sharq_moe_combine: out[t] = sum over the top_k slots of token t, in ascending expert order, of
  *     y[dest[t,j]] * w[t,j] with bf16 rounding after every product and addition, which is what the
  *     reference's sequence of index_add_ calls on a zero buffer computes. */
@@ -302,6 +305,9 @@ int sharq_linear_gemm_grouped_swiglu(const void *a_comp, const void *e, const vo
 int sharq_grouped_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, int n, int k, const int *unit_group, int groups,
                                                     const void *amax_workspace, void *a_comp, void *e, void *sfa_sparse,
                                                     void *q_res, void *sf_res, float *scale_vec_out, void *stream);
+int sharq_moe_plan(const int64_t *selected, int64_t slots, int top_k, int experts, int unit, int64_t rows, void *workspace,
+                   size_t workspace_bytes, int *dest, int *src_row, int *unit_group, void *stream);
+size_t sharq_moe_plan_workspace_bytes(int64_t slots);
 int sharq_moe_combine(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
                       int tokens, int top_k, int width, void *stream);
 

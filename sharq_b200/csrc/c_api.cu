@@ -413,6 +413,21 @@ int sharq_grouped_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, i
                     "grouped_absmax_sparse_residual_quantize_x");
 }
 
+size_t sharq_moe_plan_workspace_bytes(int64_t slots) { return slots > 0 ? sharq::moe_plan_workspace_bytes(slots) : 0; }
+
+int sharq_moe_plan(const int64_t *selected, int64_t slots, int top_k, int experts, int unit, int64_t rows, void *workspace,
+                   size_t workspace_bytes, int *dest, int *src_row, int *unit_group, void *stream) {
+  SHARQ_REQUIRE(selected && workspace && dest && src_row && unit_group, "null buffer");
+  SHARQ_REQUIRE(slots > 0 && top_k > 0 && unit > 0, "slots, top_k and unit must be positive");
+  SHARQ_REQUIRE(experts >= 1 && experts <= sharq::kGemmMaxGroups, "experts must be in [1, %d]", sharq::kGemmMaxGroups);
+  SHARQ_REQUIRE(rows % unit == 0 && rows <= 0x7fffffff && rows >= ((slots + unit - 1) / unit + experts) * unit,
+                "rows must be a multiple of unit that holds every expert's padded segment");
+  SHARQ_REQUIRE(workspace_bytes >= sharq_moe_plan_workspace_bytes(slots), "workspace is too small");
+  return check_cuda(sharq::run_moe_plan(reinterpret_cast<const long long *>(selected), slots, top_k, experts, unit, rows,
+                                        static_cast<int *>(workspace), dest, src_row, unit_group, as_stream(stream)),
+                    "moe_plan");
+}
+
 int sharq_moe_combine(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
                       int tokens, int top_k, int width, void *stream) {
   SHARQ_REQUIRE(out_bf16 && y_bf16 && dest && selected && w_bf16, "null buffer");

@@ -246,24 +246,130 @@ __global__ void __launch_bounds__(256) abs_stats_grouped_kernel(const __nv_bfloa
                                                                 const int *__restrict__ src_row) {
   __shared__ float warp_max[8];
   const int vecs = width >> 3;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long n_chunks = (rows + kGroupedChunkRows - 1) / kGroupedChunkRows;
   for (long long chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
     const long long row_lo = chunk * kGroupedChunkRows, row_hi = min(rows, row_lo + kGroupedChunkRows);
     const int grp = unit_group[row_lo / 256];
     if (grp < 0) continue;
     __nv_bfloat162 mx2 = __floats2bfloat162_rn(0.0f, 0.0f);
-    const long long n16 = (row_hi - row_lo) * vecs;
-    for (long long i = threadIdx.x; i < n16; i += blockDim.x) {
-      const long long r = row_lo + i / vecs;
+    // a warp per row, four loads in flight per lane
+    for (long long r = row_lo + warp; r < row_hi; r += 8) {
       const long long in_row = src_row != nullptr ? src_row[r] : r;  // gathered rows; < 0: a padding row
       if (in_row < 0) continue;
-      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(x + in_row * width) + (i % vecs));
-      mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.x)));
-      mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.y)));
-      mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.z)));
-      mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.w)));
+      const uint4 *row = reinterpret_cast<const uint4 *>(x + in_row * width);
+      for (int i = lane; i < vecs; i += 128) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = i + 32 * u < vecs ? __ldg(row + i + 32 * u) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u].x)));
+          mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u].y)));
+          mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u].z)));
+          mx2 = __hmax2(mx2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u].w)));
+        }
+      }
     }
     cta_absmax_to(warp_max, mx2, amax_bits + grp);
+  }
+}
+
+// Plan of a grouped mixture-of-experts step: the row of every token slot in the grouped activation (slots in ascending
+// order inside their expert's segment, segments padded to whole units), the token of every grouped row and the expert of every
+// unit.  Two launches over blocks of kPlanSlots slots: counts per block and expert, then every block adds up the counts before it and
+// ranks its own slots.  As ATen operations (argsort, scatter_add, cumsum, gathers, searchsorted) the plan of 32768
+// slots took 45 launches and 190 us.
+constexpr int kPlanThreads = 256;
+constexpr int kPlanSlots = 1024;
+constexpr int kPlanMaxExperts = 16;
+
+// expert of a slot, -1 behind the last slot or outside [0, experts)
+__device__ __forceinline__ int plan_expert(const long long *selected, long long slot, long long slots, int experts) {
+  const long long e = slot < slots ? selected[slot] : -1;
+  return e >= 0 && e < experts ? (int)e : -1;
+}
+
+__global__ void __launch_bounds__(kPlanThreads) moe_count_kernel(const long long *__restrict__ selected, long long slots, int experts,
+                                                                 int *__restrict__ counts) {
+  __shared__ int hist[kPlanMaxExperts];
+  if (threadIdx.x < kPlanMaxExperts) hist[threadIdx.x] = 0;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kPlanSlots / kPlanThreads; ++i) {
+    const int e = plan_expert(selected, (long long)blockIdx.x * kPlanSlots + i * kPlanThreads + threadIdx.x, slots, experts);
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    if (e >= 0 && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&hist[e], __popc(same));
+  }
+  __syncthreads();
+  if (threadIdx.x < kPlanMaxExperts) counts[blockIdx.x * kPlanMaxExperts + threadIdx.x] = hist[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(kPlanThreads) moe_place_kernel(const long long *__restrict__ selected, long long slots, int top_k,
+                                                                 int experts, int unit, long long rows,
+                                                                 const int *__restrict__ counts, int *__restrict__ dest,
+                                                                 int *__restrict__ src_row, int *__restrict__ unit_group) {
+  constexpr int kWarps = kPlanThreads / 32, kParts = kPlanThreads / kPlanMaxExperts;
+  __shared__ int part_before[kParts][kPlanMaxExperts], part_total[kParts][kPlanMaxExperts];
+  __shared__ int next[kPlanMaxExperts];                                  // grouped row of the expert's next slot
+  __shared__ int used_end[kPlanMaxExperts], segment_end[kPlanMaxExperts];  // ends of its rows without and with padding
+  __shared__ int warp_count[kWarps][kPlanMaxExperts];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  {
+    const int e = threadIdx.x % kPlanMaxExperts, part = threadIdx.x / kPlanMaxExperts;
+    int before = 0, total = 0;
+    for (int b = part; b < (int)gridDim.x; b += kParts) {
+      const int c = counts[b * kPlanMaxExperts + e];
+      total += c;
+      if (b < (int)blockIdx.x) before += c;
+    }
+    part_before[part][e] = before;
+    part_total[part][e] = total;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int start = 0;
+    for (int e = 0; e < experts; ++e) {
+      int before = 0, total = 0;
+      for (int q = 0; q < kParts; ++q) {
+        before += part_before[q][e];
+        total += part_total[q][e];
+      }
+      next[e] = start + before;
+      used_end[e] = start + total;
+      start += (total + unit - 1) / unit * unit;
+      segment_end[e] = start;
+    }
+  }
+  __syncthreads();
+  for (int i = 0; i < kPlanSlots / kPlanThreads; ++i) {
+    const long long slot = (long long)blockIdx.x * kPlanSlots + i * kPlanThreads + threadIdx.x;
+    const int e = plan_expert(selected, slot, slots, experts);
+    const unsigned same = __match_any_sync(0xffffffffu, e);
+    const int rank = __popc(same & ((1u << lane) - 1u));
+    if (lane < kPlanMaxExperts) warp_count[warp][lane] = 0;
+    __syncwarp();
+    if (e >= 0 && rank == 0) warp_count[warp][e] = __popc(same);
+    __syncthreads();
+    if (e >= 0) {
+      int row = next[e] + rank;
+      for (int w = 0; w < warp; ++w) row += warp_count[w][e];
+      dest[slot] = row;
+      src_row[row] = (int)(slot / top_k);
+    }
+    __syncthreads();
+    if (threadIdx.x < experts) {
+      for (int w = 0; w < kWarps; ++w) next[threadIdx.x] += warp_count[w][threadIdx.x];
+    }
+    __syncthreads();
+  }
+  // padding rows and the units' experts
+  const long long worker = (long long)blockIdx.x * kPlanThreads + threadIdx.x, workers = (long long)gridDim.x * kPlanThreads;
+  for (long long r = worker; r < rows; r += workers) {
+    int e = 0;
+    while (e < experts && r >= segment_end[e]) ++e;
+    if (e == experts || r >= used_end[e]) src_row[r] = -1;
+    if (r % unit == 0) unit_group[r / unit] = e < experts ? e : -1;
   }
 }
 
@@ -410,6 +516,21 @@ cudaError_t run_abs_stats_grouped(const void *x, long long rows, int width, unsi
   if (ctas > work) ctas = work;
   abs_stats_grouped_kernel<<<(unsigned)ctas, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(x), rows, width, amax_bits,
                                                                 unit_group, src_row);
+  return cudaGetLastError();
+}
+
+size_t moe_plan_workspace_bytes(long long slots) {
+  return (size_t)((slots + kPlanSlots - 1) / kPlanSlots) * kPlanMaxExperts * sizeof(int);
+}
+
+cudaError_t run_moe_plan(const long long *selected, long long slots, int top_k, int experts, int unit, long long rows, int *counts,
+                         int *dest, int *src_row, int *unit_group, cudaStream_t stream) {
+  if (slots <= 0 || top_k < 1 || experts < 1 || experts > kPlanMaxExperts || unit < 1) return cudaErrorInvalidValue;
+  // every expert's padding fits: rows is a whole number of units
+  if (rows % unit != 0 || rows > 0x7fffffffLL || rows < ((slots + unit - 1) / unit + experts) * unit) return cudaErrorInvalidValue;
+  const unsigned blocks = (unsigned)((slots + kPlanSlots - 1) / kPlanSlots);
+  moe_count_kernel<<<blocks, kPlanThreads, 0, stream>>>(selected, slots, experts, counts);
+  moe_place_kernel<<<blocks, kPlanThreads, 0, stream>>>(selected, slots, top_k, experts, unit, rows, counts, dest, src_row, unit_group);
   return cudaGetLastError();
 }
 

@@ -35,4 +35,10 @@ cudaError_t run_add_rmsnorm(const void *x, const void *residual, void *sum_out, 
 cudaError_t run_scatter_add_scaled(void *out, const void *y, const long long *rows, const void *w, long long n_rows,
                                    int width, long long out_rows, cudaStream_t stream);
 
+// Grouping plan of a mixture-of-experts step (see moe_place_kernel): selected [slots] (slot = token * top_k + j), at most
+// 16 experts; rows = (ceil(slots / unit) + experts) * unit or more; counts: moe_plan_workspace_bytes(slots) bytes of scratch.
+size_t moe_plan_workspace_bytes(long long slots);
+cudaError_t run_moe_plan(const long long *selected, long long slots, int top_k, int experts, int unit, long long rows, int *counts,
+                         int *dest, int *src_row, int *unit_group, cudaStream_t stream);
+
 }  // namespace sharq

@@ -458,6 +458,10 @@ def moe_grouping(selected: torch.Tensor, experts: int, unit: int = 256):
     tokens, k = selected.shape
     dev = selected.device
     slots = tokens * k
+    if selected.is_cuda and slots > 0 and experts <= 16:
+        from . import ops
+
+        return ops.moe_plan(selected.contiguous(), experts, unit)
     rows = ((slots + unit - 1) // unit + experts) * unit
     flat = selected.reshape(-1)
     order = torch.argsort(flat, stable=True)

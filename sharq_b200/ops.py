@@ -622,6 +622,24 @@ def linear_gemm_grouped_swiglu(A_comp, E, SFA_sparse, Q_res, SF_res, weights, un
     return H, amax_bits
 
 
+def moe_plan(selected: torch.Tensor, experts: int, unit: int = 256):
+    """decoder.moe_grouping on the GPU in two launches: selected int64 [tokens, top_k], experts <= 16 ->
+    (dest int32 [tokens, top_k], src_row int32 [rows], unit_group int32 [rows / unit])."""
+    _check(selected.is_cuda and selected.dtype == torch.int64 and selected.dim() == 2 and selected.is_contiguous()
+           and selected.numel() > 0, "selected must be a contiguous non-empty CUDA int64 matrix")
+    slots, dev = selected.numel(), selected.device
+    rows = ((slots + unit - 1) // unit + experts) * unit
+    L = _lib.lib()
+    ws_bytes = int(L.sharq_moe_plan_workspace_bytes(slots))
+    out = torch.empty(slots + rows + rows // unit, dtype=torch.int32, device=dev)
+    dest, src_row, unit_group = out.split((slots, rows, rows // unit))
+    ws = _u8(ws_bytes, dev)
+    with _on_device(dev):
+        _lib.check(L.sharq_moe_plan(_ptr(selected), slots, int(selected.shape[1]), int(experts), int(unit), rows, _ptr(ws), ws_bytes,
+                                    _ptr(dest), _ptr(src_row), _ptr(unit_group), _stream(dev)))
+    return dest.view(selected.shape), src_row, unit_group
+
+
 def moe_combine(y: torch.Tensor, dest: torch.Tensor, selected: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     """out[t] = sum over the top_k slots of token t, in ascending expert order, of y[dest[t, j]] * w[t, j] (bf16 roundings as
     in the reference's index_add_ loop).  dest int32 [T, top_k], selected int64 [T, top_k], w bf16 [T, top_k]."""
