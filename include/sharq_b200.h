@@ -221,6 +221,13 @@ int sharq_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, int n, in
                                             void *e, void *sfa_sparse, void *q_res, void *sf_res, float *scale_out,
                                             void *stream);
 
+/* sharq_linear_gemm_ws with a residual [M, N] (bf16, 16-byte aligned) added to the bf16 result in the epilogue, rounded as a
+ * separate bf16 add would: the residual add behind a decoder layer's last linear. */
+int sharq_linear_gemm_residual(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res,
+                               const void *qw, const void *sfw_sparse, const void *sfw_dense, int m, int n, int k, float alpha,
+                               const float *alpha_dev, const void *bias_bf16, const void *residual_bf16, void *d, void *workspace,
+                               size_t workspace_bytes, int *error_flag, void *stream);
+
 /* No counterpart in the reference.  Same work and outputs as
  * sharq_fused_rmsnorm_sparse_residual_quantize_x, for callers that cannot allocate device
  * memory and have no spare buffer to pass as workspace (a server that has given all free
@@ -310,6 +317,9 @@ int sharq_moe_plan(const int64_t *selected, int64_t slots, int top_k, int expert
 size_t sharq_moe_plan_workspace_bytes(int64_t slots);
 int sharq_moe_combine(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
                       int tokens, int top_k, int width, void *stream);
+/* ... + residual [tokens, width] (bf16, 16-byte aligned), added last and rounded as a separate bf16 add would. */
+int sharq_moe_combine_residual(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
+                               const void *residual_bf16, int tokens, int top_k, int width, void *stream);
 
 /* No counterpart in the reference (it has no tensor parallelism).  Row-parallel SharQ linear and the
  * transition to the next column-parallel one over the GPUs of one NVLink domain, with the residual

@@ -55,6 +55,9 @@ SIGNATURES = {
         c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, c_float, _P, _P, c_size_t, _P, _P]),
     "sharq_linear_gemm_ws": (
         c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, _P, _P, c_size_t, _P, _P]),
+    "sharq_linear_gemm_residual": (
+        c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, _P, _P, _P, c_size_t, _P, _P]),
+    "sharq_moe_combine_residual": (c_int, [_P, _P, _P, _P, _P, _P, c_int, c_int, c_int, _P]),
     "sharq_gemm_swiglu_pays": (c_int, [c_int, c_int, c_int]),
     "sharq_linear_gemm_swiglu": (
         c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, _P, _P, _P]),

@@ -430,13 +430,18 @@ int sharq_moe_plan(const int64_t *selected, int64_t slots, int top_k, int expert
 
 int sharq_moe_combine(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
                       int tokens, int top_k, int width, void *stream) {
+  return sharq_moe_combine_residual(out_bf16, y_bf16, dest, selected, w_bf16, nullptr, tokens, top_k, width, stream);
+}
+
+int sharq_moe_combine_residual(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
+                               const void *residual_bf16, int tokens, int top_k, int width, void *stream) {
   SHARQ_REQUIRE(out_bf16 && y_bf16 && dest && selected && w_bf16, "null buffer");
   SHARQ_REQUIRE(tokens >= 0 && top_k >= 1 && top_k <= 8 && width > 0 && width % 8 == 0,
                 "tokens >= 0, top_k in [1, 8], width a positive multiple of 8");
-  SHARQ_REQUIRE(((reinterpret_cast<uintptr_t>(out_bf16) | reinterpret_cast<uintptr_t>(y_bf16)) & 15) == 0,
-                "out and y must be 16-byte aligned");
-  return check_cuda(sharq::run_moe_combine(out_bf16, y_bf16, dest, reinterpret_cast<const long long *>(selected), w_bf16, tokens,
-                                           top_k, width, as_stream(stream)),
+  SHARQ_REQUIRE(((reinterpret_cast<uintptr_t>(out_bf16) | reinterpret_cast<uintptr_t>(y_bf16) |
+                  reinterpret_cast<uintptr_t>(residual_bf16)) & 15) == 0, "out, y and residual must be 16-byte aligned");
+  return check_cuda(sharq::run_moe_combine(out_bf16, y_bf16, dest, reinterpret_cast<const long long *>(selected), w_bf16,
+                                           residual_bf16, tokens, top_k, width, as_stream(stream)),
                     "moe_combine");
 }
 
@@ -622,6 +627,14 @@ int sharq_linear_gemm_ws(const void *a_comp, const void *e, const void *sfa_spar
                          const void *qw, const void *sfw_sparse, const void *sfw_dense, int m, int n, int k, float alpha,
                          const float *alpha_dev, const void *bias, void *d, void *workspace, size_t workspace_bytes,
                          int *error_flag, void *stream) {
+  return sharq_linear_gemm_residual(a_comp, e, sfa_sparse, q_res, sf_res, qw, sfw_sparse, sfw_dense, m, n, k, alpha, alpha_dev, bias,
+                                    nullptr, d, workspace, workspace_bytes, error_flag, stream);
+}
+
+int sharq_linear_gemm_residual(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res,
+                         const void *qw, const void *sfw_sparse, const void *sfw_dense, int m, int n, int k, float alpha,
+                         const float *alpha_dev, const void *bias, const void *residual, void *d, void *workspace, size_t workspace_bytes,
+                         int *error_flag, void *stream) {
   SHARQ_REQUIRE(m > 0 && n > 0 && k > 0, "M, N, K must be positive");
   SHARQ_REQUIRE(k % 128 == 0, "linear_gemm requires K to be a multiple of 128, got %d", k);
   SHARQ_REQUIRE(a_comp && e && sfa_sparse && q_res && sf_res && qw && sfw_sparse && sfw_dense && d && error_flag,
@@ -636,6 +649,7 @@ int sharq_linear_gemm_ws(const void *a_comp, const void *e, const void *sfa_spar
   g.sfb_sparse = sfw_sparse;
   g.sfb_dense = sfw_dense;
   g.bias = bias;
+  g.residual = residual;
   g.d = d;
   g.alpha = alpha;
   g.alpha_ptr = alpha_dev;
@@ -645,6 +659,7 @@ int sharq_linear_gemm_ws(const void *a_comp, const void *e, const void *sfa_spar
   g.tile_n = g_tile_n;
   g.error_flag = error_flag;
   g.split_k = workspace != nullptr && workspace_bytes >= sharq_gemm_workspace_bytes(m, n);
+  SHARQ_REQUIRE((reinterpret_cast<uintptr_t>(residual) & 15) == 0, "residual must be 16-byte aligned");
   SHARQ_REQUIRE(workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 15) == 0,
                 "workspace must be 16-byte aligned");
   return check_cuda(sharq::run_gemm(g, as_stream(stream)), "linear_gemm");

@@ -381,7 +381,8 @@ __global__ void __launch_bounds__(kPlanThreads) moe_place_kernel(const long long
 constexpr int kCombineMaxTopK = 8;
 __global__ void __launch_bounds__(256) moe_combine_kernel(__nv_bfloat16 *__restrict__ out, const __nv_bfloat16 *__restrict__ y,
                                                           const int *__restrict__ dest, const long long *__restrict__ selected,
-                                                          const __nv_bfloat16 *__restrict__ w, long long tokens, int top_k,
+                                                          const __nv_bfloat16 *__restrict__ w,
+                                                          const __nv_bfloat16 *__restrict__ residual, long long tokens, int top_k,
                                                           int width) {
   const int vecs = width >> 3;
   for (long long t = blockIdx.x; t < tokens; t += gridDim.x) {
@@ -405,6 +406,15 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(__nv_bfloat16 *__restr
         for (int q = 0; q < 4; ++q) {
           acc[2 * q] = round_bf16(acc[2 * q] + round_bf16(__fmul_rn(lo_f(yw[q]), wj)));
           acc[2 * q + 1] = round_bf16(acc[2 * q + 1] + round_bf16(__fmul_rn(hi_f(yw[q]), wj)));
+        }
+      }
+      if (residual != nullptr) {  // a separate bf16 add of the finished sum
+        const uint4 rv = __ldg(reinterpret_cast<const uint4 *>(residual + t * width) + v);
+        const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          acc[2 * q] += lo_f(rw[q]);
+          acc[2 * q + 1] += hi_f(rw[q]);
         }
       }
       *reinterpret_cast<uint4 *>(out + t * width + (long long)v * 8) =
@@ -535,14 +545,14 @@ cudaError_t run_moe_plan(const long long *selected, long long slots, int top_k, 
 }
 
 cudaError_t run_moe_combine(void *out, const void *y, const int *dest, const long long *selected, const void *w,
-                            long long tokens, int top_k, int width, cudaStream_t stream) {
+                            const void *residual, long long tokens, int top_k, int width, cudaStream_t stream) {
   if (top_k < 1 || top_k > kCombineMaxTopK) return cudaErrorInvalidValue;
   long long ctas = (long long)sm_count() * 8;
   if (ctas > tokens) ctas = tokens;
   if (ctas < 1) return cudaSuccess;
   moe_combine_kernel<<<(unsigned)ctas, 256, 0, stream>>>(static_cast<__nv_bfloat16 *>(out), static_cast<const __nv_bfloat16 *>(y),
-                                                          dest, selected, static_cast<const __nv_bfloat16 *>(w), tokens, top_k,
-                                                          width);
+                                                          dest, selected, static_cast<const __nv_bfloat16 *>(w),
+                                                          static_cast<const __nv_bfloat16 *>(residual), tokens, top_k, width);
   return cudaGetLastError();
 }
 

@@ -24,7 +24,7 @@ cudaError_t run_abs_stats_grouped(const void *x, long long rows, int width, unsi
 // out[t, :] = sum over the top_k slots of token t, in ascending expert order, of y[dest[t, j], :] * w[t, j]
 // with bf16 roundings after every product and every addition (selected: expert index per slot).
 cudaError_t run_moe_combine(void *out, const void *y, const int *dest, const long long *selected, const void *w,
-                            long long tokens, int top_k, int width, cudaStream_t stream);
+                            const void *residual, long long tokens, int top_k, int width, cudaStream_t stream);
 
 // out[rows, k] = bf16(s * rsqrt(mean(s^2) + eps) * gamma), s = bf16(x + residual) stored to sum_out
 // (residual == nullptr: s = x, sum_out unused); K a multiple of 8, at most 8192.

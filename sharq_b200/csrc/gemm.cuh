@@ -23,6 +23,7 @@ struct GemmArgs {
   // Epilogue: d = bf16(alpha * acc + beta * c_in), then (+ bias) in bf16.
   const void *c_in = nullptr;  // [m, n] bf16, optional
   const void *bias = nullptr;  // [n] bf16, optional
+  const void *residual = nullptr;  // [m, n] bf16, optional, 16-byte aligned: added to the bf16 result (plain output only)
   void *d = nullptr;           // [m, n] bf16
   const float *alpha_ptr = nullptr;  // device scalar; when non-null the factor is alpha * (*alpha_ptr)
   float alpha = 1.0f;

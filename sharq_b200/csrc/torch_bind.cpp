@@ -217,7 +217,8 @@ void check_weight(const Tensor &qw, const Tensor &sfs, const Tensor &sfd, const 
 // flag: the device's error flag; with split_k it also stands for the GEMM's (unwritten) workspace.
 Tensor linear_gemm(const Tensor &a_comp, const Tensor &e, const Tensor &sfa, const Tensor &q_res, const Tensor &sf_res,
                    const Tensor &qw, const Tensor &sfs, const Tensor &sfd, const std::optional<Tensor> &alpha_t, double alpha,
-                   const std::optional<Tensor> &bias, const std::optional<Tensor> &out, const Tensor &flag, bool split_k) {
+                   const std::optional<Tensor> &bias, const std::optional<Tensor> &out, const std::optional<Tensor> &residual,
+                   const Tensor &flag, bool split_k) {
   const int64_t m = q_res.size(0), k = q_res.size(1) * 2, n = qw.size(0);
   const at::Device dev = q_res.device();
   const int64_t k256 = (k + 255) / 256 * 256;
@@ -228,12 +229,16 @@ Tensor linear_gemm(const Tensor &a_comp, const Tensor &e, const Tensor &sfa, con
   check_u8(sf_res, dev, sf_bytes(m, k), "SF_res");
   check_weight(qw, sfs, sfd, dev, n, k);
   check_bias(bias, n);
+  if (residual)
+    need(is_plain(*residual, at::kBFloat16) && residual->device() == dev && residual->numel() == m * n,
+         "residual must be a contiguous CUDA bfloat16 tensor with M * N elements on the device of Q_res");
   Tensor d = output(q_res, m, n, out);
   const float *alpha_dev = alpha_t ? scale_ptr(*alpha_t, dev, "alpha") : nullptr;
   c10::cuda::OptionalCUDAGuard guard(dev);
-  check(sharq_linear_gemm_ws(ptr(a_comp), ptr(e), ptr(sfa), ptr(q_res), ptr(sf_res), ptr(qw), ptr(sfs), ptr(sfd), (int)m, (int)n,
-                             (int)k, (float)alpha, alpha_dev, bias ? ptr(*bias) : nullptr, ptr(d), split_k ? ptr(flag) : nullptr,
-                             split_k ? 16 : 0, static_cast<int *>(ptr(flag)), stream_of(q_res)));
+  check(sharq_linear_gemm_residual(ptr(a_comp), ptr(e), ptr(sfa), ptr(q_res), ptr(sf_res), ptr(qw), ptr(sfs), ptr(sfd), (int)m,
+                                   (int)n, (int)k, (float)alpha, alpha_dev, bias ? ptr(*bias) : nullptr,
+                                   residual ? ptr(*residual) : nullptr, ptr(d), split_k ? ptr(flag) : nullptr, split_k ? 16 : 0,
+                                   static_cast<int *>(ptr(flag)), stream_of(q_res)));
   return d;
 }
 

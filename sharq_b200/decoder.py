@@ -222,6 +222,8 @@ class SharqDecoderLayer(torch.nn.Module):
             else:
                 x2 = x2 + o
                 hn = _rmsnorm(x2, self.post_norm, cfg.eps)
+            if not return_delta and self.world == 1 and self.reduce_hook is None and self.fused_glue and self.grouped_experts and hn.is_cuda:
+                return self._moe_grouped(hn, *_route(hn, self.router, cfg.top_k), residual=x2).view(b, s, h)
             d = self._moe(hn)
             if return_delta:
                 return x2.view(b, s, h), d.view(b, s, h)
@@ -232,7 +234,10 @@ class SharqDecoderLayer(torch.nn.Module):
             x2 = x2 + o
             prep = self.gate_up.prepare_input_rmsnorm(x2, self.post_norm, cfg.eps)
         if self.fused_glue:
-            d = self.down.apply_prepared_reduced(self.gate_up.apply_prepared_swiglu(prep, self.down.local))
+            prep = self.gate_up.apply_prepared_swiglu(prep, self.down.local)
+            if not return_delta and self.world == 1 and self.reduce_hook is None:
+                return self.down.local.apply_prepared(prep, residual=x2).view(b, s, h)
+            d = self.down.apply_prepared_reduced(prep)
         else:
             gu = self.gate_up.apply_prepared(prep)
             f = gu.shape[1] // 2
@@ -317,7 +322,8 @@ class SharqDecoderLayer(torch.nn.Module):
         return out
 
     @torch.no_grad()
-    def _moe_grouped(self, hn: torch.Tensor, routing: torch.Tensor, selected: torch.Tensor) -> torch.Tensor:
+    def _moe_grouped(self, hn: torch.Tensor, routing: torch.Tensor, selected: torch.Tensor,
+                     residual: torch.Tensor = None) -> torch.Tensor:
         """All experts in grouped launches with no host synchronisation (so the layer can be captured in a
         CUDA graph): the token slots are sorted by expert on the device (ATen sort / cumsum: plumbing),
         every expert's segment is padded to 256 rows, and gather -> prepare -> gate_up GEMM -> SwiGLU +
@@ -345,7 +351,7 @@ class SharqDecoderLayer(torch.nn.Module):
             p2 = ops.grouped_swiglu_sparse_residual_quantize_x(ops.linear_gemm_grouped(*p1[:5], w13, unit_group, alpha13),
                                                                unit_group, e)
         y = ops.linear_gemm_grouped(*p2[:5], w2, unit_group, (p2[5] * ws2).contiguous())
-        return ops.moe_combine(y, dest, selected.contiguous(), routing.contiguous())
+        return ops.moe_combine(y, dest, selected.contiguous(), routing.contiguous(), residual=residual)
 
     @torch.no_grad()
     def _forward_comparison_tp(self, x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:

@@ -448,10 +448,12 @@ def _check_fused_operands(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, 
 
 def sharq_linear_gemm(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense, alpha,
                       bias: Optional[torch.Tensor] = None, alpha_host: float = 1.0,
-                      out: Optional[torch.Tensor] = None, scatter=None) -> Optional[torch.Tensor]:
+                      out: Optional[torch.Tensor] = None, scatter=None,
+                      residual: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """Fused sparse-main + dense-residual GEMM on a prepared activation (one launch).
     alpha: python float or 1-element CUDA float32 tensor; the factor applied is
-    alpha * alpha_host.  out: optional contiguous bf16 [M, N] tensor to write into.
+    alpha * alpha_host.  out: optional contiguous bf16 [M, N] tensor to write into.  residual: optional bf16 [M, N]
+    tensor (16-byte aligned) added to the bf16 result, rounded as a separate add.
     scatter=(rank_ptrs, rank, world): row-parallel output under tensor parallelism; the rows are dealt to the
     collection buffers of their owner GPUs (rank_ptrs: ctypes array of their mappings, see
     sharq_linear_gemm_scatter); nothing is returned."""
@@ -460,12 +462,12 @@ def sharq_linear_gemm(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_
         return _lib.native().linear_gemm(
             A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense, alpha_t,
             float(alpha_host) if alpha_t is not None else float(alpha) * float(alpha_host), bias, out,
-            _error_flag(Q_res.device), _split_k())
+            residual, _error_flag(Q_res.device), _split_k())
     M, K = int(Q_res.shape[0]), int(Q_res.shape[1]) * 2
     N = int(QW.shape[0])
     dev = Q_res.device
     _check_fused_operands(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense)
-    _check(bias is None and out is None, "scatter mode takes neither bias nor out")
+    _check(bias is None and out is None and residual is None, "scatter mode takes neither bias, out nor residual")
     rank_ptrs, rank, world = scatter
     with _on_device(dev):
         _lib.check(_lib.lib().sharq_linear_gemm_scatter(
@@ -640,18 +642,23 @@ def moe_plan(selected: torch.Tensor, experts: int, unit: int = 256):
     return dest.view(selected.shape), src_row, unit_group
 
 
-def moe_combine(y: torch.Tensor, dest: torch.Tensor, selected: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+def moe_combine(y: torch.Tensor, dest: torch.Tensor, selected: torch.Tensor, w: torch.Tensor,
+                residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out[t] = sum over the top_k slots of token t, in ascending expert order, of y[dest[t, j]] * w[t, j] (bf16 roundings as
-    in the reference's index_add_ loop).  dest int32 [T, top_k], selected int64 [T, top_k], w bf16 [T, top_k]."""
+    in the reference's index_add_ loop).  dest int32 [T, top_k], selected int64 [T, top_k], w bf16 [T, top_k].
+    residual (optional bf16 [T, width]): added to the finished sum, rounded as a separate add."""
     T, top_k = int(selected.shape[0]), int(selected.shape[1])
     _check(y.is_cuda and y.dtype == torch.bfloat16 and y.dim() == 2 and y.is_contiguous(), "y must be a contiguous CUDA bf16 matrix")
     _check(dest.dtype == torch.int32 and dest.is_contiguous() and dest.numel() == T * top_k, "dest must be int32 [T, top_k]")
     _check(selected.dtype == torch.int64 and selected.is_contiguous(), "selected must be contiguous int64 [T, top_k]")
     _check(w.dtype == torch.bfloat16 and w.is_contiguous() and w.numel() == T * top_k, "w must be contiguous bf16 [T, top_k]")
+    if residual is not None:
+        _check(residual.is_cuda and residual.device == y.device and residual.dtype == torch.bfloat16 and residual.is_contiguous()
+               and tuple(residual.shape) == (T, int(y.shape[1])), "residual must be a contiguous CUDA bf16 matrix [T, width]")
     out = torch.empty((T, int(y.shape[1])), dtype=torch.bfloat16, device=y.device)
     with _on_device(y.device):
-        _lib.check(_lib.lib().sharq_moe_combine(_ptr(out), _ptr(y), _ptr(dest), _ptr(selected), _ptr(w), T, top_k,
-                                                int(y.shape[1]), _stream(y.device)))
+        _lib.check(_lib.lib().sharq_moe_combine_residual(_ptr(out), _ptr(y), _ptr(dest), _ptr(selected), _ptr(w), _ptr(residual), T, top_k,
+                                                         int(y.shape[1]), _stream(y.device)))
     return out
 
 

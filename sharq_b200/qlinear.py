@@ -137,10 +137,14 @@ class QLinearLayer(nn.Module):
         return ("SHARQ", a_comp, e, sfa, q_res, sf_res, scale_x)
 
     @torch.no_grad()
-    def apply_prepared(self, prepared, out=None, scatter=None):
+    def apply_prepared(self, prepared, out=None, scatter=None, residual=None):
         """out: optional bf16 [M, N] tensor the fused SharQ GEMM writes into (used by the
         tensor-parallel layers to place partial sums in symmetric memory).  scatter: see
-        ops.sharq_linear_gemm (row-parallel output dealt to the owner GPUs; returns None)."""
+        ops.sharq_linear_gemm (row-parallel output dealt to the owner GPUs; returns None).  residual: optional bf16
+        [M, N] tensor, the result is residual + output (in the epilogue of the fused SharQ GEMM, same bits)."""
+        if residual is not None and not (prepared[0] == "SHARQ" and self.fused_gemm and scatter is None and residual.is_contiguous()
+                                         and residual.dtype == torch.bfloat16 and residual.data_ptr() % 16 == 0):
+            return residual + self.apply_prepared(prepared, out=out, scatter=scatter)
         tag = prepared[0]
         if scatter is not None:
             if not (tag == "SHARQ" and self.fused_gemm and self.bias is None):
@@ -156,7 +160,7 @@ class QLinearLayer(nn.Module):
             if self.fused_gemm:
                 return ops.sharq_linear_gemm(a_comp, e, sfa, q_res, sf_res, self.weight_q, self.scale_w_sparse,
                                              self.scale_w_dense, scale_x.reshape(1), bias=self.bias,
-                                             alpha_host=self.weight_scale_host, out=out)
+                                             alpha_host=self.weight_scale_host, out=out, residual=residual)
             output_scale = (scale_x * self.weight_scale).reshape(1).contiguous()
             y_sparse = ops.sparse_matmul_tensor_scale(a_comp, self.weight_q, e, sfa, self.scale_w_sparse,
                                                       q_res.shape[0], self.out_features, self.in_features,
