@@ -210,15 +210,16 @@ int sharq_linear_gemm_ws(const void *a_comp, const void *e, const void *sfa_spar
 
 /* Fused SharQ GEMM of a merged gate_up weight [2*ffn, K] (gate rows first, ffn % 128 == 0, no bias) whose epilogue
  * applies SwiGLU: h[m, ffn] = bf16(bf16(silu(gate)) * up), gate and up rounded to bf16 first, and the bits of max|h| go to
- * amax_bits (one uint32 word, 16-byte aligned rows of h).  The same bits as sharq_linear_gemm followed by sharq_swiglu, without the [m, 2*ffn]
+ * amax_bits (sharq_gemm_swiglu_absmax_words(m, ffn) uint32 words, whose largest is the maximum; 16-byte aligned rows of h).  The same bits as sharq_linear_gemm followed by sharq_swiglu, without the [m, 2*ffn]
  * intermediate.  sharq_absmax_sparse_residual_quantize_x is sharq_scaled_sparse_residual_quantize_x for an X whose max|X|
- * is already in amax_bits (no statistics pass).  sharq_gemm_swiglu_pays: 1 where this form is the faster one. */
+ * is already in amax_bits, the largest of amax_words words (no statistics pass).  sharq_gemm_swiglu_pays: 1 where this form is the faster one. */
 int sharq_gemm_swiglu_pays(int m, int ffn, int k);
 int sharq_linear_gemm_swiglu(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res,
                              const void *qw, const void *sfw_sparse, const void *sfw_dense, int m, int ffn, int k, float alpha,
                              const float *alpha_dev, void *h, void *amax_bits, int *error_flag, void *stream);
-int sharq_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, int n, int k, const void *amax_bits, void *a_comp,
-                                            void *e, void *sfa_sparse, void *q_res, void *sf_res, float *scale_out,
+int sharq_gemm_swiglu_absmax_words(int m, int ffn);
+int sharq_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, int n, int k, const void *amax_bits, int amax_words,
+                                            void *a_comp, void *e, void *sfa_sparse, void *q_res, void *sf_res, float *scale_out,
                                             void *stream);
 
 /* sharq_linear_gemm_ws with a residual [M, N] (bf16, 16-byte aligned) added to the bf16 result in the epilogue, rounded as a

@@ -122,7 +122,7 @@ int sharq_fused_add_rmsnorm_sparse_residual_quantize_x(const void *x, const void
   SHARQ_REQUIRE(workspace && workspace_bytes >= sharq::prepare_workspace_bytes(m), "workspace too small: need %zu bytes",
                 sharq::prepare_workspace_bytes(m));
   return check_cuda(sharq::run_scaled_prepare(x, gamma, eps, m, k, workspace, nullptr, a_comp, e, sfa_sparse, q_res,
-                                              sf_res, scale_out, as_stream(stream), false, residual, sum_out),
+                                              sf_res, scale_out, as_stream(stream), 0, residual, sum_out),
                     "fused_add_rmsnorm_sparse_residual_quantize_x");
 }
 
@@ -139,14 +139,15 @@ int sharq_scaled_sparse_residual_quantize_x(const void *x, int m, int n, int k, 
                     "scaled_sparse_residual_quantize_x");
 }
 
-int sharq_absmax_sparse_residual_quantize_x(const void *x, int m, int n, int k, const void *amax_bits, void *a_comp, void *e,
-                                            void *sfa_sparse, void *q_res, void *sf_res, float *scale_out, void *stream) {
+int sharq_absmax_sparse_residual_quantize_x(const void *x, int m, int n, int k, const void *amax_bits, int amax_words,
+                                            void *a_comp, void *e, void *sfa_sparse, void *q_res, void *sf_res, float *scale_out, void *stream) {
   (void)n;
   SHARQ_REQUIRE(m > 0 && k > 0, "X must be shaped [M, K]");
   SHARQ_REQUIRE(k % 128 == 0, "absmax_sparse_residual_quantize_x requires K to be a multiple of 128, got %d", k);
+  SHARQ_REQUIRE(amax_words >= 1, "amax_words must be positive");
   SHARQ_REQUIRE(x && amax_bits && a_comp && e && sfa_sparse && q_res && sf_res, "null buffer");
   return check_cuda(sharq::run_scaled_prepare(x, nullptr, 0.0f, m, k, const_cast<void *>(amax_bits), nullptr, a_comp, e,
-                                              sfa_sparse, q_res, sf_res, scale_out, as_stream(stream), /*absmax_ready=*/true),
+                                              sfa_sparse, q_res, sf_res, scale_out, as_stream(stream), amax_words),
                     "absmax_sparse_residual_quantize_x");
 }
 
@@ -205,12 +206,14 @@ int sharq_swiglu_sparse_residual_quantize_x(const void *gate_up_bf16, int m, int
   SHARQ_REQUIRE(k % 128 == 0, "swiglu_sparse_residual_quantize_x requires K to be a multiple of 128, got %d", k);
   SHARQ_REQUIRE(gate_up_bf16 && h_bf16 && a_comp && e && sfa_sparse && q_res && sf_res, "null buffer");
   SHARQ_REQUIRE(workspace && workspace_bytes >= 256, "workspace too small: need 256 bytes");
+  int words = 1;
   if (check_cuda(sharq::run_swiglu_absmax(gate_up_bf16, m, k, 2LL * k, h_bf16, static_cast<unsigned int *>(workspace),
-                                          as_stream(stream)),
+                                          as_stream(stream), nullptr, 1,
+                                          (int)(workspace_bytes / 4 < 65536 ? workspace_bytes / 4 : 65536), &words),
                  "swiglu_absmax"))
     return 1;
   return check_cuda(sharq::run_scaled_prepare(h_bf16, nullptr, 0.0f, m, k, workspace, nullptr, a_comp, e, sfa_sparse,
-                                              q_res, sf_res, scale_out, as_stream(stream), /*absmax_ready=*/true),
+                                              q_res, sf_res, scale_out, as_stream(stream), words),
                     "swiglu_sparse_residual_quantize_x");
 }
 
@@ -666,6 +669,8 @@ int sharq_linear_gemm_residual(const void *a_comp, const void *e, const void *sf
 }
 
 int sharq_gemm_swiglu_pays(int m, int ffn, int k) { return m > 0 && ffn > 0 && k > 0 && sharq::gemm_swiglu_pays(m, ffn, k); }
+
+int sharq_gemm_swiglu_absmax_words(int m, int ffn) { return m > 0 && ffn > 0 ? sharq::gemm_swiglu_absmax_words(m, ffn) : 0; }
 
 int sharq_linear_gemm_swiglu(const void *a_comp, const void *e, const void *sfa_sparse, const void *q_res, const void *sf_res,
                              const void *qw, const void *sfw_sparse, const void *sfw_dense, int m, int ffn, int k, float alpha,

@@ -20,6 +20,7 @@
 
 #include "decoder_ops.cuh"
 #include "silu.cuh"
+#include "sm100_ptx.cuh"
 
 namespace sharq {
 
@@ -159,8 +160,9 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_kernel(const __nv_bf
   }
 }
 
-// CTA-wide maximum of a packed |value| accumulator, raised into *amax_bits (may be null).  All 256 threads call it.
-__device__ __forceinline__ void cta_absmax_to(float *warp_max, __nv_bfloat162 mx2, unsigned int *amax_bits) {
+// CTA-wide maximum of a packed |value| accumulator, raised into *amax_bits (may be null) or, with `store`, stored there.
+// All 256 threads call it.
+__device__ __forceinline__ void cta_absmax_to(float *warp_max, __nv_bfloat162 mx2, unsigned int *amax_bits, bool store = false) {
   float mx = fmaxf(__bfloat162float(mx2.x), __bfloat162float(mx2.y));
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
@@ -173,7 +175,12 @@ __device__ __forceinline__ void cta_absmax_to(float *warp_max, __nv_bfloat162 mx
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     // non-negative floats order like their bit patterns
-    if (lane == 0 && amax_bits != nullptr) atomicMax(amax_bits, __float_as_uint(mx));
+    if (lane == 0 && amax_bits != nullptr) {
+      if (store)
+        *amax_bits = __float_as_uint(mx);
+      else
+        atomicMax(amax_bits, __float_as_uint(mx));
+    }
   }
 }
 
@@ -186,8 +193,10 @@ constexpr int kSwigluPieceVecs = 512;  // two vectors for each of the 256 thread
 __global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 *__restrict__ gate_up, long long rows,
                                                             int ffn, long long row_stride, __nv_bfloat16 *__restrict__ h,
                                                             unsigned int *__restrict__ amax_bits,
-                                                            const int *__restrict__ unit_group) {
+                                                            const int *__restrict__ unit_group, bool word_per_cta) {
   __shared__ float warp_max[8];
+  ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
   const int vecs = ffn >> 3;
   __nv_bfloat162 mx2 = __floats2bfloat162_rn(0.0f, 0.0f);  // running max of |h|, two lanes
   const bool grouped = unit_group != nullptr;
@@ -236,7 +245,7 @@ __global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 
      mx2 = __floats2bfloat162_rn(0.0f, 0.0f);
    }
   }
-  if (!grouped) cta_absmax_to(warp_max, mx2, amax_bits);
+  if (!grouped) cta_absmax_to(warp_max, mx2, word_per_cta ? amax_bits + blockIdx.x : amax_bits, word_per_cta);
 }
 
 // Tensor absmax per group of a grouped bf16 activation [rows, width] (see swiglu_absmax_kernel).
@@ -503,18 +512,30 @@ cudaError_t run_add_rmsnorm(const void *x, const void *residual, void *sum_out, 
 }
 
 cudaError_t run_swiglu_absmax(const void *gate_up, long long rows, int ffn, long long row_stride, void *h,
-                              unsigned int *amax_bits, cudaStream_t stream, const int *unit_group, int groups) {
-  if (amax_bits != nullptr) {
-    cudaError_t err = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int) * (unit_group != nullptr ? groups : 1), stream);
-    if (err != cudaSuccess) return err;
-  }
+                              unsigned int *amax_bits, cudaStream_t stream, const int *unit_group, int groups, int capacity,
+                              int *words) {
   long long ctas = (long long)sm_count() * 8;
   const long long work = unit_group != nullptr ? (rows + kGroupedChunkRows - 1) / kGroupedChunkRows
                                                : rows * ((ffn / 8 + kSwigluPieceVecs - 1) / kSwigluPieceVecs);
   if (ctas > work) ctas = work;
-  swiglu_absmax_kernel<<<(unsigned)ctas, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(gate_up), rows, ffn,
-                                                            row_stride, static_cast<__nv_bfloat16 *>(h), amax_bits, unit_group);
-  return cudaGetLastError();
+  // with room for a word per CTA nothing has to be zeroed before the launch
+  const bool word_per_cta = unit_group == nullptr && ctas <= capacity;
+  if (words != nullptr) *words = word_per_cta ? (int)ctas : 1;
+  if (amax_bits != nullptr && !word_per_cta) {
+    cudaError_t err = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int) * (unit_group != nullptr ? groups : 1), stream);
+    if (err != cudaSuccess) return err;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, swiglu_absmax_kernel, static_cast<const __nv_bfloat16 *>(gate_up), rows, ffn, row_stride,
+                            static_cast<__nv_bfloat16 *>(h), amax_bits, unit_group, word_per_cta);
 }
 
 cudaError_t run_abs_stats_grouped(const void *x, long long rows, int width, unsigned int *amax_bits, const int *unit_group,

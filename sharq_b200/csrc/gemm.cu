@@ -110,6 +110,7 @@ struct GemmParams {
   int *error_flag;
   // Split K: the k_splits CTAs of a cluster compute one output tile, each over its share of the K stages.
   int k_splits;
+  int a_rows;        // rows of an activation box: the rows that exist when all are in one tile, else the tile's 128
   int staged_store;  // output tiles are transposed through shared memory for coalesced stores (N % 8 == 0)
   // Scatter mode (row-parallel linear under tensor parallelism): the output rows are dealt to their owner GPUs.
   // Row r belongs to GPU o = r / scatter_rows and is stored, through the peer mapping, into d_peer[o] at row
@@ -117,7 +118,7 @@ struct GemmParams {
   // source GPU.  scatter_rows is a multiple of 128, so a tile has one owner.  scatter_rows == 0: plain output.
   __nv_bfloat16 *d_peer[kGemmMaxPeers];
   int scatter_rows, scatter_rank;
-  unsigned int *amax_bits;  // SWIGLU: bits of max|h| are raised here (one word per group when grouped)
+  unsigned int *amax_bits;  // SWIGLU: bits of max|h|, a word per CTA; grouped: a word per group, raised
 };
 
 // Grouped launch (mixture-of-experts layers): the rows of the activation are sorted by group
@@ -280,13 +281,17 @@ __device__ __forceinline__ __nv_bfloat162 swiglu_chunk(const uint32_t *gate, con
   return mx;
 }
 
-// Warp-wide maximum raised into *amax_bits (non-negative floats order like their bit patterns); the read first keeps
-// most warps from an atomic once the maximum has settled.
-__device__ __forceinline__ void raise_absmax(unsigned int *amax_bits, __nv_bfloat162 mx2, int lane) {
+__device__ __forceinline__ float warp_max(__nv_bfloat162 mx2) {
   float mx = fmaxf(__bfloat162float(mx2.x), __bfloat162float(mx2.y));
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const unsigned int bits = __float_as_uint(mx);
+  return mx;
+}
+
+// Warp-wide maximum raised into *amax_bits (non-negative floats order like their bit patterns); the read first keeps
+// most warps from an atomic once the maximum has settled.
+__device__ __forceinline__ void raise_absmax(unsigned int *amax_bits, __nv_bfloat162 mx2, int lane) {
+  const unsigned int bits = __float_as_uint(warp_max(mx2));
   if (lane == 0 && bits > *reinterpret_cast<volatile unsigned int *>(amax_bits)) atomicMax(amax_bits, bits);
 }
 
@@ -422,7 +427,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
           uint8_t *st = smem + s * L::kStageBytes;
           const int n_sp = SPARSE ? min(2, tiles_sp - 2 * it) : 0;
           const int n_d = DENSE ? min(4, tiles_d - 4 * it) : 0;
-          uint32_t tx = L::kWBytes + L::kADenseBytes + L::kACompBytes + L::kEBytes;
+          uint32_t tx = L::kWBytes + (uint32_t)p.a_rows * ((DENSE ? 128 : 0) + (SPARSE ? 64 : 0)) + L::kEBytes;
           tx += (uint32_t)(n_sp * 512 * (1 + L::kBands) + n_d * 512 * (1 + L::kBands));
           ptx::mbar_arrive_expect_tx(full_bar + s, tx);
           ptx::tma_load_2d(st + L::kOffW, tw, it * 128, w_row, full_bar + s);
@@ -719,11 +724,21 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
           epilogue_chunk(p, &acc[32 * c], row, col_base + 32 * c, alpha, beta, has_c);
       }
     }
-    if (SWIGLU && !GROUPED) raise_absmax(p.amax_bits, h_max, lane);
+    if (SWIGLU && !GROUPED) {
+      const float mx = warp_max(h_max);
+      if (lane == 0) reinterpret_cast<float *>(smem + S * L::kStageBytes + 256)[ew] = mx;
+    }
   }
 
   ptx::tc_fence_before();
   __syncthreads();
+  if (SWIGLU && !GROUPED && threadIdx.x == 0) {
+    const float *mx = reinterpret_cast<const float *>(smem + S * L::kStageBytes + 256);  // behind the barriers
+    float cta = mx[0];
+#pragma unroll
+    for (int w = 1; w < kEpiWarps; ++w) cta = fmaxf(cta, mx[w]);
+    p.amax_bits[blockIdx.x] = __float_as_uint(cta);
+  }
   if (!PAIR && k_splits > 1) {
     ptx::cluster_sync();  // every CTA's partial tile is written
     if (threadIdx.x >= 64) {
@@ -861,11 +876,16 @@ cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
   memset(&tm_ac, 0, sizeof(tm_ac));
   if (!make_tmap_bytes(&tm_w, a.b, (uint64_t)a.n, (uint64_t)a.k / 2, L::kWRows, 128, CU_TENSOR_MAP_SWIZZLE_128B))
     return cudaErrorInvalidValue;
-  if (DENSE && !make_tmap_bytes(&tm_ad, a.a_dense, (uint64_t)a.m, (uint64_t)a.k / 2, kBM, 128, CU_TENSOR_MAP_SWIZZLE_128B))
+  // With one tile of rows only those that exist are loaded (whole 8-row groups of the swizzle): a 128-row box of a decode batch
+  // is mostly zero fill, 24 of the 67 KB that a stage writes to shared memory.  The MMA then reads stale bytes for
+  // the other rows; FP4 has no NaN, their scales are zero, and their outputs are masked.
+  const int a_rows = !PAIR && a.m < kBM ? (a.m + 7) / 8 * 8 : kBM;
+  if (DENSE && !make_tmap_bytes(&tm_ad, a.a_dense, (uint64_t)a.m, (uint64_t)a.k / 2, a_rows, 128, CU_TENSOR_MAP_SWIZZLE_128B))
     return cudaErrorInvalidValue;
-  if (SPARSE && !make_tmap_bytes(&tm_ac, a.a_comp, (uint64_t)a.m, (uint64_t)a.k / 4, kBM, 64, CU_TENSOR_MAP_SWIZZLE_64B))
+  if (SPARSE && !make_tmap_bytes(&tm_ac, a.a_comp, (uint64_t)a.m, (uint64_t)a.k / 4, a_rows, 64, CU_TENSOR_MAP_SWIZZLE_64B))
     return cudaErrorInvalidValue;
   GemmParams p{};
+  p.a_rows = a_rows;
   p.staged_store = (a.n % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.scatter_world > 1 ? a.d_peer[0] : a.d) & 15) == 0);
   p.e = static_cast<const uint8_t *>(a.e);
   p.sfa_sparse = static_cast<const uint8_t *>(a.sfa_sparse);
@@ -988,6 +1008,7 @@ static cudaError_t launch_grouped(const GroupedGemmArgs &a, cudaStream_t stream)
   if (!make_tmap_bytes(&tm_ac, a.a_comp, (uint64_t)a.m, (uint64_t)a.k / 4, kBM, 64, CU_TENSOR_MAP_SWIZZLE_64B))
     return cudaErrorInvalidValue;
   GemmParams p{};
+  p.a_rows = kBM;
   p.staged_store = (a.n % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.d) & 15) == 0);
   p.e = static_cast<const uint8_t *>(a.e);
   p.sfa_sparse = static_cast<const uint8_t *>(a.sfa_sparse);
@@ -1057,8 +1078,14 @@ cudaError_t run_gemm_swiglu(const GemmArgs &a, cudaStream_t stream) {
   if (a.a_comp == nullptr || a.a_dense == nullptr || a.bias != nullptr || a.c_in != nullptr || a.scatter_world > 1 ||
       !swiglu_ok(a.n, a.d, a.amax_bits))
     return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(a.amax_bits, 0, sizeof(unsigned int), stream);
-  return e != cudaSuccess ? e : launch<256, true, true, true, false, true>(a, stream);
+  return launch<256, true, true, true, false, true>(a, stream);
+}
+
+int gemm_swiglu_absmax_words(int m, int ffn) {
+  int dev = 0, sms = 0;
+  if (device_info(&dev, &sms) != cudaSuccess) return 0;
+  const int units = ((m + 255) / 256) * (2 * ffn / 256);
+  return 2 * (units < sms / 2 ? units : sms / 2);  // the CTAs of the launch
 }
 
 cudaError_t run_gemm(const GemmArgs &a, cudaStream_t stream) {

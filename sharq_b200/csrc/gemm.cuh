@@ -37,15 +37,16 @@ struct GemmArgs {
   // block scatter_rank.  Needs m % (128 * scatter_world) == 0 and n % 8 == 0.
   void *d_peer[kGemmMaxPeers] = {};
   int scatter_world = 0, scatter_rank = 0;
-  unsigned int *amax_bits = nullptr;  // run_gemm_swiglu only: bits of max|h|
+  unsigned int *amax_bits = nullptr;  // run_gemm_swiglu only: bits of max|h|, gemm_swiglu_absmax_words(m, ffn) words
 };
 
 cudaError_t run_gemm(const GemmArgs &args, cudaStream_t stream);
 
 // Fused SharQ GEMM of a merged gate_up weight [2F, k] (n = 2F, F % 128 == 0, no bias) whose epilogue writes
-// h = bf16(bf16(silu(gate)) * up) [m, F] to d and the bits of max|h| to *amax_bits: the bits that the plain
+// h = bf16(bf16(silu(gate)) * up) [m, F] to d and every CTA's max|h| to amax_bits (nothing to zero before the launch): the h that the plain
 // GEMM followed by the SwiGLU kernel gives.
 cudaError_t run_gemm_swiglu(const GemmArgs &args, cudaStream_t stream);
+int gemm_swiglu_absmax_words(int m, int ffn);
 
 // Whether that epilogue is the better form: where the plain GEMM would run CTA pairs.  With fewer or shorter tiles the
 // GEMM runs 128-wide (or split-K) tiles that hold no gate / up pairs, and gate_up is small enough to stay in L2.

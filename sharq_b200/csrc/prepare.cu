@@ -199,6 +199,7 @@ struct PrepareParams {
   const __nv_bfloat16 *gamma;
   const float *inv_rms;
   const unsigned int *amax_bits;
+  int amax_words;    // mode 2, one tensor: the maximum is the largest of that many words
   float *scale_out;  // optional, written by one thread (modes 1, 2)
   uint8_t *a_comp;
   uint8_t *e;
@@ -286,6 +287,16 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
       amax = mx;
     } else {
       amax = __uint_as_float(*p.amax_bits);
+      if (kMode == 2 && p.amax_words > 1) {
+        __shared__ float part_max[kWarpsPerCta];
+        for (int i = threadIdx.x; i < p.amax_words; i += kPrepareThreads) amax = fmaxf(amax, __uint_as_float(p.amax_bits[i]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+        if ((threadIdx.x & 31) == 0) part_max[threadIdx.x >> 5] = amax;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kWarpsPerCta; ++w) amax = fmaxf(amax, part_max[w]);
+      }
     }
     // ATen divides a CUDA tensor by a host scalar by multiplying with the float
     // reciprocal; clamp(min=1e-9) follows (kernels/src/bindings.cpp:337 of the reference).
@@ -960,8 +971,9 @@ int prepare_timeouts() {
 
 cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int m, int k, void *workspace,
                                float *inv_rms_external, void *a_comp, void *e, void *sfa_sparse, void *q_res,
-                               void *sf_res, float *scale_out, cudaStream_t stream, bool absmax_ready,
+                               void *sf_res, float *scale_out, cudaStream_t stream, int absmax_words,
                                const void *residual, void *sum_out) {
+  const bool absmax_ready = absmax_words > 0;
   if (residual != nullptr && (gamma == nullptr || sum_out == nullptr)) return cudaErrorInvalidValue;
   // workspace: [0,4) tensor absmax bits; [256, 256+4m) inv_rms
   auto *amax_bits = static_cast<unsigned int *>(workspace);
@@ -1042,6 +1054,7 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   p.gamma = static_cast<const __nv_bfloat16 *>(gamma);
   p.inv_rms = inv_rms;
   p.amax_bits = amax_bits;
+  p.amax_words = absmax_words;
   p.scale_out = scale_out;
   p.a_comp = static_cast<uint8_t *>(a_comp);
   p.e = static_cast<uint8_t *>(e);

@@ -168,13 +168,14 @@ std::vector<Tensor> swiglu_prepare(const Tensor &gate_up, int64_t n) {
   if (f2 % 2 != 0 || k % 128 != 0)
     fail("swiglu_sparse_residual_quantize_x requires K to be a multiple of 128, got " + std::to_string(k));
   const int64_t h_bytes = m * k * 2;
-  Prepared p(gate_up, m, k, 512 + h_bytes);
+  constexpr int64_t kWs = 8192;  // a word for the maximum of every CTA of the SwiGLU kernel
+  Prepared p(gate_up, m, k, kWs + 256 + h_bytes);
   c10::cuda::OptionalCUDAGuard guard(gate_up.device());
-  check(sharq_swiglu_sparse_residual_quantize_x(ptr(gate_up), (int)m, (int)n, (int)k, p.tail() + 512, p.tail(), 256, p.a_comp(),
+  check(sharq_swiglu_sparse_residual_quantize_x(ptr(gate_up), (int)m, (int)n, (int)k, p.tail() + kWs + 256, p.tail(), (size_t)kWs, p.a_comp(),
                                                 p.e(), p.sfa(), p.q_res(), p.sf_res(),
-                                                reinterpret_cast<float *>(p.tail() + 256), stream_of(gate_up)));
+                                                reinterpret_cast<float *>(p.tail() + kWs), stream_of(gate_up)));
   std::vector<Tensor> out = p.outputs();
-  out.push_back(p.scalar(256));
+  out.push_back(p.scalar(kWs));
   return out;
 }
 
@@ -342,8 +343,9 @@ std::vector<Tensor> linear_gemm_swiglu(const Tensor &a_comp, const Tensor &e, co
   check_u8(q_res, dev, m * (k / 2), "Q_res");
   check_u8(sf_res, dev, sf_bytes(m, k), "SF_res");
   check_weight(qw, sfs, sfd, dev, n, k);
-  Tensor h = empty_like_on(q_res, {m, n / 2}, at::kBFloat16), amax = empty_like_on(q_res, {1}, at::kInt);
   c10::cuda::OptionalCUDAGuard guard(dev);
+  Tensor h = empty_like_on(q_res, {m, n / 2}, at::kBFloat16);
+  Tensor amax = empty_like_on(q_res, {sharq_gemm_swiglu_absmax_words((int)m, (int)(n / 2))}, at::kInt);
   check(sharq_linear_gemm_swiglu(ptr(a_comp), ptr(e), ptr(sfa), ptr(q_res), ptr(sf_res), ptr(qw), ptr(sfs), ptr(sfd), (int)m,
                                  (int)(n / 2), (int)k, (float)alpha, scale_ptr(alpha_t, dev, "alpha"), ptr(h), ptr(amax),
                                  static_cast<int *>(ptr(flag)), stream_of(q_res)));
@@ -353,11 +355,12 @@ std::vector<Tensor> linear_gemm_swiglu(const Tensor &a_comp, const Tensor &e, co
 std::vector<Tensor> absmax_prepare(const Tensor &x, int64_t n, const Tensor &amax_bits) {
   check_x(x);
   check_k128("absmax_sparse_residual_quantize_x", "requires", x.size(1));
-  need(amax_bits.is_cuda() && amax_bits.device() == x.device() && amax_bits.scalar_type() == at::kInt && amax_bits.numel() == 1,
-       "amax_bits must be one CUDA int32 on X's device");
+  need(amax_bits.is_cuda() && amax_bits.device() == x.device() && amax_bits.scalar_type() == at::kInt && amax_bits.is_contiguous() &&
+           amax_bits.numel() >= 1,
+       "amax_bits must be a contiguous CUDA int32 vector on X's device");
   Prepared p(x, x.size(0), x.size(1), 256);
   c10::cuda::OptionalCUDAGuard guard(x.device());
-  check(sharq_absmax_sparse_residual_quantize_x(ptr(x), (int)p.m, (int)n, (int)p.k, ptr(amax_bits), p.a_comp(), p.e(), p.sfa(),
+  check(sharq_absmax_sparse_residual_quantize_x(ptr(x), (int)p.m, (int)n, (int)p.k, ptr(amax_bits), (int)amax_bits.numel(), p.a_comp(), p.e(), p.sfa(),
                                                 p.q_res(), p.sf_res(), reinterpret_cast<float *>(p.tail()), stream_of(x)));
   std::vector<Tensor> out = p.outputs();
   out.push_back(p.scalar(0));

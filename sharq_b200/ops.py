@@ -250,7 +250,7 @@ def swiglu_sparse_residual_quantize_x(gate_up: torch.Tensor, N: int):
 
 
 def absmax_sparse_residual_quantize_x(X: torch.Tensor, N: int, amax_bits: torch.Tensor):
-    """scaled_sparse_residual_quantize_x of an X whose max|X| is already known (amax_bits: the float's bits, as
+    """scaled_sparse_residual_quantize_x of an X whose max|X| is already known (the largest word of amax_bits holds the float's bits, as
     linear_gemm_swiglu leaves them): one launch, no statistics pass."""
     return _lib.native().absmax_prepare(X, N, amax_bits)
 
@@ -486,7 +486,7 @@ def linear_gemm_swiglu_pays(M: int, ffn: int, K: int) -> bool:
 def linear_gemm_swiglu(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense, alpha: torch.Tensor,
                        alpha_host: float = 1.0):
     """Fused SharQ GEMM of a merged gate_up weight [2F, K] (F % 128 == 0, no bias) with SwiGLU in its epilogue:
-    -> (H [M, F] bf16, amax_bits [1] int32 with the bits of max|H|); the bits of swiglu(sharq_linear_gemm(...))."""
+    -> (H [M, F] bf16, amax_bits int32, the largest word holds the bits of max|H|); the bits of swiglu(sharq_linear_gemm(...))."""
     return _lib.native().linear_gemm_swiglu(A_comp, E, SFA_sparse, Q_res, SF_res, QW, SFW_sparse, SFW_dense, alpha, alpha_host,
                                             _error_flag(Q_res.device))
 

@@ -38,7 +38,7 @@ def test_gemm_swiglu_equals_gemm_then_swiglu(m, f, k):
     h, amax = ops.linear_gemm_swiglu(*a[:5], qw, sfs, sfd, a[5].reshape(1), alpha_host=40.0 * float(scale))
     ops.check_device_errors()
     assert torch.equal(h, want)
-    assert torch.equal(amax, _amax_bits(want))
+    assert torch.equal(amax.max().reshape(1), _amax_bits(want))
     if f % 128 == 0:
         p = ops.absmax_sparse_residual_quantize_x(h, 128, amax)
         q = ops.scaled_sparse_residual_quantize_x(want, 128)
