@@ -22,6 +22,9 @@
 //   * scale value and reciprocal of the 126 possible UE4M3 codes come from a shared-memory
 //     table filled with ue4m3 -> float and the IEEE reciprocal;
 //   * e2m1 encode/decode use the hardware conversions; x - q*s is one FMA (q*s is exact);
+//   * products and the FMA on packed pairs (mul / fma.rn.f32x2), max / 6 as a product, maxima of three, the tile walk
+//     without divisions: 16384 x 18944 with known absmax 285 -> 227 us (2.9 B per element: 4.0 TB/s), 2048 x 14336
+//     31.7 -> 25.7 us, an already scaled 16384 x 4096 49.1 -> 41.2 us;
 //   * x / scale (tensor scale) is y * (1/scale) when that product is provably on the same side
 //     of every bf16 rounding boundary as the IEEE quotient, and an IEEE division otherwise.
 #include "common.cuh"
@@ -218,6 +221,7 @@ struct PrepareParams {
 };
 
 constexpr int kPrepareCtasPerSm = 3;
+constexpr int kScaledCtasPerSm = 2;  // tensor-scale mode without a gather
 // Up to the first size every CTA scans the whole input for its maximum, up to the second one cluster prepares it (us per launch at
 // K = 4096, scan / cluster / cooperative grid: 16 rows 5.9 / 6.7 / 9; 32 rows 8.1 / 6.9 / 9; 64 rows 11.8 / 8.0 / 9; 128 rows - / - / 9.0;
 // RMSNorm, cluster / cooperative grid: 16 rows 8.1 / 10.8, 64 rows 9.7 / 10.8).
@@ -319,10 +323,10 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
   uint4 next[4];
   float next_inv = 0.0f;
   bool next_row_ok = true;
-  auto issue_loads = [&](int tile) {
-    const int row = (tile / k_tiles) * kRowsPerCta + row_in_tile;
-    const int group = (tile % k_tiles) * kGroupsPerWarp + group_in_tile;
-    if (tile < total_tiles && row < m && group < groups32) {
+  auto issue_loads = [&](int row_tile, int k_tile) {
+    const int row = row_tile * kRowsPerCta + row_in_tile;
+    const int group = k_tile * kGroupsPerWarp + group_in_tile;
+    if (row < m && group < groups32) {
       int in_row = row;
       if (kMode == 2 && p.src_row != nullptr) in_row = p.src_row[row];
       next_row_ok = in_row >= 0;
@@ -334,17 +338,30 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
       if (kMode == 1) next_inv = p.inv_rms[row];
     }
   };
-  issue_loads(blockIdx.x);
+  // the tile walk and the scale offsets are advanced instead of divided out per tile (the divisions were a
+  // tenth of the instructions)
+  const int step_rows = (int)gridDim.x / k_tiles, step_k = (int)gridDim.x % k_tiles;
+  int next_row_tile = (int)blockIdx.x / k_tiles, next_k_tile = (int)blockIdx.x % k_tiles;
+  // scale offset of (row, group): 512-byte tiles of 128 rows x 4 groups, see sf_offset
+  const uint32_t sf_lane = (uint32_t)row_in_tile * 16u;  // row % 32 is row_in_tile
+  const size_t band_sp = (size_t)(groups32 >> 2) * 512, band_res = (size_t)(k >> 6) * 512;
+  issue_loads(next_row_tile, next_k_tile);
 
   for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-    const int k_tile = tile % k_tiles;
-    const int row = (tile / k_tiles) * kRowsPerCta + row_in_tile;
+    const int row_tile = next_row_tile, k_tile = next_k_tile;
+    next_row_tile += step_rows;
+    next_k_tile += step_k;
+    if (next_k_tile >= k_tiles) {
+      next_k_tile -= k_tiles;
+      ++next_row_tile;
+    }
+    const int row = row_tile * kRowsPerCta + row_in_tile;
     const int group = k_tile * kGroupsPerWarp + group_in_tile;
     const bool col_ok = group < groups32;
     bool live = row < m && col_ok;
     float t_scale = scale, t_recip = recip;
     if (kMode == 2 && p.unit_group != nullptr) {  // per-group tensor scale; a 32-row tile lies inside one 256-row unit
-      const int grp = p.unit_group[((tile / k_tiles) * kRowsPerCta) >> 8];
+      const int grp = p.unit_group[(row_tile * kRowsPerCta) >> 8];
       live = live && grp >= 0;
       t_scale = round_to_bf16(fmaxf(__fmul_rn(__uint_as_float(p.amax_bits[grp < 0 ? 0 : grp]), 1.0f / 2688.0f), 1.0e-9f));
       t_recip = __frcp_rn(t_scale);
@@ -360,7 +377,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
     }
     const float inv = next_inv;
     live = live && next_row_ok;
-    issue_loads(tile + gridDim.x);
+    issue_loads(next_row_tile, next_k_tile);
 
     GroupOut o;
     o.a_comp[0] = o.a_comp[1] = 0;
@@ -379,10 +396,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
           uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
-            const uint32_t w = xw[4 * j + t];
-            const float a = __fmul_rn(__fmul_rn(lo_f(w), inv), lo_f(gw[t]));
-            const float b = __fmul_rn(__fmul_rn(hi_f(w), inv), hi_f(gw[t]));
-            xw[4 * j + t] = pack_bf16x2(a, b);
+            xw[4 * j + t] = normalise_word(xw[4 * j + t], gw[t], pair_f32(inv, inv));
           }
         }
       }
@@ -430,10 +444,13 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
       uint32_t r2 = o.sf_res;
       uint32_t r2n = __shfl_down_sync(0xffffffffu, r2, 1);
       if (col_ok) {
+        const uint32_t at = sf_lane + (uint32_t)(row_tile & 3) * 4u;
         if ((lane & 3) == 0)
-          *reinterpret_cast<uint32_t *>(p.sfa_sparse + sf_offset(row, group, groups32)) = sv | (s1 << 8) | (s2 << 16) | (s3 << 24);
+          *reinterpret_cast<uint32_t *>(p.sfa_sparse + (size_t)(row_tile >> 2) * band_sp + (uint32_t)(group >> 2) * 512u + at) =
+              sv | (s1 << 8) | (s2 << 16) | (s3 << 24);
         if ((lane & 1) == 0)
-          *reinterpret_cast<uint32_t *>(p.sf_res + sf_offset(row, 2 * group, k / 16)) = r2 | (r2n << 16);
+          *reinterpret_cast<uint32_t *>(p.sf_res + (size_t)(row_tile >> 2) * band_res + (uint32_t)(group >> 1) * 512u + at +
+                                        (uint32_t)(group & 1) * 2u) = r2 | (r2n << 16);
       }
     }
   }
@@ -681,8 +698,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
           uint32_t y[4];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            y[q] = pack_bf16x2(__fmul_rn(__fmul_rn(lo_f(xw[q]), inv), lo_f(gw[q])),
-                               __fmul_rn(__fmul_rn(hi_f(xw[q]), inv), hi_f(gw[q])));
+            y[q] = normalise_word(xw[q], gw[q], pair_f32(inv, inv));
             m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&y[q])));
           }
           row_cache[slot] = make_uint4(y[0], y[1], y[2], y[3]);
@@ -742,9 +758,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
   for (int c = chunks - 1; c >= 0; --c) {
     const bool cached = c == chunks - 1;
     const int c_rows = chunk_size(c), c_row0 = row_begin + chunk_first_row(c);
-    for (int wt = warp; wt < c_rows * tasks_per_row; wt += kFusedWarps) {
-      const int rl = wt / tasks_per_row;
-      const int group = (wt - rl * tasks_per_row) * 32 + lane;
+    int rl = warp / tasks_per_row, piece = warp % tasks_per_row;
+    const int step_rl = kFusedWarps / tasks_per_row, step_piece = kFusedWarps % tasks_per_row;
+    for (int wt = warp; wt < c_rows * tasks_per_row; wt += kFusedWarps, rl += step_rl, piece += step_piece) {
+      if (piece >= tasks_per_row) {
+        piece -= tasks_per_row;
+        ++rl;
+      }
+      const int group = piece * 32 + lane;
       const int row = c_row0 + rl;
       const bool live = group < groups32;
       uint32_t xw[16];
@@ -790,11 +811,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
               const uint4 gv = gamma_s[cache_slot(group, j)];
               const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const uint32_t w = xw[4 * j + q];
-                xw[4 * j + q] = pack_bf16x2(__fmul_rn(__fmul_rn(lo_f(w), inv), lo_f(gw[q])),
-                                            __fmul_rn(__fmul_rn(hi_f(w), inv), hi_f(gw[q])));
-              }
+              for (int q = 0; q < 4; ++q) xw[4 * j + q] = normalise_word(xw[4 * j + q], gw[q], pair_f32(inv, inv));
             }
           }
         }
@@ -830,11 +847,12 @@ static cudaError_t current_sms(int *dev_out, int *sms_out) {
   return cudaSuccess;
 }
 
-static int prepare_grid(const PrepareParams &p) {
+// As many CTAs as are resident at once: a grid of 444 for the two-CTA kernel ran its last third at one CTA per SM.
+static int prepare_grid(const PrepareParams &p, int ctas_per_sm) {
   int dev = 0, sms = 0;
   const int tiles = ((p.k + kColsPerCta - 1) / kColsPerCta) * p.row_tiles;
   if (current_sms(&dev, &sms) != cudaSuccess) return tiles < 1024 ? tiles : 1024;
-  const int full = sms * kPrepareCtasPerSm;
+  const int full = sms * ctas_per_sm;
   return tiles < full ? tiles : full;
 }
 
@@ -843,7 +861,7 @@ static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, 
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the table set-up overlaps the kernel before
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3(prepare_grid(p));
+  cfg.gridDim = dim3(prepare_grid(p, mode == 2 && p.src_row == nullptr ? kScaledCtasPerSm : kPrepareCtasPerSm));
   cfg.blockDim = dim3(kPrepareThreads);
   cfg.stream = stream;
   cfg.attrs = attr;
@@ -863,7 +881,7 @@ static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, 
     return cudaLaunchKernelEx(&cfg, prepare_kernel<1, false>, p);
   }
   if (p.src_row != nullptr) return cudaLaunchKernelEx(&cfg, prepare_kernel<2, false>, p);
-  return cudaLaunchKernelEx(&cfg, prepare_kernel<2, false, 2>, p);
+  return cudaLaunchKernelEx(&cfg, prepare_kernel<2, false, kScaledCtasPerSm>, p);
 }
 
 cudaError_t run_prepare(const void *x, int m, int k, void *a_comp, void *e, void *q_sparse_dense,

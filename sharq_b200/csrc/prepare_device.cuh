@@ -17,6 +17,31 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
   return *reinterpret_cast<uint32_t *>(&v);
 }
 
+// Two floats in a 64-bit register pair and the packed operations on them: one instruction for both lanes, each lane
+// rounded as the scalar operation rounds (the kernels are bound by instruction issue).
+__device__ __forceinline__ uint64_t pair_f32(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpair_f32(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// both bf16 values of a word times the pair b
+__device__ __forceinline__ float2 mul_word(uint32_t w, uint64_t b) { return unpair_f32(mul_f32x2(pair_f32(lo_f(w), hi_f(w)), b)); }
+
 // ---------------------------------------------------------------------------
 // The 32-element group: selection, sparse quantisation, residual quantisation.
 // ---------------------------------------------------------------------------
@@ -49,8 +74,20 @@ __device__ __forceinline__ void decode_e2m1x8(uint32_t word, uint32_t (&h)[4]) {
       : "r"(word));
 }
 
+// The group scale code of max / 6.  The product with float(1/6) stands in for the quotient: both give the same code
+// for every float of at most 13 significant bits (an exact multiple of 6 by a short value is hit exactly, every other such
+// float is further from a code boundary than the product's error), and the maximum is a bf16 value or
+// a residual x - q * s of at most 11 bits (x and q * s are multiples of 2^-9 of the power of two of s where q != 0, and the
+// residual is below 2 s; where q == 0 it is x).  A NaN stays one.
 __device__ __forceinline__ uint32_t scale_code_from_max(float mx) {
-  return float_to_ue4m3(clamp_val(__fdiv_rn(mx, kFp4Max), kScaleEps, kFp8Max));
+  return float_to_ue4m3(clamp_val(__fmul_rn(mx, 1.0f / 6.0f), kScaleEps, kFp8Max));
+}
+
+// max of three in one instruction; NaN operands are dropped as fmaxf drops them
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
 }
 
 template <bool kDebug>
@@ -62,8 +99,8 @@ __device__ __forceinline__ void quantize_group32(const uint32_t (&xw)[16], const
     x[2 * i + 1] = hi_f(xw[i]);
   }
 
-  // -- pair selection per 8-element chunk on integer keys
-  uint32_t lo_idx[4], hi_idx[4];
+  // -- pair selection per 8-element chunk on integer keys; of the selected pairs what is kept is 3 - index (the low key bits)
+  uint32_t near_pair[4], far_pair[4];  // 3 - index: the later pair has the smaller value
   uint32_t max_key = 0;
   uint32_t meta = 0;
   uint32_t second_min = 0xFFFFFFFFu;
@@ -77,14 +114,14 @@ __device__ __forceinline__ void quantize_group32(const uint32_t (&xw)[16], const
     const uint32_t m23 = max(key[2], key[3]), n23 = min(key[2], key[3]);
     const uint32_t best = max(m01, m23);
     const uint32_t second = max(min(m01, m23), max(n01, n23));
-    const uint32_t ib = 3u - (best & 3u), is = 3u - (second & 3u);
-    lo_idx[c] = min(ib, is);
-    hi_idx[c] = max(ib, is);
-    meta |= (lo_idx[c] | (hi_idx[c] << 2)) << (4 * c);
+    const uint32_t ib = best & 3u, is = second & 3u;
+    near_pair[c] = max(ib, is);
+    far_pair[c] = min(ib, is);
+    meta |= (near_pair[c] | (far_pair[c] << 2)) << (4 * c);
     max_key = max(max_key, best);
     second_min = min(second_min, second - 4u);  // an all-zero pair (key < 4) wraps to a huge value
   }
-  o.meta = meta;
+  o.meta = meta ^ 0xFFFFu;  // index = 3 - kept value, in every two-bit field
   o.second_min = second_min;
 
   // -- sparse main path scale (one UE4M3 per 32 logical elements)
@@ -95,13 +132,18 @@ __device__ __forceinline__ void quantize_group32(const uint32_t (&xw)[16], const
 
   // -- quantise every pair, mask to the selected ones, form the residual
   float r[32];
+  const uint64_t s_r2 = pair_f32(s_r, s_r), neg_s2 = pair_f32(-s_q, -s_q);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    const uint32_t all4 = pack_e2m1x8(__fmul_rn(x[8 * c + 0], s_r), __fmul_rn(x[8 * c + 1], s_r),
-                                      __fmul_rn(x[8 * c + 2], s_r), __fmul_rn(x[8 * c + 3], s_r),
-                                      __fmul_rn(x[8 * c + 4], s_r), __fmul_rn(x[8 * c + 5], s_r),
-                                      __fmul_rn(x[8 * c + 6], s_r), __fmul_rn(x[8 * c + 7], s_r));
-    const uint32_t mask4 = (0xFFu << (8 * lo_idx[c])) | (0xFFu << (8 * hi_idx[c]));
+    uint64_t xp[4];
+    float2 t[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      xp[p] = pair_f32(x[8 * c + 2 * p], x[8 * c + 2 * p + 1]);
+      t[p] = unpair_f32(mul_f32x2(xp[p], s_r2));
+    }
+    const uint32_t all4 = pack_e2m1x8(t[0].x, t[0].y, t[1].x, t[1].y, t[2].x, t[2].y, t[3].x, t[3].y);
+    const uint32_t mask4 = (0xFF000000u >> (8 * near_pair[c])) | (0xFF000000u >> (8 * far_pair[c]));
     const uint32_t dense4 = all4 & mask4;  // dropped pairs become +0,+0: their residual is x itself
     if (kDebug) o.q_sparse[c] = dense4;
     uint32_t h[4];
@@ -110,11 +152,12 @@ __device__ __forceinline__ void quantize_group32(const uint32_t (&xw)[16], const
     for (int p = 0; p < 4; ++p) {
       const float2 q = __half22float2(*reinterpret_cast<__half2 *>(&h[p]));
       // q * s_q is exact (2-bit x 4-bit significands), so the FMA rounds once like x - (q*s)
-      r[8 * c + 2 * p] = __fmaf_rn(-q.x, s_q, x[8 * c + 2 * p]);
-      r[8 * c + 2 * p + 1] = __fmaf_rn(-q.y, s_q, x[8 * c + 2 * p + 1]);
+      const float2 d = unpair_f32(fma_f32x2(pair_f32(q.x, q.y), neg_s2, xp[p]));
+      r[8 * c + 2 * p] = d.x;
+      r[8 * c + 2 * p + 1] = d.y;
     }
     // the two kept pair-bytes, ascending pair order
-    const uint32_t two = __byte_perm(dense4, 0u, lo_idx[c] | (hi_idx[c] << 4) | 0x4400u);
+    const uint32_t two = __byte_perm(dense4, 0u, 0x4433u - near_pair[c] - (far_pair[c] << 4));
     if (c & 1)
       o.a_comp[c >> 1] |= two << 16;
     else
@@ -127,16 +170,17 @@ __device__ __forceinline__ void quantize_group32(const uint32_t (&xw)[16], const
   for (int h = 0; h < 2; ++h) {
     float mx = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) mx = fmaxf(mx, fabsf(r[16 * h + i]));
+    for (int i = 0; i < 16; i += 2) mx = max3(mx, fabsf(r[16 * h + i]), fabsf(r[16 * h + i + 1]));
     const uint32_t code = scale_code_from_max(mx);
-    const float rr = tbl.recip[code];
+    const uint64_t rr2 = pair_f32(tbl.recip[code], tbl.recip[code]);
     sf_res |= code << (8 * h);
 #pragma unroll
     for (int wv = 0; wv < 2; ++wv) {
       const int i = 16 * h + 8 * wv;
-      o.q_res[2 * h + wv] =
-          pack_e2m1x8(__fmul_rn(r[i + 0], rr), __fmul_rn(r[i + 1], rr), __fmul_rn(r[i + 2], rr), __fmul_rn(r[i + 3], rr),
-                      __fmul_rn(r[i + 4], rr), __fmul_rn(r[i + 5], rr), __fmul_rn(r[i + 6], rr), __fmul_rn(r[i + 7], rr));
+      float2 t[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) t[p] = unpair_f32(mul_f32x2(pair_f32(r[i + 2 * p], r[i + 2 * p + 1]), rr2));
+      o.q_res[2 * h + wv] = pack_e2m1x8(t[0].x, t[0].y, t[1].x, t[1].y, t[2].x, t[2].y, t[3].x, t[3].y);
     }
   }
   o.sf_res = sf_res;
@@ -153,12 +197,13 @@ __device__ __forceinline__ void quantize_group32(const uint32_t (&xw)[16], const
 __device__ __forceinline__ void scale_group32(uint32_t (&w)[16], float scale, float recip) {
   uint32_t out[16];
   uint32_t nearest = 0xFFFFFFFFu;
+  const uint64_t recip2 = pair_f32(recip, recip);
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    const float qa = __fmul_rn(lo_f(w[i]), recip), qb = __fmul_rn(hi_f(w[i]), recip);
-    const uint32_t lows = __byte_perm(__float_as_uint(qa), __float_as_uint(qb), 0x5410);
+    const float2 q = mul_word(w[i], recip2);
+    const uint32_t lows = __byte_perm(__float_as_uint(q.x), __float_as_uint(q.y), 0x5410);
     nearest = __vminu2(nearest, lows + 0x80048004u);
-    out[i] = pack_bf16x2(qa, qb);
+    out[i] = pack_bf16x2(q.x, q.y);
   }
   if ((nearest & 0xFFFFu) < 10u || (nearest >> 16) < 10u) {
     // Some product of this group is close to a rounding boundary (exact ties are common when
@@ -194,6 +239,12 @@ __device__ __forceinline__ void scale_group32(uint32_t (&w)[16], float scale, fl
 // A selected pair whose score is non-zero but below 2^-118 (key = float bits | pair index).
 constexpr uint32_t kTinyKey = 0x04800000u - 4u;
 
+// RMSNorm of both bf16 values of a word: bf16((x * inv) * gamma)
+__device__ __forceinline__ uint32_t normalise_word(uint32_t x, uint32_t gamma, uint64_t inv2) {
+  const float2 y = unpair_f32(mul_f32x2(mul_f32x2(pair_f32(lo_f(x), hi_f(x)), inv2), pair_f32(lo_f(gamma), hi_f(gamma))));
+  return pack_bf16x2(y.x, y.y);
+}
+
 // float(bf16(x)): the divisor of the non-RMSNorm path.  On a CUDA device `x / scale` with a bf16
 // tensor x and a 0-dim float32 tensor scale (model/quantize.py:179-183 of the reference) casts
 // the scale to the common dtype bf16 before dividing in float.
@@ -222,7 +273,10 @@ __device__ __forceinline__ void scale_quantize_group(uint32_t (&y)[16], float di
     for (int attempt = 0; attempt < 2; ++attempt) {
       if (attempt == 0) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) y[i] = pack_bf16x2(__fmul_rn(lo_f(y[i]), recip), __fmul_rn(hi_f(y[i]), recip));
+        for (int i = 0; i < 16; ++i) {
+          const float2 q = mul_word(y[i], pair_f32(recip, recip));
+          y[i] = pack_bf16x2(q.x, q.y);
+        }
       } else {
         reload(y);
 #pragma unroll
