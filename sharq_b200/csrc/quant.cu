@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256) compress_sparse_a_kernel(const uint8_t *_
 // reduces them again in every CTA and walks the matrix from its END, so that the last ~100 MB launch 1
 // read come from L2.  As ATen passes (abs, max, float, divide, clamp, divide, cast) and a
 // quantisation kernel this took 668 us at 28672 x 4096, of which 442 us were ATen's division by a
-// 0-dim tensor; now 102 us (absmax 37 us = 6.4 TB/s, quantisation 65 us), and 85 -> 16 us at 1000 x 14336
+// 0-dim tensor; now about 96 us (absmax 37 us = 6.4 TB/s, quantisation 59 us), and 85 -> 16 us at 1000 x 14336
 // (dense).
 //
 // Arithmetic: dividing a bf16 CUDA tensor by a 0-dim float32 tensor casts the divisor to bf16 first, so
@@ -217,7 +217,7 @@ __device__ __forceinline__ void zero_scale_padding(int n, int k, uint8_t *sf_spa
 // The groups of a row are a multiple of 4, so four neighbouring lanes' scale bytes form a 32-bit word of
 // the blocked layout: gathered by shuffles and stored once.
 template <bool kShared>
-__global__ void __launch_bounds__(kScaledThreads) scaled_quantize_kernel(const uint4 *__restrict__ x, int rows, int k,
+__global__ void __launch_bounds__(kScaledThreads, kShared ? 4 : 6) scaled_quantize_kernel(const uint4 *__restrict__ x, int rows, int k,
                                                                          const float *__restrict__ partials, int n_partials,
                                                                          uint8_t *__restrict__ q,
                                                                          uint8_t *__restrict__ sf, uint8_t *__restrict__ sf2,
@@ -243,7 +243,10 @@ __global__ void __launch_bounds__(kScaledThreads) scaled_quantize_kernel(const u
   for (long long c = chunks - 1 - blockIdx.x; c >= 0; c -= gridDim.x) {
     const long long idx = c * kScaledThreads + threadIdx.x;
     const bool live = idx < total;
-    const int row = live ? (int)(idx / groups) : 0, g = live ? (int)(idx - (long long)row * groups) : 0;
+    // a 32-bit division where it will do: the 64-bit one costs a third of the group's instructions
+    int row = 0;
+    if (live) row = total <= 0xffffffffLL ? (int)((uint32_t)idx / (uint32_t)groups) : (int)(idx / groups);
+    const int g = live ? (int)(idx - (long long)row * groups) : 0;
     uint32_t code = 0;
     if (live) {
       float v[8 * kVecs];
@@ -322,7 +325,7 @@ cudaError_t run_scaled_quantize(const void *x, int rows, int k, bool shared, flo
   if (parts > cap) parts = cap;
   absmax_partials_kernel<<<(unsigned)parts, kScaledThreads, 0, stream>>>(static_cast<const uint4 *>(x), n16, partials);
   const long long chunks = ((long long)rows * (k / (shared ? 32 : 16)) + kScaledThreads - 1) / kScaledThreads;
-  const long long full = 6LL * sms;
+  const long long full = (shared ? 4LL : 6LL) * sms;  // the CTAs that are resident at once
   const unsigned grid = (unsigned)(chunks < full ? chunks : full);
   if (shared)
     scaled_quantize_kernel<true><<<grid, kScaledThreads, 0, stream>>>(
