@@ -200,6 +200,10 @@ size_t sharq_gemm_workspace_bytes(int m, int n);
 int sharq_matmul_ws(const void *a, const void *b, const void *sfa, const void *sfb, int m, int n, int k, float alpha,
                     const float *alpha_dev, const void *c_in, float beta, void *d, void *workspace,
                     size_t workspace_bytes, int *error_flag, void *stream);
+/* sharq_matmul_ws with a bias [N] (bf16) added to the bf16 result, rounded as a separate bf16 add would. */
+int sharq_matmul_bias_ws(const void *a, const void *b, const void *sfa, const void *sfb, int m, int n, int k, float alpha,
+                         const float *alpha_dev, const void *c_in, float beta, const void *bias_bf16, void *d, void *workspace,
+                         size_t workspace_bytes, int *error_flag, void *stream);
 int sharq_sparse_matmul_ws(const void *a_comp, const void *b, const void *e, const void *sfa, const void *sfb, int m,
                            int n, int k, float alpha, const float *alpha_dev, float beta, void *d, void *workspace,
                            size_t workspace_bytes, int *error_flag, void *stream);

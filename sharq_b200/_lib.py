@@ -51,6 +51,8 @@ SIGNATURES = {
         c_int, [_P, _P, _P, _P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, _P, _P, _P]),
     "sharq_gemm_workspace_bytes": (c_size_t, [c_int, c_int]),
     "sharq_matmul_ws": (c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, c_float, _P, _P, c_size_t, _P, _P]),
+    "sharq_matmul_bias_ws": (
+        c_int, [_P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, _P, c_float, _P, _P, _P, c_size_t, _P, _P]),
     "sharq_sparse_matmul_ws": (
         c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, c_float, _P, c_float, _P, _P, c_size_t, _P, _P]),
     "sharq_linear_gemm_ws": (

@@ -562,6 +562,13 @@ int sharq_matmul(const void *a, const void *b, const void *sfa, const void *sfb,
 int sharq_matmul_ws(const void *a, const void *b, const void *sfa, const void *sfb, int m, int n, int k, float alpha,
                     const float *alpha_dev, const void *c_in, float beta, void *d, void *workspace,
                     size_t workspace_bytes, int *error_flag, void *stream) {
+  return sharq_matmul_bias_ws(a, b, sfa, sfb, m, n, k, alpha, alpha_dev, c_in, beta, nullptr, d, workspace, workspace_bytes,
+                              error_flag, stream);
+}
+
+int sharq_matmul_bias_ws(const void *a, const void *b, const void *sfa, const void *sfb, int m, int n, int k, float alpha,
+                         const float *alpha_dev, const void *c_in, float beta, const void *bias, void *d, void *workspace,
+                         size_t workspace_bytes, int *error_flag, void *stream) {
   SHARQ_REQUIRE(m > 0 && n > 0 && k > 0, "M, N, K must be positive");
   SHARQ_REQUIRE(k % 64 == 0, "matmul requires K to be a multiple of 64, got %d", k);
   SHARQ_REQUIRE(a && b && sfa && sfb && d && error_flag, "null buffer");
@@ -572,6 +579,7 @@ int sharq_matmul_ws(const void *a, const void *b, const void *sfa, const void *s
   g.b = b;
   g.sfb_dense = sfb;
   g.c_in = c_in;
+  g.bias = bias;
   g.d = d;
   g.alpha = alpha;
   g.alpha_ptr = alpha_dev;

@@ -263,16 +263,17 @@ Tensor linear_forward(const Tensor &x, const Tensor &qw, const Tensor &sfs, cons
 
 Tensor dense_gemm(const Tensor &a, const Tensor &b, const Tensor &sfa, const Tensor &sfb, double alpha,
                   const std::optional<Tensor> &alpha_t, const std::optional<Tensor> &c_in, double beta,
-                  const std::optional<Tensor> &out, const Tensor &flag, bool split_k) {
+                  const std::optional<Tensor> &bias, const std::optional<Tensor> &out, const Tensor &flag, bool split_k) {
   need(a.is_cuda() && b.is_cuda() && sfa.is_cuda() && sfb.is_cuda(), "A, B, SFA and SFB must be CUDA tensors");
   const int64_t m = a.size(0), n = b.size(0), k = a.size(1) * 2;
   const at::Device dev = a.device();
+  check_bias(bias, n);
   Tensor d = output(a, m, n, out);
   const float *alpha_dev = alpha_t ? scale_ptr(*alpha_t, dev, "scale") : nullptr;
   c10::cuda::OptionalCUDAGuard guard(dev);
-  check(sharq_matmul_ws(ptr(a), ptr(b), ptr(sfa), ptr(sfb), (int)m, (int)n, (int)k, (float)alpha, alpha_dev,
-                        c_in ? ptr(*c_in) : nullptr, (float)beta, ptr(d), split_k ? ptr(flag) : nullptr, split_k ? 16 : 0,
-                        static_cast<int *>(ptr(flag)), stream_of(a)));
+  check(sharq_matmul_bias_ws(ptr(a), ptr(b), ptr(sfa), ptr(sfb), (int)m, (int)n, (int)k, (float)alpha, alpha_dev,
+                             c_in ? ptr(*c_in) : nullptr, (float)beta, bias ? ptr(*bias) : nullptr, ptr(d),
+                             split_k ? ptr(flag) : nullptr, split_k ? 16 : 0, static_cast<int *>(ptr(flag)), stream_of(a)));
   return d;
 }
 

@@ -383,8 +383,8 @@ def _split_k() -> bool:
     return os.environ.get("SHARQ_GEMM_SPLIT_K", "1") != "0"
 
 
-def _dense_gemm(A, B, SFA, SFB, alpha, alpha_t, C_in, beta, out=None):
-    return _lib.native().dense_gemm(A, B, SFA, SFB, alpha, alpha_t, C_in, beta, out, _error_flag(A.device), _split_k())
+def _dense_gemm(A, B, SFA, SFB, alpha, alpha_t, C_in, beta, out=None, bias=None):
+    return _lib.native().dense_gemm(A, B, SFA, SFB, alpha, alpha_t, C_in, beta, bias, out, _error_flag(A.device), _split_k())
 
 
 def _check_c_in(C_in, A, M, N):
@@ -402,9 +402,11 @@ def matmul(A, B, SFA, SFB, scale: float):
     return _dense_gemm(A, B, SFA, SFB, scale, None, None, 0.0)
 
 
-def matmul_tensor_scale(A, B, SFA, SFB, scale: torch.Tensor, out: Optional[torch.Tensor] = None):
-    """out (not in the reference's op): optional bf16 [M, N] tensor to write into."""
-    return _dense_gemm(A, B, SFA, SFB, 1.0, scale, None, 0.0, out=out)
+def matmul_tensor_scale(A, B, SFA, SFB, scale: torch.Tensor, out: Optional[torch.Tensor] = None,
+                        bias: Optional[torch.Tensor] = None):
+    """Not in the reference's op: out, an optional bf16 [M, N] tensor to write into; bias, an optional bf16 [N] tensor
+    added to the bf16 result, rounded as a separate add."""
+    return _dense_gemm(A, B, SFA, SFB, 1.0, scale, None, 0.0, out=out, bias=bias)
 
 
 def matmul_accum(A, B, SFA, SFB, scale: float, C_in, beta: float = 1.0):
@@ -413,9 +415,11 @@ def matmul_accum(A, B, SFA, SFB, scale: float, C_in, beta: float = 1.0):
     return _dense_gemm(A, B, SFA, SFB, scale, None, C_in, beta)
 
 
-def matmul_accum_tensor_scale(A, B, SFA, SFB, scale: torch.Tensor, C_in, beta: float = 1.0):
+def matmul_accum_tensor_scale(A, B, SFA, SFB, scale: torch.Tensor, C_in, beta: float = 1.0,
+                              bias: Optional[torch.Tensor] = None):
+    """bias: see matmul_tensor_scale."""
     _check_c_in(C_in, A, int(A.shape[0]), int(B.shape[0]))
-    return _dense_gemm(A, B, SFA, SFB, 1.0, scale, C_in, beta)
+    return _dense_gemm(A, B, SFA, SFB, 1.0, scale, C_in, beta, bias=bias)
 
 
 def _sparse_gemm(name, A_comp, B, E, SFA, SFB, M, N, K, alpha, alpha_t, beta):

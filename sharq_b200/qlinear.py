@@ -6,7 +6,7 @@ argument meaning and tuple formats, so layer wrappers written against the refere
 (one prepared activation shared by q/k/v or by gate/up) work unchanged.  With
 fused_gemm=True (default) apply_prepared runs the single-launch sparse+residual GEMM with
 the bias folded into its epilogue; with fused_gemm=False it issues the reference's two
-GEMM calls (sparse, then dense with beta=1) and a separate bias add.
+GEMM calls (sparse, then dense with beta=1; the bias add rides in the second's epilogue, rounded as a separate add).
 
 The reference's pure-PyTorch simulation modes (SHARQ_SIM, HIF4_SIM, ...) are accuracy
 tools, not part of the accelerated path; they are not provided here.
@@ -166,19 +166,17 @@ class QLinearLayer(nn.Module):
                                                       q_res.shape[0], self.out_features, self.in_features,
                                                       alpha=output_scale)
             if self.extra_fusion:
-                y = ops.matmul_accum_tensor_scale(q_res, self.weight_q, sf_res, self.scale_w_dense, output_scale,
-                                                  y_sparse, 1.0)
+                return ops.matmul_accum_tensor_scale(q_res, self.weight_q, sf_res, self.scale_w_dense, output_scale,
+                                                     y_sparse, 1.0, bias=self.bias)
             else:
                 y = y_sparse + ops.matmul_tensor_scale(q_res, self.weight_q, sf_res, self.scale_w_dense, output_scale)
         elif tag == "NVFP4":
             _, qx, scale_x, scale = prepared
-            y = ops.matmul_tensor_scale(qx, self.weight_q, scale_x, self.scale_w,
-                                        (scale * self.weight_scale).reshape(1).contiguous(), out=out)
+            return ops.matmul_tensor_scale(qx, self.weight_q, scale_x, self.scale_w,
+                                           (scale * self.weight_scale).reshape(1).contiguous(), out=out, bias=self.bias)
         else:
             raise ValueError(f"Unsupported prepared input tag: {tag}")
-        if self.bias is not None:
-            y = y + self.bias
-        return y
+        return y if self.bias is None else y + self.bias
 
     @torch.no_grad()
     def apply_prepared_swiglu(self, prepared, down: "QLinearLayer"):
