@@ -9,7 +9,9 @@
 // The kernels that take an already scaled input are written for clarity: one thread per scale
 // group, 16-byte loads and stores.
 #include "common.cuh"
+#include "prepare_device.cuh"
 #include "quant.cuh"
+#include "sm100_ptx.cuh"
 
 namespace sharq {
 
@@ -149,8 +151,8 @@ __global__ void __launch_bounds__(256) compress_sparse_a_kernel(const uint8_t *_
 // reduces them again in every CTA and walks the matrix from its END, so that the last ~100 MB launch 1
 // read come from L2.  As ATen passes (abs, max, float, divide, clamp, divide, cast) and a
 // quantisation kernel this took 668 us at 28672 x 4096, of which 442 us were ATen's division by a
-// 0-dim tensor; now about 96 us (absmax 37 us = 6.4 TB/s, quantisation 59 us), and 85 -> 16 us at 1000 x 14336
-// (dense).
+// 0-dim tensor; now about 90 us (absmax 37 us = 6.4 TB/s, quantisation 53 us; 102 us with 64-bit index divisions, IEEE divisions and
+// unpacked products, and a gap between the launches), and 85 -> 13 us at 1000 x 14336 (dense).
 //
 // Arithmetic: dividing a bf16 CUDA tensor by a 0-dim float32 tensor casts the divisor to bf16 first, so
 // y = bf16(x / float(bf16(scale))).  Quotients of two 8-bit significands are either representable
@@ -181,6 +183,8 @@ __device__ __forceinline__ float block_max_nan(float mx, float *warp_max) {
 __global__ void __launch_bounds__(kScaledThreads) absmax_partials_kernel(const uint4 *__restrict__ x, size_t n16,
                                                                          float *__restrict__ partials) {
   __shared__ float warp_max[kScaledThreads / 32];
+  ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
   __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
   const size_t stride = (size_t)gridDim.x * kScaledThreads;
   for (size_t i = (size_t)blockIdx.x * kScaledThreads + threadIdx.x; i < n16; i += 4 * stride) {
@@ -224,6 +228,8 @@ __global__ void __launch_bounds__(kScaledThreads, kShared ? 4 : 6) scaled_quanti
                                                                          float *__restrict__ scale_out) {
   constexpr int kVecs = kShared ? 4 : 2;  // 16-byte vectors of a group
   __shared__ float warp_max[kScaledThreads / 32];
+  ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
   if (kShared) zero_scale_padding(rows, k, sf, sf2);
   float mx = 0.0f;
   for (int i = threadIdx.x; i < n_partials; i += kScaledThreads) {
@@ -249,23 +255,32 @@ __global__ void __launch_bounds__(kScaledThreads, kShared ? 4 : 6) scaled_quanti
     const int g = live ? (int)(idx - (long long)row * groups) : 0;
     uint32_t code = 0;
     if (live) {
-      float v[8 * kVecs];
+      uint32_t w[4 * kVecs];
 #pragma unroll
-      for (int j = 0; j < kVecs; ++j) unpack8(__ldg(x + idx * kVecs + j), v + 8 * j);
-      float gm = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 8 * kVecs; ++i) {
-        v[i] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(v[i], recip)));
-        gm = fmaxf(gm, fabsf(v[i]));
+      for (int j = 0; j < kVecs; ++j) {
+        const uint4 t = __ldg(x + idx * kVecs + j);
+        w[4 * j] = t.x, w[4 * j + 1] = t.y, w[4 * j + 2] = t.z, w[4 * j + 3] = t.w;
       }
-      code = float_to_ue4m3(clamp_val(__fdiv_rn(gm, kFp4Max), kScaleEps, kFp8Max));
+      float gm = 0.0f;
+      const uint64_t recip2 = prep::pair_f32(recip, recip);
+#pragma unroll
+      for (int i = 0; i < 4 * kVecs; ++i) {
+        const float2 y = prep::unpair_f32(prep::mul_f32x2(prep::pair_f32(prep::lo_f(w[i]), prep::hi_f(w[i])), recip2));
+        w[i] = prep::pack_bf16x2(y.x, y.y);
+        gm = prep::max3(gm, fabsf(prep::lo_f(w[i])), fabsf(prep::hi_f(w[i])));
+      }
+      code = prep::scale_code_from_max(gm);
       const float inv = __frcp_rn(ue4m3_to_float(code));
+      const uint64_t inv2 = prep::pair_f32(inv, inv);
       uint32_t o[kVecs];
 #pragma unroll
-      for (int j = 0; j < kVecs; ++j)
-        o[j] = pack_e2m1x8(__fmul_rn(v[8 * j + 0], inv), __fmul_rn(v[8 * j + 1], inv), __fmul_rn(v[8 * j + 2], inv),
-                           __fmul_rn(v[8 * j + 3], inv), __fmul_rn(v[8 * j + 4], inv), __fmul_rn(v[8 * j + 5], inv),
-                           __fmul_rn(v[8 * j + 6], inv), __fmul_rn(v[8 * j + 7], inv));
+      for (int j = 0; j < kVecs; ++j) {
+        float2 t[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          t[i] = prep::unpair_f32(prep::mul_f32x2(prep::pair_f32(prep::lo_f(w[4 * j + i]), prep::hi_f(w[4 * j + i])), inv2));
+        o[j] = pack_e2m1x8(t[0].x, t[0].y, t[1].x, t[1].y, t[2].x, t[2].y, t[3].x, t[3].y);
+      }
       uint8_t *dst = q + (size_t)idx * (4 * kVecs);
       if (kShared)
         *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[kVecs - 1]);
@@ -323,19 +338,24 @@ cudaError_t run_scaled_quantize(const void *x, int rows, int k, bool shared, flo
   size_t parts = (n16 + 4 * kScaledThreads - 1) / (4 * kScaledThreads);
   const size_t cap = (size_t)6 * sms < (size_t)kScaledQuantPartials ? (size_t)6 * sms : (size_t)kScaledQuantPartials;
   if (parts > cap) parts = cap;
-  absmax_partials_kernel<<<(unsigned)parts, kScaledThreads, 0, stream>>>(static_cast<const uint4 *>(x), n16, partials);
+  // both launches may start while the kernel before them drains
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)parts);
+  cfg.blockDim = dim3(kScaledThreads);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const auto *xv = static_cast<const uint4 *>(x);
+  if ((err = cudaLaunchKernelEx(&cfg, absmax_partials_kernel, xv, n16, partials)) != cudaSuccess) return err;
   const long long chunks = ((long long)rows * (k / (shared ? 32 : 16)) + kScaledThreads - 1) / kScaledThreads;
   const long long full = (shared ? 4LL : 6LL) * sms;  // the CTAs that are resident at once
-  const unsigned grid = (unsigned)(chunks < full ? chunks : full);
-  if (shared)
-    scaled_quantize_kernel<true><<<grid, kScaledThreads, 0, stream>>>(
-        static_cast<const uint4 *>(x), rows, k, partials, (int)parts, static_cast<uint8_t *>(q), static_cast<uint8_t *>(sf),
-        static_cast<uint8_t *>(sf2), scale_out);
-  else
-    scaled_quantize_kernel<false><<<grid, kScaledThreads, 0, stream>>>(
-        static_cast<const uint4 *>(x), rows, k, partials, (int)parts, static_cast<uint8_t *>(q), static_cast<uint8_t *>(sf),
-        nullptr, scale_out);
-  return cudaGetLastError();
+  cfg.gridDim = dim3((unsigned)(chunks < full ? chunks : full));
+  return cudaLaunchKernelEx(&cfg, shared ? scaled_quantize_kernel<true> : scaled_quantize_kernel<false>, xv, rows, k,
+                            static_cast<const float *>(partials), (int)parts, static_cast<uint8_t *>(q),
+                            static_cast<uint8_t *>(sf), static_cast<uint8_t *>(sf2), scale_out);
 }
 
 cudaError_t run_compress_sparse_a(const void *a_dense, int m, int k, void *a_comp, void *e, cudaStream_t stream) {
