@@ -155,6 +155,8 @@ class QLinearLayer(nn.Module):
                                          scatter=scatter)
         if out is not None and not ((tag == "SHARQ" and self.fused_gemm) or (tag == "NVFP4" and self.bias is None)):
             raise ValueError("out= is only supported by the fused SharQ GEMM and the bias-free dense NVFP4 GEMM")
+        # a bias of another type (the module was cast) is added by torch
+        folded = self.bias if self.bias is not None and self.bias.dtype == torch.bfloat16 else None
         if tag == "SHARQ":
             _, a_comp, e, sfa, q_res, sf_res, scale_x = prepared
             if self.fused_gemm:
@@ -166,14 +168,16 @@ class QLinearLayer(nn.Module):
                                                       q_res.shape[0], self.out_features, self.in_features,
                                                       alpha=output_scale)
             if self.extra_fusion:
-                return ops.matmul_accum_tensor_scale(q_res, self.weight_q, sf_res, self.scale_w_dense, output_scale,
-                                                     y_sparse, 1.0, bias=self.bias)
+                y = ops.matmul_accum_tensor_scale(q_res, self.weight_q, sf_res, self.scale_w_dense, output_scale,
+                                                  y_sparse, 1.0, bias=folded)
+                return y if folded is self.bias else y + self.bias
             else:
                 y = y_sparse + ops.matmul_tensor_scale(q_res, self.weight_q, sf_res, self.scale_w_dense, output_scale)
         elif tag == "NVFP4":
             _, qx, scale_x, scale = prepared
-            return ops.matmul_tensor_scale(qx, self.weight_q, scale_x, self.scale_w,
-                                           (scale * self.weight_scale).reshape(1).contiguous(), out=out, bias=self.bias)
+            y = ops.matmul_tensor_scale(qx, self.weight_q, scale_x, self.scale_w,
+                                        (scale * self.weight_scale).reshape(1).contiguous(), out=out, bias=folded)
+            return y if folded is self.bias else y + self.bias
         else:
             raise ValueError(f"Unsupported prepared input tag: {tag}")
         return y if self.bias is None else y + self.bias
