@@ -615,9 +615,9 @@ def run_ours(args):
         "e2e": {"value": round(e2e_value, 2), "unit": UNIT, "h2d_bytes_per_step": h2d_bytes,
                 "d2h_bytes_per_step": d2h_bytes, "ms_per_step": round(ms_e2e, 4),
                 "pipeline": "copies on a second stream, double-buffered: H2D of step i+1 and D2H of step i overlap kernels"},
-        # per layer: 4 GEMMs, 2 scaled prepares, 2 RMSNorm prepares / transition kernels (replicated
-        # residual stream: 4 prepares and 2 all-reduce kernels)
-        "gpu_launches": args.steps * layers_n * (8 if (world == 1 or sp is not None) else 10),
+        # per layer: 4 GEMMs, 2 scaled prepares (statistics and quantisation launch), 2 RMSNorm prepares with the residual
+        # add / transition kernels (replicated residual stream: 2 all-reduce kernels more)
+        "gpu_launches": args.steps * layers_n * (10 if (world == 1 or sp is not None) else 12),
         "clocks": clocks,
     }
     if tp_check is not None:

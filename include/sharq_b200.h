@@ -59,6 +59,8 @@ int sharq_fused_sparse_residual_quantize_x_debug(const void *x_bf16, int m, int 
  * bytes [0,4) tensor absmax (float bits), bytes [4,8) arrival counter of the grid-wide barrier,
  * bytes [256, 256+4*M) per-row inv_rms (float).  The calls initialise what they use. */
 size_t sharq_prepare_workspace_bytes(int m);
+/* With this many bytes the prepares of some sizes save a memset between their launches. */
+size_t sharq_prepare_workspace_best_bytes(int m);
 
 /* The scaled prepare calls run statistics and quantisation in ONE cooperative launch whose CTAs
  * meet at a grid-wide barrier with a bounded wait (about one second).  Returns how many such

@@ -90,6 +90,8 @@ int sharq_fused_sparse_residual_quantize_x_debug(const void *x, int m, int n, in
 
 size_t sharq_prepare_workspace_bytes(int m) { return sharq::prepare_workspace_bytes(m); }
 
+size_t sharq_prepare_workspace_best_bytes(int m) { return m > 0 ? sharq::prepare_workspace_best_bytes(m) : 0; }
+
 int sharq_prepare_timeouts(void) { return sharq::prepare_timeouts(); }
 
 int sharq_fused_rmsnorm_sparse_residual_quantize_x(const void *x, const void *gamma, float eps, int m, int n, int k,
@@ -105,7 +107,7 @@ int sharq_fused_rmsnorm_sparse_residual_quantize_x(const void *x, const void *ga
   SHARQ_REQUIRE(workspace && workspace_bytes >= sharq::prepare_workspace_bytes(m), "workspace too small: need %zu bytes",
                 sharq::prepare_workspace_bytes(m));
   return check_cuda(sharq::run_scaled_prepare(x, gamma, eps, m, k, workspace, nullptr, a_comp, e, sfa_sparse, q_res,
-                                              sf_res, scale_out, as_stream(stream)),
+                                              sf_res, scale_out, as_stream(stream), 0, nullptr, nullptr, workspace_bytes),
                     "fused_rmsnorm_sparse_residual_quantize_x");
 }
 
@@ -122,7 +124,7 @@ int sharq_fused_add_rmsnorm_sparse_residual_quantize_x(const void *x, const void
   SHARQ_REQUIRE(workspace && workspace_bytes >= sharq::prepare_workspace_bytes(m), "workspace too small: need %zu bytes",
                 sharq::prepare_workspace_bytes(m));
   return check_cuda(sharq::run_scaled_prepare(x, gamma, eps, m, k, workspace, nullptr, a_comp, e, sfa_sparse, q_res,
-                                              sf_res, scale_out, as_stream(stream), 0, residual, sum_out),
+                                              sf_res, scale_out, as_stream(stream), 0, residual, sum_out, workspace_bytes),
                     "fused_add_rmsnorm_sparse_residual_quantize_x");
 }
 
@@ -135,7 +137,7 @@ int sharq_scaled_sparse_residual_quantize_x(const void *x, int m, int n, int k, 
   SHARQ_REQUIRE(x && a_comp && e && sfa_sparse && q_res && sf_res, "null buffer");
   SHARQ_REQUIRE(workspace && workspace_bytes >= 256, "workspace too small: need 256 bytes");
   return check_cuda(sharq::run_scaled_prepare(x, nullptr, 0.0f, m, k, workspace, nullptr, a_comp, e, sfa_sparse, q_res,
-                                              sf_res, scale_out, as_stream(stream)),
+                                              sf_res, scale_out, as_stream(stream), 0, nullptr, nullptr, workspace_bytes),
                     "scaled_sparse_residual_quantize_x");
 }
 

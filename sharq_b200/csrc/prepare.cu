@@ -54,6 +54,14 @@ __device__ __forceinline__ void raise_amax(unsigned int *amax_bits, float mx) {
   if (bits > *reinterpret_cast<volatile unsigned int *>(amax_bits)) atomicMax(amax_bits, bits);
 }
 
+// The maximum of a CTA: into the CTA's own word (nothing has to be zeroed before the launch) or raised into the first.
+__device__ __forceinline__ void publish_amax(unsigned int *amax_bits, float mx, bool word_per_cta) {
+  if (word_per_cta)
+    amax_bits[blockIdx.x] = __float_as_uint(mx);
+  else
+    raise_amax(amax_bits, mx);
+}
+
 // ---------------------------------------------------------------------------
 // Row statistics for the RMSNorm path, one CTA per row, one thread per 32-element group:
 //   inv_rms[r] = rsqrtf(sum(x^2)/K + eps) with the reference's summation order (each group
@@ -69,7 +77,9 @@ __global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 
                                                           __nv_bfloat16 *__restrict__ sum_out,
                                                           const __nv_bfloat16 *__restrict__ gamma, float eps, int k,
                                                           float *__restrict__ inv_rms,
-                                                          unsigned int *__restrict__ amax_bits) {
+                                                          unsigned int *__restrict__ amax_bits, bool word_per_cta) {
+  ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
   extern __shared__ float partial[];  // [k/32] group sums, then [0] is reused for inv_rms
   __shared__ float warp_max[32];
   const int groups = k >> 5;
@@ -112,7 +122,8 @@ __global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 
   __syncthreads();
   if (threadIdx.x == 0) {
     float total = 0.0f;
-    for (int i = 0; i < groups; i += 4) {  // groups is a multiple of 4 (K % 128 == 0)
+#pragma unroll 8
+    for (int i = 0; i < groups; i += 4) {  // groups is a multiple of 4 (K % 128 == 0); the loads run ahead of the chain
       float4 v = *reinterpret_cast<const float4 *>(partial + i);
       total = __fadd_rn(total, v.x);
       total = __fadd_rn(total, v.y);
@@ -152,13 +163,15 @@ __global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 
     mx = lane < nwarps ? warp_max[lane] : 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) raise_amax(amax_bits, mx);
+    if (lane == 0) publish_amax(amax_bits, mx, word_per_cta);
   }
 }
 
 // Tensor-wide max |x| of a bf16 tensor (non-RMSNorm path): flat grid-stride reduction.
 __global__ void __launch_bounds__(256) abs_stats_kernel(const __nv_bfloat16 *__restrict__ x, size_t n16,
-                                                         unsigned int *__restrict__ amax_bits) {
+                                                         unsigned int *__restrict__ amax_bits, bool word_per_cta) {
+  ptx::grid_launch_dependents();
+  ptx::grid_dependency_wait();
   __shared__ float warp_max[8];
   __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
   const uint4 *src = reinterpret_cast<const uint4 *>(x);
@@ -185,7 +198,7 @@ __global__ void __launch_bounds__(256) abs_stats_kernel(const __nv_bfloat16 *__r
     mx = lane < 8 ? warp_max[lane] : 0.0f;
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0) raise_amax(amax_bits, mx);
+    if (lane == 0) publish_amax(amax_bits, mx, word_per_cta);
   }
 }
 
@@ -202,7 +215,8 @@ struct PrepareParams {
   const __nv_bfloat16 *gamma;
   const float *inv_rms;
   const unsigned int *amax_bits;
-  int amax_words;    // mode 2, one tensor: the maximum is the largest of that many words
+  unsigned int *amax_out;  // optional: the bits of the maximum
+  int amax_words;    // one tensor: the maximum is the largest of that many words
   float *scale_out;  // optional, written by one thread (modes 1, 2)
   uint8_t *a_comp;
   uint8_t *e;
@@ -222,11 +236,10 @@ struct PrepareParams {
 
 constexpr int kPrepareCtasPerSm = 3;
 constexpr int kScaledCtasPerSm = 2;  // tensor-scale mode without a gather
-// Up to the first size every CTA scans the whole input for its maximum, up to the second one cluster prepares it (us per launch at
-// K = 4096, scan / cluster / cooperative grid: 16 rows 5.9 / 6.7 / 9; 32 rows 8.1 / 6.9 / 9; 64 rows 11.8 / 8.0 / 9; 128 rows - / - / 9.0;
-// RMSNorm, cluster / cooperative grid: 16 rows 8.1 / 10.8, 64 rows 9.7 / 10.8).
+// Up to this size every CTA scans the whole input for its maximum (us per launch at K = 4096, scan / statistics launch and
+// prepare: 16 rows 5.3 / 5.6, 32 rows 8.1 / 5.3).
 constexpr size_t kInlineAbsmaxElements = 64 * 1024;
-constexpr size_t kClusterElements = 256 * 1024;
+constexpr unsigned kMaxAbsmaxWords = 4096;            // words of CTA maxima that every prepare CTA reduces
 
 // kCtas: resident CTAs per SM the register allocation aims at.  The tensor-scale mode runs
 // fastest with two (no spills) except on a gathered activation (src_row), where the third CTA
@@ -291,7 +304,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
       amax = mx;
     } else {
       amax = __uint_as_float(*p.amax_bits);
-      if (kMode == 2 && p.amax_words > 1) {
+      if (p.amax_words > 1) {
         __shared__ float part_max[kWarpsPerCta];
         for (int i = threadIdx.x; i < p.amax_words; i += kPrepareThreads) amax = fmaxf(amax, __uint_as_float(p.amax_bits[i]));
 #pragma unroll
@@ -306,6 +319,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
     // reciprocal; clamp(min=1e-9) follows (kernels/src/bindings.cpp:337 of the reference).
     scale = fmaxf(__fmul_rn(amax, 1.0f / 2688.0f), 1.0e-9f);
     if (p.scale_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *p.scale_out = scale;
+    if (p.amax_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *p.amax_out = __float_as_uint(amax);
     if (kMode == 2 && p.unit_group != nullptr && blockIdx.x == 0 && (int)threadIdx.x < p.groups)
       p.scale_vec_out[threadIdx.x] = fmaxf(__fmul_rn(__uint_as_float(p.amax_bits[threadIdx.x]), 1.0f / 2688.0f), 1.0e-9f);
     if (kMode == 2) scale = round_to_bf16(scale);  // the divisor of the non-RMSNorm path, see round_to_bf16
@@ -519,11 +533,7 @@ __device__ __forceinline__ void store_group(const FusedParams &p, const GroupOut
   }
 }
 
-//
-// kCluster: the same kernel as one thread-block cluster for small inputs (decode steps).  The tensor absmax goes
-// through distributed shared memory and a cluster barrier, so nothing has to be zeroed before the launch, and the other SMs are free for
-// the CTAs of the GEMM that follows, which start early and fetch their weights meanwhile.
-template <int kMode, bool kAdd, int kFusedThreads, bool kCluster>
+template <int kMode, bool kAdd, int kFusedThreads>
 __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const FusedParams p) {
   static_assert(kMode == 1 || kMode == 2, "modes with a statistics pass");
   constexpr int kFusedWarps = kFusedThreads / 32;
@@ -537,7 +547,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
 
   __shared__ ScaleTables tbl;
   __shared__ float warp_red[32];
-  __shared__ float cta_amax;  // kCluster
   extern __shared__ uint4 fused_smem[];
   uint4 *gamma_s = fused_smem;                                      // mode 1: k bf16, pieces permuted like the cache
   uint4 *cache = fused_smem + (kMode == 1 ? row_vecs : 0);          // chunk_rows x k bf16
@@ -717,35 +726,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int w = 1; w < kFusedWarps; ++w) mx = fmaxf(mx, warp_red[w]);
-      if (kCluster) {
-        cta_amax = mx;
-      } else {
-        if (mx > 0.0f) atomicMax(p.amax_bits, __float_as_uint(mx));
-        __threadfence();
-        atomicAdd(p.arrive, 1u);
-        const long long t0 = clock64();
-        while (ld_acquire_gpu(p.arrive) < gridDim.x) {
-          if (clock64() - t0 > kGridBarrierLimitCycles) {
-            atomicAdd(&g_prepare_timeouts, 1);
-            break;
-          }
+      if (mx > 0.0f) atomicMax(p.amax_bits, __float_as_uint(mx));
+      __threadfence();
+      atomicAdd(p.arrive, 1u);
+      const long long t0 = clock64();
+      while (ld_acquire_gpu(p.arrive) < gridDim.x) {
+        if (clock64() - t0 > kGridBarrierLimitCycles) {
+          atomicAdd(&g_prepare_timeouts, 1);
+          break;
         }
       }
     }
     __syncthreads();
   }
-  float amax = 0.0f;
-  if (kCluster) {
-    ptx::cluster_sync();
-    const uint32_t at = ptx::smem_u32(&cta_amax);
-    if (lane < (int)gridDim.x) amax = ptx::ld_cluster_f32(at, lane);  // at most 16 CTAs, one per lane
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    ptx::cluster_arrive();  // the wait is at the end: no CTA leaves while another may still read its maximum
-    if (blockIdx.x == 0 && threadIdx.x == 0) *p.amax_bits = __float_as_uint(amax);
-  } else {
-    amax = __uint_as_float(ld_acquire_gpu(p.amax_bits));
-  }
+  const float amax = __uint_as_float(ld_acquire_gpu(p.amax_bits));
   // ATen divides a CUDA tensor by a host scalar by multiplying with the float
   // reciprocal; clamp(min=1e-9) follows (kernels/src/bindings.cpp:337 of the reference).
   const float scale = fmaxf(__fmul_rn(amax, 1.0f / 2688.0f), 1.0e-9f);
@@ -820,10 +814,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
       store_group(p, o, row, group, live, group < groups_padded, aligned_m, lane);
     }
   }
-  if (kCluster) {
-    __syncwarp();
-    ptx::cluster_wait();
-  }
 }
 
 }  // namespace
@@ -833,6 +823,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
 // ---------------------------------------------------------------------------
 
 size_t prepare_workspace_bytes(int m) { return 256 + (size_t)m * sizeof(float); }
+
+size_t prepare_workspace_best_bytes(int m) { return prepare_workspace_bytes(m) + kMaxAbsmaxWords * sizeof(float); }
 
 // SM count of the current device (queried once per device).
 static cudaError_t current_sms(int *dev_out, int *sms_out) {
@@ -900,77 +892,49 @@ cudaError_t run_prepare(const void *x, int m, int k, void *a_comp, void *e, void
   return launch_prepare(0, q_sparse_dense != nullptr, p, stream);
 }
 
-// One launch for statistics + prepare (see prepare_fused_kernel): a cooperative grid over all SMs, or one cluster.
-// Returns cudaErrorNotSupported when the shape does not fit or the device cannot launch it, in which
-// case the caller falls back to the other forms.
+// One cooperative launch for statistics + prepare (see prepare_fused_kernel).  Returns
+// cudaErrorNotSupported when the shape does not fit or the device cannot launch it, in which
+// case the caller falls back to the separate statistics and prepare kernels.
 // 512 threads per CTA: measured against 448, 768 and 896 (more threads spill or idle in the
 // partly filled last round of 56 warp tasks per CTA at 2048 x 4096)
-template <int kMode, bool kAdd, bool kCluster>
+template <int kMode, bool kAdd>
 static cudaError_t launch_fused(const FusedParams &p_in, cudaStream_t stream) {
   constexpr int kThreads = 512;
   static bool attr_set[64] = {};
-  static int usable[64] = {};  // 0 unknown, else the CTAs of the launch, -1 no
+  static int coop[64] = {};  // 0 unknown, 1 yes, -1 no
   int dev = 0, sms = 0;
   cudaError_t e = current_sms(&dev, &sms);
   if (e != cudaSuccess) return e;
-  auto kernel = prepare_fused_kernel<kMode, kAdd, kThreads, kCluster>;
-  if (!attr_set[dev]) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedSmemBudget + 16);
-    if (e == cudaSuccess && kCluster) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
+  if (coop[dev] == 0) {
+    int v = 0;
+    coop[dev] = (cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && v) ? 1 : -1;
   }
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
-  cfg.blockDim = dim3(kThreads);
-  cfg.stream = stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (kCluster) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    for (int c = 16; usable[dev] == 0; c /= 2) {
-      attr[0].val.clusterDim.x = (unsigned)c;
-      cfg.gridDim = dim3((unsigned)c);
-      cfg.dynamicSmemBytes = kFusedSmemBudget + 16;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) (void)cudaGetLastError();
-      if (n > 0 || c == 4) usable[dev] = n > 0 ? c : -1;
-    }
-  } else {
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    if (usable[dev] == 0) {
-      int v = 0;
-      usable[dev] = (cudaDeviceGetAttribute(&v, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && v) ? sms : -1;
-    }
-  }
-  if (usable[dev] < 0) return cudaErrorNotSupported;
-  const int ctas = usable[dev];
+  if (coop[dev] < 0) return cudaErrorNotSupported;
   FusedParams p = p_in;
   const int groups32 = p.k / 32;
-  p.rows_per_cta = (p.m + ctas - 1) / ctas;
+  p.rows_per_cta = (p.m + sms - 1) / sms;
   const size_t row_bytes = (size_t)p.k * 2 + (kMode == 1 ? (size_t)(groups32 + 4) * 4 : 0);
   const size_t fixed = (kMode == 1 ? (size_t)p.k * 2 + (size_t)p.rows_per_cta * 4 : 0);
   if (fixed + row_bytes > (size_t)kFusedSmemBudget) return cudaErrorNotSupported;
   const size_t capacity = ((size_t)kFusedSmemBudget - fixed) / row_bytes;
   p.chunk_rows = (int)(capacity < (size_t)p.rows_per_cta ? capacity : (size_t)p.rows_per_cta);
-  cfg.gridDim = dim3((unsigned)ctas);
-  cfg.dynamicSmemBytes = fixed + (size_t)p.chunk_rows * row_bytes + 16;
-  if (kCluster) {
-    attr[0].val.clusterDim.x = (unsigned)ctas;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.numAttrs = 2;
+  auto kernel = prepare_fused_kernel<kMode, kAdd, kThreads>;
+  if (!attr_set[dev]) {
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFusedSmemBudget + 16);
+    if (e != cudaSuccess) return e;
+    attr_set[dev] = true;
   }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.gridDim = dim3(sms);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = fixed + (size_t)p.chunk_rows * row_bytes + 16;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, p);
-}
-
-template <bool kCluster>
-static cudaError_t launch_fused_mode(const FusedParams &p, bool rms, cudaStream_t stream) {
-  if (!rms) return launch_fused<2, false, kCluster>(p, stream);
-  return p.residual != nullptr ? launch_fused<1, true, kCluster>(p, stream) : launch_fused<1, false, kCluster>(p, stream);
 }
 
 static bool fused_prepare_enabled() {
@@ -990,7 +954,7 @@ int prepare_timeouts() {
 cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int m, int k, void *workspace,
                                float *inv_rms_external, void *a_comp, void *e, void *sfa_sparse, void *q_res,
                                void *sf_res, float *scale_out, cudaStream_t stream, int absmax_words,
-                               const void *residual, void *sum_out) {
+                               const void *residual, void *sum_out, size_t workspace_bytes) {
   const bool absmax_ready = absmax_words > 0;
   if (residual != nullptr && (gamma == nullptr || sum_out == nullptr)) return cudaErrorInvalidValue;
   // workspace: [0,4) tensor absmax bits; [256, 256+4m) inv_rms
@@ -1002,13 +966,23 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   // a small non-RMSNorm input (a decode step): the prepare kernel finds max|x| itself
   const bool inline_absmax = !rms && !absmax_ready && (size_t)m * k <= kInlineAbsmaxElements;
   const size_t elements = (size_t)m * (size_t)k;
-  const bool one_cluster = !absmax_ready && elements <= kClusterElements && (rms || elements > kInlineAbsmaxElements);
-  // One cooperative launch pays while the per-SM row caches hold most of the tensor; beyond that
-  // the separate statistics and prepare kernels (more resident warps per SM) are faster.  Measured
-  // crossovers (us, one launch / separate): RMSNorm 4096 x 4096 35.0 / 37.0, 8192 x 4096
-  // 65.7 / 63.8, 16384 x 4096 136 / 118; tensor scale 2048 x 7168 24.9 / 25.0, 4096 x 4096 28.7 / 27.0.
-  const bool one_launch_pays = elements < (rms ? ((size_t)1 << 25) : ((size_t)1 << 24));
-  if (!absmax_ready && !inline_absmax && (one_launch_pays || one_cluster) && fused_prepare_enabled()) {
+  // statistics kernel: one CTA per row (RMSNorm) or a flat grid; its CTAs' maxima go behind the row statistics, where the
+  // caller's workspace has room for a word each
+  int dev = 0, sms = 0;
+  if (current_sms(&dev, &sms) != cudaSuccess) sms = 128;
+  const size_t flat = ((size_t)m * k / 8 + 255) / 256;
+  const unsigned stat_ctas = rms ? (unsigned)m : (unsigned)(flat < (size_t)sms * 8 ? flat : (size_t)sms * 8);
+  const size_t words_at = 256 + (rms && inv_rms_external == nullptr ? (size_t)m * sizeof(float) : 0);
+  const bool word_per_cta = stat_ctas <= kMaxAbsmaxWords && workspace_bytes >= words_at + (size_t)stat_ctas * sizeof(float);
+  // Two launches that overlap, with nothing to zero, beat one cooperative launch behind its memset (us, two launches / one: tensor scale
+  // 64 x 4096 5.3 / 8.7, 2048 x 4096 12.0 / 16.9, 4096 x 4096 19.6 / 27.1; RMSNorm 32 x 4096 7.4 / 10.5, 512 x 4096 9.8 / 12.9, 4096 x 4096
+  // 30.1 / 33.5), except with the residual add on middle sizes, where the row caches spare the second read of the sum: 512 x 4096
+  // 12.2 / 14.4, 2048 x 4096 27.3 / 25.2, 4096 x 4096 51.0 / 49.8.  Without room for the words the memset precedes both forms, and
+  // one launch pays while the row caches hold most of the tensor.
+  const bool one_launch_pays =
+      fused_prepare_enabled() && (word_per_cta ? residual != nullptr && elements >= ((size_t)1 << 22) && elements < ((size_t)1 << 25)
+                                               : elements < (rms ? ((size_t)1 << 25) : ((size_t)1 << 24)));
+  if (!absmax_ready && !inline_absmax && one_launch_pays) {
     FusedParams f{};
     f.x = static_cast<const __nv_bfloat16 *>(x);
     f.residual = static_cast<const __nv_bfloat16 *>(residual);
@@ -1026,53 +1000,60 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
     f.sf_res = static_cast<uint8_t *>(sf_res);
     f.m = m;
     f.k = k;
-    if (one_cluster) {
-      if ((err = launch_fused_mode<true>(f, rms, stream)) == cudaSuccess) return cudaSuccess;
-      (void)cudaGetLastError();
-    }
     if ((err = cudaMemsetAsync(amax_bits, 0, 2 * sizeof(unsigned int), stream)) != cudaSuccess) return err;
-    if ((err = launch_fused_mode<false>(f, rms, stream)) == cudaSuccess) return cudaSuccess;
+    err = !rms ? launch_fused<2, false>(f, stream)
+               : (residual != nullptr ? launch_fused<1, true>(f, stream) : launch_fused<1, false>(f, stream));
+    if (err == cudaSuccess) return cudaSuccess;
     (void)cudaGetLastError();  // not launchable here: the separate kernels below do the same work
     if (err != cudaErrorNotSupported && err != cudaErrorCooperativeLaunchTooLarge) return err;
     err = cudaSuccess;
   }
+  int words = absmax_words;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const auto *xb = static_cast<const __nv_bfloat16 *>(x);
   if (absmax_ready) {
     // the producer of x already left max|x| in the workspace: no statistics pass
     if (rms) return cudaErrorInvalidValue;
   } else if (inline_absmax) {
     amax_bits = nullptr;
-  } else if ((err = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int), stream)) != cudaSuccess) {
-    return err;
-  } else if (rms) {
+  } else {
     const int groups = k / 32;
-    const int threads = (groups + 31) / 32 * 32;
-    if (residual != nullptr) {
-      rms_stats_kernel<true><<<m, threads, (size_t)groups * sizeof(float), stream>>>(
-          static_cast<const __nv_bfloat16 *>(x), static_cast<const __nv_bfloat16 *>(residual),
-          static_cast<__nv_bfloat16 *>(sum_out), static_cast<const __nv_bfloat16 *>(gamma), eps, k, inv_rms, amax_bits);
+    cfg.gridDim = dim3(stat_ctas);
+    cfg.blockDim = dim3(rms ? (unsigned)((groups + 31) / 32 * 32) : 256u);
+    cfg.dynamicSmemBytes = rms ? (size_t)groups * sizeof(float) : 0;
+    if (word_per_cta) {
+      amax_bits = reinterpret_cast<unsigned int *>(static_cast<uint8_t *>(workspace) + words_at);
+      words = (int)stat_ctas;
+    } else if ((err = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int), stream)) != cudaSuccess) {
+      return err;
+    }
+    const auto *g = static_cast<const __nv_bfloat16 *>(gamma);
+    if (!rms) {
+      err = cudaLaunchKernelEx(&cfg, abs_stats_kernel, xb, (size_t)m * k / 8, amax_bits, word_per_cta);
+    } else if (residual != nullptr) {
+      err = cudaLaunchKernelEx(&cfg, rms_stats_kernel<true>, xb, static_cast<const __nv_bfloat16 *>(residual),
+                               static_cast<__nv_bfloat16 *>(sum_out), g, eps, k, inv_rms, amax_bits, word_per_cta);
       x = sum_out;  // the prepare reads the sum
     } else {
-      rms_stats_kernel<false><<<m, threads, (size_t)groups * sizeof(float), stream>>>(
-          static_cast<const __nv_bfloat16 *>(x), nullptr, nullptr, static_cast<const __nv_bfloat16 *>(gamma), eps, k,
-          inv_rms, amax_bits);
+      err = cudaLaunchKernelEx(&cfg, rms_stats_kernel<false>, xb, static_cast<const __nv_bfloat16 *>(nullptr),
+                               static_cast<__nv_bfloat16 *>(nullptr), g, eps, k, inv_rms, amax_bits, word_per_cta);
     }
-  } else {
-    const size_t n16 = (size_t)m * k / 8;
-    size_t blocks = (n16 + 255) / 256;
-    int dev = 0, sms = 0;
-    if (current_sms(&dev, &sms) != cudaSuccess) sms = 128;
-    if (blocks > (size_t)sms * 8) blocks = (size_t)sms * 8;
-    abs_stats_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16 *>(x), n16, amax_bits);
+    if (err != cudaSuccess) return err;
   }
-  err = cudaGetLastError();
-  if (err != cudaSuccess) return err;
 
   PrepareParams p{};
   p.x = static_cast<const __nv_bfloat16 *>(x);
   p.gamma = static_cast<const __nv_bfloat16 *>(gamma);
   p.inv_rms = inv_rms;
   p.amax_bits = amax_bits;
-  p.amax_words = absmax_words;
+  p.amax_words = words;
+  p.amax_out = word_per_cta && !absmax_ready && !inline_absmax ? static_cast<unsigned int *>(workspace) : nullptr;
   p.scale_out = scale_out;
   p.a_comp = static_cast<uint8_t *>(a_comp);
   p.e = static_cast<uint8_t *>(e);

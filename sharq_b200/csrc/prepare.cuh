@@ -9,6 +9,9 @@ namespace sharq {
 // [0,4) tensor absmax bits, [4,8) grid barrier counter, [256, 256 + 4*M) per-row inv_rms.
 size_t prepare_workspace_bytes(int m);
 
+// With that many bytes nothing has to be zeroed between the launches.
+size_t prepare_workspace_best_bytes(int m);
+
 // Prepare of an already scaled bf16 activation [m,k].  With q_sparse_dense != nullptr
 // the debug variant runs (dense sparse payload instead of a_comp/e).
 cudaError_t run_prepare(const void *x, int m, int k, void *a_comp, void *e, void *q_sparse_dense,
@@ -19,10 +22,11 @@ cudaError_t run_prepare(const void *x, int m, int k, void *a_comp, void *e, void
 // the workspace slot.  With absmax_words > 0 (gamma == nullptr only) the workspace already
 // holds the bits of max|x|, the largest of that many words, and the statistics pass is skipped.  With residual (RMSNorm path
 // only) the input is bf16(x + residual), which the statistics kernel also writes to sum_out.
+// workspace_bytes beyond the minimum hold the maxima of the statistics kernel's CTAs (prepare_workspace_best_bytes).
 cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int m, int k, void *workspace,
                                float *inv_rms_external, void *a_comp, void *e, void *sfa_sparse, void *q_res,
                                void *sf_res, float *scale_out, cudaStream_t stream, int absmax_words = 0,
-                               const void *residual = nullptr, void *sum_out = nullptr);
+                               const void *residual = nullptr, void *sum_out = nullptr, size_t workspace_bytes = 0);
 
 // Tensor-scale prepare of a grouped activation (mixture-of-experts layers): rows sorted by group in
 // 256-row units (m a multiple of 256), unit_group[u] < 0 = unit without rows (its outputs are

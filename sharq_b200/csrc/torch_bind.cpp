@@ -104,8 +104,8 @@ struct Scaled {
   Tensor total;
 
   Scaled(const Tensor &x, const std::optional<Tensor> &gamma, double eps, int64_t n, const std::optional<Tensor> &residual)
-      : p(x, x.size(0), x.size(1), round256(256 + 4 * x.size(0)) + 256) {
-    ws_bytes = 256 + 4 * p.m;
+      : p(x, x.size(0), x.size(1), round256((int64_t)sharq_prepare_workspace_best_bytes((int)x.size(0))) + 256) {
+    ws_bytes = (int64_t)sharq_prepare_workspace_best_bytes((int)p.m);
     scale_at = round256(ws_bytes);
     const int m = (int)p.m, k = (int)p.k;
     c10::cuda::OptionalCUDAGuard guard(x.device());
@@ -158,7 +158,7 @@ std::vector<Tensor> scaled_prepare(const Tensor &x, const std::optional<Tensor> 
   if (residual)
     out.push_back(s.total);
   else if (return_workspace)
-    out.push_back(s.p.view(s.p.o_tail, s.ws_bytes));
+    out.push_back(s.p.view(s.p.o_tail, 256 + 4 * s.p.m));
   return out;
 }
 

@@ -1,34 +1,70 @@
-"""Launches for few rows: the prepare as one thread-block cluster, and split-K GEMMs whose CTAs sum their partial tiles
-through distributed shared memory."""
+"""Launches for few rows: the prepare as a statistics launch that leaves a maximum per CTA and a quantisation launch that
+overlap, and split-K GEMMs whose CTAs sum their partial tiles through distributed shared memory."""
+import ctypes
+
+import numpy as np
 import pytest
 import torch
 
 from tests import helpers as H
-from tests import test_prepare_gpu as prepare
+from tests.test_prepare_gpu import _compare
 
 pytestmark = pytest.mark.gpu
 
 
-# one row per CTA, one more than the CTAs, the largest input of the form, the longest row, the next size up
-@pytest.mark.parametrize("m,k", [(1, 4096), (16, 4096), (17, 4096), (64, 4096), (8, 32768), (65, 4096)])
-def test_small_rmsnorm_prepare_matches_oracle(oracle, m, k):
-    prepare.test_rmsnorm_prepare_matches_oracle(oracle, m, k)
+def _prepare(m, k, x, gamma, eps=1e-6):
+    """The scaled (RMSNorm) prepare with the workspace that takes the two overlapping launches -> outputs, absmax, scale, inv_rms."""
+    from sharq_b200 import _lib
+    from tests.gpu_util import Buf, call, dptr, sizes5, stream_ptr
+
+    bufs = [Buf(s) for s in sizes5(m, 128, k)]
+    ws_bytes = int(_lib.lib().sharq_prepare_workspace_best_bytes(m))
+    ws, scale = Buf(ws_bytes), Buf(4)
+    xd = x.cuda()
+    tail = (m, 128, k, ws.ptr, ws_bytes, *[b.ptr for b in bufs], scale.ptr, stream_ptr())
+    if gamma is None:
+        call("sharq_scaled_sparse_residual_quantize_x", dptr(xd), *tail)
+    else:
+        gd = gamma.cuda()
+        call("sharq_fused_rmsnorm_sparse_residual_quantize_x", dptr(xd), dptr(gd), ctypes.c_float(eps), *tail)
+    wsh = ws.get()
+    return ([b.get() for b in bufs], wsh[:4].view(np.float32)[0], scale.get().view(np.float32)[0],
+            wsh[256:256 + 4 * m].view(np.float32))
 
 
-@pytest.mark.parametrize("m,k", [(8, 4096), (9, 4096), (33, 1152), (64, 4096), (65, 4096)])
-def test_small_scaled_prepare_matches_oracle(oracle, m, k):
-    prepare.test_scaled_prepare_matches_oracle(oracle, m, k)
+# one row, around one and two CTAs per SM, the longest row, rows of a chunk, the largest number of CTA maxima and one row more
+@pytest.mark.parametrize("m,k", [(1, 4096), (17, 4096), (149, 256), (8, 32768), (300, 1152), (4096, 128), (4097, 128)])
+def test_rmsnorm_prepare_in_two_launches_matches_oracle(oracle, m, k):
+    x, gamma = H.config0_x(m, k, seed=m + k), H.config0_gamma(k, seed=m)
+    got, amax, scale, inv = _prepare(m, k, x, gamma)
+    inv_cpu, _, _ = oracle.rmsnorm_row_stats(H.bits(x), H.bits(gamma), 1e-6)
+    ulp = np.abs(inv.view(np.int32).astype(np.int64) - inv_cpu.view(np.int32).astype(np.int64))
+    assert ulp.max() <= 2  # the sum of squares is order-exact, rsqrtf a <= 2 ulp approximation
+    _, amax_rows, _ = oracle.rmsnorm_row_stats(H.bits(x), H.bits(gamma), 1e-6, inv_rms_in=inv)
+    assert np.float32(amax_rows.max()) == amax and oracle.tensor_scale(amax, cuda_mode=True) == scale
+    _compare(got, oracle.rmsnorm_prepare(H.bits(x), H.bits(gamma), inv, scale), f"rmsnorm {m}x{k}")
 
 
-def test_small_add_rmsnorm_prepare_equals_the_prepare_of_the_sum():
+# around the size up to which every CTA scans the input, a ragged row, more input than CTAs
+@pytest.mark.parametrize("m,k", [(16, 4096), (17, 4096), (33, 1152), (65, 4096), (700, 4096)])
+def test_scaled_prepare_in_two_launches_matches_oracle(oracle, m, k):
+    x = H.config0_x(m, k, seed=m)
+    got, _, scale, _ = _prepare(m, k, x, None)
+    s = oracle.tensor_scale(oracle.absmax_bf16(H.bits(x)), cuda_mode=True)
+    assert scale == s
+    _compare(got, oracle.prepare(oracle.scale_bf16(H.bits(x), s, cuda_mode=True)), f"scaled {m}x{k}")
+
+
+# two launches, the cooperative launch, and two launches again
+@pytest.mark.parametrize("m,k", [(5, 4096), (48, 2048), (1100, 4096), (4096, 8192)])
+def test_add_rmsnorm_prepare_equals_the_prepare_of_the_sum(m, k):
     from sharq_b200 import ops
 
-    for m, k in ((5, 4096), (48, 2048)):
-        x, r, g = H.config0_x(m, k, m).cuda(), H.config0_x(m, k, m + 1).cuda(), H.config0_gamma(k, m).cuda()
-        got = ops.fused_add_rmsnorm_sparse_residual_quantize_x(x, r, g, 1e-6, 128)
-        assert torch.equal(got[6], x + r)
-        want = ops.fused_rmsnorm_sparse_residual_quantize_x(x + r, g, 1e-6, 128)
-        assert all(torch.equal(a, b) for a, b in zip(got[:6], want))
+    x, r, g = H.config0_x(m, k, m).cuda(), H.config0_x(m, k, m + 1).cuda(), H.config0_gamma(k, m).cuda()
+    got = ops.fused_add_rmsnorm_sparse_residual_quantize_x(x, r, g, 1e-6, 128)
+    assert torch.equal(got[6], x + r)
+    want = ops.fused_rmsnorm_sparse_residual_quantize_x(x + r, g, 1e-6, 128)
+    assert all(torch.equal(a, b) for a, b in zip(got[:6], want))
 
 
 # rows: one, a quadrant of the accumulator and one more, a full tile, two tiles with a ragged second; columns: one tile,
