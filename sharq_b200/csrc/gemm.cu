@@ -47,7 +47,9 @@ namespace {
 constexpr int kBM = 128;
 constexpr int kBK = 256;  // logical K per stage
 constexpr int kEpiWarps = 8;
-constexpr int kPrefetchStages = 8;  // K stages of weights a CTA prefetches into L2 while the activation is still being prepared
+// K stages of weights a CTA prefetches into L2 while the activation is still being prepared: about what the ring holds.
+// (Linears of a 32-token decode step, us: none 89.7, 3 87.3, 8 87.4; 28672 x 4096 at M = 32 right behind another GEMM 20.6 / 20.0 / 21.5.)
+constexpr int kPrefetchStages = 3;
 constexpr int kMaxSplits = 8;  // CTAs of a split-K cluster (the portable cluster size)
 constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 
@@ -1056,13 +1058,19 @@ static cudaError_t choose_tile_n(int m, int n, int k, int *tile_n) {
   cudaError_t e = device_info(&dev, &sms);
   if (e != cudaSuccess) return e;
   const int pair_units = ((m + 255) / 256) * ((n + 255) / 256);
+  const int units_128 = ((m + 127) / 128) * ((n + 127) / 128);
   if (m <= 128 || n <= 128) {
-    *tile_n = n > 128 ? 256 : 128;
-  } else if (pair_units * 4 <= sms || k <= 512) {
+    // one row of tiles: narrow ones while they fit the GPU at once (split K fills it: 4096 x 4096 at M = 32 / 128 8.1 / 11.1 us
+    // against 9.7 / 16.3 with 256-wide tiles, 4096 x 14336 13.7 / 16.4 against 15.8 / 22.5); beyond that both take the
+    // same time (28672 x 4096) and the wide ones read the activation half as often
+    *tile_n = n > 128 && units_128 > sms ? 256 : 128;
+  } else if (pair_units * 4 <= sms || k <= 512 || units_128 <= sms) {
     // 256 x 256 pair tiles would keep at most half of the SMs busy, or the K loop is too
     // short to hide the drain of a 256-wide accumulator: 128 x 128 tiles (measured at the
-    // 8-way tensor-parallel shapes: 14.6 vs 18.8 us for N = 768, 12.7 vs 16.7 us for K = 512)
-    *tile_n = 128;
+    // 8-way tensor-parallel shapes: 14.6 vs 18.8 us for N = 768, 12.7 vs 16.7 us for K = 512); also while these fit the GPU
+    // at once (6144 x 4096 at M = 384: 12.6 against 16.1 us).  Where K is long and they fill more than half of it, so that K is not
+    // split, 256-wide tiles with K split move fewer bytes through L2 (3584 x 18944 at M = 384: 30.0 against 36.4 us).
+    *tile_n = k > 16384 && 2 * units_128 > sms && units_128 <= sms ? 256 : 128;
   } else {
     *tile_n = 512;
   }
