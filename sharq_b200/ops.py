@@ -26,7 +26,7 @@ import torch
 from . import _lib
 
 _ERROR_FLAGS: dict[int, torch.Tensor] = {}
-_NO_FLAG = torch.zeros(1, dtype=torch.int32)
+_NO_FLAG = torch.zeros(1, dtype=torch.int32, device="cpu")
 _PREPARE_TIMEOUTS_SEEN = 0
 
 

@@ -203,7 +203,9 @@ class QLinearLayer(nn.Module):
         else:
             x_orig, bsz, q_len = x, None, x.shape[0]
         x2 = x_orig.reshape(-1, x_orig.shape[-1]).to(torch.bfloat16)
-        if self.quant_type == "SHARQ" and self.fused_gemm:
+        cls = type(self)
+        if (self.quant_type == "SHARQ" and self.fused_gemm and cls.prepare_input is QLinearLayer.prepare_input
+                and cls.apply_prepared is QLinearLayer.apply_prepared):  # a subclass may put its own steps there
             y = ops.sharq_linear_forward(x2, self.weight_q, self.scale_w_sparse, self.scale_w_dense, self.weight_scale_host,
                                          bias=self.bias)
         else:
