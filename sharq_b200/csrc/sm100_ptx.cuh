@@ -69,11 +69,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Four consecutive floats added to global memory without a return value (16-byte aligned).
-__device__ __forceinline__ void red_add_v4_f32(float *addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 // Bounded wait.  Returns false on timeout or when *abort_flag became non-zero.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
@@ -123,22 +118,7 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// A float / 16 bytes of another CTA's shared memory (addr: this CTA's address of the same variable).
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t cta_rank) {
-  float v;
-  asm volatile(
-      "{\n\t"
-      ".reg .b32 remote;\n\t"
-      "mapa.shared::cluster.u32 remote, %1, %2;\n\t"
-      "ld.shared::cluster.f32 %0, [remote];\n\t"
-      "}"
-      : "=f"(v)
-      : "r"(addr), "r"(cta_rank)
-      : "memory");
-  return v;
-}
+// 16 bytes of another CTA's shared memory (addr: this CTA's address of the same variable).
 __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr, uint32_t cta_rank) {
   float4 v;
   asm volatile(
