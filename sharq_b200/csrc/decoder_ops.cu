@@ -190,10 +190,9 @@ __device__ __forceinline__ void cta_absmax_to(float *warp_max, __nv_bfloat162 mx
 constexpr int kGroupedChunkRows = 64;
 constexpr int kSwigluPieceVecs = 512;  // two vectors for each of the 256 threads
 
-__global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 *__restrict__ gate_up, long long rows,
-                                                            int ffn, long long row_stride, __nv_bfloat16 *__restrict__ h,
-                                                            unsigned int *__restrict__ amax_bits,
-                                                            const int *__restrict__ unit_group, bool word_per_cta) {
+__global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 *gate_up, long long rows, int ffn,
+                                                            long long row_stride, __nv_bfloat16 *h, unsigned int *amax_bits,
+                                                            const int *unit_group, bool word_per_cta) {
   __shared__ float warp_max[8];
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();
@@ -219,8 +218,8 @@ __global__ void __launch_bounds__(256) swiglu_absmax_kernel(const __nv_bfloat16 
       for (int t = 0; t < 2; ++t) {
         const int v = v0 + t * blockDim.x;
         if (v < v_hi) {
-          g4[t] = __ldg(reinterpret_cast<const uint4 *>(grow + v * 8));
-          u4[t] = __ldg(reinterpret_cast<const uint4 *>(grow + ffn + v * 8));
+          g4[t] = *reinterpret_cast<const uint4 *>(grow + v * 8);
+          u4[t] = *reinterpret_cast<const uint4 *>(grow + ffn + v * 8);
         }
       }
 #pragma unroll

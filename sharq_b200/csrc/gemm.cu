@@ -169,7 +169,7 @@ __device__ __forceinline__ void epilogue_8(const GemmParams &p, const float (&ac
     // bias is added to the bf16 result, as a separate bf16 add would (a bf16 add rounds the
     // exact sum once, which is what the fp32 add + rounding of two bf16 values gives)
     if (full && (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0) {
-      const uint4 bv = __ldg(reinterpret_cast<const uint4 *>(p.bias + col));
+      const uint4 bv = *reinterpret_cast<const uint4 *>(p.bias + col);
       const uint32_t bw[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -194,7 +194,7 @@ __device__ __forceinline__ void epilogue_8(const GemmParams &p, const float (&ac
 // o + residual[off, off + 8), every sum rounded to bf16; off a multiple of 8.  In place of an add pass of 6 bytes per element behind a
 // layer's last linear (8 us at 2048 x 4096, 48 us at 16384 x 3584).
 __device__ __forceinline__ void add_residual_8(const GemmParams &p, uint32_t (&o)[4], size_t off) {
-  const uint4 rv = __ldg(reinterpret_cast<const uint4 *>(p.residual + off));
+  const uint4 rv = __ldcg(reinterpret_cast<const uint4 *>(p.residual + off));  // read once; the plain load cost 8 bytes of spills
   const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {

@@ -72,12 +72,9 @@ __device__ __forceinline__ void publish_amax(unsigned int *amax_bits, float mx, 
 // With kAdd the row is first formed as bf16(x + residual) (the decoder's residual add, rounded
 // like the ATen add), stored to sum_out, and the statistics are those of the sum.
 template <bool kAdd>
-__global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 *__restrict__ x,
-                                                          const __nv_bfloat16 *__restrict__ residual,
-                                                          __nv_bfloat16 *__restrict__ sum_out,
-                                                          const __nv_bfloat16 *__restrict__ gamma, float eps, int k,
-                                                          float *__restrict__ inv_rms,
-                                                          unsigned int *__restrict__ amax_bits, bool word_per_cta) {
+__global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *residual,
+                                                          __nv_bfloat16 *sum_out, const __nv_bfloat16 *gamma, float eps, int k,
+                                                          float *inv_rms, unsigned int *amax_bits, bool word_per_cta) {
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();
   extern __shared__ float partial[];  // [k/32] group sums, then [0] is reused for inv_rms
@@ -91,7 +88,7 @@ __global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 
     const uint4 *src = reinterpret_cast<const uint4 *>(x + (size_t)row * k + (size_t)g * 32);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      uint4 v = __ldg(src + j);
+      uint4 v = src[j];
       w[4 * j + 0] = v.x;
       w[4 * j + 1] = v.y;
       w[4 * j + 2] = v.z;
@@ -100,10 +97,12 @@ __global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 
     if (kAdd) {
       const uint4 *rsrc = reinterpret_cast<const uint4 *>(residual + (size_t)row * k + (size_t)g * 32);
       uint4 *dst = reinterpret_cast<uint4 *>(sum_out + (size_t)row * k + (size_t)g * 32);
+      uint4 r[4];  // all loads ahead of the first store, which they may not pass
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[j] = rsrc[j];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const uint4 r = __ldg(rsrc + j);
-        const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+        const uint32_t rw[4] = {r[j].x, r[j].y, r[j].z, r[j].w};
 #pragma unroll
         for (int t = 0; t < 4; ++t)
           w[4 * j + t] = pack_bf16x2(__fadd_rn(lo_f(w[4 * j + t]), lo_f(rw[t])), __fadd_rn(hi_f(w[4 * j + t]), hi_f(rw[t])));
@@ -143,7 +142,7 @@ __global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 
     __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      uint4 gv = __ldg(gsrc + j);
+      uint4 gv = gsrc[j];
       uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
@@ -168,8 +167,8 @@ __global__ void __launch_bounds__(1024, 2) rms_stats_kernel(const __nv_bfloat16 
 }
 
 // Tensor-wide max |x| of a bf16 tensor (non-RMSNorm path): flat grid-stride reduction.
-__global__ void __launch_bounds__(256) abs_stats_kernel(const __nv_bfloat16 *__restrict__ x, size_t n16,
-                                                         unsigned int *__restrict__ amax_bits, bool word_per_cta) {
+__global__ void __launch_bounds__(256) abs_stats_kernel(const __nv_bfloat16 *x, size_t n16, unsigned int *amax_bits,
+                                                         bool word_per_cta) {
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();
   __shared__ float warp_max[8];
@@ -179,7 +178,7 @@ __global__ void __launch_bounds__(256) abs_stats_kernel(const __nv_bfloat16 *__r
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += 4 * stride) {
     uint4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = (i + u * stride < n16) ? __ldg(src + i + u * stride) : make_uint4(0, 0, 0, 0);
+    for (int u = 0; u < 4; ++u) v[u] = (i + u * stride < n16) ? src[i + u * stride] : make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       m2 = __hmax2(m2, __habs2(*reinterpret_cast<__nv_bfloat162 *>(&v[u].x)));
@@ -262,7 +261,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
   ptx::grid_dependency_wait();
   if (kMode == 1) {
     const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
-    for (int i = threadIdx.x; i < k / 8; i += blockDim.x) gamma_smem[i] = __ldg(gsrc + i);
+    for (int i = threadIdx.x; i < k / 8; i += blockDim.x) gamma_smem[i] = gsrc[i];
   }
   __syncthreads();
 
@@ -287,7 +286,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
       const size_t n16 = (size_t)m * k / 8;
       __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
       for (size_t i = threadIdx.x; i < n16; i += blockDim.x) {
-        const uint4 v = __ldg(all + i);
+        const uint4 v = all[i];
         m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.x)));
         m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.y)));
         m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.z)));
@@ -347,7 +346,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
       if (in_row >= 0) {
         const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)in_row * k + (size_t)group * 32);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) next[j] = __ldg(src + j);
+        for (int j = 0; j < 4; ++j) next[j] = src[j];
       }
       if (kMode == 1) next_inv = p.inv_rms[row];
     }
@@ -420,7 +419,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
         const uint4 *src = reinterpret_cast<const uint4 *>(p.x + (size_t)in_row * k + (size_t)group * 32);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const uint4 v = __ldg(src + j);
+          const uint4 v = src[j];
           w[4 * j + 0] = v.x;
           w[4 * j + 1] = v.y;
           w[4 * j + 2] = v.z;
@@ -562,7 +561,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
   ptx::grid_dependency_wait();
   if (kMode == 1) {
     const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
-    for (int i = threadIdx.x; i < row_vecs; i += kFusedThreads) gamma_s[cache_slot(i >> 2, i & 3)] = __ldg(gsrc + i);
+    for (int i = threadIdx.x; i < row_vecs; i += kFusedThreads) gamma_s[cache_slot(i >> 2, i & 3)] = gsrc[i];
   }
 
   // ---- zero what no owner thread writes: padding rows of the metadata and scale-factor
@@ -627,11 +626,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
           const size_t off = (size_t)(c_row0 + rl[u]) * k + (size_t)g[u] * 32;
           const uint4 *xs = reinterpret_cast<const uint4 *>(p.x + off);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) xv[u][j] = __ldg(xs + j);
+          for (int j = 0; j < 4; ++j) xv[u][j] = xs[j];
           if (kAdd) {
             const uint4 *rs = reinterpret_cast<const uint4 *>(p.residual + off);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) rv[u][j] = __ldg(rs + j);
+            for (int j = 0; j < 4; ++j) rv[u][j] = rs[j];
           }
         }
       }

@@ -180,8 +180,7 @@ __device__ __forceinline__ float block_max_nan(float mx, float *warp_max) {
   return mx;
 }
 
-__global__ void __launch_bounds__(kScaledThreads) absmax_partials_kernel(const uint4 *__restrict__ x, size_t n16,
-                                                                         float *__restrict__ partials) {
+__global__ void __launch_bounds__(kScaledThreads) absmax_partials_kernel(const uint4 *x, size_t n16, float *partials) {
   __shared__ float warp_max[kScaledThreads / 32];
   ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();
@@ -190,7 +189,7 @@ __global__ void __launch_bounds__(kScaledThreads) absmax_partials_kernel(const u
   for (size_t i = (size_t)blockIdx.x * kScaledThreads + threadIdx.x; i < n16; i += 4 * stride) {
     uint4 v[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = (i + u * stride < n16) ? __ldg(x + i + u * stride) : make_uint4(0, 0, 0, 0);
+    for (int u = 0; u < 4; ++u) v[u] = (i + u * stride < n16) ? x[i + u * stride] : make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
@@ -221,11 +220,9 @@ __device__ __forceinline__ void zero_scale_padding(int n, int k, uint8_t *sf_spa
 // The groups of a row are a multiple of 4, so four neighbouring lanes' scale bytes form a 32-bit word of
 // the blocked layout: gathered by shuffles and stored once.
 template <bool kShared>
-__global__ void __launch_bounds__(kScaledThreads, kShared ? 4 : 6) scaled_quantize_kernel(const uint4 *__restrict__ x, int rows, int k,
-                                                                         const float *__restrict__ partials, int n_partials,
-                                                                         uint8_t *__restrict__ q,
-                                                                         uint8_t *__restrict__ sf, uint8_t *__restrict__ sf2,
-                                                                         float *__restrict__ scale_out) {
+__global__ void __launch_bounds__(kScaledThreads, kShared ? 4 : 6) scaled_quantize_kernel(const uint4 *x, int rows, int k, const float *partials,
+                                                                         int n_partials, uint8_t *q, uint8_t *sf, uint8_t *sf2,
+                                                                         float *scale_out) {
   constexpr int kVecs = kShared ? 4 : 2;  // 16-byte vectors of a group
   __shared__ float warp_max[kScaledThreads / 32];
   ptx::grid_launch_dependents();
@@ -258,7 +255,7 @@ __global__ void __launch_bounds__(kScaledThreads, kShared ? 4 : 6) scaled_quanti
       uint32_t w[4 * kVecs];
 #pragma unroll
       for (int j = 0; j < kVecs; ++j) {
-        const uint4 t = __ldg(x + idx * kVecs + j);
+        const uint4 t = x[idx * kVecs + j];
         w[4 * j] = t.x, w[4 * j + 1] = t.y, w[4 * j + 2] = t.z, w[4 * j + 3] = t.w;
       }
       float gm = 0.0f;

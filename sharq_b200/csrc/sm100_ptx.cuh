@@ -136,6 +136,9 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr, uint32_t cta_r
 // ---------------------------------------------------------------- programmatic dependent launch
 // Waits until the kernels this launch depends on have finished and their writes are visible; returns at once in a
 // kernel that was launched without the attribute.
+// A kernel with this wait may be alive while the kernels ahead of it still write what it reads, and the read-only path (__ldg, or
+// a const __restrict__ parameter, which the compiler may load through it) is defined only for data that nothing
+// writes during the kernel's life: such kernels read global memory with ordinary loads and declare no pointer __restrict__.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets a dependent kernel that was launched with the attribute start its blocks (it waits itself before it reads).
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -99,3 +99,17 @@ def test_scaled_quantisation_keeps_a_nan_like_the_torch_passes():
     assert bool(torch.isnan(scale))
     for got, want in zip((qw, sfs, sfd), ops.quantize_w32_shared(scaled)):
         assert torch.equal(got, want)
+
+
+def test_scaled_quantisations_back_to_back_without_a_synchronisation():
+    """Calls whose kernels are all dependents of one another, with the scratch of each handed to the next by the
+    allocator: every call gets its own scale (absmax 1, 2, 4, ...), whatever the one before it left there."""
+    from sharq_b200 import ops, quantize
+
+    x = H.config0_x(512, 1024, seed=2).cuda()
+    x = x / x.abs().max()
+    inputs = [x * 2.0 ** i for i in range(24)]
+    torch.cuda.synchronize()
+    scales = [(ops.scaled_quantize_w32_shared if i % 2 else ops.scaled_quantize_nvfp4)(v)[-1] for i, v in enumerate(inputs)]
+    for got, v in zip(scales, inputs):
+        assert torch.equal(got, quantize.global_nvfp4_scale(v))
