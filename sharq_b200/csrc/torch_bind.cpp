@@ -204,9 +204,10 @@ Tensor output(const Tensor &ref, int64_t m, int64_t n, const std::optional<Tenso
   return *out;
 }
 
-void check_bias(const std::optional<Tensor> &bias, int64_t n) {
-  if (bias)
-    need(is_plain(*bias, at::kBFloat16) && bias->numel() == n, "bias must be a contiguous CUDA bfloat16 tensor with N elements");
+void check_bias(const std::optional<Tensor> &bias, int64_t n, const at::Device &dev) {
+  if (!bias) return;
+  need(is_plain(*bias, at::kBFloat16) && bias->numel() == n, "bias must be a contiguous CUDA bfloat16 tensor with N elements");
+  need(bias->device() == dev, "bias must be on the same device as the inputs");
 }
 
 void check_weight(const Tensor &qw, const Tensor &sfs, const Tensor &sfd, const at::Device &dev, int64_t n, int64_t k) {
@@ -229,7 +230,7 @@ Tensor linear_gemm(const Tensor &a_comp, const Tensor &e, const Tensor &sfa, con
   check_u8(q_res, dev, m * (k / 2), "Q_res");
   check_u8(sf_res, dev, sf_bytes(m, k), "SF_res");
   check_weight(qw, sfs, sfd, dev, n, k);
-  check_bias(bias, n);
+  check_bias(bias, n, dev);
   if (residual)
     need(is_plain(*residual, at::kBFloat16) && residual->device() == dev && residual->numel() == m * n,
          "residual must be a contiguous CUDA bfloat16 tensor with M * N elements on the device of Q_res");
@@ -250,7 +251,7 @@ Tensor linear_forward(const Tensor &x, const Tensor &qw, const Tensor &sfs, cons
   const int64_t m = x.size(0), k = x.size(1), n = qw.size(0);
   check_k128("scaled_sparse_residual_quantize_x", "requires", k);
   check_weight(qw, sfs, sfd, x.device(), n, k);
-  check_bias(bias, n);
+  check_bias(bias, n, x.device());
   Scaled s(x, std::nullopt, 0.0, n, std::nullopt);
   Tensor d = empty_like_on(x, {m, n}, at::kBFloat16);
   c10::cuda::OptionalCUDAGuard guard(x.device());
@@ -267,7 +268,7 @@ Tensor dense_gemm(const Tensor &a, const Tensor &b, const Tensor &sfa, const Ten
   need(a.is_cuda() && b.is_cuda() && sfa.is_cuda() && sfb.is_cuda(), "A, B, SFA and SFB must be CUDA tensors");
   const int64_t m = a.size(0), n = b.size(0), k = a.size(1) * 2;
   const at::Device dev = a.device();
-  check_bias(bias, n);
+  check_bias(bias, n, dev);
   Tensor d = output(a, m, n, out);
   const float *alpha_dev = alpha_t ? scale_ptr(*alpha_t, dev, "scale") : nullptr;
   c10::cuda::OptionalCUDAGuard guard(dev);
