@@ -298,9 +298,11 @@ int sharq_allreduce_bf16_peer(void *const *rank_data_ptrs, void *const *rank_fla
  *   sharq_moe_plan: the grouping itself from selected [tokens * top_k] (expert of every token slot, experts <= 16, unit 256
  *     for the entry points below): dest[slot] = its grouped row (ascending slots inside an expert), src_row[row] = its
  *     token or -1, unit_group as above; rows >= (ceil(slots / unit) + experts) * unit, a multiple of unit.
+ *     A slot whose expert is outside [0, experts) has no row: dest is -1.  sharq_moe_plan_flagged also stores the code
+ *     0x401 in *error_flag (device) then.
  *   sharq_moe_combine: out[t] = sum over the top_k slots of token t, in ascending expert order, of
  *     y[dest[t,j]] * w[t,j] with bf16 rounding after every product and addition, which is what the
- *     reference's sequence of index_add_ calls on a zero buffer computes. */
+ *     reference's sequence of index_add_ calls on a zero buffer computes.  dest < 0: the token's row is NaN. */
 int sharq_grouped_sparse_residual_quantize_x(const void *x_bf16, const int *src_row, int m, int n, int k,
                                             const int *unit_group, int groups, void *amax_workspace, void *a_comp, void *e,
                                             void *sfa_sparse, void *q_res, void *sf_res, float *scale_vec_out, void *stream);
@@ -321,6 +323,8 @@ int sharq_grouped_absmax_sparse_residual_quantize_x(const void *x_bf16, int m, i
                                                     void *q_res, void *sf_res, float *scale_vec_out, void *stream);
 int sharq_moe_plan(const int64_t *selected, int64_t slots, int top_k, int experts, int unit, int64_t rows, void *workspace,
                    size_t workspace_bytes, int *dest, int *src_row, int *unit_group, void *stream);
+int sharq_moe_plan_flagged(const int64_t *selected, int64_t slots, int top_k, int experts, int unit, int64_t rows, void *workspace,
+                           size_t workspace_bytes, int *dest, int *src_row, int *unit_group, int *error_flag, void *stream);
 size_t sharq_moe_plan_workspace_bytes(int64_t slots);
 int sharq_moe_combine(void *out_bf16, const void *y_bf16, const int *dest, const int64_t *selected, const void *w_bf16,
                       int tokens, int top_k, int width, void *stream);

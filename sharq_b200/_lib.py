@@ -83,6 +83,7 @@ SIGNATURES = {
     "sharq_grouped_absmax_sparse_residual_quantize_x": (
         c_int, [_P, c_int, c_int, c_int, _P, c_int, _P, _P, _P, _P, _P, _P, _P, _P]),
     "sharq_moe_plan": (c_int, [_P, c_int64, c_int, c_int, c_int, c_int64, _P, c_size_t, _P, _P, _P, _P]),
+    "sharq_moe_plan_flagged": (c_int, [_P, c_int64, c_int, c_int, c_int, c_int64, _P, c_size_t, _P, _P, _P, _P, _P]),
     "sharq_moe_plan_workspace_bytes": (c_size_t, [c_int64]),
     "sharq_moe_combine": (c_int, [_P, _P, _P, _P, _P, c_int, c_int, c_int, _P]),
     "sharq_linear_gemm_scatter": (

@@ -422,6 +422,12 @@ size_t sharq_moe_plan_workspace_bytes(int64_t slots) { return slots > 0 ? sharq:
 
 int sharq_moe_plan(const int64_t *selected, int64_t slots, int top_k, int experts, int unit, int64_t rows, void *workspace,
                    size_t workspace_bytes, int *dest, int *src_row, int *unit_group, void *stream) {
+  return sharq_moe_plan_flagged(selected, slots, top_k, experts, unit, rows, workspace, workspace_bytes, dest, src_row, unit_group,
+                                nullptr, stream);
+}
+
+int sharq_moe_plan_flagged(const int64_t *selected, int64_t slots, int top_k, int experts, int unit, int64_t rows, void *workspace,
+                           size_t workspace_bytes, int *dest, int *src_row, int *unit_group, int *error_flag, void *stream) {
   SHARQ_REQUIRE(selected && workspace && dest && src_row && unit_group, "null buffer");
   SHARQ_REQUIRE(slots > 0 && top_k > 0 && unit > 0, "slots, top_k and unit must be positive");
   SHARQ_REQUIRE(experts >= 1 && experts <= sharq::kGemmMaxGroups, "experts must be in [1, %d]", sharq::kGemmMaxGroups);
@@ -429,7 +435,7 @@ int sharq_moe_plan(const int64_t *selected, int64_t slots, int top_k, int expert
                 "rows must be a multiple of unit that holds every expert's padded segment");
   SHARQ_REQUIRE(workspace_bytes >= sharq_moe_plan_workspace_bytes(slots), "workspace is too small");
   return check_cuda(sharq::run_moe_plan(reinterpret_cast<const long long *>(selected), slots, top_k, experts, unit, rows,
-                                        static_cast<int *>(workspace), dest, src_row, unit_group, as_stream(stream)),
+                                        static_cast<int *>(workspace), dest, src_row, unit_group, error_flag, as_stream(stream)),
                     "moe_plan");
 }
 

@@ -291,6 +291,7 @@ __global__ void __launch_bounds__(256) abs_stats_grouped_kernel(const __nv_bfloa
 constexpr int kPlanThreads = 256;
 constexpr int kPlanSlots = 1024;
 constexpr int kPlanMaxExperts = 16;
+constexpr int kPlanBadExpert = 0x401;  // error code: an expert outside [0, experts)
 
 // expert of a slot, -1 behind the last slot or outside [0, experts)
 __device__ __forceinline__ int plan_expert(const long long *selected, long long slot, long long slots, int experts) {
@@ -299,13 +300,15 @@ __device__ __forceinline__ int plan_expert(const long long *selected, long long 
 }
 
 __global__ void __launch_bounds__(kPlanThreads) moe_count_kernel(const long long *__restrict__ selected, long long slots, int experts,
-                                                                 int *__restrict__ counts) {
+                                                                 int *__restrict__ counts, int *error_flag) {
   __shared__ int hist[kPlanMaxExperts];
   if (threadIdx.x < kPlanMaxExperts) hist[threadIdx.x] = 0;
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < kPlanSlots / kPlanThreads; ++i) {
-    const int e = plan_expert(selected, (long long)blockIdx.x * kPlanSlots + i * kPlanThreads + threadIdx.x, slots, experts);
+    const long long slot = (long long)blockIdx.x * kPlanSlots + i * kPlanThreads + threadIdx.x;
+    const int e = plan_expert(selected, slot, slots, experts);
+    if (slot < slots && e < 0 && error_flag != nullptr) atomicExch(error_flag, kPlanBadExpert);
     const unsigned same = __match_any_sync(0xffffffffu, e);
     if (e >= 0 && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&hist[e], __popc(same));
   }
@@ -364,6 +367,8 @@ __global__ void __launch_bounds__(kPlanThreads) moe_place_kernel(const long long
       for (int w = 0; w < warp; ++w) row += warp_count[w][e];
       dest[slot] = row;
       src_row[row] = (int)(slot / top_k);
+    } else if (slot < slots) {
+      dest[slot] = -1;  // no expert has that number; see moe_combine_kernel
     }
     __syncthreads();
     if (threadIdx.x < experts) {
@@ -385,7 +390,7 @@ __global__ void __launch_bounds__(kPlanThreads) moe_place_kernel(const long long
 // outputs y[dest[t, j], :] * w[t, j] in ascending order of the expert index, every product and every
 // partial sum rounded to bf16 - the arithmetic of the reference's per-expert loop
 // `final.index_add_(0, top_x, y * w[top_x, idx, None])` (model/qMixtralLayer.py:223-231), which
-// visits the experts in that order on a zero-initialised buffer.
+// visits the experts in that order on a zero-initialised buffer.  A slot without a row (dest < 0) makes its token NaN.
 constexpr int kCombineMaxTopK = 8;
 __global__ void __launch_bounds__(256) moe_combine_kernel(__nv_bfloat16 *__restrict__ out, const __nv_bfloat16 *__restrict__ y,
                                                           const int *__restrict__ dest, const long long *__restrict__ selected,
@@ -408,7 +413,9 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(__nv_bfloat16 *__restr
       for (int j = 0; j < top_k; ++j) {
         const int slot = order[j];
         const float wj = __bfloat162float(w[t * top_k + slot]);
-        const uint4 yv = __ldg(reinterpret_cast<const uint4 *>(y + (long long)dest[t * top_k + slot] * width) + v);
+        const int from = dest[t * top_k + slot];
+        const uint4 yv = from >= 0 ? __ldg(reinterpret_cast<const uint4 *>(y + (long long)from * width) + v)
+                                   : make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u);
         const uint32_t yw[4] = {yv.x, yv.y, yv.z, yv.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -554,12 +561,12 @@ size_t moe_plan_workspace_bytes(long long slots) {
 }
 
 cudaError_t run_moe_plan(const long long *selected, long long slots, int top_k, int experts, int unit, long long rows, int *counts,
-                         int *dest, int *src_row, int *unit_group, cudaStream_t stream) {
+                         int *dest, int *src_row, int *unit_group, int *error_flag, cudaStream_t stream) {
   if (slots <= 0 || top_k < 1 || experts < 1 || experts > kPlanMaxExperts || unit < 1) return cudaErrorInvalidValue;
   // every expert's padding fits: rows is a whole number of units
   if (rows % unit != 0 || rows > 0x7fffffffLL || rows < ((slots + unit - 1) / unit + experts) * unit) return cudaErrorInvalidValue;
   const unsigned blocks = (unsigned)((slots + kPlanSlots - 1) / kPlanSlots);
-  moe_count_kernel<<<blocks, kPlanThreads, 0, stream>>>(selected, slots, experts, counts);
+  moe_count_kernel<<<blocks, kPlanThreads, 0, stream>>>(selected, slots, experts, counts, error_flag);
   moe_place_kernel<<<blocks, kPlanThreads, 0, stream>>>(selected, slots, top_k, experts, unit, rows, counts, dest, src_row, unit_group);
   return cudaGetLastError();
 }

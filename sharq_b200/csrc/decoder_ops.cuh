@@ -38,9 +38,9 @@ cudaError_t run_scatter_add_scaled(void *out, const void *y, const long long *ro
                                    int width, long long out_rows, cudaStream_t stream);
 
 // Grouping plan of a mixture-of-experts step (see moe_place_kernel): selected [slots] (slot = token * top_k + j), at most
-// 16 experts; rows = (ceil(slots / unit) + experts) * unit or more; counts: moe_plan_workspace_bytes(slots) bytes of scratch.
+// 16 experts; a slot whose expert is outside [0, experts) gets dest -1 and stores a code in *error_flag (may be null); rows = (ceil(slots / unit) + experts) * unit or more; counts: moe_plan_workspace_bytes(slots) bytes of scratch.
 size_t moe_plan_workspace_bytes(long long slots);
 cudaError_t run_moe_plan(const long long *selected, long long slots, int top_k, int experts, int unit, long long rows, int *counts,
-                         int *dest, int *src_row, int *unit_group, cudaStream_t stream);
+                         int *dest, int *src_row, int *unit_group, int *error_flag, cudaStream_t stream);
 
 }  // namespace sharq

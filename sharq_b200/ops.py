@@ -28,6 +28,7 @@ from . import _lib
 _ERROR_FLAGS: dict[int, torch.Tensor] = {}
 _NO_FLAG = torch.zeros(1, dtype=torch.int32, device="cpu")
 _PREPARE_TIMEOUTS_SEEN = 0
+_BAD_EXPERT = 0x401  # kPlanBadExpert of csrc/decoder_ops.cu
 
 
 def _check(cond: bool, msg: str) -> None:
@@ -55,8 +56,8 @@ def _error_flag(device: torch.device) -> torch.Tensor:
 
 
 def check_device_errors(device=None) -> None:
-    """Synchronising check of the kernels' bounded waits: the GEMM / all-reduce error flag of each
-    device and the grid barrier of the one-launch prepare."""
+    """Synchronising check of the kernels' bounded waits, the GEMM / all-reduce error flag of each device and the grid
+    barrier of the one-launch prepare, and of the expert ids that a mixture-of-experts plan was given."""
     global _PREPARE_TIMEOUTS_SEEN
     if torch.cuda.is_available() and torch.cuda.is_initialized():
         torch.cuda.synchronize()
@@ -70,6 +71,8 @@ def check_device_errors(device=None) -> None:
         code = int(flag.item())
         if code != 0:
             flag.zero_()
+            if code == _BAD_EXPERT:
+                raise RuntimeError(f"sharq_b200 moe_plan: an expert id was outside [0, experts) on cuda:{idx}")
             raise RuntimeError(f"sharq_b200 GEMM kernel reported a timed-out wait (code {code}) on cuda:{idx}")
 
 
@@ -630,7 +633,8 @@ def linear_gemm_grouped_swiglu(A_comp, E, SFA_sparse, Q_res, SF_res, weights, un
 
 def moe_plan(selected: torch.Tensor, experts: int, unit: int = 256):
     """decoder.moe_grouping on the GPU in two launches: selected int64 [tokens, top_k], experts <= 16 ->
-    (dest int32 [tokens, top_k], src_row int32 [rows], unit_group int32 [rows / unit])."""
+    (dest int32 [tokens, top_k], src_row int32 [rows], unit_group int32 [rows / unit]).  An expert outside [0, experts) is
+    reported by check_device_errors; its slot has no row (dest -1) and moe_combine makes its token NaN."""
     _check(selected.is_cuda and selected.dtype == torch.int64 and selected.dim() == 2 and selected.is_contiguous()
            and selected.numel() > 0, "selected must be a contiguous non-empty CUDA int64 matrix")
     slots, dev = selected.numel(), selected.device
@@ -641,8 +645,9 @@ def moe_plan(selected: torch.Tensor, experts: int, unit: int = 256):
     dest, src_row, unit_group = out.split((slots, rows, rows // unit))
     ws = _u8(ws_bytes, dev)
     with _on_device(dev):
-        _lib.check(L.sharq_moe_plan(_ptr(selected), slots, int(selected.shape[1]), int(experts), int(unit), rows, _ptr(ws), ws_bytes,
-                                    _ptr(dest), _ptr(src_row), _ptr(unit_group), _stream(dev)))
+        _lib.check(L.sharq_moe_plan_flagged(
+            _ptr(selected), slots, int(selected.shape[1]), int(experts), int(unit), rows, _ptr(ws), ws_bytes, _ptr(dest),
+            _ptr(src_row), _ptr(unit_group), _ptr(_error_flag(dev)), _stream(dev)))
     return dest.view(selected.shape), src_row, unit_group
 
 

@@ -18,3 +18,26 @@ def test_plan_equals_the_aten_plan(tokens, experts, top_k):
     got = moe_grouping(selected.cuda(), experts)
     for a, b in zip(got, want):
         assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(a.cpu(), b)
+
+
+# first and last slot of a token, of a block, negative and too large; the range of int32 exceeded
+@pytest.mark.parametrize("at,expert", [((0, 0), -1), ((1023, 1), 8), ((511, 1), 2 ** 33), ((1299, 0), -2 ** 40)])
+def test_an_expert_outside_the_range_is_reported_and_reads_nothing(at, expert):
+    from sharq_b200 import ops
+
+    tokens, experts, width = 1300, 8, 64
+    selected = torch.rand(tokens, experts, generator=torch.Generator().manual_seed(1)).topk(2, dim=1).indices.cuda()
+    good_dest = ops.moe_plan(selected, experts)[0]
+    selected[at] = expert
+    dest, src_row, _ = ops.moe_plan(selected, experts)
+    with pytest.raises(RuntimeError, match="expert id"):
+        ops.check_device_errors()
+    ops.check_device_errors()  # reported once
+    assert int(dest[at]) == -1 and int((dest < 0).sum()) == 1 and int(good_dest.min()) >= 0
+    valid = dest >= 0
+    assert torch.equal(src_row[dest[valid].long()].long(), valid.nonzero()[:, 0])
+    y = torch.ones(src_row.numel(), width, dtype=torch.bfloat16, device="cuda")
+    out = ops.moe_combine(y, dest, selected, torch.full((tokens, 2), 0.5, dtype=torch.bfloat16, device="cuda"))
+    bad = torch.zeros(tokens, dtype=torch.bool, device="cuda")
+    bad[at[0]] = True
+    assert torch.equal(out.isnan().all(dim=1), bad) and bool((out[~bad] == 1).all())
