@@ -27,6 +27,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 
+from .qlinear import QLinearLayer, methods_kept
 from .tp import RowParallelSharqLinear, head_layout, padded_size, shard_bounds
 
 
@@ -163,8 +164,6 @@ class SharqDecoderLayer(torch.nn.Module):
             del wq, wk, wv, wo, wg, wu, wd
         if mode == "NVFP4":
             # dense NVFP4 baseline: unfused RMSNorm, dense activation quantisation, dense GEMM
-            from .qlinear import QLinearLayer
-
             def dense(w, b=None):
                 lin = torch.nn.Linear(w.shape[1], w.shape[0], bias=b is not None, device=device, dtype=torch.bfloat16)
                 lin.weight.data.copy_(w)
@@ -222,7 +221,8 @@ class SharqDecoderLayer(torch.nn.Module):
             else:
                 x2 = x2 + o
                 hn = _rmsnorm(x2, self.post_norm, cfg.eps)
-            if not return_delta and self.world == 1 and self.reduce_hook is None and self.fused_glue and self.grouped_experts and hn.is_cuda:
+            if (not return_delta and self.world == 1 and self.reduce_hook is None and self.fused_glue and self.grouped_experts
+                    and hn.is_cuda and methods_kept(self, _LAYER_METHODS, "_moe", "_moe_grouped")):
                 return self._moe_grouped(hn, *_route(hn, self.router, cfg.top_k), residual=x2).view(b, s, h)
             d = self._moe(hn)
             if return_delta:
@@ -234,9 +234,9 @@ class SharqDecoderLayer(torch.nn.Module):
             x2 = x2 + o
             prep = self.gate_up.prepare_input_rmsnorm(x2, self.post_norm, cfg.eps)
         if self.fused_glue:
-            prep = self.gate_up.apply_prepared_swiglu(prep, self.down.local)
-            if not return_delta and self.world == 1 and self.reduce_hook is None:
-                return self.down.local.apply_prepared(prep, residual=x2).view(b, s, h)
+            prep = _prepare_down(self.gate_up, prep, self.down.local)
+            if not return_delta and isinstance(self.down, RowParallelSharqLinear):
+                return self.down.apply_prepared_residual(prep, x2).view(b, s, h)
             d = self.down.apply_prepared_reduced(prep)
         else:
             gu = self.gate_up.apply_prepared(prep)
@@ -262,7 +262,7 @@ class SharqDecoderLayer(torch.nn.Module):
         attn2 = attn.transpose(1, 2).reshape(b * s, self.local_heads * cfg.head_dim)
         self.o_proj.local.apply_prepared(self.o_proj.local.prepare_input(attn2), scatter=sp.scatter)
         prepared, x_local = sp.transition(x_local, self.post_norm, cfg.eps)
-        self.down.local.apply_prepared(self.gate_up.apply_prepared_swiglu(prepared, self.down.local), scatter=sp.scatter)
+        self.down.local.apply_prepared(_prepare_down(self.gate_up, prepared, self.down.local), scatter=sp.scatter)
         return sp.transition(x_local, next_gamma, cfg.eps)
 
     @torch.no_grad()
@@ -453,6 +453,9 @@ class SharqDecoderLayer(torch.nn.Module):
         return x2.view(b, s, h)
 
 
+_LAYER_METHODS = {name: vars(SharqDecoderLayer)[name] for name in ("_moe", "_moe_grouped")}
+
+
 def moe_grouping(selected: torch.Tensor, experts: int, unit: int = 256):
     """Device-side plan of a grouped mixture-of-experts step, without host synchronisation.
     selected [tokens, top_k] (expert of every token slot) ->
@@ -518,6 +521,13 @@ def _split_heads(qkv: torch.Tensor, b: int, s: int, heads: int, kv_heads: int, d
     return q, k, v
 
 
+def _prepare_down(gate_up, prepared, down):
+    """down.prepare_input_swiglu(gate_up.apply_prepared(prepared)), for a QLinearLayer in one GEMM launch where it can be."""
+    if isinstance(gate_up, QLinearLayer):
+        return gate_up.apply_prepared_swiglu(prepared, down)
+    return down.prepare_input_swiglu(gate_up.apply_prepared(prepared))
+
+
 def _swiglu(gu: torch.Tensor, fused: bool) -> torch.Tensor:
     if fused and gu.is_cuda:
         from . import ops
@@ -531,8 +541,6 @@ def _local_column(w_local: torch.Tensor, w_full: torch.Tensor, bias):
     """Column-parallel linear from an already gathered local slice; the weight tensor scale is
     taken over the FULL weight so that shards agree with the unsharded layer."""
     from . import ops
-    from .qlinear import QLinearLayer
-
     scale = torch.clamp(w_full.abs().max().float() / (448.0 * 6.0), min=1e-9)
     q, sfs, sfd = ops.quantize_w32_shared((w_local / scale).to(torch.bfloat16).contiguous())
     return QLinearLayer.from_quantized(w_local.shape[1], w_local.shape[0], q, sfs, sfd, scale, bias=bias)

@@ -29,6 +29,14 @@ from .quantize import (
 )
 
 
+def methods_kept(layer, own: dict, *names: str) -> bool:
+    """Whether the methods `names` of layer are the functions of `own`: neither overridden by a subclass, nor replaced on the
+    class (a profiler's wrappers), nor set on the instance.  A call that does the work of several methods at once
+    is taken only then."""
+    methods = (getattr(layer, name, None) for name in names)
+    return all(getattr(m, "__func__", None) is own[name] and m.__self__ is layer for m, name in zip(methods, names))
+
+
 class QLinearLayer(nn.Module):
     def __init__(self, original_layer: nn.Linear, select_num=None, reorder_index=None, out_reorder_index=None,
                  quant_type: str = "NVFP4", extra_fusion: bool = True, fused_gemm: bool = True,
@@ -187,7 +195,8 @@ class QLinearLayer(nn.Module):
         """down.prepare_input_swiglu(self.apply_prepared(prepared)) for a merged gate_up layer whose output nothing
         else reads: where the shape allows, SwiGLU and the absmax run in the GEMM epilogue and the [M, 2F] product
         is never stored (same bits)."""
-        if (prepared[0] == "SHARQ" and down.quant_type == "SHARQ" and self.fused_gemm and self.bias is None
+        if (methods_kept(self, QLINEAR_METHODS, "apply_prepared") and methods_kept(down, QLINEAR_METHODS, "prepare_input_swiglu")
+                and prepared[0] == "SHARQ" and down.quant_type == "SHARQ" and self.fused_gemm and self.bias is None
                 and self.out_features % 256 == 0
                 and ops.linear_gemm_swiglu_pays(prepared[4].shape[0], self.out_features // 2, self.in_features)):
             _, a_comp, e, sfa, q_res, sf_res, scale_x = prepared
@@ -203,9 +212,7 @@ class QLinearLayer(nn.Module):
         else:
             x_orig, bsz, q_len = x, None, x.shape[0]
         x2 = x_orig.reshape(-1, x_orig.shape[-1]).to(torch.bfloat16)
-        cls = type(self)
-        if (self.quant_type == "SHARQ" and self.fused_gemm and cls.prepare_input is QLinearLayer.prepare_input
-                and cls.apply_prepared is QLinearLayer.apply_prepared):  # a subclass may put its own steps there
+        if self.quant_type == "SHARQ" and self.fused_gemm and methods_kept(self, QLINEAR_METHODS, "prepare_input", "apply_prepared"):
             y = ops.sharq_linear_forward(x2, self.weight_q, self.scale_w_sparse, self.scale_w_dense, self.weight_scale_host,
                                          bias=self.bias)
         else:
@@ -213,3 +220,6 @@ class QLinearLayer(nn.Module):
         if bsz is not None:
             return y.reshape(bsz, q_len, -1)
         return y.reshape(q_len, -1)
+
+
+QLINEAR_METHODS = {name: vars(QLinearLayer)[name] for name in ("prepare_input", "prepare_input_swiglu", "apply_prepared")}

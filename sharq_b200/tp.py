@@ -451,10 +451,24 @@ class RowParallelSharqLinear(_ShardedBase):
         buf.sum_(slot, nbytes)
         return view + self.bias if self.bias is not None else view
 
+    def apply_prepared_residual(self, prepared, residual: torch.Tensor) -> torch.Tensor:
+        """residual + apply_prepared_reduced(prepared).  Where nothing is summed over ranks or added in between, the
+        add rides in the epilogue of the fused GEMM (same bits)."""
+        from .qlinear import QLINEAR_METHODS, methods_kept
+
+        if (self.world == 1 and self.reduce_hook is None and self.bias is None
+                and methods_kept(self, _ROW_PARALLEL_METHODS, "reduce", "apply_prepared_reduced")
+                and methods_kept(self.local, QLINEAR_METHODS, "apply_prepared")):
+            return self.local.apply_prepared(prepared, residual=residual)
+        return residual + self.apply_prepared_reduced(prepared)
+
     def forward(self, x_local):
         x2 = x_local.reshape(-1, x_local.shape[-1]).to(torch.bfloat16)
         y = self.apply_prepared_reduced(self.local.prepare_input(x2))
         return y.reshape(*x_local.shape[:-1], y.shape[-1])
+
+
+_ROW_PARALLEL_METHODS = {name: vars(RowParallelSharqLinear)[name] for name in ("reduce", "apply_prepared_reduced")}
 
 
 def all_reduce_sum_(t: torch.Tensor, group=None) -> torch.Tensor:
