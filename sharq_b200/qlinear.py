@@ -163,8 +163,7 @@ class QLinearLayer(nn.Module):
                                          scatter=scatter)
         if out is not None and not ((tag == "SHARQ" and self.fused_gemm) or (tag == "NVFP4" and self.bias is None)):
             raise ValueError("out= is only supported by the fused SharQ GEMM and the bias-free dense NVFP4 GEMM")
-        # a bias of another type (the module was cast) is added by torch
-        folded = self.bias if self.bias is not None and self.bias.dtype == torch.bfloat16 else None
+        folded = self.bias if self._bias_folds() else None
         if tag == "SHARQ":
             _, a_comp, e, sfa, q_res, sf_res, scale_x = prepared
             if self.fused_gemm:
@@ -189,6 +188,13 @@ class QLinearLayer(nn.Module):
         else:
             raise ValueError(f"Unsupported prepared input tag: {tag}")
         return y if self.bias is None else y + self.bias
+
+    def _bias_folds(self) -> bool:
+        """Whether the epilogue of the dense GEMM takes the bias as it is; one of another type (the module was cast), stride, shape
+        or device is left to torch's add, which broadcasts, promotes or raises."""
+        b = self.bias
+        return (b is not None and b.dtype == torch.bfloat16 and b.dim() == 1 and b.shape[0] == self.out_features
+                and b.is_contiguous() and b.device == self.weight_q.device)
 
     @torch.no_grad()
     def apply_prepared_swiglu(self, prepared, down: "QLinearLayer"):
