@@ -208,14 +208,17 @@ int sharq_swiglu_sparse_residual_quantize_x(const void *gate_up_bf16, int m, int
   SHARQ_REQUIRE(k % 128 == 0, "swiglu_sparse_residual_quantize_x requires K to be a multiple of 128, got %d", k);
   SHARQ_REQUIRE(gate_up_bf16 && h_bf16 && a_comp && e && sfa_sparse && q_res && sf_res, "null buffer");
   SHARQ_REQUIRE(workspace && workspace_bytes >= 256, "workspace too small: need 256 bytes");
-  int words = 1;
-  if (check_cuda(sharq::run_swiglu_absmax(gate_up_bf16, m, k, 2LL * k, h_bf16, static_cast<unsigned int *>(workspace),
-                                          as_stream(stream), nullptr, 1,
-                                          (int)(workspace_bytes / 4 < 65536 ? workspace_bytes / 4 : 65536), &words),
+  // max|H| ends up in the first word either way; the maxima of the CTAs lie behind the first 256 bytes
+  auto *amax = static_cast<unsigned int *>(workspace);
+  const size_t room = (workspace_bytes - 256) / sizeof(unsigned int);
+  int words = 0;
+  if (check_cuda(sharq::run_swiglu_absmax(gate_up_bf16, m, k, 2LL * k, h_bf16, amax, as_stream(stream), nullptr, 1, amax + 64,
+                                          (int)(room < 65536 ? room : 65536), &words),
                  "swiglu_absmax"))
     return 1;
-  return check_cuda(sharq::run_scaled_prepare(h_bf16, nullptr, 0.0f, m, k, workspace, nullptr, a_comp, e, sfa_sparse,
-                                              q_res, sf_res, scale_out, as_stream(stream), words),
+  return check_cuda(sharq::run_scaled_prepare(h_bf16, nullptr, 0.0f, m, k, words > 0 ? amax + 64 : amax, nullptr, a_comp, e,
+                                              sfa_sparse, q_res, sf_res, scale_out, as_stream(stream), words > 0 ? words : 1,
+                                              nullptr, nullptr, 0, words > 0 ? amax : nullptr),
                     "swiglu_sparse_residual_quantize_x");
 }
 

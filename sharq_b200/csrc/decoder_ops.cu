@@ -518,15 +518,16 @@ cudaError_t run_add_rmsnorm(const void *x, const void *residual, void *sum_out, 
 }
 
 cudaError_t run_swiglu_absmax(const void *gate_up, long long rows, int ffn, long long row_stride, void *h,
-                              unsigned int *amax_bits, cudaStream_t stream, const int *unit_group, int groups, int capacity,
-                              int *words) {
+                              unsigned int *amax_bits, cudaStream_t stream, const int *unit_group, int groups,
+                              unsigned int *cta_words, int capacity, int *words) {
   long long ctas = (long long)sm_count() * 8;
   const long long work = unit_group != nullptr ? (rows + kGroupedChunkRows - 1) / kGroupedChunkRows
                                                : rows * ((ffn / 8 + kSwigluPieceVecs - 1) / kSwigluPieceVecs);
   if (ctas > work) ctas = work;
   // with room for a word per CTA nothing has to be zeroed before the launch
-  const bool word_per_cta = unit_group == nullptr && ctas <= capacity;
-  if (words != nullptr) *words = word_per_cta ? (int)ctas : 1;
+  const bool word_per_cta = unit_group == nullptr && cta_words != nullptr && ctas <= capacity;
+  if (words != nullptr) *words = word_per_cta ? (int)ctas : 0;
+  if (word_per_cta) amax_bits = cta_words;
   if (amax_bits != nullptr && !word_per_cta) {
     cudaError_t err = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int) * (unit_group != nullptr ? groups : 1), stream);
     if (err != cudaSuccess) return err;

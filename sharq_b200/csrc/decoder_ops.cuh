@@ -10,13 +10,13 @@ cudaError_t run_rope_inplace(void *x, long long rows, long long row_stride, int 
                              const void *cos_t, const void *sin_t, cudaStream_t stream);
 
 // h[rows, ffn] = silu(gate) * up from gate_up[rows, 2*ffn] (gate first); amax_bits (optional) is
-// zeroed and then raised to the bits of max|h| or, where it has room for a word per CTA (capacity words), gets every CTA's
-// maximum (*words of them, the largest is max|h|) and nothing has to be zeroed.
+// zeroed and then raised to the bits of max|h|, unless cta_words has room for a word per CTA (capacity words): then it is
+// not touched, cta_words gets every CTA's maximum (*words of them, the largest is max|h|; else *words = 0) and nothing is zeroed.
 // With unit_group (device, one int per 256 rows, < 0 = unit without rows) the rows are a grouped
 // activation: amax_bits has `groups` words, one per group, and rows of empty units are skipped.
 cudaError_t run_swiglu_absmax(const void *gate_up, long long rows, int ffn, long long row_stride, void *h,
                               unsigned int *amax_bits, cudaStream_t stream, const int *unit_group = nullptr, int groups = 1,
-                              int capacity = 0, int *words = nullptr);
+                              unsigned int *cta_words = nullptr, int capacity = 0, int *words = nullptr);
 
 // max|x| per group of a grouped bf16 activation [rows, width] into amax_bits[groups] (zeroed first).
 // With src_row, grouped row r is input row src_row[r] of x (< 0: a padding row without data).

@@ -953,7 +953,7 @@ int prepare_timeouts() {
 cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int m, int k, void *workspace,
                                float *inv_rms_external, void *a_comp, void *e, void *sfa_sparse, void *q_res,
                                void *sf_res, float *scale_out, cudaStream_t stream, int absmax_words,
-                               const void *residual, void *sum_out, size_t workspace_bytes) {
+                               const void *residual, void *sum_out, size_t workspace_bytes, unsigned int *amax_out) {
   const bool absmax_ready = absmax_words > 0;
   if (residual != nullptr && (gamma == nullptr || sum_out == nullptr)) return cudaErrorInvalidValue;
   // workspace: [0,4) tensor absmax bits; [256, 256+4m) inv_rms
@@ -1052,7 +1052,7 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   p.inv_rms = inv_rms;
   p.amax_bits = amax_bits;
   p.amax_words = words;
-  p.amax_out = word_per_cta && !absmax_ready && !inline_absmax ? static_cast<unsigned int *>(workspace) : nullptr;
+  p.amax_out = word_per_cta && !absmax_ready && !inline_absmax ? static_cast<unsigned int *>(workspace) : amax_out;
   p.scale_out = scale_out;
   p.a_comp = static_cast<uint8_t *>(a_comp);
   p.e = static_cast<uint8_t *>(e);

@@ -22,11 +22,13 @@ cudaError_t run_prepare(const void *x, int m, int k, void *a_comp, void *e, void
 // the workspace slot.  With absmax_words > 0 (gamma == nullptr only) the workspace already
 // holds the bits of max|x|, the largest of that many words, and the statistics pass is skipped.  With residual (RMSNorm path
 // only) the input is bf16(x + residual), which the statistics kernel also writes to sum_out.
+// amax_out (optional, with absmax_words) receives the bits of the largest word.
 // workspace_bytes beyond the minimum hold the maxima of the statistics kernel's CTAs (prepare_workspace_best_bytes).
 cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int m, int k, void *workspace,
                                float *inv_rms_external, void *a_comp, void *e, void *sfa_sparse, void *q_res,
                                void *sf_res, float *scale_out, cudaStream_t stream, int absmax_words = 0,
-                               const void *residual = nullptr, void *sum_out = nullptr, size_t workspace_bytes = 0);
+                               const void *residual = nullptr, void *sum_out = nullptr, size_t workspace_bytes = 0,
+                               unsigned int *amax_out = nullptr);
 
 // Tensor-scale prepare of a grouped activation (mixture-of-experts layers): rows sorted by group in
 // 256-row units (m a multiple of 256), unit_group[u] < 0 = unit without rows (its outputs are

@@ -168,7 +168,7 @@ std::vector<Tensor> swiglu_prepare(const Tensor &gate_up, int64_t n) {
   if (f2 % 2 != 0 || k % 128 != 0)
     fail("swiglu_sparse_residual_quantize_x requires K to be a multiple of 128, got " + std::to_string(k));
   const int64_t h_bytes = m * k * 2;
-  constexpr int64_t kWs = 8192;  // a word for the maximum of every CTA of the SwiGLU kernel
+  constexpr int64_t kWs = 256 + 8192;  // with a word for the maximum of every CTA of the SwiGLU kernel
   Prepared p(gate_up, m, k, kWs + 256 + h_bytes);
   c10::cuda::OptionalCUDAGuard guard(gate_up.device());
   check(sharq_swiglu_sparse_residual_quantize_x(ptr(gate_up), (int)m, (int)n, (int)k, p.tail() + kWs + 256, p.tail(), (size_t)kWs, p.a_comp(),

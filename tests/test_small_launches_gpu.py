@@ -97,3 +97,21 @@ def test_split_k_against_one_pass(m, n, k, monkeypatch):
         # cancels the orders of addition differ by K * 2^-24 of the terms, far below 2^-10 of the largest element
         d, size = (s.float() - w.float()).abs(), w.float().abs()
         assert bool((d <= size * 2.0 ** -7 + float(size.max()) * 2.0 ** -10).all())
+
+
+# one CTA, more CTAs than the smallest workspace has words; the smallest workspace, a word short of one per CTA, plenty
+@pytest.mark.parametrize("m,k", [(1, 128), (100, 4096), (700, 8192)])
+@pytest.mark.parametrize("ws_bytes", [256, 259, 260, 8192])
+def test_swiglu_prepare_leaves_the_absmax_in_the_first_word(m, k, ws_bytes):
+    from sharq_b200 import ops
+    from tests.gpu_util import Buf, call, dptr, sizes5, stream_ptr
+
+    gate_up = H.config0_x(m, 2 * k, seed=m).cuda()
+    bufs, ws, scale, h = [Buf(s) for s in sizes5(m, 128, k)], Buf(ws_bytes), Buf(4), Buf(m * k * 2)
+    call("sharq_swiglu_sparse_residual_quantize_x", dptr(gate_up), m, 128, k, h.ptr, ws.ptr, ws_bytes, *[b.ptr for b in bufs],
+         scale.ptr, stream_ptr())
+    want_h = ops.swiglu(gate_up)
+    want = ops.scaled_sparse_residual_quantize_x(want_h, 128)
+    assert ws.get()[:4].view(np.float32)[0] == float(want_h.float().abs().max())
+    assert scale.get().view(np.float32)[0] == float(want[5])
+    assert np.array_equal(bufs[3].get().ravel(), want[3].cpu().numpy().ravel())
