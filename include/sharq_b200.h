@@ -383,6 +383,9 @@ int sharq_set_wait_limit_cycles(long long cycles);
 /* Test/tuning hook: force the GEMM kernel variant (0 = automatic; 128 or 256 = single-CTA kernel
  * with that tile width; 512 = CTA-pair kernel, 256 x 256 tile per pair).  Process-wide. */
 int sharq_set_gemm_tile_n(int tile_n);
+/* Test/tuning hook: the variant that the automatic choice takes for a shape on a GPU of `sms` SMs (128, 256 or 512 as above);
+ * split_k: whether the call gives leave to split K.  Runs nothing. */
+int sharq_gemm_tile_n(int m, int n, int k, int split_k, int sms);
 
 #ifdef __cplusplus
 }

@@ -687,6 +687,10 @@ int sharq_linear_gemm_residual(const void *a_comp, const void *e, const void *sf
   return check_cuda(sharq::run_gemm(g, as_stream(stream)), "linear_gemm");
 }
 
+int sharq_gemm_tile_n(int m, int n, int k, int split_k, int sms) {
+  return m > 0 && n > 0 && k > 0 && sms > 0 ? sharq::gemm_tile_n(m, n, k, split_k != 0, sms) : 0;
+}
+
 int sharq_gemm_swiglu_pays(int m, int ffn, int k) { return m > 0 && ffn > 0 && k > 0 && sharq::gemm_swiglu_pays(m, ffn, k); }
 
 int sharq_gemm_swiglu_absmax_words(int m, int ffn) { return m > 0 && ffn > 0 ? sharq::gemm_swiglu_absmax_words(m, ffn) : 0; }

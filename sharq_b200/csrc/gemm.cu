@@ -1052,34 +1052,41 @@ cudaError_t run_gemm_grouped(const GroupedGemmArgs &a, cudaStream_t stream) {
   return e != cudaSuccess ? e : launch_grouped<true>(a, stream);
 }
 
-// Tile width of a fused or single GEMM (128 / 256 = single CTAs, 512 = CTA pairs of 256 x 256).
-static cudaError_t choose_tile_n(int m, int n, int k, int *tile_n) {
-  int dev = 0, sms = 0;
-  cudaError_t e = device_info(&dev, &sms);
-  if (e != cudaSuccess) return e;
+int gemm_tile_n(int m, int n, int k, bool split_k, int sms) {
   const int pair_units = ((m + 255) / 256) * ((n + 255) / 256);
   const int units_128 = ((m + 127) / 128) * ((n + 127) / 128);
+  const int units_256 = ((m + 127) / 128) * ((n + 255) / 256);
   if (m <= 128 || n <= 128) {
     // one row of tiles: narrow ones while they fit the GPU at once (split K fills it: 4096 x 4096 at M = 32 / 128 8.1 / 11.1 us
-    // against 9.7 / 16.3 with 256-wide tiles, 4096 x 14336 13.7 / 16.4 against 15.8 / 22.5); beyond that both take the
-    // same time (28672 x 4096) and the wide ones read the activation half as often
-    *tile_n = n > 128 && units_128 > sms ? 256 : 128;
-  } else if (pair_units * 4 <= sms || k <= 512 || units_128 <= sms) {
+    // against 9.7 / 16.3 with 256-wide tiles, 4096 x 14336 13.7 / 16.4 against 15.8 / 22.5; without split K 10.3 / 10.9 against
+    // 14.7 / 16.2 and 26.2 / 27.0 against 38.1 / 40.3); beyond that both take the same time (28672 x 4096) and the wide ones read the
+    // activation half as often
+    return n > 128 && units_128 > sms ? 256 : 128;
+  }
+  if (pair_units * 4 <= sms || k <= 512 || units_128 <= sms) {
     // 256 x 256 pair tiles would keep at most half of the SMs busy, or the K loop is too
     // short to hide the drain of a 256-wide accumulator: 128 x 128 tiles (measured at the
     // 8-way tensor-parallel shapes: 14.6 vs 18.8 us for N = 768, 12.7 vs 16.7 us for K = 512); also while these fit the GPU
-    // at once (6144 x 4096 at M = 384: 12.6 against 16.1 us).  Where K is long and they fill more than half of it, so that K is not
-    // split, 256-wide tiles with K split move fewer bytes through L2 (3584 x 18944 at M = 384: 30.0 against 36.4 us).
-    *tile_n = k > 16384 && 2 * units_128 > sms && units_128 <= sms ? 256 : 128;
-  } else {
-    *tile_n = 512;
+    // at once (6144 x 4096 at M = 384: 12.6 against 16.1 us).  Where these fill more than half of it, so that their K is not split, and
+    // 256-wide ones leave room for two CTAs per tile, the wide ones move fewer bytes through L2 and pay once a long K has
+    // earned back the cluster sum (128-wide / 256-wide with K split, us, 84 to 140 narrow tiles of N = 2560 to 5120: K = 8192
+    // 18.2 / 20.6, 12288 25.3 / 25.9, 14336 28.6 / 28.4, 16384 32.1 / 31.4, 18944 36.3 / 34.8; dense 16384 26.8 / 26.0, sparse 16384 21.5 / 21.4,
+    // 18944 24.2 / 23.3).  Unsplit they never do (18944: 51.9).
+    return split_k && k > 16384 && 2 * units_128 > sms && units_128 <= sms && 2 * units_256 <= sms ? 256 : 128;
   }
-  return cudaSuccess;
+  return 512;
+}
+
+static cudaError_t choose_tile_n(int m, int n, int k, bool split_k, int *tile_n) {
+  int dev = 0, sms = 0;
+  cudaError_t e = device_info(&dev, &sms);
+  if (e == cudaSuccess) *tile_n = gemm_tile_n(m, n, k, split_k, sms);
+  return e;
 }
 
 bool gemm_swiglu_pays(int m, int ffn, int k) {
   int tile_n = 0;
-  return ffn % 128 == 0 && choose_tile_n(m, 2 * ffn, k, &tile_n) == cudaSuccess && tile_n == 512;
+  return ffn % 128 == 0 && choose_tile_n(m, 2 * ffn, k, true, &tile_n) == cudaSuccess && tile_n == 512;
 }
 
 cudaError_t run_gemm_swiglu(const GemmArgs &a, cudaStream_t stream) {
@@ -1103,7 +1110,7 @@ cudaError_t run_gemm(const GemmArgs &a, cudaStream_t stream) {
   // tile_n: 0 = automatic, 128 / 256 = single-CTA tiles of that width, 512 = CTA pairs (256 x 256)
   int tile_n = a.tile_n;
   if (tile_n == 0) {
-    cudaError_t e = choose_tile_n(a.m, a.n, a.k, &tile_n);
+    cudaError_t e = choose_tile_n(a.m, a.n, a.k, a.split_k && a.scatter_world <= 1, &tile_n);
     if (e != cudaSuccess) return e;
   }
   const bool pair = tile_n == 512;

@@ -42,6 +42,9 @@ struct GemmArgs {
 
 cudaError_t run_gemm(const GemmArgs &args, cudaStream_t stream);
 
+// Tile width that run_gemm takes on a GPU of `sms` SMs: 128 / 256 = single CTAs, 512 = CTA pairs of 256 x 256.
+int gemm_tile_n(int m, int n, int k, bool split_k, int sms);
+
 // Fused SharQ GEMM of a merged gate_up weight [2F, k] (n = 2F, F % 128 == 0, no bias) whose epilogue writes
 // h = bf16(bf16(silu(gate)) * up) [m, F] to d and every CTA's max|h| to amax_bits (nothing to zero before the launch): the h that the plain
 // GEMM followed by the SwiGLU kernel gives.
