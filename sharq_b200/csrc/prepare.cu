@@ -235,9 +235,11 @@ struct PrepareParams {
 
 constexpr int kPrepareCtasPerSm = 3;
 constexpr int kScaledCtasPerSm = 2;  // tensor-scale mode without a gather
-// Up to this size every CTA scans the whole input for its maximum (us per launch at K = 4096, scan / statistics launch and
-// prepare: 16 rows 5.3 / 5.6, 32 rows 8.1 / 5.3).
+// Up to this size every CTA scans the whole input for its maximum.  us per call in a graph, scan / statistics launch and prepare: 16 x 4096
+// 4.5 / 4.9, 17 x 4096 5.1 / 4.6, 32 x 4096 6.7 / 4.7.  Without room for a word per CTA the other form is a cooperative launch behind
+// a memset, and the scan pays longer: 17 x 4096 5.1 / 8.4, 8 x 14336 6.4 / 10.3, 48 x 4096 8.5 / 8.4, 64 x 4096 10.4 / 8.4.
 constexpr size_t kInlineAbsmaxElements = 64 * 1024;
+constexpr size_t kInlineAbsmaxElementsNoWords = 192 * 1024;
 constexpr unsigned kMaxAbsmaxWords = 4096;            // words of CTA maxima that every prepare CTA reduces
 
 // kCtas: resident CTAs per SM the register allocation aims at.  The tensor-scale mode runs
@@ -962,8 +964,6 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
                                     : reinterpret_cast<float *>(static_cast<uint8_t *>(workspace) + 256);
   cudaError_t err = cudaSuccess;
   const bool rms = gamma != nullptr;
-  // a small non-RMSNorm input (a decode step): the prepare kernel finds max|x| itself
-  const bool inline_absmax = !rms && !absmax_ready && (size_t)m * k <= kInlineAbsmaxElements;
   const size_t elements = (size_t)m * (size_t)k;
   // statistics kernel: one CTA per row (RMSNorm) or a flat grid; its CTAs' maxima go behind the row statistics, where the
   // caller's workspace has room for a word each
@@ -973,6 +973,9 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   const unsigned stat_ctas = rms ? (unsigned)m : (unsigned)(flat < (size_t)sms * 8 ? flat : (size_t)sms * 8);
   const size_t words_at = 256 + (rms && inv_rms_external == nullptr ? (size_t)m * sizeof(float) : 0);
   const bool word_per_cta = stat_ctas <= kMaxAbsmaxWords && workspace_bytes >= words_at + (size_t)stat_ctas * sizeof(float);
+  // a small non-RMSNorm input (a decode step): the prepare kernel finds max|x| itself
+  const bool inline_absmax =
+      !rms && !absmax_ready && elements <= (word_per_cta ? kInlineAbsmaxElements : kInlineAbsmaxElementsNoWords);
   // Two launches that overlap, with nothing to zero, beat one cooperative launch behind its memset (us, two launches / one: tensor scale
   // 64 x 4096 5.3 / 8.7, 2048 x 4096 12.0 / 16.9, 4096 x 4096 19.6 / 27.1; RMSNorm 32 x 4096 7.4 / 10.5, 512 x 4096 9.8 / 12.9, 4096 x 4096
   // 30.1 / 33.5), except with the residual add on middle sizes, where the row caches spare the second read of the sum: 512 x 4096

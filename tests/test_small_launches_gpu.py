@@ -115,3 +115,22 @@ def test_swiglu_prepare_leaves_the_absmax_in_the_first_word(m, k, ws_bytes):
     assert ws.get()[:4].view(np.float32)[0] == float(want_h.float().abs().max())
     assert scale.get().view(np.float32)[0] == float(want[5])
     assert np.array_equal(bufs[3].get().ravel(), want[3].cpu().numpy().ravel())
+
+
+# the largest input that is scanned by the prepare itself and one row more, with and without room for the CTAs' maxima; the
+# workspace is written only where there is a statistics pass
+@pytest.mark.parametrize("m,k,minimal,scanned", [(16, 4096, False, True), (17, 4096, False, False), (17, 4096, True, True),
+                                                 (48, 4096, True, True), (49, 4096, True, False), (13, 14336, True, True)])
+def test_small_input_is_scanned_by_the_prepare(oracle, m, k, minimal, scanned):
+    from sharq_b200 import _lib
+    from tests.gpu_util import Buf, SENTINEL, call, dptr, sizes5, stream_ptr
+
+    x = H.config0_x(m, k, seed=m)
+    ws_bytes = 256 if minimal else int(_lib.lib().sharq_prepare_workspace_best_bytes(m))
+    bufs, ws, scale, xd = [Buf(s) for s in sizes5(m, 128, k)], Buf(ws_bytes), Buf(4), x.cuda()
+    call("sharq_scaled_sparse_residual_quantize_x", dptr(xd), m, 128, k, ws.ptr, ws_bytes, *[b.ptr for b in bufs], scale.ptr,
+         stream_ptr())
+    assert bool((ws.get()[:4] == SENTINEL).all()) == scanned
+    s = oracle.tensor_scale(oracle.absmax_bf16(H.bits(x)), cuda_mode=True)
+    assert scale.get().view(np.float32)[0] == s
+    _compare([b.get() for b in bufs], oracle.prepare(oracle.scale_bf16(H.bits(x), s, cuda_mode=True)), f"scaled {m}x{k}")
