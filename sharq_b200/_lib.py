@@ -130,8 +130,13 @@ def native():
         import torch  # noqa: F401  (the binding links against its libraries)
 
         lib()  # the library it calls; also the check that the build is there
+        from . import _build
+
         if not NATIVE_PATH.exists():
             raise ImportError(f"{NATIVE_PATH} is missing: build it with `python -m sharq_b200._build`")
+        if not _build.binding_matches():
+            raise ImportError(f"{NATIVE_PATH} was built against another torch or Python than the running {_build.binding_tag()}: "
+                              "build it again with `python -m sharq_b200._build`")
         spec = importlib.util.spec_from_file_location("sharq_native", NATIVE_PATH)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
