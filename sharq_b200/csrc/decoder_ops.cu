@@ -412,10 +412,11 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(__nv_bfloat16 *__restr
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       for (int j = 0; j < top_k; ++j) {
         const int slot = order[j];
-        const float wj = __bfloat162float(w[t * top_k + slot]);
+        // a missing slot reads row 0 with a NaN weight (a branch around the load: 63 instead of 49 us at 8192 x 4096)
         const int from = dest[t * top_k + slot];
-        const uint4 yv = from >= 0 ? __ldg(reinterpret_cast<const uint4 *>(y + (long long)from * width) + v)
-                                   : make_uint4(0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u, 0x7fc07fc0u);
+        const uint32_t w_bits = (uint32_t)__bfloat16_as_ushort(w[t * top_k + slot]) << 16;
+        const float wj = __uint_as_float(w_bits | (uint32_t)((from >> 31) & 0x7fff0000));  // all ones: NaN
+        const uint4 yv = __ldg(reinterpret_cast<const uint4 *>(y + (long long)max(from, 0) * width) + v);
         const uint32_t yw[4] = {yv.x, yv.y, yv.z, yv.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
