@@ -44,15 +44,25 @@ __device__ __forceinline__ float rope1(float x, float r, float c, float s) {
 // A thread rotates 8 elements of the first half of a head with their 8 partners in the
 // second half (rotate_half pairs element d with d + D/2).  One CTA per row, one thread per 16-byte vector of the row's
 // half heads: the row, its position and the head are found without 64-bit divisions per vector, which bound the kernel
-// when a grid-stride loop took the vectors of all rows (16384 rows x 32 heads x 128: 63 -> 53 us, 5.1 TB/s).
-__global__ void __launch_bounds__(1024) rope_kernel(__nv_bfloat16 *__restrict__ x, long long row_stride, int seq_len, int heads,
-                                                    int head_dim, const __nv_bfloat16 *__restrict__ cos_t,
+// when a grid-stride loop took the vectors of all rows (16384 rows x 32 heads x 128: 63 -> 53 us, 5.1 TB/s).  Rows of many
+// vectors loop in CTAs of 256 threads, several per row while there are few rows; short rows share a CTA (see run_rope_inplace).
+template <bool kShortRows>
+__global__ void __launch_bounds__(512) rope_kernel(__nv_bfloat16 *__restrict__ x, long long row_stride, unsigned rows,
+                                                    unsigned rows_per_cta, int seq_len, int heads, int head_dim,
+                                                    const __nv_bfloat16 *__restrict__ cos_t,
                                                     const __nv_bfloat16 *__restrict__ sin_t) {
   const int half = head_dim >> 1;
   const unsigned vecs = (unsigned)half >> 3;  // 16-byte vectors per half head
-  const unsigned row = blockIdx.x;
+  const unsigned per_row = (unsigned)heads * vecs;
+  unsigned i = blockIdx.y * blockDim.x + threadIdx.x, row = blockIdx.x;
+  if (kShortRows) {
+    const unsigned in_cta = i / per_row;
+    i -= in_cta * per_row;
+    row = row * rows_per_cta + in_cta;
+    if (in_cta >= rows_per_cta || row >= rows) return;
+  }
   const size_t table = (size_t)(row % (unsigned)seq_len) * head_dim;
-  for (unsigned i = threadIdx.x; i < (unsigned)heads * vecs; i += blockDim.x) {
+  for (; i < per_row; i += gridDim.y * blockDim.x) {
     const unsigned head = i / vecs, v = i % vecs;
     __nv_bfloat16 *p = x + row * row_stride + (size_t)head * head_dim + v * 8;
     const __nv_bfloat16 *c = cos_t + table + v * 8;
@@ -481,11 +491,23 @@ int sm_count() {
 cudaError_t run_rope_inplace(void *x, long long rows, long long row_stride, int seq_len, int heads, int head_dim,
                              const void *cos_t, const void *sin_t, cudaStream_t stream) {
   if (rows <= 0 || rows > 0x7fffffffLL) return cudaErrorInvalidValue;
-  int threads = (heads * (head_dim / 16) + 31) / 32 * 32;
-  if (threads > 1024) threads = 256;
-  rope_kernel<<<(unsigned)rows, threads, 0, stream>>>(static_cast<__nv_bfloat16 *>(x), row_stride, seq_len, heads, head_dim,
-                                                      static_cast<const __nv_bfloat16 *>(cos_t),
-                                                      static_cast<const __nv_bfloat16 *>(sin_t));
+  // A thread per vector up to 512.  Beyond, CTAs of 256 threads that loop, and enough of them per row to fill the SMs (us, 136 heads x 128:
+  // 1 row in one CTA 4.7, in five 2.2; 16384 rows 204 and 238; 128 heads x 128, 16384 rows in CTAs of 1024 threads 345).  Rows of fewer
+  // than 64 vectors share a CTA (3 heads x 16, 16384 rows: a CTA each 10.0, this 2.8).
+  const long long per_row = (long long)heads * (head_dim / 16);
+  const int rows_per_cta = per_row < 64 ? (int)(128 / per_row) : 1;
+  const int threads = per_row > 512 ? 256 : (int)((rows_per_cta * per_row + 31) / 32 * 32);
+  long long pieces = 1;
+  if (per_row > 512) {
+    const long long most = (per_row + 255) / 256, fill = (8LL * sm_count() + rows - 1) / rows;
+    pieces = most < fill ? most : fill;
+    if (pieces > 65535) pieces = 65535;
+  }
+  const dim3 grid((unsigned)((rows + rows_per_cta - 1) / rows_per_cta), (unsigned)pieces);
+  const auto kernel = rows_per_cta > 1 ? rope_kernel<true> : rope_kernel<false>;
+  kernel<<<grid, threads, 0, stream>>>(static_cast<__nv_bfloat16 *>(x), row_stride, (unsigned)rows, (unsigned)rows_per_cta, seq_len,
+                                       heads, head_dim, static_cast<const __nv_bfloat16 *>(cos_t),
+                                       static_cast<const __nv_bfloat16 *>(sin_t));
   return cudaGetLastError();
 }
 

@@ -37,6 +37,21 @@ def test_rope_inplace_equals_aten(b, s, heads, kv, d):
     assert torch.equal(got[:, nq + nk:], v_before)  # value heads untouched
 
 
+# heads * head_dim / 16 vectors of a row: 1 and 63 (rows share a CTA, the last one ragged), 64 and 512 (a CTA each), 520, 1088 and
+# 2048 (several CTAs of a row, or a loop)
+@pytest.mark.parametrize("s,heads,d", [(1, 1, 16), (300, 1, 16), (41, 63, 16), (41, 64, 16), (3, 64, 128), (3, 65, 128), (7, 136, 128),
+                                       (1, 128, 256), (700, 136, 128), (1500, 65, 128)])
+def test_rope_of_short_and_long_rows(s, heads, d):
+    from sharq_b200 import ops
+    from sharq_b200.decoder import apply_rope
+
+    qkv = torch.randn(s, (heads + 1) * d, generator=torch.Generator().manual_seed(s)).to(torch.bfloat16).cuda()
+    cos, sin = _rope_tables(s, d)
+    want = apply_rope(qkv[:, :heads * d].view(1, s, heads, d).transpose(1, 2), cos, sin).transpose(1, 2).reshape(s, heads * d)
+    got = ops.rope_inplace_(qkv.clone(), heads, d, cos, sin, s)
+    assert torch.equal(got[:, :heads * d], want) and torch.equal(got[:, heads * d:], qkv[:, heads * d:])
+
+
 @pytest.mark.parametrize("m,f", [(2048, 14336), (300, 1024), (17, 128)])
 def test_swiglu_equals_aten(m, f):
     from sharq_b200 import ops
