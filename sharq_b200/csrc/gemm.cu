@@ -229,6 +229,57 @@ __device__ __forceinline__ void store_8(const GemmParams &p, uint32_t (&o)[4], i
   }
 }
 
+// epilogue_8 on 32 columns.  Where all of them exist the loads of C_in (and then of the bias) are issued together: a load and its
+// checks per 8 columns cost a latency each (28672 x 4096 at M = 127 with C_in 18.3 against 16.6 us).
+__device__ __forceinline__ void epilogue_32(const GemmParams &p, const uint32_t *acc, int row, int col0, float alpha, float beta,
+                                            bool has_c, uint32_t (&o)[4][4]) {
+  const bool vec = col0 + 32 <= p.n && (p.n & 7) == 0 &&
+                   ((reinterpret_cast<uintptr_t>(p.c_in) | reinterpret_cast<uintptr_t>(p.bias)) & 15) == 0;
+  if (!vec) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      float f[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(acc[8 * v + i]);
+      epilogue_8(p, f, row, col0 + 8 * v, alpha, beta, has_c, o[v]);
+    }
+    return;
+  }
+  auto pack = [](float a, float b) {
+    __nv_bfloat162 pair = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t *>(&pair);
+  };
+  if (has_c) {
+    const uint4 *c = reinterpret_cast<const uint4 *>(p.c_in + (size_t)row * p.n + col0);
+    const uint4 cv[4] = {c[0], c[1], c[2], c[3]};
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const uint32_t cw[4] = {cv[v].x, cv[v].y, cv[v].z, cv[v].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        o[v][i] = pack(__fmaf_rn(beta, bf16_bits_to_float(cw[i] & 0xFFFFu), alpha * __uint_as_float(acc[8 * v + 2 * i])),
+                       __fmaf_rn(beta, bf16_bits_to_float(cw[i] >> 16), alpha * __uint_as_float(acc[8 * v + 2 * i + 1])));
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      o[i >> 2][i & 3] = pack(alpha * __uint_as_float(acc[2 * i]), alpha * __uint_as_float(acc[2 * i + 1]));
+  }
+  if (p.bias != nullptr) {
+    const uint4 *b = reinterpret_cast<const uint4 *>(p.bias + col0);
+    const uint4 bv[4] = {b[0], b[1], b[2], b[3]};
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const uint32_t bw[4] = {bv[v].x, bv[v].y, bv[v].z, bv[v].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 sum = __hadd2(*reinterpret_cast<__nv_bfloat162 *>(&o[v][i]), *reinterpret_cast<const __nv_bfloat162 *>(&bw[i]));
+        o[v][i] = *reinterpret_cast<const uint32_t *>(&sum);
+      }
+    }
+  }
+}
+
 // Epilogue of 32 accumulator columns held in registers; rows >= M and columns >= N are masked.  A thread owns one row
 // and stores 64 contiguous bytes.
 // With `stage` non-null the 64 bytes go to row `stage_row` of a 32-row x 64-byte shared-memory
@@ -242,13 +293,11 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams &p, const uint32
                                                int chunk_base = 0) {
   if (stage == nullptr && (row >= p.m || col0 >= p.n)) return;
   if (row >= p.m || col0 >= p.n) has_c = false;  // masked by the caller's store; C_in must not be read out of range
+  uint32_t all[4][4];
+  epilogue_32(p, acc, row, col0, alpha, beta, has_c, all);
 #pragma unroll
   for (int v = 0; v < 4; ++v) {  // 8 columns per 16-byte store
-    float f[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = __uint_as_float(acc[8 * v + i]);
-    uint32_t o[4];
-    epilogue_8(p, f, row, col0 + 8 * v, alpha, beta, has_c, o);
+    uint32_t(&o)[4] = all[v];
     if (stage != nullptr) {
       uint8_t *slot = kWide ? stage + stage_row * 128 + (((chunk_base + v) ^ (stage_row & 7)) << 4)
                             : stage + stage_row * 64 + ((v ^ ((stage_row >> 1) & 3)) << 4);
