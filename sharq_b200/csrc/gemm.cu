@@ -996,9 +996,16 @@ cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
     // takes as many SMs as possible): the most CTAs per tile for which all clusters run at the same time, each
     // with at least two K stages.  Sums through distributed shared memory took the place of a memset, fp32 atomics and a
     // second kernel (4.5 us of 20 per launch at M = 32), for which only M <= 64 or K >= 8192 had paid.
-    if (a.split_k && a.scatter_world <= 1) {
+    // The sum costs more the more rows a tile has and is set against K stages of 0.40 us (fused), 0.30 (dense) or 0.23 (sparse): split / one
+    // pass of 4096 x 1024 at M = 129 took 8.6 / 6.4 us, 768 x 4096 sparse at M = 256 10.9 / 8.0, 1024 x 2048 at M = 64 7.0 / 7.2 and at M = 1 5.0 / 7.0,
+    // 512 x 8192 at M = 256 12.1 / 16.8.  The line below lies within 6 % of the better form over M = 1 to 512, N = 128 to 6144, K = 512 to
+    // 14336, but for 11 % at 16 x 4096 x 2048 sparse.  Rows of D that allow no 16-byte stores (N % 8 != 0) are always better dealt over
+    // the threads of a cluster (300 x 1152 at M = 128 9.0 / 23.1 us).
+    const int k_stages = (a.k + kBK - 1) / kBK;
+    const int rows = a.m < kBM ? a.m : kBM;
+    const bool split_pays = p.staged_store == 0 || k_stages >= 4 + rows / (SPARSE && DENSE ? 9 : (DENSE ? 8 : 5));
+    if (a.split_k && split_pays && a.scatter_world <= 1) {
       static int capacity[64][kMaxSplits + 1] = {};  // clusters of a size that the device holds at once; 0 = not asked yet
-      const int k_stages = (a.k + kBK - 1) / kBK;
       int s = k_stages / 2 < kMaxSplits ? k_stages / 2 : kMaxSplits;
       if (s > sms / units) s = sms / units;
       for (; s >= 2; --s) {

@@ -99,6 +99,13 @@ def test_split_k_against_one_pass(m, n, k, monkeypatch):
         assert bool((d <= size * 2.0 ** -7 + float(size.max()) * 2.0 ** -10).all())
 
 
+# full tiles on both sides of the K from which the fused (18 stages of 256), dense (20) and sparse (29) GEMM are split, with a ragged last stage
+@pytest.mark.parametrize("m", [128, 300])
+@pytest.mark.parametrize("n,k", [(264, 4480), (300, 5248), (264, 7552)])
+def test_split_k_of_full_tiles_against_one_pass(m, n, k, monkeypatch):
+    test_split_k_against_one_pass(m, n, k, monkeypatch)
+
+
 # one CTA, more CTAs than the smallest workspace has words; the smallest workspace, a word short of one per CTA, plenty
 @pytest.mark.parametrize("m,k", [(1, 128), (100, 4096), (700, 8192)])
 @pytest.mark.parametrize("ws_bytes", [256, 259, 260, 8192])
