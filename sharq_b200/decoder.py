@@ -234,10 +234,11 @@ class SharqDecoderLayer(torch.nn.Module):
             x2 = x2 + o
             prep = self.gate_up.prepare_input_rmsnorm(x2, self.post_norm, cfg.eps)
         if self.fused_glue:
-            prep = _prepare_down(self.gate_up, prep, self.down.local)
-            if not return_delta and isinstance(self.down, RowParallelSharqLinear):
-                return self.down.apply_prepared_residual(prep, x2).view(b, s, h)
-            d = self.down.apply_prepared_reduced(prep)
+            down = self.down
+            prep = _prepare_down(self.gate_up, prep, down.local)
+            if not return_delta and isinstance(down, RowParallelSharqLinear):
+                return down.apply_prepared_residual(prep, x2).view(b, s, h)
+            d = down.apply_prepared_reduced(prep)
         else:
             gu = self.gate_up.apply_prepared(prep)
             f = gu.shape[1] // 2

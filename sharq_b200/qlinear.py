@@ -33,8 +33,11 @@ def methods_kept(layer, own: dict, *names: str) -> bool:
     """Whether the methods `names` of layer are the functions of `own`: neither overridden by a subclass, nor replaced on the
     class (a profiler's wrappers), nor set on the instance.  A call that does the work of several methods at once
     is taken only then."""
-    methods = (getattr(layer, name, None) for name in names)
-    return all(getattr(m, "__func__", None) is own[name] and m.__self__ is layer for m, name in zip(methods, names))
+    cls, instance = type(layer), getattr(layer, "__dict__", ())
+    for name in names:  # 0.3 us for two; a generator over bound methods took 1.3 us of a 20 us call
+        if name in instance or getattr(cls, name, None) is not own[name]:
+            return False
+    return True
 
 
 class QLinearLayer(nn.Module):

@@ -34,6 +34,8 @@ import torch
 import torch.distributed as dist
 import torch.nn as nn
 
+from .qlinear import QLINEAR_METHODS, QLinearLayer, methods_kept
+
 K_ALIGN = 128  # the prepare kernels need K % 128 == 0 per shard
 N_ALIGN = 128  # scale-factor tiles cover 128 rows
 
@@ -367,7 +369,6 @@ class ColumnParallelSharqLinear(_ShardedBase):
     def __init__(self, weight: torch.Tensor, bias: Optional[torch.Tensor] = None, group=None, fused_gemm: bool = True):
         super().__init__(group)
         from . import ops
-        from .qlinear import QLinearLayer
 
         n, k = weight.shape
         b, e = shard_bounds(n, self.world, self.rank, N_ALIGN)
@@ -403,7 +404,6 @@ class RowParallelSharqLinear(_ShardedBase):
         several ranks in one process)."""
         super().__init__(group)
         from . import ops
-        from .qlinear import QLinearLayer
 
         if world_rank is not None:
             self.world, self.rank = int(world_rank[0]), int(world_rank[1])
@@ -454,12 +454,11 @@ class RowParallelSharqLinear(_ShardedBase):
     def apply_prepared_residual(self, prepared, residual: torch.Tensor) -> torch.Tensor:
         """residual + apply_prepared_reduced(prepared).  Where nothing is summed over ranks or added in between, the
         add rides in the epilogue of the fused GEMM (same bits)."""
-        from .qlinear import QLINEAR_METHODS, methods_kept
-
+        local = self.local
         if (self.world == 1 and self.reduce_hook is None and self.bias is None
                 and methods_kept(self, _ROW_PARALLEL_METHODS, "reduce", "apply_prepared_reduced")
-                and methods_kept(self.local, QLINEAR_METHODS, "apply_prepared")):
-            return self.local.apply_prepared(prepared, residual=residual)
+                and methods_kept(local, QLINEAR_METHODS, "apply_prepared")):
+            return local.apply_prepared(prepared, residual=residual)
         return residual + self.apply_prepared_reduced(prepared)
 
     def forward(self, x_local):
