@@ -59,19 +59,19 @@ int sharq_fused_sparse_residual_quantize_x_debug(const void *x_bf16, int m, int 
  * bytes [0,4) tensor absmax (float bits), bytes [4,8) arrival counter of the grid-wide barrier,
  * bytes [256, 256+4*M) per-row inv_rms (float).  The calls initialise what they use. */
 size_t sharq_prepare_workspace_bytes(int m);
-/* With this many bytes the prepares of some sizes save a memset between their launches. */
+/* With this many bytes (room for a maximum per CTA of the statistics launch, up to 4096 of them) nothing is zeroed between the launches. */
 size_t sharq_prepare_workspace_best_bytes(int m);
 
-/* The scaled prepare calls run statistics and quantisation in ONE cooperative launch whose CTAs
- * meet at a grid-wide barrier with a bounded wait (about one second).  Returns how many such
+/* A scaled prepare call runs its statistics and its quantisation as two launches or, with the smaller workspace and with the
+ * residual add on middle sizes, as one cooperative launch whose CTAs meet at a grid-wide barrier with a bounded wait (about one
+ * second).  Returns how many such
  * waits ran out on the current device since the library was loaded: 0 in a healthy process (the
  * outputs of a call that timed out are undefined), -1 if the counter cannot be read.  Synchronises
  * nothing itself: call it after synchronising the stream.  No counterpart in the reference. */
 int sharq_prepare_timeouts(void);
 
 /* fused_rmsnorm_sparse_residual_quantize_x(X, rmsnorm_weight, eps, N): RMSNorm, tensor
- * scale = clamp(amax/2688, 1e-9) and prepare: an 8-byte memset and one cooperative launch (row
- * statistics, grid barrier, quantisation; the rows of a CTA stay in shared memory in between).
+ * scale = clamp(amax/2688, 1e-9) and prepare, in two launches or one (see sharq_prepare_timeouts).
  * The normalised values are divided by the float32 scale, as the reference's kernel does
  * (kernels/src/fused_rmsnorm_sparse_prepare.cu:195-204).
  * K % 128 == 0 and K/32 <= 1024.  scale_out: one device float.  bindings.cpp:291-355 */
@@ -118,7 +118,8 @@ int sharq_scaled_sparse_residual_quantize_x(const void *x_bf16, int m, int n, in
  * scaled prepare of H for down_proj in two launches instead of the reference's five passes
  * (silu, mul, amax, divide, prepare): the SwiGLU kernel leaves max|H| in the workspace, so
  * the statistics pass of sharq_scaled_sparse_residual_quantize_x is not needed.  Outputs
- * equal sharq_scaled_sparse_residual_quantize_x(H). */
+ * equal sharq_scaled_sparse_residual_quantize_x(H).  workspace: 256 bytes, whose first word gets the bits of max|H|; with 8 KB behind them
+ * (a maximum per CTA) nothing is zeroed first. */
 int sharq_rope_inplace(void *x_bf16, int rows, int row_stride, int seq_len, int heads, int head_dim,
                        const void *cos_bf16, const void *sin_bf16, void *stream);
 /* sharq_scatter_add_scaled: out[rows[i], :] += y[i, :] * w[i] in bf16 with the roundings of

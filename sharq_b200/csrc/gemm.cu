@@ -929,7 +929,8 @@ cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
     return cudaErrorInvalidValue;
   // With one tile of rows only those that exist are loaded (whole 8-row groups of the swizzle): a 128-row box of a decode batch
   // is mostly zero fill, 24 of the 67 KB that a stage writes to shared memory.  The MMA then reads stale bytes for
-  // the other rows; FP4 has no NaN, their scales are zero, and their outputs are masked.
+  // the other rows, and whatever scales their padding holds (the dense quantisation leaves it unwritten): the rows of an
+  // accumulator are independent, and those are masked.
   const int a_rows = !PAIR && a.m < kBM ? (a.m + 7) / 8 * 8 : kBM;
   if (DENSE && !make_tmap_bytes(&tm_ad, a.a_dense, (uint64_t)a.m, (uint64_t)a.k / 2, a_rows, 128, CU_TENSOR_MAP_SWIZZLE_128B))
     return cudaErrorInvalidValue;
@@ -974,7 +975,7 @@ cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
   const int units = m_units * n_tiles;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  // see grid_dependency_wait in gemm_body; the linears of a 32-token decode step, with split K and the cluster prepare: 123 -> 100 us
+  // see grid_dependency_wait in gemm_body; the linears of a 32-token decode step 90.8 -> 83.6 us, of 2048 tokens 429.6 -> 423.6
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;

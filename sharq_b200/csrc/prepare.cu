@@ -977,9 +977,9 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   const bool inline_absmax =
       !rms && !absmax_ready && elements <= (word_per_cta ? kInlineAbsmaxElements : kInlineAbsmaxElementsNoWords);
   // Two launches that overlap, with nothing to zero, beat one cooperative launch behind its memset (us, two launches / one: tensor scale
-  // 64 x 4096 5.3 / 8.7, 2048 x 4096 12.0 / 16.9, 4096 x 4096 19.6 / 27.1; RMSNorm 32 x 4096 7.4 / 10.5, 512 x 4096 9.8 / 12.9, 4096 x 4096
-  // 30.1 / 33.5), except with the residual add on middle sizes, where the row caches spare the second read of the sum: 512 x 4096
-  // 12.2 / 14.4, 2048 x 4096 27.3 / 25.2, 4096 x 4096 51.0 / 49.8.  Without room for the words the memset precedes both forms, and
+  // 64 x 4096 5.0 / 8.4, 2048 x 4096 12.0 / 16.9, 4096 x 4096 19.6 / 27.1; RMSNorm 33 x 4096 7.0 / 10.5, 512 x 4096 9.1 / 12.5, 4096 x 4096
+  // 29.8 / 33.0), except with the residual add on middle sizes, where the row caches spare the second read of the sum: 512 x 4096
+  // 10.8 / 12.7, 2048 x 4096 24.7 / 24.9, 2048 x 8192 49.4 / 45.6, 700 x 14336 37.2 / 30.7.  Without room for the words the memset precedes both forms, and
   // one launch pays while the row caches hold most of the tensor.
   const bool one_launch_pays =
       fused_prepare_enabled() && (word_per_cta ? residual != nullptr && elements >= ((size_t)1 << 22) && elements < ((size_t)1 << 25)

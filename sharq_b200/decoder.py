@@ -326,7 +326,7 @@ class SharqDecoderLayer(torch.nn.Module):
     def _moe_grouped(self, hn: torch.Tensor, routing: torch.Tensor, selected: torch.Tensor,
                      residual: torch.Tensor = None) -> torch.Tensor:
         """All experts in grouped launches with no host synchronisation (so the layer can be captured in a
-        CUDA graph): the token slots are sorted by expert on the device (ATen sort / cumsum: plumbing),
+        CUDA graph): the token slots are grouped by expert on the device (moe_grouping),
         every expert's segment is padded to 256 rows, and gather -> prepare -> gate_up GEMM -> SwiGLU +
         prepare -> down GEMM -> weighted combine each run once for all experts.  Same arithmetic per
         token as the per-expert loop (each expert's rows get that expert's own tensor scales)."""

@@ -124,8 +124,8 @@ def test_gemm_argument_errors():
 
 @pytest.mark.parametrize("m,n,k", [(16, 6144, 4096), (128, 4096, 14336), (100, 1000, 1024), (1, 4096, 4096)])
 def test_small_m_split_k_agrees_with_single_pass(oracle, m, n, k, monkeypatch):
-    """M <= 128 with caller scratch: K split over the SMs (fp32 vector reductions + a finalize
-    kernel with alpha / beta / bias) against the same GEMM computed in one pass per tile, and
+    """M <= 128 with leave to split K: K dealt over the CTAs of a cluster, which sum their partial tiles on
+    chip, against the same GEMM computed in one pass per tile, and
     both against the float32 product of the dequantised operands (plain PyTorch index
     arithmetic, no kernel of this project) at the real decode-step shapes."""
     from sharq_b200 import ops
