@@ -27,6 +27,7 @@ from dataclasses import dataclass
 import torch
 import torch.nn.functional as F
 
+from . import ops
 from .qlinear import QLinearLayer, methods_kept
 from .tp import RowParallelSharqLinear, head_layout, padded_size, shard_bounds
 
@@ -214,8 +215,6 @@ class SharqDecoderLayer(torch.nn.Module):
         o = self.o_proj(attn2)
         if cfg.experts > 0:
             if self.fused_glue and h <= 8192:
-                from . import ops
-
                 # residual add + norm in one launch (the router and the experts read hn)
                 hn, x2 = ops.add_rmsnorm(o.contiguous(), self.post_norm, cfg.eps, residual=x2.contiguous())
             else:
@@ -308,8 +307,6 @@ class SharqDecoderLayer(torch.nn.Module):
                 f = gu.shape[1] // 2
                 y = down.apply_prepared(down.prepare_input((F.silu(gu[:, :f]) * gu[:, f:]).contiguous()))
             if self.fused_glue:
-                from . import ops
-
                 ops.scatter_add_scaled_(out, y, top_x.contiguous(), routing[top_x, idx].contiguous())
             else:
                 out.index_add_(0, top_x, y * routing[top_x, idx, None])
@@ -330,8 +327,6 @@ class SharqDecoderLayer(torch.nn.Module):
         every expert's segment is padded to 256 rows, and gather -> prepare -> gate_up GEMM -> SwiGLU +
         prepare -> down GEMM -> weighted combine each run once for all experts.  Same arithmetic per
         token as the per-expert loop (each expert's rows get that expert's own tensor scales)."""
-        from . import ops
-
         cfg = self.cfg
         m, h = hn.shape
         e, k = cfg.experts, cfg.top_k
@@ -469,8 +464,6 @@ def moe_grouping(selected: torch.Tensor, experts: int, unit: int = 256):
     dev = selected.device
     slots = tokens * k
     if selected.is_cuda and slots > 0 and experts <= 16:
-        from . import ops
-
         return ops.moe_plan(selected.contiguous(), experts, unit)
     rows = ((slots + unit - 1) // unit + experts) * unit
     flat = selected.reshape(-1)
@@ -511,8 +504,6 @@ def _split_heads(qkv: torch.Tensor, b: int, s: int, heads: int, kv_heads: int, d
     views.  fused: one in-place kernel on the q and k columns; else the ATen composition."""
     nq, nk = heads * d, kv_heads * d
     if fused and qkv.is_cuda:
-        from . import ops
-
         ops.rope_inplace_(qkv, heads + kv_heads, d, cos, sin, s)
     q = qkv[:, :nq].view(b, s, heads, d).transpose(1, 2)
     k = qkv[:, nq:nq + nk].view(b, s, kv_heads, d).transpose(1, 2)
@@ -531,8 +522,6 @@ def _prepare_down(gate_up, prepared, down):
 
 def _swiglu(gu: torch.Tensor, fused: bool) -> torch.Tensor:
     if fused and gu.is_cuda:
-        from . import ops
-
         return ops.swiglu(gu.contiguous())
     f = gu.shape[1] // 2
     return F.silu(gu[:, :f]) * gu[:, f:]
@@ -541,7 +530,6 @@ def _swiglu(gu: torch.Tensor, fused: bool) -> torch.Tensor:
 def _local_column(w_local: torch.Tensor, w_full: torch.Tensor, bias):
     """Column-parallel linear from an already gathered local slice; the weight tensor scale is
     taken over the FULL weight so that shards agree with the unsharded layer."""
-    from . import ops
     scale = torch.clamp(w_full.abs().max().float() / (448.0 * 6.0), min=1e-9)
     q, sfs, sfd = ops.quantize_w32_shared((w_local / scale).to(torch.bfloat16).contiguous())
     return QLinearLayer.from_quantized(w_local.shape[1], w_local.shape[0], q, sfs, sfd, scale, bias=bias)
