@@ -504,7 +504,8 @@ def sharq_linear_forward(x: torch.Tensor, qw: torch.Tensor, sfw_sparse: torch.Te
     op the reference's vLLM plugin calls when present (benchmarks/vllm/sharq.py:199-213).
     Two prepare launches and one GEMM launch; the activation scale stays on the device."""
     _check(x.dim() == 2, "x must be shaped [M, K]")
-    x = x.contiguous().to(torch.bfloat16)
+    if x.dtype != torch.bfloat16 or not x.is_contiguous():  # the two cost 0.8 us when there is nothing to do
+        x = x.contiguous().to(torch.bfloat16)
     return _lib.native().linear_forward(x, qw, sfw_sparse, sfw_dense, weight_scale, bias, _error_flag(x.device), _split_k())
 
 
