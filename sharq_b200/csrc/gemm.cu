@@ -22,8 +22,9 @@
 //              conversions), a transpose through a small shared-memory tile and coalesced
 //              global stores overlap the next tile's MMAs.
 // Few tiles (decode batches, short chunks): K is split over the CTAs of a cluster, one tile per cluster; every
-// CTA leaves its fp32 partial tile in its own shared memory and the cluster's epilogue threads sum the tiles
-// in rank order through distributed shared memory (no scratch, no second kernel, a fixed order of additions).
+// CTA sends the columns of its fp32 partial tile to the CTAs that own them (asynchronous stores to distributed shared
+// memory that count on the owner's barrier) and sums its own columns in rank order (no scratch, no second
+// kernel, a fixed order of additions).
 // CTA-pair mode (cta_group::2, cluster of 2): the pair computes a 256 x 256 tile; CTA r owns
 // rows [128r,128r+128) (its A operands, scales, metadata, accumulator) and loads weight rows
 // [128r,128r+128) of the tile; the tensor cores of both SMs read both halves.  Every CTA
@@ -52,6 +53,21 @@ constexpr int kEpiWarps = 8;
 constexpr int kPrefetchStages = 3;
 constexpr int kMaxSplits = 8;  // CTAs of a split-K cluster (the portable cluster size)
 constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
+
+// Split launches: the columns of a tile are dealt over the CTAs of the cluster in runs of 8; run u belongs to rank
+// u * splits / runs.
+__host__ __device__ constexpr int first_run(int rank, int splits, int runs) { return (rank * runs + splits - 1) / splits; }
+constexpr int kRecvPad = 4;  // floats behind each received row: neighbouring rows start on distinct banks
+constexpr int max_recv_bytes(int bn) {
+  int most = 0;
+  for (int s = 2; s <= kMaxSplits; ++s)
+    for (int r = 0; r < s; ++r) {
+      const int cols = 8 * (first_run(r + 1, s, bn / 8) - first_run(r, s, bn / 8));
+      const int bytes = s * kBM * (cols + kRecvPad) * 4;
+      most = bytes > most ? bytes : most;
+    }
+  return most;
+}
 
 // Shared-memory stage and tensor-memory column layout.  In pair mode BN is the pair's tile
 // width (256) and each CTA stores half of the weight tile.
@@ -89,8 +105,7 @@ struct StageLayout {
   static constexpr int kColSfbD = kColSfaD + 16;
   static constexpr int kColEnd = kColSfbD + 4 * (BN / 32);
   static constexpr int kTmemCols = kColEnd <= 256 ? 256 : 512;
-  static constexpr int kPartStride = BN + 4;  // floats per row of a split launch's partial tile (row starts on distinct banks)
-  static_assert(PAIR || kBM * kPartStride * 4 <= kStages * kStageBytes, "the partial tile takes the place of the stages");
+  static_assert(PAIR || max_recv_bytes(BN) <= kStages * kStageBytes, "the received parts take the place of the stages");
   static constexpr int kSmemBytes =
       kStages * kStageBytes + kOutStageBytes + 1024 /*alignment slack*/ + 512 /*barriers*/;
 };
@@ -366,8 +381,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   uint64_t *peer_bar = empty_bar + S;  // pair mode, leader CTA: "the peer has loaded stage s"
   uint64_t *acc_full_bar = peer_bar + S;
   uint64_t *acc_empty_bar = acc_full_bar + 1;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty_bar + 1);
+  uint64_t *recv_bar = acc_empty_bar + 1;  // split launch: the parts of this CTA's columns have arrived
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(recv_bar + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  volatile int *never_set = abort_flag + 1;  // for the wait that another role's abort does not end
+  int2 *recv_tab = reinterpret_cast<int2 *>(smem + S * L::kStageBytes + 256);  // split launch, see recv_entry
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -390,6 +408,20 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   // this CTA's share of the K stages
   const int k_rank = PAIR ? 0 : (int)blockIdx.x % k_splits;  // the rank in the cluster of a split launch
   const int it_begin = k_stages * k_rank / k_splits, it_end = k_stages * (k_rank + 1) / k_splits;
+  const bool split = !PAIR && k_splits > 1;
+  // Split launch: the rows of the cluster's tile, and where a rank receives the parts of its columns: in the stages that it is
+  // done with first (its last use of a slot lies furthest back).
+  const int split_rows = split ? min(kBM, p.m - (unit0 % m_units) * kBM) : 0;
+  constexpr int kRuns = BN / 8;
+  // What the senders need of a rank: byte offset of its column 0 in row 0 (of rank 0's part), and bytes per row.
+  auto recv_entry = [&](int rank, int *slot0, int *slots) {
+    const int run0 = first_run(rank, k_splits, kRuns);
+    const int stride = 4 * (8 * (first_run(rank + 1, k_splits, kRuns) - run0) + kRecvPad);
+    const int oldest = (k_stages * (rank + 1) / k_splits - k_stages * rank / k_splits) % S;
+    *slots = (k_splits * split_rows * stride + L::kStageBytes - 1) / L::kStageBytes;
+    *slot0 = oldest + *slots <= S ? oldest : 0;
+    return make_int2(*slot0 * L::kStageBytes - 32 * run0, stride);
+  };
 
   if (threadIdx.x == 32) {
     // fetch the tensor maps while the barriers and tensor memory are being set up
@@ -405,8 +437,17 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     }
     ptx::mbar_init(acc_full_bar, 1);
     ptx::mbar_init(acc_empty_bar, PAIR ? 2 * kEpiWarps : kEpiWarps);
+    ptx::mbar_init(recv_bar, 1);
     *abort_flag = 0;
+    *never_set = 0;
     ptx::fence_barrier_init();
+    if (split)
+      ptx::mbar_arrive_expect_tx(recv_bar, (uint32_t)(k_splits * split_rows * 32 *
+                                                      (first_run(k_rank + 1, k_splits, kRuns) - first_run(k_rank, k_splits, kRuns))));
+  }
+  if (split && threadIdx.x >= 64 && (int)threadIdx.x - 64 < k_splits) {
+    int slot0, slots;
+    recv_tab[threadIdx.x - 64] = recv_entry((int)threadIdx.x - 64, &slot0, &slots);
   }
   if (warp == 1) {
     ptx::tmem_alloc<CG>(tmem_slot, L::kTmemCols);
@@ -418,10 +459,64 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // The set-up above and the prefetch below overlap the end of the kernel that prepares the activation; from here on
+  auto stage_bytes = [&](int it) {
+    const int n_sp = SPARSE ? min(2, tiles_sp - 2 * it) : 0, n_d = DENSE ? min(4, tiles_d - 4 * it) : 0;
+    return L::kWBytes + (uint32_t)p.a_rows * ((DENSE ? 128 : 0) + (SPARSE ? 64 : 0)) + L::kEBytes +
+           (uint32_t)((n_sp + n_d) * 512 * (1 + L::kBands));
+  };
+  // The metadata and scale-factor copies are plain bulk copies without bounds checks.  A
+  // tile may hang over the last 128-row band (the second CTA of a pair when ceil(M/128) is
+  // odd, the second weight band of a 256-wide tile when ceil(N/128) is odd): such a band
+  // is loaded from the last band that exists.  Its rows / columns are masked on output.
+  auto load_weight = [&](int it, int s, int n_tile, const CUtensorMap *tw, const uint8_t *sfb_dense, const uint8_t *sfb_sparse) {
+    uint8_t *st = smem + s * L::kStageBytes;
+    ptx::tma_load_2d(st + L::kOffW, tw, it * 128,
+                     SWIGLU ? n_tile * 128 + (int)cta_rank * ffn : n_tile * BN + (PAIR ? (int)cta_rank * (BN / 2) : 0), full_bar + s);
+#pragma unroll
+    for (int b = 0; b < L::kBands; ++b) {
+      const size_t band = SWIGLU ? n_tile + b * (ffn / 128) : min(n_tile * L::kBands + b, b_bands - 1);
+      if (DENSE)
+        ptx::bulk_load_1d(st + L::kOffSfbD + b * 2048, sfb_dense + (band * tiles_d + 4 * (size_t)it) * 512,
+                          (uint32_t)min(4, tiles_d - 4 * it) * 512, full_bar + s);
+      if (SPARSE)
+        ptx::bulk_load_1d(st + L::kOffSfbSp + b * 1024, sfb_sparse + (band * tiles_sp + 2 * (size_t)it) * 512,
+                          (uint32_t)min(2, tiles_sp - 2 * it) * 512, full_bar + s);
+    }
+  };
+  auto load_activation = [&](int it, int s, int m_tile) {
+    uint8_t *st = smem + s * L::kStageBytes;
+    const int a_band = min(m_tile, a_bands - 1);
+    if (DENSE) {
+      ptx::tma_load_2d(st + L::kOffADense, &tm_a_dense, it * 128, m_tile * kBM, full_bar + s);
+      ptx::bulk_load_1d(st + L::kOffSfaD, p.sfa_dense + ((size_t)a_band * tiles_d + 4 * (size_t)it) * 512,
+                        (uint32_t)min(4, tiles_d - 4 * it) * 512, full_bar + s);
+    }
+    if (SPARSE) {
+      ptx::tma_load_2d(st + L::kOffAComp, &tm_a_comp, it * 64, m_tile * kBM, full_bar + s);
+      ptx::bulk_load_1d(st + L::kOffE, p.e + ((size_t)it * aligned_m + (size_t)a_band * 128) * 16, 2048, full_bar + s);
+      ptx::bulk_load_1d(st + L::kOffSfaSp, p.sfa_sparse + ((size_t)a_band * tiles_sp + 2 * (size_t)it) * 512,
+                        (uint32_t)min(2, tiles_sp - 2 * it) * 512, full_bar + s);
+    }
+  };
+
+  // The set-up above and the loads below overlap the end of the kernel that prepares the activation; from the wait on
   // every role reads or writes what earlier kernels may still use.
-  if (!PAIR && warp == 0 && unit0 < num_units) {
-    // weight tiles of this CTA's first stages into L2: nothing of them depends on the activation
+  // The fused GEMM's weight is not written by a kernel that lets its dependents start early (see grid_launch_dependents): its first
+  // stages are loaded here, as many as the ring holds (with the epilogues below the linears of a 32-token decode step 83.6 -> 79.9 us).
+  constexpr bool kPreload = SPARSE && DENSE && !GROUPED;
+  int preloaded = 0;
+  if (kPreload && warp == 0 && unit0 < num_units) {
+    preloaded = min(S, it_end - it_begin);
+    if (ptx::elect_one()) {
+      for (int i = 0; i < preloaded; ++i) {
+        ptx::mbar_arrive_expect_tx(full_bar + i, stage_bytes(it_begin + i));
+        load_weight(it_begin + i, i, unit0 / m_units, &tm_w, p.sfb_dense, p.sfb_sparse);
+      }
+    }
+    __syncwarp();
+  }
+  if (!kPreload && !PAIR && warp == 0 && unit0 < num_units) {
+    // the operands of the single-pass GEMMs may come from any kernel: into L2, where a prefetch cannot make stale data visible
     if (ptx::elect_one()) {
       const int n_tile = unit0 / m_units;
       const int ahead = min(it_end, it_begin + kPrefetchStages);
@@ -456,58 +551,44 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         const uint8_t *sfb_sparse = GROUPED ? gt->sfb_sparse[grp] : p.sfb_sparse;
         const int m_tile = PAIR ? 2 * (tile % m_units) + (int)cta_rank : (tile % m_units);
         const int n_tile = tile / m_units;
-        const int w_row = SWIGLU ? n_tile * 128 + (int)cta_rank * ffn : n_tile * BN + (PAIR ? (int)cta_rank * (BN / 2) : 0);
-        // The metadata and scale-factor copies are plain bulk copies without bounds checks.  A
-        // tile may hang over the last 128-row band (the second CTA of a pair when ceil(M/128) is
-        // odd, the second weight band of a 256-wide tile when ceil(N/128) is odd): such a band
-        // is loaded from the last band that exists.  Its rows / columns are masked on output.
-        const int a_band = min(m_tile, a_bands - 1);
-        int b_band[L::kBands];
-#pragma unroll
-        for (int b = 0; b < L::kBands; ++b)
-          b_band[b] = SWIGLU ? n_tile + b * (ffn / 128) : min(n_tile * L::kBands + b, b_bands - 1);
         for (int it = it_begin; it < it_end; ++it, ++g) {
           const int s = (int)(g % S);
-          const uint32_t ph = (g / S) & 1u;
-          if (!ptx::mbar_wait(empty_bar + s, ph ^ 1u, abort_flag)) {
-            *abort_flag = 1;
-            atomicExch(p.error_flag, 1);
-            ok = false;
-            break;
+          if ((int)g >= preloaded) {
+            if (!ptx::mbar_wait(empty_bar + s, ((g / S) & 1u) ^ 1u, abort_flag)) {
+              *abort_flag = 1;
+              atomicExch(p.error_flag, 1);
+              ok = false;
+              break;
+            }
+            ptx::mbar_arrive_expect_tx(full_bar + s, stage_bytes(it));
+            load_weight(it, s, n_tile, tw, sfb_dense, sfb_sparse);
           }
-          uint8_t *st = smem + s * L::kStageBytes;
-          const int n_sp = SPARSE ? min(2, tiles_sp - 2 * it) : 0;
-          const int n_d = DENSE ? min(4, tiles_d - 4 * it) : 0;
-          uint32_t tx = L::kWBytes + (uint32_t)p.a_rows * ((DENSE ? 128 : 0) + (SPARSE ? 64 : 0)) + L::kEBytes;
-          tx += (uint32_t)(n_sp * 512 * (1 + L::kBands) + n_d * 512 * (1 + L::kBands));
-          ptx::mbar_arrive_expect_tx(full_bar + s, tx);
-          ptx::tma_load_2d(st + L::kOffW, tw, it * 128, w_row, full_bar + s);
-          if (DENSE) {
-            ptx::tma_load_2d(st + L::kOffADense, &tm_a_dense, it * 128, m_tile * kBM, full_bar + s);
-            ptx::bulk_load_1d(st + L::kOffSfaD, p.sfa_dense + ((size_t)a_band * tiles_d + 4 * (size_t)it) * 512,
-                              (uint32_t)n_d * 512, full_bar + s);
-#pragma unroll
-            for (int b = 0; b < L::kBands; ++b)
-              ptx::bulk_load_1d(st + L::kOffSfbD + b * 2048,
-                                sfb_dense + ((size_t)b_band[b] * tiles_d + 4 * (size_t)it) * 512,
-                                (uint32_t)n_d * 512, full_bar + s);
-          }
-          if (SPARSE) {
-            ptx::tma_load_2d(st + L::kOffAComp, &tm_a_comp, it * 64, m_tile * kBM, full_bar + s);
-            ptx::bulk_load_1d(st + L::kOffE, p.e + ((size_t)it * aligned_m + (size_t)a_band * 128) * 16, 2048,
-                              full_bar + s);
-            ptx::bulk_load_1d(st + L::kOffSfaSp, p.sfa_sparse + ((size_t)a_band * tiles_sp + 2 * (size_t)it) * 512,
-                              (uint32_t)n_sp * 512, full_bar + s);
-#pragma unroll
-            for (int b = 0; b < L::kBands; ++b)
-              ptx::bulk_load_1d(st + L::kOffSfbSp + b * 1024,
-                                sfb_sparse + ((size_t)b_band[b] * tiles_sp + 2 * (size_t)it) * 512,
-                                (uint32_t)n_sp * 512, full_bar + s);
-          }
+          load_activation(it, s, m_tile);
+        }
+      }
+      if (split) {
+        // the slots that take the received parts are free once their last stage has been consumed
+        int slot0, slots;
+        recv_entry(k_rank, &slot0, &slots);
+        const int n = it_end - it_begin;
+        for (int s = slot0; s < slot0 + slots && ok; ++s) {
+          if (s >= n) continue;
+          ok = ptx::mbar_wait(empty_bar + s, (uint32_t)((n - 1 - s) / S) & 1u, abort_flag);
+        }
+        if (!ok) {
+          *abort_flag = 1;
+          atomicExch(p.error_flag, 6);
         }
       }
     }
+    if (split) {
+      __syncwarp();
+      ptx::cluster_arrive();
+      ptx::cluster_wait();  // all CTAs can receive
+      ptx::cluster_arrive();
+    }
   } else if (warp == 1) {
+    if (split) ptx::cluster_arrive();
     if (ptx::elect_one()) {
       if (PAIR && !leader) {
         // ---------------------------------------------------------- peer CTA: report loaded stages
@@ -631,6 +712,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         }
       }
     }
+    if (split) {
+      __syncwarp();
+      ptx::cluster_wait();
+      ptx::cluster_arrive();
+    }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..9)
     const int ew = warp - 2;
@@ -647,13 +733,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     uint8_t *stage = p.staged_store ? smem + S * L::kStageBytes + 512 + ew * 2048 : nullptr;
     uint32_t tile_iter = 0;
     __nv_bfloat162 h_max = __floats2bfloat162_rn(0.0f, 0.0f);  // SWIGLU: running max |h|
-    for (int u = unit0; u < num_units; u += unit_stride) {
-      const int tile = u;
-      const int grp = GROUPED ? gt->unit_group[tile % m_units] : 0;
-      if (GROUPED && grp < 0) continue;
-      const float alpha = GROUPED ? alpha0 * gt->alpha[grp] : alpha0;
-      const int m_tile = PAIR ? 2 * (tile % m_units) + (int)cta_rank : (tile % m_units);
-      const int n_tile = tile / m_units;
+    auto wait_acc = [&]() {  // the next tile's accumulator is complete (uniform over the warp)
       bool ok = ptx::mbar_wait(acc_full_bar, tile_iter & 1u, abort_flag);
       ++tile_iter;
       if (!ok) {
@@ -661,8 +741,127 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         atomicExch(p.error_flag, 3);
       }
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
       ptx::tc_fence_after();
+      return ok;
+    };
+    if constexpr (!PAIR && !SWIGLU && !WIDE) {
+      if (split) {
+        // The first of two passes only runs the code of the sum on one item, unstored, while the stages are still being
+        // consumed: fetched when the last stage is done, it took longer than the sum.  From the last stage's MMAs to the end of the
+        // launch 4096 x 4096 at M = 32 takes 2.6 us (3.6 with a cluster barrier, a sum that reads the other CTAs' memory, and a second
+        // barrier), at M = 1 1.5 (2.6).
+        const int run0 = first_run(k_rank, k_splits, kRuns), n_runs = first_run(k_rank + 1, k_splits, kRuns) - run0;
+        const int m_tile = unit0 % m_units, n_tile = unit0 / m_units;
+        const uint32_t ring = ptx::smem_u32(smem);
+        const int items = split_rows * n_runs;
+        bool ok = true;
+        ptx::cluster_arrive();
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+          if (pass == 1) {
+            ok = wait_acc();
+            ptx::cluster_wait();  // all CTAs can receive
+            const int r = quad * 32 + lane;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::kColAcc + half * kColsPerEpiWarp);
+            if (ok && quad * 32 < split_rows) {
+#pragma unroll 1
+              for (int c = 0; c < kColsPerEpiWarp / 32; ++c) {
+                uint32_t acc[32];
+                ptx::tmem_ld_32x32b_x32(taddr + 32 * c, acc);
+                ptx::tmem_ld_wait();
+                if (r < split_rows) {
+#pragma unroll
+                  for (int v = 0; v < 4; ++v) {
+                    const int run = (half * kColsPerEpiWarp + 32 * c) / 8 + v;
+                    const int owner = run * k_splits / kRuns;
+                    const int2 entry = recv_tab[owner];
+                    const uint32_t at = ring + (uint32_t)(entry.x + (k_rank * split_rows + r) * entry.y + 32 * run);
+                    ptx::st_async_cluster_x4(at, recv_bar, owner, acc[8 * v], acc[8 * v + 1], acc[8 * v + 2], acc[8 * v + 3]);
+                    ptx::st_async_cluster_x4(at + 16, recv_bar, owner, acc[8 * v + 4], acc[8 * v + 5], acc[8 * v + 6], acc[8 * v + 7]);
+                  }
+                }
+              }
+            }
+            __syncwarp();
+            ptx::cluster_arrive();
+            // parts that are under way are waited for also when another role has given up
+            if (!ptx::mbar_wait_cluster_acquire(recv_bar, 0, never_set)) {
+              *abort_flag = 1;
+              atomicExch(p.error_flag, 7);
+              ok = false;
+            }
+            ok = __all_sync(0xffffffffu, ok);
+          }
+#pragma unroll 1
+          for (int i = (int)threadIdx.x - 64; i < items && ok; i += 32 * kEpiWarps) {
+            const int r = i / n_runs, c8 = i % n_runs;
+            const int row = m_tile * kBM + r, col = n_tile * BN + 8 * (run0 + c8);
+            if (col >= p.n) continue;
+            float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            const int2 entry = recv_tab[k_rank];
+            const uint32_t at = ring + (uint32_t)(entry.x + r * entry.y + 32 * (run0 + c8)), step = (uint32_t)(split_rows * entry.y);
+#pragma unroll
+            for (int s = 0; s < kMaxSplits; ++s) {
+              if (s < k_splits) {
+                const float4 lo = ptx::ld_shared_f32x4(at + s * step), hi = ptx::ld_shared_f32x4(at + s * step + 16);
+                f[0] += lo.x, f[1] += lo.y, f[2] += lo.z, f[3] += lo.w;
+                f[4] += hi.x, f[5] += hi.y, f[6] += hi.z, f[7] += hi.w;
+              }
+            }
+            uint32_t o[4];
+            epilogue_8(p, f, row, col, alpha0, beta, has_c, o);
+            asm volatile("" : "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]));  // computed in both passes
+            if (pass == 0) break;
+            store_8(p, o, row, col);
+          }
+        }
+      }
+    }
+    for (int u = unit0; u < num_units && !split; u += unit_stride) {
+      const int tile = u;
+      const int grp = GROUPED ? gt->unit_group[tile % m_units] : 0;
+      if (GROUPED && grp < 0) continue;
+      const float alpha = GROUPED ? alpha0 * gt->alpha[grp] : alpha0;
+      const int m_tile = PAIR ? 2 * (tile % m_units) + (int)cta_rank : (tile % m_units);
+      const int n_tile = tile / m_units;
+      if constexpr (!SWIGLU && !WIDE) {
+        if (stage != nullptr && u + unit_stride >= num_units) {
+          // The CTA's last tile: nothing waits for the tensor memory, so it is drained 32 columns at a time by a loop whose code is
+          // a quarter of the unrolled form's, and which runs once on no rows ahead of the wait (28672 x 4096 at M = 32: 2.6 us behind the last MMA against 4.6, of which 2.8 went into
+          // fetching code).
+          const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::kColAcc + half * kColsPerEpiWarp);
+          const int row0 = m_tile * kBM + quad * 32;
+          bool ok = true;
+#pragma unroll 1
+          for (int c = -1; c < kColsPerEpiWarp / 32; ++c) {
+            uint32_t acc[32] = {};
+            if (c == 0) ok = wait_acc();
+            if (!ok) break;
+            if (c >= 0) {
+              ptx::tmem_ld_32x32b_x32(taddr + 32 * c, acc);
+              ptx::tmem_ld_wait();
+            }
+            const int rows = c < 0 ? 0 : p.m, col0 = n_tile * BN + half * kColsPerEpiWarp + 32 * max(c, 0);
+            epilogue_chunk(p, acc, c < 0 ? p.m : row0 + lane, col0, alpha, beta, has_c, stage, lane);
+            __syncwarp();
+            const int gcol = col0 + (lane & 3) * 8;
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+              const int r = it * 8 + (lane >> 2);
+              const uint4 v = *reinterpret_cast<const uint4 *>(stage + r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) << 4));
+              if (row0 + r < rows && gcol < p.n) {
+                const size_t off = (size_t)(row0 + r) * p.n + gcol;
+                uint32_t o[4] = {v.x, v.y, v.z, v.w};
+                if (p.residual != nullptr) add_residual_8(p, o, off);
+                *reinterpret_cast<uint4 *>(p.d + off) = make_uint4(o[0], o[1], o[2], o[3]);
+              }
+            }
+            __syncwarp();
+          }
+          break;
+        }
+      }
+      if (!wait_acc()) break;
       uint32_t acc[kColsPerEpiWarp];
       // SWIGLU: 64 gate columns and the 64 up columns that belong to them, else neighbouring columns
       const uint32_t taddr =
@@ -702,16 +901,6 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         if (GROUPED) {  // the unit's rows belong to one group
           raise_absmax(p.amax_bits + grp, h_max, lane);
           h_max = __floats2bfloat162_rn(0.0f, 0.0f);
-        }
-        continue;
-      }
-      if (!PAIR && k_splits > 1) {
-        // this CTA's partial tile into its own shared memory: the last stage has been consumed, nothing else is loaded
-        if (row < p.m) {
-          float *dst = reinterpret_cast<float *>(smem) + (size_t)(quad * 32 + lane) * L::kPartStride + half * kColsPerEpiWarp;
-#pragma unroll
-          for (int i = 0; i < kColsPerEpiWarp; i += 4)
-            *reinterpret_cast<uint4 *>(dst + i) = make_uint4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
         }
         continue;
       }
@@ -790,44 +979,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     for (int w = 1; w < kEpiWarps; ++w) cta = fmaxf(cta, mx[w]);
     p.amax_bits[blockIdx.x] = __float_as_uint(cta);
   }
-  if (!PAIR && k_splits > 1) {
-    ptx::cluster_sync();  // every CTA's partial tile is written
-    if (threadIdx.x >= 64) {
-      const int m_tile = unit0 % m_units, n_tile = unit0 / m_units;
-      const int rows = min(kBM, p.m - m_tile * kBM);
-      const float alpha = p.alpha_ptr ? p.alpha * (*p.alpha_ptr) : p.alpha;
-      const bool has_c = (p.c_in != nullptr) && (p.beta != 0.0f);
-      const uint32_t part = ptx::smem_u32(smem);
-      // 8 columns per thread, dealt over the threads of all CTAs: neighbouring lanes read neighbouring 32 bytes
-      for (int i = (int)threadIdx.x - 64 + k_rank * 32 * kEpiWarps; i < rows * (BN / 8); i += k_splits * 32 * kEpiWarps) {
-        const int r = i / (BN / 8), c8 = i % (BN / 8);
-        const int row = m_tile * kBM + r, col = n_tile * BN + 8 * c8;
-        if (col >= p.n) continue;
-        const uint32_t at = part + (uint32_t)(r * L::kPartStride + 8 * c8) * 4u;
-        float4 lo[kMaxSplits], hi[kMaxSplits];
-#pragma unroll
-        for (int s = 0; s < kMaxSplits; ++s) {
-          if (s < k_splits) {
-            lo[s] = ptx::ld_cluster_f32x4(at, s);
-            hi[s] = ptx::ld_cluster_f32x4(at + 16, s);
-          }
-        }
-        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int s = 0; s < kMaxSplits; ++s) {
-          if (s < k_splits) {
-            f[0] += lo[s].x, f[1] += lo[s].y, f[2] += lo[s].z, f[3] += lo[s].w;
-            f[4] += hi[s].x, f[5] += hi[s].y, f[6] += hi[s].z, f[7] += hi[s].w;
-          }
-        }
-        uint32_t o[4];
-        epilogue_8(p, f, row, col, alpha, p.beta, has_c, o);
-        store_8(p, o, row, col);
-      }
-    }
-    __syncwarp();
-    ptx::cluster_sync();  // no CTA leaves while another may still read its partial tile
-  }
+  if (split) ptx::cluster_wait();  // every CTA has sent its parts
   if (PAIR) ptx::cluster_sync();  // neither CTA leaves (or frees tensor memory) while its peer may still use it
   if (warp == 1) {
     ptx::tc_fence_after();

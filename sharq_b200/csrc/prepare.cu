@@ -252,7 +252,6 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
   const int groups32 = k >> 5;
   const int aligned_m = (m + 127) / 128 * 128;
 
-  ptx::grid_launch_dependents();
   __shared__ ScaleTables tbl;
   extern __shared__ uint4 gamma_smem[];  // mode 1: the whole RMSNorm weight, k bf16
   if (threadIdx.x < 128) {
@@ -261,6 +260,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
     tbl.recip[threadIdx.x] = __frcp_rn(v);  // code 0 is never looked up (scales are clamped to >= 2^-9)
   }
   ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();  // behind the wait: a GEMM that follows loads its weight before its own wait
   if (kMode == 1) {
     const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
     for (int i = threadIdx.x; i < k / 8; i += blockDim.x) gamma_smem[i] = gsrc[i];
@@ -554,13 +554,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
   float *partial = reinterpret_cast<float *>(cache + (size_t)p.chunk_rows * row_vecs);  // mode 1: chunk_rows x partial_stride
   float *inv_s = partial + (kMode == 1 ? p.chunk_rows * partial_stride : 0);            // mode 1: rows_per_cta
 
-  ptx::grid_launch_dependents();
   if (threadIdx.x < 128) {
     const float v = ue4m3_to_float(threadIdx.x);
     tbl.value[threadIdx.x] = v;
     tbl.recip[threadIdx.x] = __frcp_rn(v);  // code 0 is never looked up (scales are clamped to >= 2^-9)
   }
   ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();  // see prepare_kernel
   if (kMode == 1) {
     const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
     for (int i = threadIdx.x; i < row_vecs; i += kFusedThreads) gamma_s[cache_slot(i >> 2, i & 3)] = gsrc[i];

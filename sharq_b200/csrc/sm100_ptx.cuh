@@ -81,8 +81,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
   }
 }
 
-// Same, with acquire semantics at cluster scope: for barriers that another CTA of the
-// cluster arrives on.
+// For barriers that another CTA of the cluster arrives on; orders no memory.
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -107,6 +106,31 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity
   }
 }
 
+// For what other CTAs stored and counted on the barrier: acquire at cluster scope.
+__device__ __forceinline__ bool mbar_try_wait_cluster_acquire(uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait_cluster_acquire(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+  if (mbar_try_wait_cluster_acquire(bar, parity)) return true;
+  const long long start = clock64();
+  while (true) {
+    for (int i = 0; i < 64; ++i)
+      if (mbar_try_wait_cluster_acquire(bar, parity)) return true;
+    if (*abort_flag != 0) return false;
+    if (clock64() - start > kWaitLimitCycles) return false;
+  }
+}
+
 // ---------------------------------------------------------------- clusters
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -118,18 +142,26 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// 16 bytes of another CTA's shared memory (addr: this CTA's address of the same variable).
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr, uint32_t cta_rank) {
-  float4 v;
+// The two halves of cluster_sync, for what lies between them; executed alternately by every thread of the cluster, warps converged.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// 16 bytes into the shared memory of CTA `cta_rank` (addr, bar: this CTA's addresses of the same variables), counted on its barrier.
+__device__ __forceinline__ void st_async_cluster_x4(uint32_t addr, uint64_t *bar, uint32_t cta_rank, uint32_t a, uint32_t b, uint32_t c,
+                                                    uint32_t d) {
   asm volatile(
       "{\n\t"
-      ".reg .b32 remote;\n\t"
-      "mapa.shared::cluster.u32 remote, %4, %5;\n\t"
-      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [remote];\n\t"
-      "}"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "r"(addr), "r"(cta_rank)
+      ".reg .b32 remote, remote_bar;\n\t"
+      "mapa.shared::cluster.u32 remote, %0, %2;\n\t"
+      "mapa.shared::cluster.u32 remote_bar, %1, %2;\n\t"
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [remote], {%3, %4, %5, %6}, [remote_bar];\n\t"
+      "}" ::"r"(addr),
+      "r"(smem_u32(bar)), "r"(cta_rank), "r"(a), "r"(b), "r"(c), "r"(d)
       : "memory");
+}
+__device__ __forceinline__ float4 ld_shared_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
 
@@ -140,7 +172,9 @@ __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr, uint32_t cta_r
 // a const __restrict__ parameter, which the compiler may load through it) is defined only for data that nothing
 // writes during the kernel's life: such kernels read global memory with ordinary loads and declare no pointer __restrict__.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Lets a dependent kernel that was launched with the attribute start its blocks (it waits itself before it reads).
+// Lets a dependent kernel that was launched with the attribute start its blocks (it waits itself before it reads; the fused GEMM
+// loads its weight before that: a kernel that may write a weight does not call this, and one that may stand between such a
+// kernel and the GEMM calls it behind its own wait, when all that came before it is complete and visible).
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- TMA
