@@ -57,6 +57,7 @@ constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 // Split launches: the columns of a tile are dealt over the CTAs of the cluster in runs of 8; run u belongs to rank
 // u * splits / runs.
 __host__ __device__ constexpr int first_run(int rank, int splits, int runs) { return (rank * runs + splits - 1) / splits; }
+constexpr int kRegisterRows = 32;  // rows of a tile whose parts are sent from registers, see send_offset
 constexpr int kRecvPad = 4;  // floats behind each received row: neighbouring rows start on distinct banks
 constexpr int max_recv_bytes(int bn) {
   int most = 0;
@@ -385,7 +386,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(recv_bar + 1);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   volatile int *never_set = abort_flag + 1;  // for the wait that another role's abort does not end
-  int2 *recv_tab = reinterpret_cast<int2 *>(smem + S * L::kStageBytes + 256);  // split launch, see recv_entry
+  int4 *recv_tab = reinterpret_cast<int4 *>(smem + S * L::kStageBytes + 256);  // split launch, see recv_entry
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -413,14 +414,25 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   // done with first (its last use of a slot lies furthest back).
   const int split_rows = split ? min(kBM, p.m - (unit0 % m_units) * kBM) : 0;
   constexpr int kRuns = BN / 8;
-  // What the senders need of a rank: byte offset of its column 0 in row 0 (of rank 0's part), and bytes per row.
+  // What the senders need of a rank: byte offset of the tile's column 0 in row 0 of rank 0's part, bytes per row, its first run.
   auto recv_entry = [&](int rank, int *slot0, int *slots) {
     const int run0 = first_run(rank, k_splits, kRuns);
     const int stride = 4 * (8 * (first_run(rank + 1, k_splits, kRuns) - run0) + kRecvPad);
     const int oldest = (k_stages * (rank + 1) / k_splits - k_stages * rank / k_splits) % S;
     *slots = (k_splits * split_rows * stride + L::kStageBytes - 1) / L::kStageBytes;
     *slot0 = oldest + *slots <= S ? oldest : 0;
-    return make_int2(*slot0 * L::kStageBytes - 32 * run0, stride);
+    return make_int4(*slot0 * L::kStageBytes - 32 * run0, stride, run0, 0);
+  };
+  // Where a CTA lays its parts out, one block per owner, to be sent by block copies (-1: they go from registers, 16 bytes at a time: up
+  // to 32 rows, where that is faster, and where the stages beside the receiving slots do not hold the blocks).  us, registers / blocks:
+  // 4096 x 4096 at M = 1 6.1 / 7.1, 32 7.2 / 7.5, 64 9.1 / 8.6, 96 11.1 / 10.2; 4096 x 14336 at M = 32 11.9 / 12.2, 64 13.7 / 13.1,
+  // 128 17.5 / 16.3.
+  auto send_offset = [&](int rank) {
+    if (split_rows <= kRegisterRows) return -1;
+    int slot0, slots;
+    recv_entry(rank, &slot0, &slots);
+    const int need = (split_rows * (BN + k_splits * kRecvPad) * 4 + L::kStageBytes - 1) / L::kStageBytes;
+    return slot0 >= need ? 0 : (S - slot0 - slots >= need ? (slot0 + slots) * L::kStageBytes : -1);
   };
 
   if (threadIdx.x == 32) {
@@ -441,9 +453,13 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     *abort_flag = 0;
     *never_set = 0;
     ptx::fence_barrier_init();
-    if (split)
-      ptx::mbar_arrive_expect_tx(recv_bar, (uint32_t)(k_splits * split_rows * 32 *
-                                                      (first_run(k_rank + 1, k_splits, kRuns) - first_run(k_rank, k_splits, kRuns))));
+    if (split) {
+      // what arrives: the columns, and with a block copy their padding too
+      int bytes = k_splits * split_rows * 32 * (first_run(k_rank + 1, k_splits, kRuns) - first_run(k_rank, k_splits, kRuns));
+      if (split_rows > kRegisterRows)
+        for (int s = 0; s < k_splits; ++s) bytes += send_offset(s) >= 0 ? split_rows * 4 * kRecvPad : 0;
+      ptx::mbar_arrive_expect_tx(recv_bar, (uint32_t)bytes);
+    }
   }
   if (split && threadIdx.x >= 64 && (int)threadIdx.x - 64 < k_splits) {
     int slot0, slots;
@@ -763,7 +779,38 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
             ptx::cluster_wait();  // all CTAs can receive
             const int r = quad * 32 + lane;
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::kColAcc + half * kColsPerEpiWarp);
-            if (ok && quad * 32 < split_rows) {
+            const int send = send_offset(k_rank);
+            if (send >= 0) {
+              if (ok && quad * 32 < split_rows) {
+#pragma unroll 1
+                for (int c = 0; c < kColsPerEpiWarp / 32; ++c) {
+                  uint32_t acc[32];
+                  ptx::tmem_ld_32x32b_x32(taddr + 32 * c, acc);
+                  ptx::tmem_ld_wait();
+                  if (r < split_rows) {
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                      const int run = (half * kColsPerEpiWarp + 32 * c) / 8 + v;
+                      const int owner = run * k_splits / kRuns;
+                      const int4 entry = recv_tab[owner];
+                      // the blocks ahead hold run0 runs and `owner` paddings per row
+                      uint4 *dst = reinterpret_cast<uint4 *>(smem + send + split_rows * (32 * entry.z + 4 * kRecvPad * owner) +
+                                                             r * entry.y + 32 * (run - entry.z));
+                      dst[0] = make_uint4(acc[8 * v], acc[8 * v + 1], acc[8 * v + 2], acc[8 * v + 3]);
+                      dst[1] = make_uint4(acc[8 * v + 4], acc[8 * v + 5], acc[8 * v + 6], acc[8 * v + 7]);
+                    }
+                  }
+                }
+              }
+              ptx::fence_proxy_async();
+              ptx::named_sync(1, 32 * kEpiWarps);
+              if (ok && ew == 0 && lane < k_splits) {
+                const int4 entry = recv_tab[lane];
+                ptx::bulk_copy_cluster(ring + (uint32_t)(entry.x + k_rank * split_rows * entry.y + 32 * entry.z),
+                                       smem + send + split_rows * (32 * entry.z + 4 * kRecvPad * lane), (uint32_t)(split_rows * entry.y),
+                                       recv_bar, lane);
+              }
+            } else if (ok && quad * 32 < split_rows) {
 #pragma unroll 1
               for (int c = 0; c < kColsPerEpiWarp / 32; ++c) {
                 uint32_t acc[32];
@@ -774,7 +821,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
                   for (int v = 0; v < 4; ++v) {
                     const int run = (half * kColsPerEpiWarp + 32 * c) / 8 + v;
                     const int owner = run * k_splits / kRuns;
-                    const int2 entry = recv_tab[owner];
+                    const int4 entry = recv_tab[owner];
                     const uint32_t at = ring + (uint32_t)(entry.x + (k_rank * split_rows + r) * entry.y + 32 * run);
                     ptx::st_async_cluster_x4(at, recv_bar, owner, acc[8 * v], acc[8 * v + 1], acc[8 * v + 2], acc[8 * v + 3]);
                     ptx::st_async_cluster_x4(at + 16, recv_bar, owner, acc[8 * v + 4], acc[8 * v + 5], acc[8 * v + 6], acc[8 * v + 7]);
@@ -783,7 +830,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
               }
             }
             __syncwarp();
-            ptx::cluster_arrive();
+            // A CTA may leave once its parts are on their way; where they may be read from its memory, once they have arrived.
+            if (split_rows <= kRegisterRows) ptx::cluster_arrive();
             // parts that are under way are waited for also when another role has given up
             if (!ptx::mbar_wait_cluster_acquire(recv_bar, 0, never_set)) {
               *abort_flag = 1;
@@ -791,6 +839,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
               ok = false;
             }
             ok = __all_sync(0xffffffffu, ok);
+            if (split_rows > kRegisterRows) ptx::cluster_arrive();
           }
 #pragma unroll 1
           for (int i = (int)threadIdx.x - 64; i < items && ok; i += 32 * kEpiWarps) {
@@ -798,7 +847,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
             const int row = m_tile * kBM + r, col = n_tile * BN + 8 * (run0 + c8);
             if (col >= p.n) continue;
             float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            const int2 entry = recv_tab[k_rank];
+            const int4 entry = recv_tab[k_rank];
             const uint32_t at = ring + (uint32_t)(entry.x + r * entry.y + 32 * (run0 + c8)), step = (uint32_t)(split_rows * entry.y);
 #pragma unroll
             for (int s = 0; s < kMaxSplits; ++s) {
@@ -979,7 +1028,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     for (int w = 1; w < kEpiWarps; ++w) cta = fmaxf(cta, mx[w]);
     p.amax_bits[blockIdx.x] = __float_as_uint(cta);
   }
-  if (split) ptx::cluster_wait();  // every CTA has sent its parts
+  if (split) ptx::cluster_wait();  // no CTA is sent to or read from any more
   if (PAIR) ptx::cluster_sync();  // neither CTA leaves (or frees tensor memory) while its peer may still use it
   if (warp == 1) {
     ptx::tc_fence_after();

@@ -28,6 +28,9 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Named barrier of `threads` threads.
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -157,6 +160,19 @@ __device__ __forceinline__ void st_async_cluster_x4(uint32_t addr, uint64_t *bar
       "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [remote], {%3, %4, %5, %6}, [remote_bar];\n\t"
       "}" ::"r"(addr),
       "r"(smem_u32(bar)), "r"(cta_rank), "r"(a), "r"(b), "r"(c), "r"(d)
+      : "memory");
+}
+// `bytes` (a multiple of 16) of this CTA's shared memory to CTA `cta_rank` (dst, bar: this CTA's addresses of the same variables),
+// counted on its barrier; what was written through the generic proxy needs fence_proxy_async first.
+__device__ __forceinline__ void bulk_copy_cluster(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar, uint32_t cta_rank) {
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 remote, remote_bar;\n\t"
+      "mapa.shared::cluster.u32 remote, %0, %4;\n\t"
+      "mapa.shared::cluster.u32 remote_bar, %3, %4;\n\t"
+      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [remote], [%1], %2, [remote_bar];\n\t"
+      "}" ::"r"(dst),
+      "r"(smem_u32(src)), "r"(bytes), "r"(smem_u32(bar)), "r"(cta_rank)
       : "memory");
 }
 __device__ __forceinline__ float4 ld_shared_f32x4(uint32_t addr) {
