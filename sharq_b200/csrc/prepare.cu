@@ -201,6 +201,27 @@ __global__ void __launch_bounds__(256) abs_stats_kernel(const __nv_bfloat16 *x, 
   }
 }
 
+// Zeros in the padding rows [m, ceil128(m)) of the metadata and of both scale buffers.
+__device__ __forceinline__ void zero_padding_rows(uint8_t *e, uint8_t *sfa_sparse, uint8_t *sf_res, int m, int k, int worker, int workers) {
+  const int groups32 = k >> 5, aligned_m = (m + 127) / 128 * 128;
+  const int pad_rows = aligned_m - m;
+  const int k_tiles = (k + 255) / 256;
+  const int w_sp = groups32 >> 2, w_res = k >> 6;  // 32-bit scale words per row
+  const int per_row = k_tiles * 4 + w_sp + w_res;  // 32-bit words to clear per padding row
+  for (int i = worker; i < pad_rows * per_row; i += workers) {
+    const int row = m + i / per_row;
+    int j = i % per_row;
+    if (j < k_tiles * 4) {
+      *reinterpret_cast<uint32_t *>(e + ((size_t)(j >> 2) * aligned_m + row) * 16 + (size_t)(j & 3) * 4) = 0u;
+    } else if ((j -= k_tiles * 4) < w_sp) {
+      *reinterpret_cast<uint32_t *>(sfa_sparse + sf_offset(row, 4 * j, groups32)) = 0u;
+    } else {
+      j -= w_sp;
+      *reinterpret_cast<uint32_t *>(sf_res + sf_offset(row, 4 * j, k / 16)) = 0u;
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Prepare kernel.
 //   kMode 0: input already scaled (drop-in for fused_sparse_residual_quantize_x)
@@ -235,18 +256,32 @@ struct PrepareParams {
 
 constexpr int kPrepareCtasPerSm = 3;
 constexpr int kScaledCtasPerSm = 2;  // tensor-scale mode without a gather
-// Up to this size every CTA scans the whole input for its maximum.  us per call in a graph, scan / statistics launch and prepare: 16 x 4096
-// 4.5 / 4.9, 17 x 4096 5.1 / 4.6, 32 x 4096 6.7 / 4.7.  Without room for a word per CTA the other form is a cooperative launch behind
-// a memset, and the scan pays longer: 17 x 4096 5.1 / 8.4, 8 x 14336 6.4 / 10.3, 48 x 4096 8.5 / 8.4, 64 x 4096 10.4 / 8.4.
+// An input of up to kClusterScanElements needs no statistics launch: every CTA scans it for its maximum, or (from kCtaScanElements) every
+// cluster of kScanCtas CTAs.  us per call in a graph, CTA / cluster / statistics launch and prepare: 1 x 4096 2.6 / 4.0 / -, 8 x 4096
+// 3.1 / 3.9 / -, 16 x 4096 4.5 / 3.1 / 4.9, 32 x 4096 6.7 / 3.7 / 4.4, 64 x 4096 10.4 / 4.2 / 4.8, 16 x 14336 - / 4.8 / 4.4, 32 x 14336 - / 6.0 / 4.7.  A
+// launch less is also 2 us less host time (16 x 14336 and its GEMM, eager: 21.4 -> 19.2 us).
+constexpr size_t kCtaScanElements = 40 * 1024;
+constexpr size_t kClusterScanElements = 256 * 1024;
+constexpr int kClusterScanTiles = 256;  // CTAs that leave room for every cluster at once (8 x 18944, 296 of them: 6.6 us, launch 4.7)
+constexpr int kScanCtas = 8;
+// The scanning forms leave the maximum in the workspace only above these sizes (with and without room for a word per statistics CTA).
 constexpr size_t kInlineAbsmaxElements = 64 * 1024;
 constexpr size_t kInlineAbsmaxElementsNoWords = 192 * 1024;
+// Up to this size, with the maximum ready and more than one 32-row tile, a lane takes 8 elements (prepare_narrow_kernel).  us, statistics and
+// wide / narrow prepare: RMSNorm 48 x 4096 6.1 / 5.3, 128 x 4096 6.5 / 5.8, 200 x 4096 6.5 / 6.7, 256 x 4096 6.7 / 7.4; tensor scale 128 x 4096
+// 5.0 / 4.5, 200 x 4096 5.1 / 6.1.  Up to 32 rows the narrow form is as much faster by itself, but it spreads over all SMs, on which the
+// GEMM behind it then starts to load its weight sooner, in the prepare's way: linears of a layer with 8 / 32 / 64 / 128 tokens wide 73.8 /
+// 80.0 / 85.8 / 94.0, narrow 78.1 / 82.1 / 85.3 / 93.5.
+constexpr size_t kNarrowElements = 640 * 1024;
 constexpr unsigned kMaxAbsmaxWords = 4096;            // words of CTA maxima that every prepare CTA reduces
 
 // kCtas: resident CTAs per SM the register allocation aims at.  The tensor-scale mode runs
 // fastest with two (no spills) except on a gathered activation (src_row), where the third CTA
 // hides more of the gather's latency (measured: 2048 x 14336 43.3 -> 41.1 us with two,
 // 34816 x 4096 grouped 253 -> 264 us).
-template <int kMode, bool kDebug, int kCtas = kPrepareCtasPerSm>
+// kCluster (mode 2): a small input without a statistics launch: the CTAs of a cluster of kScanCtas CTAs look for the maximum of the whole input
+// together, each over its share, and exchange what they found through distributed shared memory.
+template <int kMode, bool kDebug, int kCtas = kPrepareCtasPerSm, bool kCluster = false>
 __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const PrepareParams p) {
   const int m = p.m, k = p.k;
   const int groups32 = k >> 5;
@@ -259,74 +294,10 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
     tbl.value[threadIdx.x] = v;
     tbl.recip[threadIdx.x] = __frcp_rn(v);  // code 0 is never looked up (scales are clamped to >= 2^-9)
   }
+  __shared__ float scan_max[kScanCtas];  // kCluster
+  if (kCluster) ptx::cluster_arrive();
   ptx::grid_dependency_wait();
   ptx::grid_launch_dependents();  // behind the wait: a GEMM that follows loads its weight before its own wait
-  if (kMode == 1) {
-    const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
-    for (int i = threadIdx.x; i < k / 8; i += blockDim.x) gamma_smem[i] = gsrc[i];
-  }
-  __syncthreads();
-
-  // zero what no owner thread writes: the spare tail of the scale buffers and of A_comp
-  {
-    const int worker = blockIdx.x * blockDim.x + threadIdx.x;
-    const int workers = gridDim.x * blockDim.x;
-    const size_t bands = (size_t)aligned_m / 128;
-    zero_range(p.sfa_sparse, bands * (size_t)(groups32 / 4) * 512, sf_alloc_bytes(m, k), worker, workers);
-    zero_range(p.sf_res, bands * (size_t)(k / 16 / 4) * 512, sf_alloc_bytes(m, k), worker, workers);
-    if (!kDebug) zero_range(p.a_comp, (size_t)m * (k / 4), a_comp_bytes(m, k), worker, workers);
-  }
-
-  float scale = 1.0f, recip = 1.0f;
-  if (kMode != 0) {
-    float amax;
-    if (kMode == 2 && p.amax_bits == nullptr) {
-      // Small input (a decode step): every CTA finds max|x| of the whole tensor itself, which
-      // replaces the memset and the statistics launch; the tensor is read from L2.
-      __shared__ float cta_max[kWarpsPerCta];
-      const uint4 *all = reinterpret_cast<const uint4 *>(p.x);
-      const size_t n16 = (size_t)m * k / 8;
-      __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
-      for (size_t i = threadIdx.x; i < n16; i += blockDim.x) {
-        const uint4 v = all[i];
-        m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.x)));
-        m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.y)));
-        m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.z)));
-        m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.w)));
-      }
-      float mx = fmaxf(__bfloat162float(m2.x), __bfloat162float(m2.y));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      if ((threadIdx.x & 31) == 0) cta_max[threadIdx.x >> 5] = mx;
-      __syncthreads();
-      mx = cta_max[0];
-#pragma unroll
-      for (int w = 1; w < kWarpsPerCta; ++w) mx = fmaxf(mx, cta_max[w]);
-      amax = mx;
-    } else {
-      amax = __uint_as_float(*p.amax_bits);
-      if (p.amax_words > 1) {
-        __shared__ float part_max[kWarpsPerCta];
-        for (int i = threadIdx.x; i < p.amax_words; i += kPrepareThreads) amax = fmaxf(amax, __uint_as_float(p.amax_bits[i]));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        if ((threadIdx.x & 31) == 0) part_max[threadIdx.x >> 5] = amax;
-        __syncthreads();
-#pragma unroll
-        for (int w = 0; w < kWarpsPerCta; ++w) amax = fmaxf(amax, part_max[w]);
-      }
-    }
-    // ATen divides a CUDA tensor by a host scalar by multiplying with the float
-    // reciprocal; clamp(min=1e-9) follows (kernels/src/bindings.cpp:337 of the reference).
-    scale = fmaxf(__fmul_rn(amax, 1.0f / 2688.0f), 1.0e-9f);
-    if (p.scale_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *p.scale_out = scale;
-    if (p.amax_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *p.amax_out = __float_as_uint(amax);
-    if (kMode == 2 && p.unit_group != nullptr && blockIdx.x == 0 && (int)threadIdx.x < p.groups)
-      p.scale_vec_out[threadIdx.x] = fmaxf(__fmul_rn(__uint_as_float(p.amax_bits[threadIdx.x]), 1.0f / 2688.0f), 1.0e-9f);
-    if (kMode == 2) scale = round_to_bf16(scale);  // the divisor of the non-RMSNorm path, see round_to_bf16
-    recip = __frcp_rn(scale);
-  }
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k_tiles = (k + kColsPerCta - 1) / kColsPerCta;
   const int total_tiles = k_tiles * p.row_tiles;
@@ -361,6 +332,77 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
   const uint32_t sf_lane = (uint32_t)row_in_tile * 16u;  // row % 32 is row_in_tile
   const size_t band_sp = (size_t)(groups32 >> 2) * 512, band_res = (size_t)(k >> 6) * 512;
   issue_loads(next_row_tile, next_k_tile);
+
+  // What the CTA needs first is loaded together, with one barrier behind it: its first tile (above), its words of the maximum, its
+  // RMSNorm weight.  One after the other they were three latencies of a launch that lasts about four on a decode step (RMSNorm 32 x 4096
+  // with its statistics 6.6 -> 6.1 us, 1 x 4096 with its scan 3.0 -> 2.6).
+  float amax = 0.0f;
+  if (kMode == 2 && p.amax_bits == nullptr) {
+    // Small input (a decode step): every CTA, or every cluster, finds max|x| of the whole tensor itself, which
+    // replaces the statistics launch; the tensor is read from L2.
+    const uint4 *all = reinterpret_cast<const uint4 *>(p.x);
+    const int n16 = m * (k / 8);
+    __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
+    const int share = kCluster ? (int)ptx::cluster_ctarank() : 0, shares = kCluster ? kScanCtas : 1;
+    for (int i = share * kPrepareThreads + (int)threadIdx.x; i < n16; i += shares * kPrepareThreads) {
+      const uint4 v = all[i];
+      m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.x)));
+      m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.y)));
+      m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.z)));
+      m2 = __hmax2(m2, __habs2(*reinterpret_cast<const __nv_bfloat162 *>(&v.w)));
+    }
+    amax = fmaxf(__bfloat162float(m2.x), __bfloat162float(m2.y));
+  } else if (kMode != 0) {
+    amax = __uint_as_float(*p.amax_bits);
+    for (int i = threadIdx.x; i < p.amax_words; i += kPrepareThreads) amax = fmaxf(amax, __uint_as_float(p.amax_bits[i]));
+  }
+  if (kMode == 1) {
+    // the columns this CTA will meet: those of its one tile, or all
+    const bool one_tile = total_tiles <= (int)gridDim.x;
+    const int lo = one_tile ? next_k_tile * (kColsPerCta / 8) : 0, hi = one_tile ? min(k / 8, lo + kColsPerCta / 8) : k / 8;
+    const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
+    for (int i = lo + (int)threadIdx.x; i < hi; i += blockDim.x) gamma_smem[i] = gsrc[i];
+  }
+
+  // zero what no owner thread writes: the spare tail of the scale buffers and of A_comp
+  {
+    const int worker = blockIdx.x * blockDim.x + threadIdx.x;
+    const int workers = gridDim.x * blockDim.x;
+    const size_t bands = (size_t)aligned_m / 128;
+    zero_range(p.sfa_sparse, bands * (size_t)(groups32 / 4) * 512, sf_alloc_bytes(m, k), worker, workers);
+    zero_range(p.sf_res, bands * (size_t)(k / 16 / 4) * 512, sf_alloc_bytes(m, k), worker, workers);
+    if (!kDebug) zero_range(p.a_comp, (size_t)m * (k / 4), a_comp_bytes(m, k), worker, workers);
+  }
+
+  __shared__ float part_max[kWarpsPerCta];
+  if (kMode != 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) part_max[warp] = amax;
+  }
+  __syncthreads();
+  float scale = 1.0f, recip = 1.0f;
+  if (kMode != 0) {
+#pragma unroll
+    for (int w = 0; w < kWarpsPerCta; ++w) amax = fmaxf(amax, part_max[w]);
+    if (kCluster) {
+      ptx::cluster_wait();  // the CTAs of the cluster are running
+      if (threadIdx.x < kScanCtas) ptx::st_cluster_f32(&scan_max[ptx::cluster_ctarank()], threadIdx.x, amax);
+      __syncwarp();
+      ptx::cluster_sync();  // behind it no CTA writes to another
+#pragma unroll
+      for (int c = 0; c < kScanCtas; ++c) amax = fmaxf(amax, scan_max[c]);
+    }
+    // ATen divides a CUDA tensor by a host scalar by multiplying with the float
+    // reciprocal; clamp(min=1e-9) follows (kernels/src/bindings.cpp:337 of the reference).
+    scale = fmaxf(__fmul_rn(amax, 1.0f / 2688.0f), 1.0e-9f);
+    if (p.scale_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *p.scale_out = scale;
+    if (p.amax_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *p.amax_out = __float_as_uint(amax);
+    if (kMode == 2 && p.unit_group != nullptr && blockIdx.x == 0 && (int)threadIdx.x < p.groups)
+      p.scale_vec_out[threadIdx.x] = fmaxf(__fmul_rn(__uint_as_float(p.amax_bits[threadIdx.x]), 1.0f / 2688.0f), 1.0e-9f);
+    if (kMode == 2) scale = round_to_bf16(scale);  // the divisor of the non-RMSNorm path, see round_to_bf16
+    recip = __frcp_rn(scale);
+  }
 
   for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
     const int row_tile = next_row_tile, k_tile = next_k_tile;
@@ -473,6 +515,121 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
 
 
 // ---------------------------------------------------------------------------
+// Prepare of a small input: latency is all there is, and one group per lane makes a serial chain of some 700 instructions that eight
+// warps of a few SMs walk while the others idle.  Here a lane owns 8 elements, a warp 256 columns of one row, and a CTA has one task per
+// warp (RMSNorm 48 x 4096 with its statistics 6.1 -> 5.3 us).  Modes as in prepare_kernel (the maximum is ready), same bytes.
+// ---------------------------------------------------------------------------
+// Warps of a CTA: the tensor-scale mode has up to 8 maxima per SM to reduce in every CTA, the RMSNorm mode one per row.  us with 4 / 8
+// warps: 96 x 4096 5.3 / 4.4, 32 x 14336 6.0 / 4.7 (tensor scale).
+__host__ __device__ constexpr int narrow_warps(int mode) { return mode == 2 ? 8 : 4; }
+
+template <int kMode>
+__global__ void __launch_bounds__(32 * narrow_warps(kMode)) prepare_narrow_kernel(const PrepareParams p) {
+  constexpr int kNarrowWarps = narrow_warps(kMode);
+  const int m = p.m, k = p.k, groups32 = k >> 5;
+  const int aligned_m = (m + 127) / 128 * 128;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ ScaleTables tbl;
+  __shared__ float part_max[kNarrowWarps];
+  if (threadIdx.x < 128) {
+    const float v = ue4m3_to_float(threadIdx.x);
+    tbl.value[threadIdx.x] = v;
+    tbl.recip[threadIdx.x] = __frcp_rn(v);  // code 0 is never looked up (scales are clamped to >= 2^-9)
+  }
+  ptx::grid_dependency_wait();
+  ptx::grid_launch_dependents();  // see prepare_kernel
+
+  const int k_tiles = (k + 255) / 256;
+  const int task = (int)blockIdx.x * kNarrowWarps + warp;
+  const int row = task / k_tiles, k_tile = task - row * k_tiles;
+  const int col8 = k_tile * 32 + lane;  // in units of 8 columns
+  const bool live = row < m && col8 < (k >> 3);
+  uint4 v = make_uint4(0, 0, 0, 0), gv = make_uint4(0, 0, 0, 0);
+  float inv = 0.0f;
+  if (live) {
+    v = reinterpret_cast<const uint4 *>(p.x)[(size_t)row * (k >> 3) + col8];
+    if (kMode == 1) {
+      gv = reinterpret_cast<const uint4 *>(p.gamma)[col8];
+      inv = p.inv_rms[row];
+    }
+  }
+  float amax = 0.0f;
+  if (kMode != 0) {
+    amax = __uint_as_float(*p.amax_bits);
+    for (int i = threadIdx.x; i < p.amax_words; i += 32 * kNarrowWarps) amax = fmaxf(amax, __uint_as_float(p.amax_bits[i]));
+  }
+  {
+    const int worker = (int)(blockIdx.x * blockDim.x + threadIdx.x), workers = (int)(gridDim.x * blockDim.x);
+    const size_t bands = (size_t)aligned_m / 128;
+    zero_range(p.sfa_sparse, bands * (size_t)(groups32 / 4) * 512, sf_alloc_bytes(m, k), worker, workers);
+    zero_range(p.sf_res, bands * (size_t)(k / 16 / 4) * 512, sf_alloc_bytes(m, k), worker, workers);
+    zero_range(p.a_comp, (size_t)m * (k / 4), a_comp_bytes(m, k), worker, workers);
+    zero_padding_rows(p.e, p.sfa_sparse, p.sf_res, m, k, worker, workers);
+  }
+  if (kMode != 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) part_max[warp] = amax;
+  }
+  __syncthreads();
+  float scale = 1.0f, recip = 1.0f;
+  if (kMode != 0) {
+#pragma unroll
+    for (int w = 0; w < kNarrowWarps; ++w) amax = fmaxf(amax, part_max[w]);
+    scale = fmaxf(__fmul_rn(amax, 1.0f / 2688.0f), 1.0e-9f);  // as in prepare_kernel
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (p.scale_out != nullptr) *p.scale_out = scale;
+      if (p.amax_out != nullptr) *p.amax_out = __float_as_uint(amax);
+    }
+    if (kMode == 2) scale = round_to_bf16(scale);
+    recip = __frcp_rn(scale);
+  }
+  if (row >= m) return;
+
+  uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  if (kMode == 1) {
+    const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = normalise_word(w[i], gw[i], pair_f32(inv, inv));
+    scale_words(w, scale, recip);
+  } else if (kMode == 2) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 q = mul_word(w[i], pair_f32(recip, recip));
+      w[i] = pack_bf16x2(q.x, q.y);
+    }
+  }
+  ChunkPick pick = pick_pairs(w);
+  if (kMode == 2 && pick.second - 4u < kTinyKey) {  // rare, see scale_quantize_group: a subnormal quotient takes part in the selection
+    const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = pack_bf16x2(__fdiv_rn(lo_f(x[i]), scale), __fdiv_rn(hi_f(x[i]), scale));
+    pick = pick_pairs(w);
+  }
+  __syncwarp();
+  ChunkOut o;
+  quantize_chunk8(w, pick, tbl, o);
+  if (!live) o = ChunkOut{};
+
+  if (live) *reinterpret_cast<uint32_t *>(p.q_res + (size_t)row * (k / 2) + (size_t)col8 * 4) = o.q_res;
+  const uint32_t comp = o.a_comp | (__shfl_down_sync(0xffffffffu, o.a_comp, 1) << 16);
+  if (live && (lane & 1) == 0) *reinterpret_cast<uint32_t *>(p.a_comp + (size_t)row * (k / 4) + (size_t)col8 * 2) = comp;
+  uint32_t meta = o.meta << (4 * (lane & 7));  // 8 lanes: the metadata of two groups
+  meta |= __shfl_xor_sync(0xffffffffu, meta, 1);
+  meta |= __shfl_xor_sync(0xffffffffu, meta, 2);
+  meta |= __shfl_xor_sync(0xffffffffu, meta, 4);
+  if ((lane & 7) == 0) *reinterpret_cast<uint32_t *>(p.e + ((size_t)k_tile * aligned_m + row) * 16 + (size_t)(lane >> 3) * 4) = meta;
+  uint32_t res = o.sf_res << (8 * ((lane >> 1) & 3));  // 8 lanes: four 16-groups
+  res |= __shfl_xor_sync(0xffffffffu, res, 2);
+  res |= __shfl_xor_sync(0xffffffffu, res, 4);
+  if (live && (lane & 7) == 0) *reinterpret_cast<uint32_t *>(p.sf_res + sf_offset(row, col8 >> 1, k / 16)) = res;
+  uint32_t sp = o.sf_sparse << (8 * ((lane >> 2) & 3));  // 16 lanes: four 32-groups
+  sp |= __shfl_xor_sync(0xffffffffu, sp, 4);
+  sp |= __shfl_xor_sync(0xffffffffu, sp, 8);
+  if (live && (lane & 15) == 0) *reinterpret_cast<uint32_t *>(p.sfa_sparse + sf_offset(row, col8 >> 2, groups32)) = sp;
+}
+
+// ---------------------------------------------------------------------------
 // One-launch scaled prepare (modes 1 and 2 with their statistics pass folded in).
 //
 // A cooperative grid of one CTA per SM; CTA b owns a contiguous block of rows.  Phase 1: the
@@ -575,22 +732,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
     zero_range(p.sfa_sparse, bands * (size_t)(groups32 / 4) * 512, sf_alloc_bytes(m, k), worker, workers);
     zero_range(p.sf_res, bands * (size_t)(k / 16 / 4) * 512, sf_alloc_bytes(m, k), worker, workers);
     zero_range(p.a_comp, (size_t)m * (k / 4), a_comp_bytes(m, k), worker, workers);
-    const int pad_rows = aligned_m - m;
-    const int k_tiles = groups_padded >> 3;
-    const int w_sp = groups32 >> 2, w_res = k >> 6;  // 32-bit scale words per row
-    const int per_row = k_tiles * 4 + w_sp + w_res;  // 32-bit words to clear per padding row
-    for (long long i = worker; i < (long long)pad_rows * per_row; i += workers) {
-      const int row = m + (int)(i / per_row);
-      int j = (int)(i % per_row);
-      if (j < k_tiles * 4) {
-        *reinterpret_cast<uint32_t *>(p.e + ((size_t)(j >> 2) * aligned_m + row) * 16 + (size_t)(j & 3) * 4) = 0u;
-      } else if ((j -= k_tiles * 4) < w_sp) {
-        *reinterpret_cast<uint32_t *>(p.sfa_sparse + sf_offset(row, 4 * j, groups32)) = 0u;
-      } else {
-        j -= w_sp;
-        *reinterpret_cast<uint32_t *>(p.sf_res + sf_offset(row, 4 * j, k / 16)) = 0u;
-      }
-    }
+    zero_padding_rows(p.e, p.sfa_sparse, p.sf_res, m, k, worker, workers);
   }
 
   const int row_begin = min(m, (int)blockIdx.x * p.rows_per_cta);
@@ -840,18 +982,25 @@ static cudaError_t current_sms(int *dev_out, int *sms_out) {
   return cudaSuccess;
 }
 
+// 32-row x 256-column tiles of the padded activation.
+static int prepare_tiles(int m, int k) { return (k + kColsPerCta - 1) / kColsPerCta * ((m + 127) / 128 * 128 / kRowsPerCta); }
+
 // As many CTAs as are resident at once: a grid of 444 for the two-CTA kernel ran its last third at one CTA per SM.
 static int prepare_grid(const PrepareParams &p, int ctas_per_sm) {
   int dev = 0, sms = 0;
-  const int tiles = ((p.k + kColsPerCta - 1) / kColsPerCta) * p.row_tiles;
+  const int tiles = prepare_tiles(p.m, p.k);
   if (current_sms(&dev, &sms) != cudaSuccess) return tiles < 1024 ? tiles : 1024;
   const int full = sms * ctas_per_sm;
   return tiles < full ? tiles : full;
 }
 
 static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, cudaStream_t stream) {
+  const size_t elements = (size_t)p.m * p.k;
+  const bool narrow = !debug && p.m > kRowsPerCta && elements <= kNarrowElements && p.unit_group == nullptr && p.src_row == nullptr &&
+                      (mode != 2 || p.amax_bits != nullptr);
+  const bool cluster = mode == 2 && p.amax_bits == nullptr && elements > kCtaScanElements;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the table set-up overlaps the kernel before
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(prepare_grid(p, mode == 2 && p.src_row == nullptr ? kScaledCtasPerSm : kPrepareCtasPerSm));
@@ -859,6 +1008,20 @@ static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (narrow) {
+    const int warps = narrow_warps(mode);
+    cfg.gridDim = dim3((unsigned)((p.m * ((p.k + 255) / 256) + warps - 1) / warps));
+    cfg.blockDim = dim3((unsigned)(32 * warps));
+    if (mode == 0) return cudaLaunchKernelEx(&cfg, prepare_narrow_kernel<0>, p);
+    return cudaLaunchKernelEx(&cfg, mode == 1 ? prepare_narrow_kernel<1> : prepare_narrow_kernel<2>, p);
+  }
+  if (cluster) {
+    cfg.gridDim.x = (cfg.gridDim.x + kScanCtas - 1) / kScanCtas * kScanCtas;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = kScanCtas;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
   if (debug) return cudaLaunchKernelEx(&cfg, prepare_kernel<0, true>, p);
   if (mode == 0) return cudaLaunchKernelEx(&cfg, prepare_kernel<0, false>, p);
   if (mode == 1) {
@@ -874,6 +1037,7 @@ static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, 
     return cudaLaunchKernelEx(&cfg, prepare_kernel<1, false>, p);
   }
   if (p.src_row != nullptr) return cudaLaunchKernelEx(&cfg, prepare_kernel<2, false>, p);
+  if (cluster) return cudaLaunchKernelEx(&cfg, prepare_kernel<2, false, kScaledCtasPerSm, true>, p);
   return cudaLaunchKernelEx(&cfg, prepare_kernel<2, false, kScaledCtasPerSm>, p);
 }
 
@@ -974,8 +1138,10 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   const size_t words_at = 256 + (rms && inv_rms_external == nullptr ? (size_t)m * sizeof(float) : 0);
   const bool word_per_cta = stat_ctas <= kMaxAbsmaxWords && workspace_bytes >= words_at + (size_t)stat_ctas * sizeof(float);
   // a small non-RMSNorm input (a decode step): the prepare kernel finds max|x| itself
-  const bool inline_absmax =
-      !rms && !absmax_ready && elements <= (word_per_cta ? kInlineAbsmaxElements : kInlineAbsmaxElementsNoWords);
+  const bool inline_absmax = !rms && !absmax_ready && elements <= kClusterScanElements &&
+                             (elements <= kCtaScanElements || prepare_tiles(m, k) <= kClusterScanTiles ||
+                              (!word_per_cta && elements <= kInlineAbsmaxElementsNoWords));
+  const bool leave_absmax = !inline_absmax || elements > (word_per_cta ? kInlineAbsmaxElements : kInlineAbsmaxElementsNoWords);
   // Two launches that overlap, with nothing to zero, beat one cooperative launch behind its memset (us, two launches / one: tensor scale
   // 64 x 4096 5.0 / 8.4, 2048 x 4096 12.0 / 16.9, 4096 x 4096 19.6 / 27.1; RMSNorm 33 x 4096 7.0 / 10.5, 512 x 4096 9.1 / 12.5, 4096 x 4096
   // 29.8 / 33.0), except with the residual add on middle sizes, where the row caches spare the second read of the sum: 512 x 4096
@@ -1058,7 +1224,7 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   p.inv_rms = inv_rms;
   p.amax_bits = amax_bits;
   p.amax_words = words;
-  p.amax_out = word_per_cta && !absmax_ready && !inline_absmax ? static_cast<unsigned int *>(workspace) : amax_out;
+  p.amax_out = !absmax_ready && (inline_absmax ? leave_absmax : word_per_cta) ? static_cast<unsigned int *>(workspace) : amax_out;
   p.scale_out = scale_out;
   p.a_comp = static_cast<uint8_t *>(a_comp);
   p.e = static_cast<uint8_t *>(e);

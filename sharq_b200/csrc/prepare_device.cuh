@@ -186,20 +186,21 @@ __device__ __forceinline__ void quantize_group32(const uint32_t (&xw)[16], const
   o.sf_res = sf_res;
 }
 
-// bf16(y / scale) of a whole 32-element group, y already bf16-exact floats.
+// bf16(y / scale) of 2 * kWords elements (a 32-element group, or a lane's part of one), y already bf16-exact floats.
 // q = y * recip is within 2 ulp of the true quotient; when q is more than 4 ulp away from
 // every bf16 rounding boundary (low 16 bits == 0x8000) the IEEE quotient rounds to the same
 // bf16 value.  The boundary test is done on packed halves: the low
 // 16 bits of both products of a word go into one register (one byte permute), 0x8004 is added
 // to each half (a carry out of the low half can only raise the high half by one, which the
 // wider threshold absorbs), and a packed unsigned minimum over the group is compared once.
-// A group in which any product lies within the window is redone with IEEE divisions.
-__device__ __forceinline__ void scale_group32(uint32_t (&w)[16], float scale, float recip) {
-  uint32_t out[16];
+// Where any product lies within the window the words concerned are redone.
+template <int kWords>
+__device__ __forceinline__ void scale_words(uint32_t (&w)[kWords], float scale, float recip) {
+  uint32_t out[kWords];
   uint32_t nearest = 0xFFFFFFFFu;
   const uint64_t recip2 = pair_f32(recip, recip);
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
+  for (int i = 0; i < kWords; ++i) {
     const float2 q = mul_word(w[i], recip2);
     const uint32_t lows = __byte_perm(__float_as_uint(q.x), __float_as_uint(q.y), 0x5410);
     nearest = __vminu2(nearest, lows + 0x80048004u);
@@ -212,7 +213,7 @@ __device__ __forceinline__ void scale_group32(uint32_t (&w)[16], float scale, fl
     // multiply-adds (the classic division refinement, exact because recip is the correctly
     // rounded reciprocal), or an IEEE division for tiny operands or a subnormal quotient.
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
+    for (int i = 0; i < kWords; ++i) {
       const float ya = lo_f(w[i]), yb = hi_f(w[i]);
       float qa = __fmul_rn(ya, recip), qb = __fmul_rn(yb, recip);
       const uint32_t ta = (__float_as_uint(qa) + 0x8004u) & 0xFFFFu;
@@ -233,7 +234,7 @@ __device__ __forceinline__ void scale_group32(uint32_t (&w)[16], float scale, fl
     }
   }
 #pragma unroll
-  for (int i = 0; i < 16; ++i) w[i] = out[i];
+  for (int i = 0; i < kWords; ++i) w[i] = out[i];
 }
 
 // A selected pair whose score is non-zero but below 2^-118 (key = float bits | pair index).
@@ -252,7 +253,7 @@ __device__ __forceinline__ float round_to_bf16(float x) { return __bfloat162floa
 
 // Tensor-scale division and quantisation of one group.
 //   kMode 1: the divisor is the float32 scale (the reference's RMSNorm kernel divides by it with
-//            __fdiv_rn): products with a boundary test, see scale_group32.
+//            __fdiv_rn): products with a boundary test, see scale_words.
 //   kMode 2: the divisor has an 8-bit significand (see round_to_bf16), and so has y.  The exact
 //            quotient of two such numbers is either representable in 8 bits or at least a
 //            relative 2^-17 away from every value with a 9-bit significand, i.e. from every bf16
@@ -266,7 +267,7 @@ template <int kMode, bool kDebug, typename Reload>
 __device__ __forceinline__ void scale_quantize_group(uint32_t (&y)[16], float div, float recip, const ScaleTables &tbl,
                                                      GroupOut &o, Reload reload) {
   if (kMode == 1) {
-    scale_group32(y, div, recip);
+    scale_words(y, div, recip);
     quantize_group32<kDebug>(y, tbl, o);
   } else if (kMode == 2) {
 #pragma unroll 1
@@ -288,6 +289,73 @@ __device__ __forceinline__ void scale_quantize_group(uint32_t (&y)[16], float di
   } else {
     quantize_group32<kDebug>(y, tbl, o);
   }
+}
+
+// An 8-element chunk of a group whose four chunks lie in four neighbouring lanes (lane & 3): the arithmetic of quantize_group32, a
+// quarter of the serial chain per lane.
+struct ChunkOut {
+  uint32_t q_res;      // 4 B dense residual payload
+  uint32_t a_comp;     // 2 B compressed sparse payload
+  uint32_t meta;       // a nibble
+  uint32_t sf_sparse;  // the group's scale code, in all four lanes
+  uint32_t sf_res;     // the 16-group's scale code, in both of its lanes
+};
+
+struct ChunkPick {
+  uint32_t near_pair, far_pair;  // 3 - index of the kept pairs
+  uint32_t best, second;         // their keys
+};
+
+__device__ __forceinline__ ChunkPick pick_pairs(const uint32_t (&xw)[4]) {
+  uint32_t key[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) key[p] = __float_as_uint(fmaxf(fabsf(lo_f(xw[p])), fabsf(hi_f(xw[p])))) | (uint32_t)(3 - p);
+  const uint32_t m01 = max(key[0], key[1]), n01 = min(key[0], key[1]);
+  const uint32_t m23 = max(key[2], key[3]), n23 = min(key[2], key[3]);
+  ChunkPick c;
+  c.best = max(m01, m23);
+  c.second = max(min(m01, m23), max(n01, n23));
+  c.near_pair = max(c.best & 3u, c.second & 3u);
+  c.far_pair = min(c.best & 3u, c.second & 3u);
+  return c;
+}
+
+__device__ __forceinline__ void quantize_chunk8(const uint32_t (&xw)[4], const ChunkPick &pick, const ScaleTables &tbl, ChunkOut &o) {
+  o.meta = (pick.near_pair | (pick.far_pair << 2)) ^ 0xFu;
+  uint32_t max_key = pick.best;
+  max_key = max(max_key, __shfl_xor_sync(0xffffffffu, max_key, 1));
+  max_key = max(max_key, __shfl_xor_sync(0xffffffffu, max_key, 2));
+  o.sf_sparse = scale_code_from_max(__uint_as_float(max_key & 0xFFFF0000u));
+  const float s_q = tbl.value[o.sf_sparse], s_r = tbl.recip[o.sf_sparse];
+  const uint64_t s_r2 = pair_f32(s_r, s_r), neg_s2 = pair_f32(-s_q, -s_q);
+  uint64_t xp[4];
+  float2 t[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    xp[p] = pair_f32(lo_f(xw[p]), hi_f(xw[p]));
+    t[p] = unpair_f32(mul_f32x2(xp[p], s_r2));
+  }
+  const uint32_t all4 = pack_e2m1x8(t[0].x, t[0].y, t[1].x, t[1].y, t[2].x, t[2].y, t[3].x, t[3].y);
+  const uint32_t mask4 = (0xFF000000u >> (8 * pick.near_pair)) | (0xFF000000u >> (8 * pick.far_pair));
+  const uint32_t dense4 = all4 & mask4;
+  uint32_t h[4];
+  decode_e2m1x8(dense4, h);
+  float mx = 0.0f;
+  uint64_t r[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float2 q = __half22float2(*reinterpret_cast<__half2 *>(&h[p]));
+    r[p] = fma_f32x2(pair_f32(q.x, q.y), neg_s2, xp[p]);
+    const float2 d = unpair_f32(r[p]);
+    mx = max3(mx, fabsf(d.x), fabsf(d.y));
+  }
+  o.a_comp = __byte_perm(dense4, 0u, 0x4433u - pick.near_pair - (pick.far_pair << 4));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  o.sf_res = scale_code_from_max(mx);
+  const float rr = tbl.recip[o.sf_res];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) t[p] = unpair_f32(mul_f32x2(r[p], pair_f32(rr, rr)));
+  o.q_res = pack_e2m1x8(t[0].x, t[0].y, t[1].x, t[1].y, t[2].x, t[2].y, t[3].x, t[3].y);
 }
 
 __device__ __forceinline__ void zero_range(uint8_t *base, size_t begin, size_t end, int worker, int workers) {

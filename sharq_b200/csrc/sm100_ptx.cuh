@@ -149,6 +149,18 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
+// A float into the same variable of CTA `cta_rank`; visible behind a cluster barrier.
+__device__ __forceinline__ void st_cluster_f32(float *var, uint32_t cta_rank, float v) {
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %0, %1;\n\t"
+      "st.shared::cluster.f32 [remote], %2;\n\t"
+      "}" ::"r"(smem_u32(var)),
+      "r"(cta_rank), "f"(v)
+      : "memory");
+}
+
 // 16 bytes into the shared memory of CTA `cta_rank` (addr, bar: this CTA's addresses of the same variables), counted on its barrier.
 __device__ __forceinline__ void st_async_cluster_x4(uint32_t addr, uint64_t *bar, uint32_t cta_rank, uint32_t a, uint32_t b, uint32_t c,
                                                     uint32_t d) {
