@@ -515,24 +515,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     }
   };
 
-  // The set-up above and the loads below overlap the end of the kernel that prepares the activation; from the wait on
-  // every role reads or writes what earlier kernels may still use.
-  // The fused GEMM's weight is not written by a kernel that lets its dependents start early (see grid_launch_dependents): its first
-  // stages are loaded here, as many as the ring holds (with the epilogues below the linears of a 32-token decode step 83.6 -> 79.9 us).
-  constexpr bool kPreload = SPARSE && DENSE && !GROUPED;
-  int preloaded = 0;
-  if (kPreload && warp == 0 && unit0 < num_units) {
-    preloaded = min(S, it_end - it_begin);
-    if (ptx::elect_one()) {
-      for (int i = 0; i < preloaded; ++i) {
-        ptx::mbar_arrive_expect_tx(full_bar + i, stage_bytes(it_begin + i));
-        load_weight(it_begin + i, i, unit0 / m_units, &tm_w, p.sfb_dense, p.sfb_sparse);
-      }
-    }
-    __syncwarp();
-  }
-  if (!kPreload && !PAIR && warp == 0 && unit0 < num_units) {
-    // the operands of the single-pass GEMMs may come from any kernel: into L2, where a prefetch cannot make stale data visible
+  // The set-up above and the prefetch below overlap the end of the kernel that prepares the activation; from the wait on
+  // every role reads or writes what earlier kernels may still use.  The prefetch goes to L2, where it cannot make stale data visible.
+  // Loads of the weight into the ring ahead of the wait were no faster (linears of a layer with 8 / 32 / 64 / 128 tokens 73.3 / 79.2 / 84.5 / 93.3 us,
+  // prefetched 73.1 / 79.2 / 83.5 / 92.2): they get in the prepare's way.
+  if (!PAIR && warp == 0 && unit0 < num_units) {
+    // weight tiles of this CTA's first stages: nothing of them depends on the activation
     if (ptx::elect_one()) {
       const int n_tile = unit0 / m_units;
       const int ahead = min(it_end, it_begin + kPrefetchStages);
@@ -569,16 +557,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         const int n_tile = tile / m_units;
         for (int it = it_begin; it < it_end; ++it, ++g) {
           const int s = (int)(g % S);
-          if ((int)g >= preloaded) {
-            if (!ptx::mbar_wait(empty_bar + s, ((g / S) & 1u) ^ 1u, abort_flag)) {
-              *abort_flag = 1;
-              atomicExch(p.error_flag, 1);
-              ok = false;
-              break;
-            }
-            ptx::mbar_arrive_expect_tx(full_bar + s, stage_bytes(it));
-            load_weight(it, s, n_tile, tw, sfb_dense, sfb_sparse);
+          if (!ptx::mbar_wait(empty_bar + s, ((g / S) & 1u) ^ 1u, abort_flag)) {
+            *abort_flag = 1;
+            atomicExch(p.error_flag, 1);
+            ok = false;
+            break;
           }
+          ptx::mbar_arrive_expect_tx(full_bar + s, stage_bytes(it));
+          load_weight(it, s, n_tile, tw, sfb_dense, sfb_sparse);
           load_activation(it, s, m_tile);
         }
       }

@@ -269,9 +269,8 @@ constexpr size_t kInlineAbsmaxElements = 64 * 1024;
 constexpr size_t kInlineAbsmaxElementsNoWords = 192 * 1024;
 // Up to this size, with the maximum ready and more than one 32-row tile, a lane takes 8 elements (prepare_narrow_kernel).  us, statistics and
 // wide / narrow prepare: RMSNorm 48 x 4096 6.1 / 5.3, 128 x 4096 6.5 / 5.8, 200 x 4096 6.5 / 6.7, 256 x 4096 6.7 / 7.4; tensor scale 128 x 4096
-// 5.0 / 4.5, 200 x 4096 5.1 / 6.1.  Up to 32 rows the narrow form is as much faster by itself, but it spreads over all SMs, on which the
-// GEMM behind it then starts to load its weight sooner, in the prepare's way: linears of a layer with 8 / 32 / 64 / 128 tokens wide 73.8 /
-// 80.0 / 85.8 / 94.0, narrow 78.1 / 82.1 / 85.3 / 93.5.
+// 5.0 / 4.5, 200 x 4096 5.1 / 6.1.  Up to 32 rows it is faster by itself (RMSNorm 32 x 4096 6.1 / 5.1) but not between GEMMs: linears of a
+// Llama-3-8B layer with 8 / 32 / 64 / 128 tokens wide 72.4 / 78.4 / 85.8 / 94.0, narrow 77.2 / 80.9 / 83.9 / 91.9.
 constexpr size_t kNarrowElements = 640 * 1024;
 constexpr unsigned kMaxAbsmaxWords = 4096;            // words of CTA maxima that every prepare CTA reduces
 
@@ -287,6 +286,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
   const int groups32 = k >> 5;
   const int aligned_m = (m + 127) / 128 * 128;
 
+  ptx::grid_launch_dependents();
   __shared__ ScaleTables tbl;
   extern __shared__ uint4 gamma_smem[];  // mode 1: the whole RMSNorm weight, k bf16
   if (threadIdx.x < 128) {
@@ -297,7 +297,6 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
   __shared__ float scan_max[kScanCtas];  // kCluster
   if (kCluster) ptx::cluster_arrive();
   ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();  // behind the wait: a GEMM that follows loads its weight before its own wait
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k_tiles = (k + kColsPerCta - 1) / kColsPerCta;
   const int total_tiles = k_tiles * p.row_tiles;
@@ -529,6 +528,7 @@ __global__ void __launch_bounds__(32 * narrow_warps(kMode)) prepare_narrow_kerne
   const int m = p.m, k = p.k, groups32 = k >> 5;
   const int aligned_m = (m + 127) / 128 * 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  ptx::grid_launch_dependents();
   __shared__ ScaleTables tbl;
   __shared__ float part_max[kNarrowWarps];
   if (threadIdx.x < 128) {
@@ -537,7 +537,6 @@ __global__ void __launch_bounds__(32 * narrow_warps(kMode)) prepare_narrow_kerne
     tbl.recip[threadIdx.x] = __frcp_rn(v);  // code 0 is never looked up (scales are clamped to >= 2^-9)
   }
   ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();  // see prepare_kernel
 
   const int k_tiles = (k + 255) / 256;
   const int task = (int)blockIdx.x * kNarrowWarps + warp;
@@ -711,13 +710,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) prepare_fused_kernel(const F
   float *partial = reinterpret_cast<float *>(cache + (size_t)p.chunk_rows * row_vecs);  // mode 1: chunk_rows x partial_stride
   float *inv_s = partial + (kMode == 1 ? p.chunk_rows * partial_stride : 0);            // mode 1: rows_per_cta
 
+  ptx::grid_launch_dependents();
   if (threadIdx.x < 128) {
     const float v = ue4m3_to_float(threadIdx.x);
     tbl.value[threadIdx.x] = v;
     tbl.recip[threadIdx.x] = __frcp_rn(v);  // code 0 is never looked up (scales are clamped to >= 2^-9)
   }
   ptx::grid_dependency_wait();
-  ptx::grid_launch_dependents();  // see prepare_kernel
   if (kMode == 1) {
     const uint4 *gsrc = reinterpret_cast<const uint4 *>(p.gamma);
     for (int i = threadIdx.x; i < row_vecs; i += kFusedThreads) gamma_s[cache_slot(i >> 2, i & 3)] = gsrc[i];

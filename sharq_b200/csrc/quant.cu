@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kScaledThreads, kShared ? 4 : 6) scaled_quanti
                                                                          float *scale_out) {
   constexpr int kVecs = kShared ? 4 : 2;  // 16-byte vectors of a group
   __shared__ float warp_max[kScaledThreads / 32];
-  // no early launch of dependents: a GEMM behind this kernel may load the weight ahead of its wait
+  ptx::grid_launch_dependents();
   ptx::grid_dependency_wait();
   if (kShared) zero_scale_padding(rows, k, sf, sf2);
   float mx = 0.0f;

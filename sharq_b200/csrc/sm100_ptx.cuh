@@ -200,9 +200,7 @@ __device__ __forceinline__ float4 ld_shared_f32x4(uint32_t addr) {
 // a const __restrict__ parameter, which the compiler may load through it) is defined only for data that nothing
 // writes during the kernel's life: such kernels read global memory with ordinary loads and declare no pointer __restrict__.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Lets a dependent kernel that was launched with the attribute start its blocks (it waits itself before it reads; the fused GEMM
-// loads its weight before that: a kernel that may write a weight does not call this, and one that may stand between such a
-// kernel and the GEMM calls it behind its own wait, when all that came before it is complete and visible).
+// Lets a dependent kernel that was launched with the attribute start its blocks (it waits itself before it reads).
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------- TMA
