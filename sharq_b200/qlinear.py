@@ -26,6 +26,7 @@ from .quantize import (
     quantize_activation_sparse_residual_nvfp4,
     quantize_weight_nvfp4,
     quantize_weight_shared_nvfp4,
+    without_grad,
 )
 
 
@@ -101,7 +102,7 @@ class QLinearLayer(nn.Module):
         # the fused GEMM takes the weight tensor scale as a host scalar: keep it in step with the buffer
         self.weight_scale_host = float(self.weight_scale.item())
 
-    @torch.no_grad()
+    @without_grad
     def prepare_input(self, x_2d: torch.Tensor, out_features_hint: Optional[int] = None):
         x_2d = x_2d.to(torch.bfloat16)
         if self.quant_type == "SHARQ":
@@ -111,7 +112,7 @@ class QLinearLayer(nn.Module):
         qx, scale_x, scale = quantize_activation_nvfp4(x_2d)
         return ("NVFP4", qx, scale_x, scale)
 
-    @torch.no_grad()
+    @without_grad
     def prepare_input_rmsnorm(self, x_2d: torch.Tensor, rmsnorm_weight: torch.Tensor, rmsnorm_eps: float,
                               out_features_hint: Optional[int] = None):
         if self.quant_type == "SHARQ" and self.extra_fusion:
@@ -122,7 +123,7 @@ class QLinearLayer(nn.Module):
         x_norm = apply_rmsnorm(x_2d.to(torch.bfloat16), rmsnorm_weight, rmsnorm_eps)
         return self.prepare_input(x_norm, out_features_hint=out_features_hint)
 
-    @torch.no_grad()
+    @without_grad
     def prepare_input_add_rmsnorm(self, x_2d: torch.Tensor, residual_2d: torch.Tensor, rmsnorm_weight: torch.Tensor,
                                   rmsnorm_eps: float, out_features_hint: Optional[int] = None):
         """(prepared activation of rmsnorm(x + residual), x + residual): the residual add of the
@@ -136,7 +137,7 @@ class QLinearLayer(nn.Module):
         total = x_2d + residual_2d
         return self.prepare_input_rmsnorm(total, rmsnorm_weight, rmsnorm_eps, out_features_hint), total
 
-    @torch.no_grad()
+    @without_grad
     def prepare_input_swiglu(self, gate_up_2d: torch.Tensor, out_features_hint: Optional[int] = None):
         """Prepared activation of act_fn(gate) * up for this (down_proj) layer from the merged
         gate_up output [M, 2 * in_features]: the three ATen passes of
@@ -147,7 +148,7 @@ class QLinearLayer(nn.Module):
         a_comp, e, sfa, q_res, sf_res, scale_x = ops.swiglu_sparse_residual_quantize_x(gate_up_2d, n)
         return ("SHARQ", a_comp, e, sfa, q_res, sf_res, scale_x)
 
-    @torch.no_grad()
+    @without_grad
     def apply_prepared(self, prepared, out=None, scatter=None, residual=None):
         """out: optional bf16 [M, N] tensor the fused SharQ GEMM writes into (used by the
         tensor-parallel layers to place partial sums in symmetric memory).  scatter: see
@@ -209,7 +210,7 @@ class QLinearLayer(nn.Module):
             return ("SHARQ", *ops.absmax_sparse_residual_quantize_x(h, down.out_features, amax_bits))
         return down.prepare_input_swiglu(self.apply_prepared(prepared))
 
-    @torch.no_grad()
+    @without_grad
     def forward(self, x):
         if isinstance(x, tuple):
             x_orig, bsz, q_len = x
