@@ -424,11 +424,12 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     return make_int4(*slot0 * L::kStageBytes - 32 * run0, stride, run0, 0);
   };
   // Where a CTA lays its parts out, one block per owner, to be sent by block copies (-1: they go from registers, 16 bytes at a time: up
-  // to 32 rows, where that is faster, and where the stages beside the receiving slots do not hold the blocks).  us, registers / blocks:
+  // to 32 rows and between two CTAs, where that is faster, and where the stages beside the receiving slots do not hold the blocks).  us, registers / blocks:
   // 4096 x 4096 at M = 1 6.1 / 7.1, 32 7.2 / 7.5, 64 9.1 / 8.6, 96 11.1 / 10.2; 4096 x 14336 at M = 32 11.9 / 12.2, 64 13.7 / 13.1,
-  // 128 17.5 / 16.3.
+  // 128 17.5 / 16.3; between two CTAs 3584 x 18944 at M = 211 24.5 / 25.4, 256 24.8 / 25.1.
+  const bool blocks = split && k_splits > 2 && split_rows > kRegisterRows;
   auto send_offset = [&](int rank) {
-    if (split_rows <= kRegisterRows) return -1;
+    if (!blocks) return -1;
     int slot0, slots;
     recv_entry(rank, &slot0, &slots);
     const int need = (split_rows * (BN + k_splits * kRecvPad) * 4 + L::kStageBytes - 1) / L::kStageBytes;
@@ -456,7 +457,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     if (split) {
       // what arrives: the columns, and with a block copy their padding too
       int bytes = k_splits * split_rows * 32 * (first_run(k_rank + 1, k_splits, kRuns) - first_run(k_rank, k_splits, kRuns));
-      if (split_rows > kRegisterRows)
+      if (blocks)
         for (int s = 0; s < k_splits; ++s) bytes += send_offset(s) >= 0 ? split_rows * 4 * kRecvPad : 0;
       ptx::mbar_arrive_expect_tx(recv_bar, (uint32_t)bytes);
     }
@@ -817,7 +818,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
             }
             __syncwarp();
             // A CTA may leave once its parts are on their way; where they may be read from its memory, once they have arrived.
-            if (split_rows <= kRegisterRows) ptx::cluster_arrive();
+            if (!blocks) ptx::cluster_arrive();
             // parts that are under way are waited for also when another role has given up
             if (!ptx::mbar_wait_cluster_acquire(recv_bar, 0, never_set)) {
               *abort_flag = 1;
@@ -825,7 +826,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
               ok = false;
             }
             ok = __all_sync(0xffffffffu, ok);
-            if (split_rows > kRegisterRows) ptx::cluster_arrive();
+            if (blocks) ptx::cluster_arrive();
           }
 #pragma unroll 1
           for (int i = (int)threadIdx.x - 64; i < items && ok; i += 32 * kEpiWarps) {
