@@ -70,6 +70,10 @@ constexpr int max_recv_bytes(int bn) {
   return most;
 }
 
+// A wait that ran out: the first code of a launch stays.  Whatever gives up makes others give up behind it (a CTA that sends nothing lets the
+// waits of its cluster run out), and their codes would hide the role that failed first.
+__device__ __forceinline__ void report(int *error_flag, int code) { atomicCAS(error_flag, 0, code); }
+
 // Shared-memory stage and tensor-memory column layout.  In pair mode BN is the pair's tile
 // width (256) and each CTA stores half of the weight tile.
 template <int BN, bool SPARSE, bool DENSE, bool PAIR>
@@ -560,7 +564,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
           const int s = (int)(g % S);
           if (!ptx::mbar_wait(empty_bar + s, ((g / S) & 1u) ^ 1u, abort_flag)) {
             *abort_flag = 1;
-            atomicExch(p.error_flag, 1);
+            report(p.error_flag, 1);
             ok = false;
             break;
           }
@@ -577,10 +581,10 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
         for (int s = slot0; s < slot0 + slots && ok; ++s) {
           if (s >= n) continue;
           ok = ptx::mbar_wait(empty_bar + s, (uint32_t)((n - 1 - s) / S) & 1u, abort_flag);
-        }
-        if (!ok) {
-          *abort_flag = 1;
-          atomicExch(p.error_flag, 6);
+          if (!ok) {
+            *abort_flag = 1;
+            report(p.error_flag, 6);
+          }
         }
       }
     }
@@ -603,7 +607,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
             const int s = (int)(g % S);
             if (!ptx::mbar_wait(full_bar + s, (g / S) & 1u, abort_flag)) {
               *abort_flag = 1;
-              atomicExch(p.error_flag, 4);
+              report(p.error_flag, 4);
               ok = false;
               break;
             }
@@ -624,7 +628,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
                                     : ptx::mbar_wait(acc_empty_bar, (tile_iter & 1u) ^ 1u, abort_flag);
           if (!drained) {
             *abort_flag = 1;
-            atomicExch(p.error_flag, 5);
+            report(p.error_flag, 5);
             break;
           }
           ptx::tc_fence_after();
@@ -636,7 +640,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
             if (PAIR && got) got = ptx::mbar_wait_cluster(peer_bar + s, ph, abort_flag);
             if (!got) {
               *abort_flag = 1;
-              atomicExch(p.error_flag, 2);
+              report(p.error_flag, 2);
               ok = false;
               break;
             }
@@ -741,7 +745,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
       ++tile_iter;
       if (!ok) {
         *abort_flag = 1;
-        atomicExch(p.error_flag, 3);
+        report(p.error_flag, 3);
       }
       ok = __all_sync(0xffffffffu, ok);
       ptx::tc_fence_after();
@@ -822,7 +826,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
             // parts that are under way are waited for also when another role has given up
             if (!ptx::mbar_wait_cluster_acquire(recv_bar, 0, never_set)) {
               *abort_flag = 1;
-              atomicExch(p.error_flag, 7);
+              report(p.error_flag, 7);
               ok = false;
             }
             ok = __all_sync(0xffffffffu, ok);
