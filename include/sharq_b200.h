@@ -387,6 +387,10 @@ int sharq_set_gemm_tile_n(int tile_n);
 /* Test/tuning hook: the variant that the automatic choice takes for a shape on a GPU of `sms` SMs (128, 256 or 512 as above);
  * split_k: whether the call gives leave to split K.  Runs nothing. */
 int sharq_gemm_tile_n(int m, int n, int k, int split_k, int sms);
+/* Test hook: how the fp32 parts of an output tile with `rows` rows (1..128) meet when K is split over `splits` CTAs (2..8) of a
+ * single-CTA kernel (tile_n 128 or 256): 0 = sent to the CTAs that sum them, from registers; 1 = by block copies; 2 = read behind a
+ * cluster barrier; -1 for other arguments.  Runs nothing. */
+int sharq_gemm_exchange(int tile_n, int sparse, int dense, int rows, int k, int splits);
 
 #ifdef __cplusplus
 }

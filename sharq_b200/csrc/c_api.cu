@@ -691,6 +691,11 @@ int sharq_gemm_tile_n(int m, int n, int k, int split_k, int sms) {
   return m > 0 && n > 0 && k > 0 && sms > 0 ? sharq::gemm_tile_n(m, n, k, split_k != 0, sms) : 0;
 }
 
+int sharq_gemm_exchange(int tile_n, int sparse, int dense, int rows, int k, int splits) {
+  if ((tile_n != 128 && tile_n != 256) || (!sparse && !dense) || rows < 1 || rows > 128 || k < 1 || splits < 2 || splits > 8) return -1;
+  return sharq::gemm_exchange(tile_n, sparse != 0, dense != 0, rows, k, splits);
+}
+
 int sharq_gemm_swiglu_pays(int m, int ffn, int k) { return m > 0 && ffn > 0 && k > 0 && sharq::gemm_swiglu_pays(m, ffn, k); }
 
 int sharq_gemm_swiglu_absmax_words(int m, int ffn) { return m > 0 && ffn > 0 ? sharq::gemm_swiglu_absmax_words(m, ffn) : 0; }

@@ -21,10 +21,9 @@
 //              tensor memory back to the MMA warp at once, then alpha/beta/bias, bf16 (packed
 //              conversions), a transpose through a small shared-memory tile and coalesced
 //              global stores overlap the next tile's MMAs.
-// Few tiles (decode batches, short chunks): K is split over the CTAs of a cluster, one tile per cluster; every
-// CTA sends the columns of its fp32 partial tile to the CTAs that own them (asynchronous stores to distributed shared
-// memory that count on the owner's barrier) and sums its own columns in rank order (no scratch, no second
-// kernel, a fixed order of additions).
+// Few tiles (decode batches, short chunks): K is split over the CTAs of a cluster, one tile per cluster; the fp32 partial tiles meet in
+// distributed shared memory, where every element is summed in rank order (no scratch, no second kernel, a fixed order of
+// additions).  How they meet depends on the rows of the tile, see Exchange.
 // CTA-pair mode (cta_group::2, cluster of 2): the pair computes a 256 x 256 tile; CTA r owns
 // rows [128r,128r+128) (its A operands, scales, metadata, accumulator) and loads weight rows
 // [128r,128r+128) of the tile; the tensor cores of both SMs read both halves.  Every CTA
@@ -57,14 +56,27 @@ constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 // Split launches: the columns of a tile are dealt over the CTAs of the cluster in runs of 8; run u belongs to rank
 // u * splits / runs.
 __host__ __device__ constexpr int first_run(int rank, int splits, int runs) { return (rank * runs + splits - 1) / splits; }
-constexpr int kRegisterRows = 32;  // rows of a tile whose parts are sent from registers, see send_offset
 constexpr int kRecvPad = 4;  // floats behind each received row: neighbouring rows start on distinct banks
+
+// How the partial tiles of a split launch meet:
+//   kSendRegisters: every CTA sends the columns of its part to the CTAs that own them, 16 bytes at a time from its registers
+//     (asynchronous stores that count on the owner's barrier), and sums its own columns.
+//   kSendBlocks: the same by one block copy per owner, out of stages beside the receiving ones.
+//   kPull: every CTA leaves its part in its own shared memory, and behind a cluster barrier all threads of the cluster read the others'.
+// Sending saves the latency of the reads and a barrier, but its 16-byte stores and its few receiving CTAs are slower per byte.  us of a prepare
+// and its fused GEMM, registers / blocks / pull: 1024 x 8192 (8 CTAs per tile) at M = 16 9.7 / 9.9 / 11.2, 32 11.1 / 11.1 / 12.1, 48 12.7 / 12.1 / 12.9,
+// 64 14.7 / 13.4 / 13.8, 96 17.5 / 15.9 / 15.7, 128 21.2 / 19.1 / 18.2; 3584 x 18944 (4) at 48 20.6 / 20.2 / 20.4, 64 22.0 / 21.2 / 21.4, 128 27.3 / 26.0 / 24.0,
+// 384 (3, wide tiles) 44.7 / 44.6 / 40.0; 6144 x 4096 (3) at 64 13.8 / 14.2 / 13.3; 3584 x 18944 (2) at 211 33.5 / 33.8 / 31.1.
+enum Exchange { kSendRegisters = 0, kSendBlocks = 1, kPull = 2 };
+constexpr int kRegisterRows = 32;  // rows of a tile up to which parts are sent from registers
+constexpr int kBlockSplits = 4;    // fewer CTAs per tile: blocks are no faster than reads
+constexpr int block_rows(int splits) { return 48 + 4 * splits; }  // rows up to which they are
 constexpr int max_recv_bytes(int bn) {
   int most = 0;
   for (int s = 2; s <= kMaxSplits; ++s)
     for (int r = 0; r < s; ++r) {
       const int cols = 8 * (first_run(r + 1, s, bn / 8) - first_run(r, s, bn / 8));
-      const int bytes = s * kBM * (cols + kRecvPad) * 4;
+      const int bytes = s * block_rows(s) * (cols + kRecvPad) * 4;
       most = bytes > most ? bytes : most;
     }
   return most;
@@ -110,10 +122,39 @@ struct StageLayout {
   static constexpr int kColSfbD = kColSfaD + 16;
   static constexpr int kColEnd = kColSfbD + 4 * (BN / 32);
   static constexpr int kTmemCols = kColEnd <= 256 ? 256 : 512;
-  static_assert(PAIR || max_recv_bytes(BN) <= kStages * kStageBytes, "the received parts take the place of the stages");
+  static constexpr int kPartStride = BN + 4;  // floats per row of a partial tile that is pulled (row starts on distinct banks)
+  static_assert(PAIR || (max_recv_bytes(BN) <= kStages * kStageBytes && kBM * kPartStride * 4 <= kStages * kStageBytes),
+                "the parts take the place of the stages");
   static constexpr int kSmemBytes =
       kStages * kStageBytes + kOutStageBytes + 1024 /*alignment slack*/ + 512 /*barriers*/;
 };
+
+// Where a rank receives the parts of its columns: in the stages that it is done with first (its last use of a slot lies furthest back).
+struct RecvSlots {
+  int first, count;
+};
+template <class L>
+__host__ __device__ constexpr RecvSlots recv_slots(int rank, int splits, int rows, int k_stages, int runs) {
+  const int stride = 4 * (8 * (first_run(rank + 1, splits, runs) - first_run(rank, splits, runs)) + kRecvPad);
+  const int oldest = (k_stages * (rank + 1) / splits - k_stages * rank / splits) % L::kStages;
+  const int count = (splits * rows * stride + L::kStageBytes - 1) / L::kStageBytes;
+  return {oldest + count <= L::kStages ? oldest : 0, count};
+}
+// The stage that the blocks of a rank are laid out from: the first ones, or those behind the receiving slots; -1: neither holds them.
+template <class L>
+__host__ __device__ constexpr int send_slot(int rank, int splits, int rows, int k_stages, int bn) {
+  const RecvSlots r = recv_slots<L>(rank, splits, rows, k_stages, bn / 8);
+  const int need = (rows * (bn + splits * kRecvPad) * 4 + L::kStageBytes - 1) / L::kStageBytes;
+  return r.first >= need ? 0 : (L::kStages - r.first - r.count >= need ? r.first + r.count : -1);
+}
+template <class L>
+constexpr Exchange exchange_form(int rows, int splits, int k_stages, int bn) {
+  if (rows <= kRegisterRows) return kSendRegisters;
+  if (rows > block_rows(splits) || splits < kBlockSplits) return kPull;
+  for (int r = 0; r < splits; ++r)
+    if (send_slot<L>(r, splits, rows, k_stages, bn) < 0) return kPull;  // all CTAs of a cluster do the same
+  return kSendBlocks;
+}
 
 struct GemmParams {
   const uint8_t *e;
@@ -132,6 +173,7 @@ struct GemmParams {
   int *error_flag;
   // Split K: the k_splits CTAs of a cluster compute one output tile, each over its share of the K stages.
   int k_splits;
+  Exchange exchange, exchange_last;  // of the full tiles and of the last row of tiles
   int a_rows;        // rows of an activation box: the rows that exist when all are in one tile, else the tile's 128
   int staged_store;  // output tiles are transposed through shared memory for coalesced stores (N % 8 == 0)
   // Scatter mode (row-parallel linear under tensor parallelism): the output rows are dealt to their owner GPUs.
@@ -414,30 +456,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
   const int k_rank = PAIR ? 0 : (int)blockIdx.x % k_splits;  // the rank in the cluster of a split launch
   const int it_begin = k_stages * k_rank / k_splits, it_end = k_stages * (k_rank + 1) / k_splits;
   const bool split = !PAIR && k_splits > 1;
-  // Split launch: the rows of the cluster's tile, and where a rank receives the parts of its columns: in the stages that it is
-  // done with first (its last use of a slot lies furthest back).
-  const int split_rows = split ? min(kBM, p.m - (unit0 % m_units) * kBM) : 0;
+  const int split_rows = split ? min(kBM, p.m - (unit0 % m_units) * kBM) : 0;  // the rows of the cluster's tile
   constexpr int kRuns = BN / 8;
+  const Exchange exchange = !split ? kPull : (split_rows < kBM ? p.exchange_last : p.exchange);
   // What the senders need of a rank: byte offset of the tile's column 0 in row 0 of rank 0's part, bytes per row, its first run.
-  auto recv_entry = [&](int rank, int *slot0, int *slots) {
+  auto recv_entry = [&](int rank) {
     const int run0 = first_run(rank, k_splits, kRuns);
     const int stride = 4 * (8 * (first_run(rank + 1, k_splits, kRuns) - run0) + kRecvPad);
-    const int oldest = (k_stages * (rank + 1) / k_splits - k_stages * rank / k_splits) % S;
-    *slots = (k_splits * split_rows * stride + L::kStageBytes - 1) / L::kStageBytes;
-    *slot0 = oldest + *slots <= S ? oldest : 0;
-    return make_int4(*slot0 * L::kStageBytes - 32 * run0, stride, run0, 0);
-  };
-  // Where a CTA lays its parts out, one block per owner, to be sent by block copies (-1: they go from registers, 16 bytes at a time: up
-  // to 32 rows and between two CTAs, where that is faster, and where the stages beside the receiving slots do not hold the blocks).  us, registers / blocks:
-  // 4096 x 4096 at M = 1 6.1 / 7.1, 32 7.2 / 7.5, 64 9.1 / 8.6, 96 11.1 / 10.2; 4096 x 14336 at M = 32 11.9 / 12.2, 64 13.7 / 13.1,
-  // 128 17.5 / 16.3; between two CTAs 3584 x 18944 at M = 211 24.5 / 25.4, 256 24.8 / 25.1.
-  const bool blocks = split && k_splits > 2 && split_rows > kRegisterRows;
-  auto send_offset = [&](int rank) {
-    if (!blocks) return -1;
-    int slot0, slots;
-    recv_entry(rank, &slot0, &slots);
-    const int need = (split_rows * (BN + k_splits * kRecvPad) * 4 + L::kStageBytes - 1) / L::kStageBytes;
-    return slot0 >= need ? 0 : (S - slot0 - slots >= need ? (slot0 + slots) * L::kStageBytes : -1);
+    return make_int4(recv_slots<L>(rank, k_splits, split_rows, k_stages, kRuns).first * L::kStageBytes - 32 * run0, stride, run0, 0);
   };
 
   if (threadIdx.x == 32) {
@@ -458,18 +484,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     *abort_flag = 0;
     *never_set = 0;
     ptx::fence_barrier_init();
-    if (split) {
+    if (exchange != kPull) {
       // what arrives: the columns, and with a block copy their padding too
-      int bytes = k_splits * split_rows * 32 * (first_run(k_rank + 1, k_splits, kRuns) - first_run(k_rank, k_splits, kRuns));
-      if (blocks)
-        for (int s = 0; s < k_splits; ++s) bytes += send_offset(s) >= 0 ? split_rows * 4 * kRecvPad : 0;
-      ptx::mbar_arrive_expect_tx(recv_bar, (uint32_t)bytes);
+      const int cols = 8 * (first_run(k_rank + 1, k_splits, kRuns) - first_run(k_rank, k_splits, kRuns));
+      ptx::mbar_arrive_expect_tx(recv_bar, (uint32_t)(k_splits * split_rows * 4 * (cols + (exchange == kSendBlocks ? kRecvPad : 0))));
     }
   }
-  if (split && threadIdx.x >= 64 && (int)threadIdx.x - 64 < k_splits) {
-    int slot0, slots;
-    recv_tab[threadIdx.x - 64] = recv_entry((int)threadIdx.x - 64, &slot0, &slots);
-  }
+  if (exchange != kPull && threadIdx.x >= 64 && (int)threadIdx.x - 64 < k_splits)
+    recv_tab[threadIdx.x - 64] = recv_entry((int)threadIdx.x - 64);
   if (warp == 1) {
     ptx::tmem_alloc<CG>(tmem_slot, L::kTmemCols);
     ptx::tmem_relinquish<CG>();
@@ -573,12 +595,11 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
           load_activation(it, s, m_tile);
         }
       }
-      if (split) {
+      if (exchange != kPull) {
         // the slots that take the received parts are free once their last stage has been consumed
-        int slot0, slots;
-        recv_entry(k_rank, &slot0, &slots);
-        const int n = it_end - it_begin;
-        for (int s = slot0; s < slot0 + slots && ok; ++s) {
+        const RecvSlots slots = recv_slots<L>(k_rank, k_splits, split_rows, k_stages, kRuns);
+        const int slot0 = slots.first, n = it_end - it_begin;
+        for (int s = slot0; s < slot0 + slots.count && ok; ++s) {
           if (s >= n) continue;
           ok = ptx::mbar_wait(empty_bar + s, (uint32_t)((n - 1 - s) / S) & 1u, abort_flag);
           if (!ok) {
@@ -591,7 +612,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
     if (split) {
       __syncwarp();
       ptx::cluster_arrive();
-      ptx::cluster_wait();  // all CTAs can receive
+      ptx::cluster_wait();  // all CTAs can receive, or all parts are written
       ptx::cluster_arrive();
     }
   } else if (warp == 1) {
@@ -752,7 +773,57 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
       return ok;
     };
     if constexpr (!PAIR && !SWIGLU && !WIDE) {
-      if (split) {
+      if (exchange == kPull && split) {
+        bool ok = wait_acc();
+        const uint32_t part = ptx::smem_u32(smem);
+        const int r0 = quad * 32 + lane;
+        if (ok && quad * 32 < split_rows) {
+          const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::kColAcc + half * kColsPerEpiWarp);
+#pragma unroll 1
+          for (int c = 0; c < kColsPerEpiWarp / 32; ++c) {
+            uint32_t acc[32];
+            ptx::tmem_ld_32x32b_x32(taddr + 32 * c, acc);
+            ptx::tmem_ld_wait();
+            if (r0 < split_rows) {
+              uint4 *dst = reinterpret_cast<uint4 *>(smem + ((size_t)r0 * L::kPartStride + half * kColsPerEpiWarp + 32 * c) * 4);
+#pragma unroll
+              for (int v = 0; v < 8; ++v) dst[v] = make_uint4(acc[4 * v], acc[4 * v + 1], acc[4 * v + 2], acc[4 * v + 3]);
+            }
+          }
+        }
+        __syncwarp();
+        ptx::cluster_arrive();
+        ptx::cluster_wait();  // every CTA's part is written
+        const int m_tile = unit0 % m_units, n_tile = unit0 / m_units;
+        // 8 columns per thread, dealt over the threads of all CTAs: neighbouring lanes read neighbouring 32 bytes
+        for (int i = (int)threadIdx.x - 64 + k_rank * 32 * kEpiWarps; i < split_rows * kRuns && ok; i += k_splits * 32 * kEpiWarps) {
+          const int r = i / kRuns, c8 = i % kRuns;
+          const int row = m_tile * kBM + r, col = n_tile * BN + 8 * c8;
+          if (col >= p.n) continue;
+          const uint32_t at = part + (uint32_t)(r * L::kPartStride + 8 * c8) * 4u;
+          float4 lo[kMaxSplits], hi[kMaxSplits];
+#pragma unroll
+          for (int s = 0; s < kMaxSplits; ++s) {
+            if (s < k_splits) {
+              lo[s] = ptx::ld_cluster_f32x4(at, s);
+              hi[s] = ptx::ld_cluster_f32x4(at + 16, s);
+            }
+          }
+          float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int s = 0; s < kMaxSplits; ++s) {
+            if (s < k_splits) {
+              f[0] += lo[s].x, f[1] += lo[s].y, f[2] += lo[s].z, f[3] += lo[s].w;
+              f[4] += hi[s].x, f[5] += hi[s].y, f[6] += hi[s].z, f[7] += hi[s].w;
+            }
+          }
+          uint32_t o[4];
+          epilogue_8(p, f, row, col, alpha0, beta, has_c, o);
+          store_8(p, o, row, col);
+        }
+        __syncwarp();
+        ptx::cluster_arrive();
+      } else if (split) {
         // The first of two passes only runs the code of the sum on one item, unstored, while the stages are still being
         // consumed: fetched when the last stage is done, it took longer than the sum.  From the last stage's MMAs to the end of the
         // launch 4096 x 4096 at M = 32 takes 2.6 us (3.6 with a cluster barrier, a sum that reads the other CTAs' memory, and a second
@@ -770,8 +841,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
             ptx::cluster_wait();  // all CTAs can receive
             const int r = quad * 32 + lane;
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::kColAcc + half * kColsPerEpiWarp);
-            const int send = send_offset(k_rank);
-            if (send >= 0) {
+            if (exchange == kSendBlocks) {
+              const int send = send_slot<L>(k_rank, k_splits, split_rows, k_stages, BN) * L::kStageBytes;
               if (ok && quad * 32 < split_rows) {
 #pragma unroll 1
                 for (int c = 0; c < kColsPerEpiWarp / 32; ++c) {
@@ -822,7 +893,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
             }
             __syncwarp();
             // A CTA may leave once its parts are on their way; where they may be read from its memory, once they have arrived.
-            if (!blocks) ptx::cluster_arrive();
+            if (exchange == kSendRegisters) ptx::cluster_arrive();
             // parts that are under way are waited for also when another role has given up
             if (!ptx::mbar_wait_cluster_acquire(recv_bar, 0, never_set)) {
               *abort_flag = 1;
@@ -830,7 +901,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
               ok = false;
             }
             ok = __all_sync(0xffffffffu, ok);
-            if (blocks) ptx::cluster_arrive();
+            if (exchange == kSendBlocks) ptx::cluster_arrive();
           }
 #pragma unroll 1
           for (int i = (int)threadIdx.x - 64; i < items && ok; i += 32 * kEpiWarps) {
@@ -1217,7 +1288,11 @@ cudaError_t launch(const GemmArgs &a, cudaStream_t stream) {
         }
         if (capacity[dev][s] >= units) break;
       }
-      if (s >= 2) p.k_splits = s;
+      if (s >= 2) {
+        p.k_splits = s;
+        p.exchange = exchange_form<L>(kBM, s, k_stages, BN);
+        p.exchange_last = exchange_form<L>(a.m - (m_units - 1) * kBM, s, k_stages, BN);
+      }
     }
     attr[1].val.clusterDim.x = (unsigned)p.k_splits;
     cfg.gridDim = dim3(p.k_splits > 1 ? units * p.k_splits : (units < sms ? units : sms));
@@ -1324,6 +1399,18 @@ int gemm_tile_n(int m, int n, int k, bool split_k, int sms) {
     return split_k && k > 16384 && 2 * units_128 > sms && units_128 <= sms && 2 * units_256 <= sms ? 256 : 128;
   }
   return 512;
+}
+
+int gemm_exchange(int tile_n, bool sparse, bool dense, int rows, int k, int splits) {
+  const int k_stages = (k + kBK - 1) / kBK;
+  if (tile_n == 256) {
+    if (sparse && dense) return exchange_form<StageLayout<256, true, true, false>>(rows, splits, k_stages, 256);
+    return sparse ? exchange_form<StageLayout<256, true, false, false>>(rows, splits, k_stages, 256)
+                  : exchange_form<StageLayout<256, false, true, false>>(rows, splits, k_stages, 256);
+  }
+  if (sparse && dense) return exchange_form<StageLayout<128, true, true, false>>(rows, splits, k_stages, 128);
+  return sparse ? exchange_form<StageLayout<128, true, false, false>>(rows, splits, k_stages, 128)
+                : exchange_form<StageLayout<128, false, true, false>>(rows, splits, k_stages, 128);
 }
 
 static cudaError_t choose_tile_n(int m, int n, int k, bool split_k, int *tile_n) {

@@ -45,6 +45,10 @@ cudaError_t run_gemm(const GemmArgs &args, cudaStream_t stream);
 // Tile width that run_gemm takes on a GPU of `sms` SMs: 128 / 256 = single CTAs, 512 = CTA pairs of 256 x 256.
 int gemm_tile_n(int m, int n, int k, bool split_k, int sms);
 
+// How the partial tiles of a tile with `rows` rows and K split over `splits` CTAs meet: 0 = sent from registers, 1 = sent by block copies,
+// 2 = read behind a cluster barrier.
+int gemm_exchange(int tile_n, bool sparse, bool dense, int rows, int k, int splits);
+
 // Fused SharQ GEMM of a merged gate_up weight [2F, k] (n = 2F, F % 128 == 0, no bias) whose epilogue writes
 // h = bf16(bf16(silu(gate)) * up) [m, F] to d and every CTA's max|h| to amax_bits (nothing to zero before the launch): the h that the plain
 // GEMM followed by the SwiGLU kernel gives.

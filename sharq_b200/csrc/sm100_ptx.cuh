@@ -149,6 +149,21 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
+// 16 bytes of another CTA's shared memory (addr: this CTA's address of the same variable).
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t addr, uint32_t cta_rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t"
+      ".reg .b32 remote;\n\t"
+      "mapa.shared::cluster.u32 remote, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [remote];\n\t"
+      "}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(addr), "r"(cta_rank)
+      : "memory");
+  return v;
+}
+
 // A float into the same variable of CTA `cta_rank`; visible behind a cluster barrier.
 __device__ __forceinline__ void st_cluster_f32(float *var, uint32_t cta_rank, float v) {
   asm volatile(
