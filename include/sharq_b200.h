@@ -56,7 +56,8 @@ int sharq_fused_sparse_residual_quantize_x_debug(const void *x_bf16, int m, int 
                                                  void *sfa_sparse, void *q_res, void *sf_res, void *stream);
 
 /* Scratch bytes needed by the scaled prepare calls below for M rows.  Layout:
- * bytes [0,4) tensor absmax (float bits), bytes [4,8) arrival counter of the grid-wide barrier,
+ * bytes [0,4) tensor absmax (float bits; not written by a call without RMSNorm on up to 64 K elements, or up to 192 K where there
+ * is no room for a word per CTA, see below), bytes [4,8) arrival counter of the grid-wide barrier,
  * bytes [256, 256+4*M) per-row inv_rms (float).  The calls initialise what they use. */
 size_t sharq_prepare_workspace_bytes(int m);
 /* With this many bytes (room for a maximum per CTA of the statistics launch, up to 4096 of them) nothing is zeroed between the launches. */
@@ -391,6 +392,11 @@ int sharq_gemm_tile_n(int m, int n, int k, int split_k, int sms);
  * single-CTA kernel (tile_n 128 or 256): 0 = sent to the CTAs that sum them, from registers; 1 = by block copies; 2 = read behind a
  * cluster barrier; -1 for other arguments.  Runs nothing. */
 int sharq_gemm_exchange(int tile_n, int sparse, int dense, int rows, int k, int splits);
+
+/* Test hook: the form that a scaled prepare call takes on a GPU of `sms` SMs with that workspace: 0 = every CTA scans the input for its
+ * maximum, 1 = every cluster of CTAs does, 2 = a statistics launch and 8 elements per lane, 3 = a statistics launch (none with absmax_ready)
+ * and a group per lane, 4 = one cooperative launch; -1 for other arguments.  Runs nothing. */
+int sharq_scaled_prepare_form(int m, int k, int rms, int residual, int absmax_ready, size_t workspace_bytes, int sms);
 
 #ifdef __cplusplus
 }

@@ -69,6 +69,7 @@ SIGNATURES = {
     "sharq_set_gemm_tile_n": (c_int, [c_int]),
     "sharq_gemm_tile_n": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "sharq_gemm_exchange": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int]),
+    "sharq_scaled_prepare_form": (c_int, [c_int, c_int, c_int, c_int, c_int, c_size_t, c_int]),
     "sharq_set_wait_limit_cycles": (c_int, [c_longlong]),
     "sharq_allreduce_bf16_multimem": (c_int, [_P, POINTER(c_void_p), c_int, c_int, c_size_t, c_int, _P, _P]),
     "sharq_allreduce_flag_bytes": (c_size_t, []),

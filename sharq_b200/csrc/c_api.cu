@@ -696,6 +696,11 @@ int sharq_gemm_exchange(int tile_n, int sparse, int dense, int rows, int k, int 
   return sharq::gemm_exchange(tile_n, sparse != 0, dense != 0, rows, k, splits);
 }
 
+int sharq_scaled_prepare_form(int m, int k, int rms, int residual, int absmax_ready, size_t workspace_bytes, int sms) {
+  if (m < 1 || k < 128 || k % 128 != 0 || sms < 1 || (residual && !rms) || (absmax_ready && rms)) return -1;
+  return sharq::scaled_prepare_form(m, k, rms != 0, residual != 0, absmax_ready != 0, workspace_bytes, sms);
+}
+
 int sharq_gemm_swiglu_pays(int m, int ffn, int k) { return m > 0 && ffn > 0 && k > 0 && sharq::gemm_swiglu_pays(m, ffn, k); }
 
 int sharq_gemm_swiglu_absmax_words(int m, int ffn) { return m > 0 && ffn > 0 ? sharq::gemm_swiglu_absmax_words(m, ffn) : 0; }

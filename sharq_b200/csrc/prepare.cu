@@ -256,21 +256,26 @@ struct PrepareParams {
 
 constexpr int kPrepareCtasPerSm = 3;
 constexpr int kScaledCtasPerSm = 2;  // tensor-scale mode without a gather
-// An input of up to kClusterScanElements needs no statistics launch: every CTA scans it for its maximum, or (from kCtaScanElements) every
-// cluster of kScanCtas CTAs.  us per call in a graph, CTA / cluster / statistics launch and prepare: 1 x 4096 2.6 / 4.0 / -, 8 x 4096
-// 3.1 / 3.9 / -, 16 x 4096 4.5 / 3.1 / 4.9, 32 x 4096 6.7 / 3.7 / 4.4, 64 x 4096 10.4 / 4.2 / 4.8, 16 x 14336 - / 4.8 / 4.4, 32 x 14336 - / 6.0 / 4.7.  A
-// launch less is also 2 us less host time (16 x 14336 and its GEMM, eager: 21.4 -> 19.2 us).
+// A tensor-scale input of up to kClusterScanElements needs no statistics launch: every CTA scans it for its maximum, or (from kCtaScanElements)
+// every cluster of kScanCtas CTAs.  A prepare is followed by its GEMM, and what counts is the pair: us of both in a graph (o_proj of 4096
+// columns behind it), clusters / statistics launch: 12 x 4096 9.9 / 10.4, 32 x 4096 11.9 / 11.8, 40 x 4096 12.5 / 12.2, 64 x 4096 13.6 / 14.5, 16 x 8192 12.1 / 13.0,
+// 16 x 14336 15.5 / 16.1.  The prepare by itself behind a memset is slower from about 16 x 4096 on (16 x 14336 5.9 / 5.3).  A launch less is also 2 us
+// less on the host (16 x 14336 and its GEMM, eager: 21.4 -> 19.2).  CTA / cluster by themselves: 8 x 4096 3.1 / 3.9, 16 x 4096 4.5 / 3.1.
 constexpr size_t kCtaScanElements = 40 * 1024;
 constexpr size_t kClusterScanElements = 256 * 1024;
-constexpr int kClusterScanTiles = 256;  // CTAs that leave room for every cluster at once (8 x 18944, 296 of them: 6.6 us, launch 4.7)
+constexpr int kClusterScanTiles = 256;  // CTAs that leave room for every cluster at once (8 x 18944, 296 of them: with its GEMM 19.2, launch 17.5)
 constexpr int kScanCtas = 8;
-// The scanning forms leave the maximum in the workspace only above these sizes (with and without room for a word per statistics CTA).
+// The scanning forms leave the maximum in the workspace only above these sizes (with and without room for a word per statistics CTA); up to
+// the second one an input is scanned in any case where there is no such room.
 constexpr size_t kInlineAbsmaxElements = 64 * 1024;
 constexpr size_t kInlineAbsmaxElementsNoWords = 192 * 1024;
-// Up to this size, with the maximum ready and more than one 32-row tile, a lane takes 8 elements (prepare_narrow_kernel).  us, statistics and
-// wide / narrow prepare: RMSNorm 48 x 4096 6.1 / 5.3, 128 x 4096 6.5 / 5.8, 200 x 4096 6.5 / 6.7, 256 x 4096 6.7 / 7.4; tensor scale 128 x 4096
-// 5.0 / 4.5, 200 x 4096 5.1 / 6.1.  Up to 32 rows it is faster by itself (RMSNorm 32 x 4096 6.1 / 5.1) but not between GEMMs: linears of a
-// Llama-3-8B layer with 8 / 32 / 64 / 128 tokens wide 72.4 / 78.4 / 85.8 / 94.0, narrow 77.2 / 80.9 / 83.9 / 91.9.
+// Behind a statistics launch of its own and with more than one 32-row tile a lane takes 8 elements (prepare_narrow_kernel): RMSNorm up to
+// kNarrowElements, tensor scale while its CTAs are at most one per SM.  us of the calls and their GEMM (4096 columns) in a graph, wide / narrow: RMSNorm
+// 33 x 4096 14.4 / 13.8, 64 x 4096 15.4 / 15.2, 128 x 4096 17.3 / 16.7, 200 x 4096 17.9 / 17.9, 256 x 4096 18.3 / 18.8; tensor scale 72 x 4096 (144 CTAs) 15.4 / 13.9,
+// 80 x 4096 (160) 15.8 / 17.9, 36 x 8192 (144) 15.5 / 13.9, 40 x 8192 (160) 15.6 / 17.5, 512 x 1152 (320) 12.6 / 14.9.  With a maximum that another kernel left
+// (SwiGLU) 48 x 4096 14.6 / 13.1, but 72 x 4096 16.5 / 18.7, 128 x 1152 11.2 / 15.1 and 48 x 14336 19.6 / 20.2, and for an input that needs none 64 x 4096 11.1 / 12.7:
+// these two keep the wide form.  Up to 32 rows the narrow one is faster by itself (RMSNorm 32 x 4096 6.1 / 5.1) but not between GEMMs: linears of a
+// Llama-3-8B layer with 8 / 32 tokens wide 72.4 / 78.4, narrow 77.2 / 80.9.
 constexpr size_t kNarrowElements = 640 * 1024;
 constexpr unsigned kMaxAbsmaxWords = 4096;            // words of CTA maxima that every prepare CTA reduces
 
@@ -516,7 +521,7 @@ __global__ void __launch_bounds__(kPrepareThreads, kCtas) prepare_kernel(const P
 // ---------------------------------------------------------------------------
 // Prepare of a small input: latency is all there is, and one group per lane makes a serial chain of some 700 instructions that eight
 // warps of a few SMs walk while the others idle.  Here a lane owns 8 elements, a warp 256 columns of one row, and a CTA has one task per
-// warp (RMSNorm 48 x 4096 with its statistics 6.1 -> 5.3 us).  Modes as in prepare_kernel (the maximum is ready), same bytes.
+// warp (RMSNorm 48 x 4096 with its statistics 6.1 -> 5.3 us).  Modes 1 and 2 of prepare_kernel, the maximum ready; same bytes.
 // ---------------------------------------------------------------------------
 // Warps of a CTA: the tensor-scale mode has up to 8 maxima per SM to reduce in every CTA, the RMSNorm mode one per row.  us with 4 / 8
 // warps: 96 x 4096 5.3 / 4.4, 32 x 14336 6.0 / 4.7 (tensor scale).
@@ -552,11 +557,8 @@ __global__ void __launch_bounds__(32 * narrow_warps(kMode)) prepare_narrow_kerne
       inv = p.inv_rms[row];
     }
   }
-  float amax = 0.0f;
-  if (kMode != 0) {
-    amax = __uint_as_float(*p.amax_bits);
-    for (int i = threadIdx.x; i < p.amax_words; i += 32 * kNarrowWarps) amax = fmaxf(amax, __uint_as_float(p.amax_bits[i]));
-  }
+  float amax = __uint_as_float(*p.amax_bits);
+  for (int i = threadIdx.x; i < p.amax_words; i += 32 * kNarrowWarps) amax = fmaxf(amax, __uint_as_float(p.amax_bits[i]));
   {
     const int worker = (int)(blockIdx.x * blockDim.x + threadIdx.x), workers = (int)(gridDim.x * blockDim.x);
     const size_t bands = (size_t)aligned_m / 128;
@@ -565,24 +567,19 @@ __global__ void __launch_bounds__(32 * narrow_warps(kMode)) prepare_narrow_kerne
     zero_range(p.a_comp, (size_t)m * (k / 4), a_comp_bytes(m, k), worker, workers);
     zero_padding_rows(p.e, p.sfa_sparse, p.sf_res, m, k, worker, workers);
   }
-  if (kMode != 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (lane == 0) part_max[warp] = amax;
-  }
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (lane == 0) part_max[warp] = amax;
   __syncthreads();
-  float scale = 1.0f, recip = 1.0f;
-  if (kMode != 0) {
 #pragma unroll
-    for (int w = 0; w < kNarrowWarps; ++w) amax = fmaxf(amax, part_max[w]);
-    scale = fmaxf(__fmul_rn(amax, 1.0f / 2688.0f), 1.0e-9f);  // as in prepare_kernel
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      if (p.scale_out != nullptr) *p.scale_out = scale;
-      if (p.amax_out != nullptr) *p.amax_out = __float_as_uint(amax);
-    }
-    if (kMode == 2) scale = round_to_bf16(scale);
-    recip = __frcp_rn(scale);
+  for (int w = 0; w < kNarrowWarps; ++w) amax = fmaxf(amax, part_max[w]);
+  float scale = fmaxf(__fmul_rn(amax, 1.0f / 2688.0f), 1.0e-9f);  // as in prepare_kernel
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (p.scale_out != nullptr) *p.scale_out = scale;
+    if (p.amax_out != nullptr) *p.amax_out = __float_as_uint(amax);
   }
+  if (kMode == 2) scale = round_to_bf16(scale);
+  const float recip = __frcp_rn(scale);
   if (row >= m) return;
 
   uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -591,7 +588,7 @@ __global__ void __launch_bounds__(32 * narrow_warps(kMode)) prepare_narrow_kerne
 #pragma unroll
     for (int i = 0; i < 4; ++i) w[i] = normalise_word(w[i], gw[i], pair_f32(inv, inv));
     scale_words(w, scale, recip);
-  } else if (kMode == 2) {
+  } else {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float2 q = mul_word(w[i], pair_f32(recip, recip));
@@ -981,6 +978,15 @@ static cudaError_t current_sms(int *dev_out, int *sms_out) {
   return cudaSuccess;
 }
 
+// How a scaled prepare finds its maximum and quantises (scaled_prepare_form names them by number).
+enum class PrepareForm {
+  kCtaScan = 0,      // prepare_kernel, every CTA scans the input
+  kClusterScan = 1,  // prepare_kernel, every cluster scans it
+  kNarrow = 2,       // statistics launch, prepare_narrow_kernel
+  kWide = 3,         // statistics launch (none where the maximum is ready), prepare_kernel
+  kOneLaunch = 4     // prepare_fused_kernel
+};
+
 // 32-row x 256-column tiles of the padded activation.
 static int prepare_tiles(int m, int k) { return (k + kColsPerCta - 1) / kColsPerCta * ((m + 127) / 128 * 128 / kRowsPerCta); }
 
@@ -993,11 +999,11 @@ static int prepare_grid(const PrepareParams &p, int ctas_per_sm) {
   return tiles < full ? tiles : full;
 }
 
-static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, cudaStream_t stream) {
-  const size_t elements = (size_t)p.m * p.k;
-  const bool narrow = !debug && p.m > kRowsPerCta && elements <= kNarrowElements && p.unit_group == nullptr && p.src_row == nullptr &&
-                      (mode != 2 || p.amax_bits != nullptr);
-  const bool cluster = mode == 2 && p.amax_bits == nullptr && elements > kCtaScanElements;
+// CTAs of prepare_narrow_kernel.
+static int narrow_ctas(int mode, int m, int k) { return (m * ((k + 255) / 256) + narrow_warps(mode) - 1) / narrow_warps(mode); }
+
+static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, cudaStream_t stream, PrepareForm form = PrepareForm::kWide) {
+  const bool cluster = form == PrepareForm::kClusterScan;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the table set-up overlaps the kernel before
@@ -1007,11 +1013,9 @@ static cudaError_t launch_prepare(int mode, bool debug, const PrepareParams &p, 
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (narrow) {
-    const int warps = narrow_warps(mode);
-    cfg.gridDim = dim3((unsigned)((p.m * ((p.k + 255) / 256) + warps - 1) / warps));
-    cfg.blockDim = dim3((unsigned)(32 * warps));
-    if (mode == 0) return cudaLaunchKernelEx(&cfg, prepare_narrow_kernel<0>, p);
+  if (form == PrepareForm::kNarrow) {
+    cfg.gridDim = dim3((unsigned)narrow_ctas(mode, p.m, p.k));
+    cfg.blockDim = dim3((unsigned)(32 * narrow_warps(mode)));
     return cudaLaunchKernelEx(&cfg, mode == 1 ? prepare_narrow_kernel<1> : prepare_narrow_kernel<2>, p);
   }
   if (cluster) {
@@ -1115,6 +1119,48 @@ int prepare_timeouts() {
   return v;
 }
 
+struct ScaledPlan {
+  PrepareForm form;
+  bool narrow;         // the quantisation behind a statistics launch
+  unsigned stat_ctas;  // statistics launch: one CTA per row (RMSNorm) or a flat grid
+  bool word_per_cta;   // its CTAs' maxima go behind the row statistics, where the caller's workspace has room for a word each
+  size_t words_at;
+};
+
+static ScaledPlan plan_scaled_prepare(int m, int k, bool rms, bool residual, bool absmax_ready, bool inv_rms_external, size_t workspace_bytes,
+                                      int sms) {
+  ScaledPlan q{};
+  const size_t elements = (size_t)m * (size_t)k;
+  const size_t flat = (elements / 8 + 255) / 256;
+  q.stat_ctas = rms ? (unsigned)m : (unsigned)(flat < (size_t)sms * 8 ? flat : (size_t)sms * 8);
+  q.words_at = 256 + (rms && !inv_rms_external ? (size_t)m * sizeof(float) : 0);
+  q.word_per_cta = q.stat_ctas <= kMaxAbsmaxWords && workspace_bytes >= q.words_at + (size_t)q.stat_ctas * sizeof(float);
+  q.narrow = !absmax_ready && m > kRowsPerCta && (rms ? elements <= kNarrowElements : narrow_ctas(2, m, k) <= sms);
+  q.form = q.narrow ? PrepareForm::kNarrow : PrepareForm::kWide;
+  if (absmax_ready) return q;
+  // Without room for the words the other forms are a cooperative launch behind a memset, and the scan pays longer: by every CTA where the
+  // clusters would not fit at once (us per call in a graph, CTA / cluster: 2 x 18944 3.5 / 5.6, 8 x 18944 5.8 / 6.5, 10 x 18944 6.6 / 6.6).
+  const bool clusters_fit = prepare_tiles(m, k) <= kClusterScanTiles;
+  if (!rms && (elements <= kCtaScanElements || (clusters_fit && elements <= kClusterScanElements) ||
+               (!q.word_per_cta && elements <= kInlineAbsmaxElementsNoWords))) {
+    q.form = elements > kCtaScanElements && clusters_fit ? PrepareForm::kClusterScan : PrepareForm::kCtaScan;
+    return q;
+  }
+  // Two launches that overlap, with nothing to zero, beat one cooperative launch behind its memset (us, two launches / one: tensor scale
+  // 64 x 4096 5.0 / 8.4, 2048 x 4096 12.0 / 16.9, 4096 x 4096 19.6 / 27.1; RMSNorm 33 x 4096 7.0 / 10.5, 512 x 4096 9.1 / 12.5, 4096 x 4096
+  // 29.8 / 33.0), except with the residual add on middle sizes, where the row caches spare the second read of the sum: 512 x 4096
+  // 10.8 / 12.7, 2048 x 4096 24.7 / 24.9, 2048 x 8192 49.4 / 45.6, 700 x 14336 37.2 / 30.7.  Without room for the words the memset precedes both forms, and
+  // one launch pays while the row caches hold most of the tensor.
+  if (fused_prepare_enabled() && (q.word_per_cta ? residual && elements >= ((size_t)1 << 22) && elements < ((size_t)1 << 25)
+                                                 : elements < (rms ? ((size_t)1 << 25) : ((size_t)1 << 24))))
+    q.form = PrepareForm::kOneLaunch;
+  return q;
+}
+
+int scaled_prepare_form(int m, int k, bool rms, bool residual, bool absmax_ready, size_t workspace_bytes, int sms) {
+  return (int)plan_scaled_prepare(m, k, rms, residual, absmax_ready, false, workspace_bytes, sms).form;
+}
+
 cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int m, int k, void *workspace,
                                float *inv_rms_external, void *a_comp, void *e, void *sfa_sparse, void *q_res,
                                void *sf_res, float *scale_out, cudaStream_t stream, int absmax_words,
@@ -1128,28 +1174,13 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   cudaError_t err = cudaSuccess;
   const bool rms = gamma != nullptr;
   const size_t elements = (size_t)m * (size_t)k;
-  // statistics kernel: one CTA per row (RMSNorm) or a flat grid; its CTAs' maxima go behind the row statistics, where the
-  // caller's workspace has room for a word each
   int dev = 0, sms = 0;
   if (current_sms(&dev, &sms) != cudaSuccess) sms = 128;
-  const size_t flat = ((size_t)m * k / 8 + 255) / 256;
-  const unsigned stat_ctas = rms ? (unsigned)m : (unsigned)(flat < (size_t)sms * 8 ? flat : (size_t)sms * 8);
-  const size_t words_at = 256 + (rms && inv_rms_external == nullptr ? (size_t)m * sizeof(float) : 0);
-  const bool word_per_cta = stat_ctas <= kMaxAbsmaxWords && workspace_bytes >= words_at + (size_t)stat_ctas * sizeof(float);
-  // a small non-RMSNorm input (a decode step): the prepare kernel finds max|x| itself
-  const bool inline_absmax = !rms && !absmax_ready && elements <= kClusterScanElements &&
-                             (elements <= kCtaScanElements || prepare_tiles(m, k) <= kClusterScanTiles ||
-                              (!word_per_cta && elements <= kInlineAbsmaxElementsNoWords));
-  const bool leave_absmax = !inline_absmax || elements > (word_per_cta ? kInlineAbsmaxElements : kInlineAbsmaxElementsNoWords);
-  // Two launches that overlap, with nothing to zero, beat one cooperative launch behind its memset (us, two launches / one: tensor scale
-  // 64 x 4096 5.0 / 8.4, 2048 x 4096 12.0 / 16.9, 4096 x 4096 19.6 / 27.1; RMSNorm 33 x 4096 7.0 / 10.5, 512 x 4096 9.1 / 12.5, 4096 x 4096
-  // 29.8 / 33.0), except with the residual add on middle sizes, where the row caches spare the second read of the sum: 512 x 4096
-  // 10.8 / 12.7, 2048 x 4096 24.7 / 24.9, 2048 x 8192 49.4 / 45.6, 700 x 14336 37.2 / 30.7.  Without room for the words the memset precedes both forms, and
-  // one launch pays while the row caches hold most of the tensor.
-  const bool one_launch_pays =
-      fused_prepare_enabled() && (word_per_cta ? residual != nullptr && elements >= ((size_t)1 << 22) && elements < ((size_t)1 << 25)
-                                               : elements < (rms ? ((size_t)1 << 25) : ((size_t)1 << 24)));
-  if (!absmax_ready && !inline_absmax && one_launch_pays) {
+  const ScaledPlan plan = plan_scaled_prepare(m, k, rms, residual != nullptr, absmax_ready, inv_rms_external != nullptr, workspace_bytes, sms);
+  const bool scan = plan.form == PrepareForm::kCtaScan || plan.form == PrepareForm::kClusterScan;
+  const bool leave_absmax = scan ? elements > (plan.word_per_cta ? kInlineAbsmaxElements : kInlineAbsmaxElementsNoWords) : plan.word_per_cta;
+  PrepareForm form = plan.form;
+  if (form == PrepareForm::kOneLaunch) {
     FusedParams f{};
     f.x = static_cast<const __nv_bfloat16 *>(x);
     f.residual = static_cast<const __nv_bfloat16 *>(residual);
@@ -1174,6 +1205,7 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
     (void)cudaGetLastError();  // not launchable here: the separate kernels below do the same work
     if (err != cudaErrorNotSupported && err != cudaErrorCooperativeLaunchTooLarge) return err;
     err = cudaSuccess;
+    form = plan.narrow ? PrepareForm::kNarrow : PrepareForm::kWide;
   }
   int words = absmax_words;
   cudaLaunchConfig_t cfg = {};
@@ -1190,29 +1222,29 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   if (absmax_ready) {
     // the producer of x already left max|x| in the workspace: no statistics pass
     if (rms) return cudaErrorInvalidValue;
-  } else if (inline_absmax) {
+  } else if (scan) {
     amax_bits = nullptr;
   } else {
     const int groups = k / 32;
-    cfg.gridDim = dim3(stat_ctas);
+    cfg.gridDim = dim3(plan.stat_ctas);
     cfg.blockDim = dim3(rms ? (unsigned)((groups + 31) / 32 * 32) : 256u);
     cfg.dynamicSmemBytes = rms ? (size_t)groups * sizeof(float) : 0;
-    if (word_per_cta) {
-      amax_bits = reinterpret_cast<unsigned int *>(static_cast<uint8_t *>(workspace) + words_at);
-      words = (int)stat_ctas;
+    if (plan.word_per_cta) {
+      amax_bits = reinterpret_cast<unsigned int *>(static_cast<uint8_t *>(workspace) + plan.words_at);
+      words = (int)plan.stat_ctas;
     } else if ((err = cudaMemsetAsync(amax_bits, 0, sizeof(unsigned int), stream)) != cudaSuccess) {
       return err;
     }
     const auto *g = static_cast<const __nv_bfloat16 *>(gamma);
     if (!rms) {
-      err = cudaLaunchKernelEx(&cfg, abs_stats_kernel, xb, (size_t)m * k / 8, amax_bits, word_per_cta);
+      err = cudaLaunchKernelEx(&cfg, abs_stats_kernel, xb, (size_t)m * k / 8, amax_bits, plan.word_per_cta);
     } else if (residual != nullptr) {
       err = cudaLaunchKernelEx(&cfg, rms_stats_kernel<true>, xb, static_cast<const __nv_bfloat16 *>(residual),
-                               static_cast<__nv_bfloat16 *>(sum_out), g, eps, k, inv_rms, amax_bits, word_per_cta);
+                               static_cast<__nv_bfloat16 *>(sum_out), g, eps, k, inv_rms, amax_bits, plan.word_per_cta);
       x = sum_out;  // the prepare reads the sum
     } else {
       err = cudaLaunchKernelEx(&cfg, rms_stats_kernel<false>, xb, static_cast<const __nv_bfloat16 *>(nullptr),
-                               static_cast<__nv_bfloat16 *>(nullptr), g, eps, k, inv_rms, amax_bits, word_per_cta);
+                               static_cast<__nv_bfloat16 *>(nullptr), g, eps, k, inv_rms, amax_bits, plan.word_per_cta);
     }
     if (err != cudaSuccess) return err;
   }
@@ -1223,7 +1255,7 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   p.inv_rms = inv_rms;
   p.amax_bits = amax_bits;
   p.amax_words = words;
-  p.amax_out = !absmax_ready && (inline_absmax ? leave_absmax : word_per_cta) ? static_cast<unsigned int *>(workspace) : amax_out;
+  p.amax_out = !absmax_ready && leave_absmax ? static_cast<unsigned int *>(workspace) : amax_out;
   p.scale_out = scale_out;
   p.a_comp = static_cast<uint8_t *>(a_comp);
   p.e = static_cast<uint8_t *>(e);
@@ -1233,7 +1265,7 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
   p.m = m;
   p.k = k;
   p.row_tiles = (m + 127) / 128 * 128 / kRowsPerCta;
-  return launch_prepare(rms ? 1 : 2, false, p, stream);
+  return launch_prepare(rms ? 1 : 2, false, p, stream, form);
 }
 
 cudaError_t run_grouped_prepare(const void *x, int m, int k, const unsigned int *amax_bits, const int *unit_group, int groups,

@@ -6,7 +6,8 @@
 namespace sharq {
 
 // Bytes of scratch the scaled / RMSNorm-fused prepare needs for M rows:
-// [0,4) tensor absmax bits, [4,8) grid barrier counter, [256, 256 + 4*M) per-row inv_rms.
+// [0,4) tensor absmax bits (not written for a tensor-scale input of up to 64 K elements, 192 K without room for a word per
+// CTA), [4,8) grid barrier counter, [256, 256 + 4*M) per-row inv_rms.
 size_t prepare_workspace_bytes(int m);
 
 // With that many bytes nothing has to be zeroed between the launches.
@@ -29,6 +30,10 @@ cudaError_t run_scaled_prepare(const void *x, const void *gamma, float eps, int 
                                void *sf_res, float *scale_out, cudaStream_t stream, int absmax_words = 0,
                                const void *residual = nullptr, void *sum_out = nullptr, size_t workspace_bytes = 0,
                                unsigned int *amax_out = nullptr);
+
+// The form that run_scaled_prepare takes on a GPU of `sms` SMs: 0 = every CTA scans the input for its maximum, 1 = every cluster of CTAs,
+// 2 = a statistics launch and 8 elements per lane, 3 = a statistics launch (none with absmax_ready) and a 32-element group per lane, 4 = one cooperative launch.
+int scaled_prepare_form(int m, int k, bool rms, bool residual, bool absmax_ready, size_t workspace_bytes, int sms);
 
 // Tensor-scale prepare of a grouped activation (mixture-of-experts layers): rows sorted by group in
 // 256-row units (m a multiple of 256), unit_group[u] < 0 = unit without rows (its outputs are
