@@ -544,8 +544,8 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
 
   // The set-up above and the prefetch below overlap the end of the kernel that prepares the activation; from the wait on
   // every role reads or writes what earlier kernels may still use.  The prefetch goes to L2, where it cannot make stale data visible.
-  // Loads of the weight into the ring ahead of the wait were no faster (linears of a layer with 8 / 32 / 64 / 128 tokens 73.3 / 79.2 / 84.5 / 93.3 us,
-  // prefetched 73.1 / 79.2 / 83.5 / 92.2): they get in the prepare's way.
+  // Loads of the weight into the ring ahead of the wait were no faster (linears of a layer with 8 to 128 tokens within 2 % either way): they get
+  // in the prepare's way.
   if (!PAIR && warp == 0 && unit0 < num_units) {
     // weight tiles of this CTA's first stages: nothing of them depends on the activation
     if (ptx::elect_one()) {
@@ -938,7 +938,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap &tm_w, const CUtenso
       if constexpr (!SWIGLU && !WIDE) {
         if (stage != nullptr && u + unit_stride >= num_units) {
           // The CTA's last tile: nothing waits for the tensor memory, so it is drained 32 columns at a time by a loop whose code is
-          // a quarter of the unrolled form's, and which runs once on no rows ahead of the wait (28672 x 4096 at M = 32: 2.6 us behind the last MMA against 4.6, of which 2.8 went into
+          // a quarter of the unrolled form's, and which runs once on no rows ahead of the wait (28672 x 4096 at M = 32: 3.0 us behind the last MMA against 4.6, of which 2.8 went into
           // fetching code).
           const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(L::kColAcc + half * kColsPerEpiWarp);
           const int row0 = m_tile * kBM + quad * 32;
